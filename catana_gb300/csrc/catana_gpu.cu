@@ -273,7 +273,7 @@ catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double
         s = split_raw_accumulate(ctx, pts_d, w_d, npoints, lmax, nmax, rmax, kln_d, facc, err_d, st,
                                  (flags & CATANA_SPLIT_ACCURATE) != 0);
     } else {
-        s = fp64_raw_accumulate(ctx, pts_d, w_d, npoints, lmax, nmax, resolve_jl(flags, npoints), kln_d, facc,
+        s = fp64_raw_accumulate(ctx, pts_d, w_d, npoints, lmax, nmax, rmax, resolve_jl(flags, npoints), kln_d, facc,
                                 err_d, st);
     }
     if (s != CATANA_OK) return s;
@@ -396,7 +396,7 @@ catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats,
     } else {
         for (int c = 0; c < ncat; ++c) {
             const catana_catalog_t &C = cats[c];
-            s = fp64_raw_accumulate(ctx, C.points, C.weights, C.npoints, C.lmax, C.nmax,
+            s = fp64_raw_accumulate(ctx, C.points, C.weights, C.npoints, C.lmax, C.nmax, C.rmax,
                                     resolve_jl(flags, C.npoints), C.k_ln, facc[c], err_d, st);
             if (s != CATANA_OK) return s;
             if (C.kmax > 0.0 && C.lmax > 0 && C.nmax > 0) {

@@ -92,6 +92,14 @@ struct DeviceContext {
     std::vector<double> tab_dxinv, tab_zmax;  // per l
     DevBuf poly;       // piecewise FP64 j_l polynomials [l][interval][12] (CATANA_JL_POLY)
     int poly_lmax = -1, poly_nint = -1;
+    // plain path on the tensor cores (plain_tc.cu)
+    DevBuf tc_ws;      // sort scratch, point records, Legendre rows, phase tables
+    DevBuf tc_coef;    // (beta, A) of the monic recurrence
+    DevBuf tc_tab;     // (y0 - dy, dy) lerp tables, dx^-1 and z_max per l
+    DevBuf tc_jarr;    // j_l arrays of the modes without a table
+    int tc_coef_lmax = -1, tc_tab_lmax = -1, tc_tab_nmax = -1;
+    size_t tc_tab_off = 0;
+    bool attr_tc = false;
 };
 
 DeviceContext *get_context(int *status);
@@ -119,7 +127,13 @@ enum JlMode { JL_MODE_LERP = 0, JL_MODE_EXACT = 1, JL_MODE_POLY = 2 };
 // FP64 plain raw path (sfb_fp64.cu).  All pointers device.  Accumulates into
 // f_acc (complex, packed by l, un-normalised); the caller normalises.
 catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
-                                    int64_t npoints, int lmax, int nmax, JlMode jl, const double *kln_dev,
+                                    int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev,
+                                    double *f_acc_dev, int *err_dev, cudaStream_t st);
+// The same sum with its contraction on the tensor cores (plain_tc.cu), where the device has them and
+// lmax <= 512; with JL_MODE_POLY the caller has prepared ctx->poly.
+bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax);
+catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
+                                    int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev,
                                     double *f_acc_dev, int *err_dev, cudaStream_t st);
 // f *= norm; c_ln from f (device).
 catana_status_t finish_flmn_cln(double *f_dev, double norm, int lmax, int nmax, double *c_ln_dev,

@@ -1,0 +1,1041 @@
+// plain_tc.cu -- the plain (FP64-accurate) raw SFB sum with its contraction on the tcgen05
+// tensor cores.
+//
+//   f_l(m, n) = k_ln sum_i w_i j_l(k_ln r_i) P_lm(cos theta_i) e^{-i m phi_i}   (sfb_raw.cpp:56-84)
+//
+// GB300 issues two FP64 FMAs per SM and cycle, so the FP64 contraction (k_fp64_raw_l,
+// 2 nmax (l + 1) FMAs per point and l) leaves everything else idle.  Here both factors become
+// fixed-point numbers cut into signed 8-bit digits, and the digit products run as FP16 MMAs whose
+// FP32 accumulators hold exact integers:
+//   J[n][i]    = j_l(k_ln r_i) 2^(63 - EJ_n)                             -> digits J_0 .. J_7
+//   Y[m,ri][i] = w_i P_lm(x_i) (cos, -sin)(m phi_i) 2^(55 - EP_m - EW)   -> digits Y_0 .. Y_6
+//   D_d = sum_{a + b = d} Y_a J_b^T,  d = 0 .. 7   (35 digit products)
+// A digit is in [-128, 127], so a D_d entry of 128 points is at most 7 * 128 * 2^14 < 2^24: every
+// FP32 sum is exact.  After 128 points the eight D_d are added, as integers with weights
+// 256^(7 - d), to one 64-bit register per (m, ri, n), which holds the slab's whole sum.
+// What is rounded: the operands (Y to 2^-55 of its row's bound, J to 2^-63), the products of digits
+// a + b > 7 (2^-64), and each group's sum (2^-54 to 2^-51 of the slab's largest term).  (With seven digits of J,
+// 28 products, the sums erred by 30% more, at the same speed.)  The rows' bounds are kept close to
+// the values: points are sorted by radius, a CTA owns a contiguous slab of at most 2048 of them, EJ
+// bounds |j_l| over the slab's radii (Debye's and Watson's inequalities), EP bounds
+// |P_lm| over the slab's points from the two levels before, EW the slab's weights.
+//
+// What a point costs besides the MMAs (CUDA cores):
+//   * P_lm: the monic recurrence Q_l = x Q_{l-1} - beta_lm Q_{l-2} (P_lm = A_lm Q_lm, A_lm applied
+//     at the slab's end) in FP64, two operations per (point, m);
+//   * the phase e^{-i m phi} w as a 58-bit table per (point, m), written once per call;
+//     Y = the upper half of a 64 x 64-bit integer product;
+//   * j_l from the reference's linear table (SBesselInterpolator.cpp:10-26): the table position
+//     k r / dx is a 64 x 64-bit integer product, the interpolation one FP64 FMA on (y0 - dy, dy);
+//     or, in the other j_l modes, read from an array that another kernel filled.
+// FP64 work: 3 operations per (point, m) and (point, n) instead of 2 nmax (l + 1).
+//
+// Schedule: one CTA per slab walks every level of the launch (its Legendre rows are its own, so
+// levels need no grid-wide wait), 64 complex m x up to 64 radial orders at a time.  Warps 0..10
+// write the digits of 32-point tiles into two shared-memory buffers (units of four m or eight
+// radial orders, dealt round robin across tiles), warp 11 issues the MMAs (all digits J_0 .. J_{7-a}
+// of B in one N <= 256 instruction, since D_{a + b} lie side by side), warps 12..19 fold.  D lies in
+// two regions, so that MMAs run while sums are folded: with at most 32 radial orders they take the
+// groups in turn (each folded by all eight warps), otherwise the radial orders below and from 32
+// (each folded by four warps).  Slab sums go to HBM as FP64 and are added in slab
+// order (k_ptc_reduce): results do not depend on timing.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "common.cuh"
+#include "special.cuh"
+#include "tc05.cuh"
+
+namespace catana_gpu {
+
+namespace {
+
+constexpr int TC_KT = 32;        // points per tile (two K = 16 MMA steps)
+constexpr int TC_GROUP = 4;      // tiles per exact FP32 sum (128 points)
+constexpr int TC_DY = 7;         // 8-bit digits of Y
+constexpr int TC_DG = 8;         // 8-bit digits of J, digit sums
+constexpr int TC_MB = 64;        // complex m per block (128 MMA rows)
+constexpr int TC_NB = 64;        // most radial orders per block
+constexpr int TC_OPW = 11;       // operand warps
+constexpr int TC_OPT = 32 * TC_OPW;
+constexpr int TC_FOLD0 = 12;     // first fold warp (warp 11 issues the MMAs)
+constexpr int TC_THREADS = 640;  // 12 + 8 warps
+constexpr int TC_SLAB_TILES = 64;  // most tiles per slab
+constexpr int TC_LMAX = 512;     // |Q_lm| and A_lm stay inside FP64 up to here
+constexpr uint64_t TC_WAIT_NS = 1000000000ull;
+constexpr uint64_t TC_OFF_Y = 0x0080808080808080ull;  // 128 in every digit
+constexpr uint64_t TC_OFF_J = 0x8080808080808080ull;
+constexpr int TC_NH = 32;        // radial orders per D region
+constexpr uint32_t TC_DREG = TC_DG * TC_NH;  // columns of a D region
+
+// shared memory from a 1024-aligned base: two operand buffers, then the block tables
+constexpr uint32_t TC_YD = 8192;                       // one Y digit: 4 k-groups x 2 atoms of 1 KB
+constexpr uint32_t TC_SY = TC_DY * TC_YD;
+constexpr uint32_t TC_SJ = 8 * 4 * 1024;               // J digits: 4 k-groups x up to 2 x 4 atoms
+constexpr uint32_t TC_BUF = TC_SY + TC_SJ;
+constexpr uint32_t TC_RING = 8;                        // block tables in flight (the fold may be five blocks behind)
+constexpr uint32_t TC_OFF_N = 2 * TC_BUF;              // uint4 per n: (kd hi, kd lo, shift, EJ)
+constexpr uint32_t TC_OFF_M = TC_OFF_N + TC_RING * TC_NB * 16;  // per m: (beta, EP)
+constexpr uint32_t TC_OFF_MX = TC_OFF_M + TC_RING * TC_MB * 16; // max |Q| (upper words), three levels
+constexpr uint32_t TC_SMEM = TC_OFF_MX + 3 * TC_LMAX * 4 + 1024;
+static_assert(TC_SMEM <= 232448 - 1024, "k_ptc_main shared memory");
+
+struct TcSlab {
+    double rmin, rmax;  // of |r|
+    int ew;             // |w| < 2^ew
+    int pad;
+};
+
+struct TcArgs {
+    int l0, l1;                 // levels of the launch
+    int nmax, lmp;              // radial orders; row pitch in m (lmax rounded up to 4)
+    int tiles, tslab;           // tiles of the chunk, tiles per slab
+    const ulonglong2 *phase;    // [tile][lmp][32]: w cos, -w sin of m phi, times 2^(58 - EW), words split at
+                                // 2^32 into two signed halves
+    double *rows;               // [2][tile][lmp][32]: Q_l by the parity of l
+    const uint64_t *rint;       // [point]: r 2^(62 - er)
+    const double2 *xs;          // [point]: cos theta, sin theta
+    const TcSlab *slab;
+    const double2 *coef;        // (beta, A) per (l, m)
+    const uint4 *ntab;          // [slab][l - l0][n]: (kd hi, kd lo, shift, EJ)
+    const double2 *tab;         // lerp tables [l][npts]: (y_i - dy_i, dy_i), or null
+    int npts;
+    const double *jarr;         // [l - l0][tile][nmax][32] where tab is null
+    uint32_t *maxq;             // [slab][3][TC_LMAX]: level maxima between launches
+    double *partial;            // [slab][l - l0][n][2 (l + 1)]
+    int64_t pslab;              // doubles per slab in partial
+    int *err;
+};
+
+__device__ __forceinline__ uint64_t shr64(uint64_t v, int s) {  // 0 past 63
+    uint64_t r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+    return r;
+}
+
+// x as upper and lower words that are both signed: x = hi 2^32 + lo
+__device__ __forceinline__ uint64_t signed_halves(int64_t x) { return (uint64_t)x + ((uint64_t)(x & 0x80000000ll) << 1); }
+
+// Byte `byte` of eight consecutive rows' or columns' values at one point as FP16 digits, 16 bytes:
+// 0x6400 | b is 1024 + b, minus 1152 is b - 128.
+template <int BYTE>
+__device__ __forceinline__ void store_digit(uint8_t *p, const uint64_t (&u)[8]) {
+    const __half2 c = __half2half2(__ushort_as_half(0x6480));  // 1152
+    constexpr uint32_t b = BYTE & 3;
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t x = BYTE >= 4 ? (uint32_t)(u[2 * k] >> 32) : (uint32_t)u[2 * k];
+        const uint32_t y = BYTE >= 4 ? (uint32_t)(u[2 * k + 1] >> 32) : (uint32_t)u[2 * k + 1];
+        uint32_t t = __byte_perm(x, y, b | (b << 4) | ((4 + b) << 8) | ((4 + b) << 12));
+        t = (t & 0x00ff00ffu) | 0x64006400u;
+        const __half2 h = __hsub2(*reinterpret_cast<__half2 *>(&t), c);
+        w[k] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+    *reinterpret_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+template <int A, int N>
+struct Digits {
+    template <class F>
+    static __device__ __forceinline__ void each(F &&at, const uint64_t (&u)[8]) {  // digit A of N at at(A)
+        store_digit<N - 1 - A>(at(A), u);
+        if constexpr (A + 1 < N) Digits<A + 1, N>::each(at, u);
+    }
+};
+
+// FP64 load where pred holds, 0 elsewhere (rows that this kernel also writes)
+__device__ __forceinline__ double ld_if(const double *p, bool pred) {
+    double v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.f64 %0, 0d0000000000000000;\n@q ld.global.L1::no_allocate.f64 %0, [%1];\n}"
+                 : "=d"(v)
+                 : "l"(p), "r"((int)pred)
+                 : "memory");
+    return v;
+}
+
+// the same for a pair of read-only words; L1 is left to the j_l table
+__device__ __forceinline__ ulonglong2 ld_if(const ulonglong2 *p, bool pred) {
+    ulonglong2 v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %3, 0;\nmov.u64 %0, 0;\nmov.u64 %1, 0;\n"
+                 "@q ld.global.nc.L1::no_allocate.v2.u64 {%0, %1}, [%2];\n}"
+                 : "=l"(v.x), "=l"(v.y)
+                 : "l"(p), "r"((int)pred));
+    return v;
+}
+
+// log2 of a bound on |j_l| over [z1, z2] (FP32; checked to exceed log2 |j_l| up to 1e-6 for every l < 512):
+// below l + 1/2 Debye's inequality at z2, beyond it Watson's M^2 < 2 / (pi sqrt(z^2 - nu^2)) at z1, never
+// more than the maximum of j_l, 0.89 (l + 1/2)^(-5/6)
+__device__ __forceinline__ float jl_log2_bound(int l, float z1, float z2) {
+    const float nu = (float)l + 0.5f;
+    const float mx = fminf(0.f, -0.1681228f - 0.8333333f * log2f(nu));
+    float b = mx;
+    if (z2 < nu) {
+        const float z = fmaxf(z2, 1e-30f);
+        const float s = sqrtf((nu - z) * (nu + z));
+        b = (s - nu * logf((nu + s) / z)) * 1.4426950f - 1.f - 0.5f * log2f(z) - 0.5f * log2f(s);
+    } else if (z1 > nu) {
+        b = -0.5f * log2f(z1) - 0.25f * log2f((z1 - nu) * (z1 + nu));
+    }
+    return fminf(b, mx);
+}
+
+__device__ __forceinline__ void op_bar() { asm volatile("barrier.sync 2, 352;" ::: "memory"); }
+__device__ __forceinline__ void tc_arrive(uint64_t *mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc05::smem_u32(mbar)) : "memory");
+}
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t (&v)[2]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr));
+}
+
+// Block (l, m-block, n-block) sequence of the launch, walked alike by the operand and the fold warps.
+struct TcBlock {
+    int l, mb0, mcount, n0, ncount;
+    int nb0, nb1;  // columns per digit (multiples of 16) of the radial orders below TC_NH and from it
+};
+template <class F>
+__device__ __forceinline__ void tc_blocks(const TcArgs &a, F &&body) {
+    int seq = 0;
+    for (int l = a.l0; l < a.l1; ++l)
+        for (int mb0 = 0; mb0 <= l; mb0 += TC_MB)
+            for (int n0 = 0; n0 < a.nmax; n0 += TC_NB) {
+                TcBlock b;
+                b.l = l;
+                b.mb0 = mb0;
+                b.mcount = min(TC_MB, l + 1 - mb0);
+                b.n0 = n0;
+                b.ncount = min(TC_NB, a.nmax - n0);
+                b.nb0 = min(TC_NH, (b.ncount + 15) & ~15);
+                b.nb1 = max(0, ((b.ncount + 15) & ~15) - TC_NH);
+                body(b, seq++);
+            }
+}
+
+// What bounds it at 64 m x 64 n: the FP64 pipe (2 operations per (point, m), 1 per (point, n), 16 cycles
+// each per warp: ~3.1k cycles per tile), the issue slots (~9k warp instructions per tile) and the tensor
+// core (70 MMAs of 128 x 64 x 16 per tile, ~2.2k cycles) are of one size.
+template <bool LERP>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
+    extern __shared__ uint8_t tc_smem[];
+    uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(tc_smem) + 1023) & ~uintptr_t(1023));
+    __shared__ uint64_t full[2], empty[2], gdone[2], dfree[2];
+    __shared__ uint32_t tmem_sh;
+    __shared__ int abort_sh;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int slab = blockIdx.x;
+    const int t0 = slab * a.tslab, t1 = min(a.tiles, t0 + a.tslab);
+    const bool alt = a.nmax <= TC_NH;  // the D regions take the groups in turn
+    constexpr uint32_t tcols = 512;
+    uint4 *s_n = reinterpret_cast<uint4 *>(sm + TC_OFF_N);
+    double2 *s_m = reinterpret_cast<double2 *>(sm + TC_OFF_M);  // (beta, EP as int bits)
+    uint32_t *s_mx = reinterpret_cast<uint32_t *>(sm + TC_OFF_MX);
+    volatile int *abort_v = &abort_sh;
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b) {
+            tc05::mbar_init(&full[b], TC_OPW);
+            tc05::mbar_init(&empty[b], 1);
+            tc05::mbar_init(&gdone[b], 1);
+            tc05::mbar_init(&dfree[b], alt ? 256 : 128);
+        }
+        abort_sh = 0;
+    }
+    // level maxima carried over from the launch before (levels l0 - 1, l0 - 2)
+    for (int k = tid; k < 3 * TC_LMAX; k += TC_THREADS)
+        s_mx[k] = a.l0 > 0 ? a.maxq[(size_t)slab * 3 * TC_LMAX + k] : 0u;
+    if (warp == TC_FOLD0) tc05::tmem_alloc(&tmem_sh, tcols);
+    tc05::fence_before();
+    __syncthreads();
+    tc05::fence_after();
+    const uint32_t tmem = tmem_sh;
+    // a bounded wait; once one ran out every later wait of the CTA returns at once
+    auto wait = [&](uint64_t *bar, uint32_t parity, bool &dead) {
+        if (dead || __all_sync(0xffffffffu, tc05::mbar_try(bar, parity))) return;
+        dead = __any_sync(0xffffffffu, *abort_v || !tc05::mbar_wait(bar, parity, TC_WAIT_NS));
+        if (dead) *abort_v = 1;
+    };
+
+    if (warp < TC_OPW) {
+        uint32_t use = 0;  // tiles written so far
+        int ofs = 0;       // units dealt so far, mod TC_OPW
+        bool dead = false;
+        const uint32_t lk = (uint32_t)(lane >> 3), lr = (uint32_t)(lane & 7);  // K row of this point: group, row
+        const size_t lset = (size_t)a.tiles * a.lmp * TC_KT;
+        tc_blocks(a, [&](const TcBlock &b, int seq) {
+            const int l = b.l;
+            const int ring = seq & (int)(TC_RING - 1);
+            uint4 *tn = s_n + ring * TC_NB;
+            double2 *tm = s_m + ring * TC_MB;
+            // past the count: zero digits
+            uint4 e = make_uint4(0u, 0u, 31u, 2022u << 20);
+            double beta = 0.0;
+            if (tid < b.ncount) e = a.ntab[((size_t)slab * (a.l1 - a.l0) + (l - a.l0)) * a.nmax + b.n0 + tid];
+            if (tid >= 64 && tid < 64 + b.mcount) beta = a.coef[(size_t)l * (l + 1) / 2 + b.mb0 + tid - 64].x;
+            op_bar();  // rows and maxima of the block before are written, its tables read
+            if (tid < b.nb0 + b.nb1) {
+                tn[tid] = e;
+            } else if (tid >= 64 && tid < 64 + b.mcount) {
+                const int m = b.mb0 + tid - 64;
+                // |Q_l| <= max |Q_{l-1}| + beta max |Q_{l-2}|
+                auto mx = [&](int lv, int mm) {
+                    const uint32_t h = s_mx[(lv % 3) * TC_LMAX + mm];
+                    return __hiloint2double((int)h, h ? -1 : 0);
+                };
+                double bd = 1.0;
+                if (l > 0) {
+                    if (m == l) bd = mx(l - 1, m - 1);
+                    else if (m == l - 1) bd = mx(l - 1, m);
+                    else bd = fma(beta, mx(l - 2, m), mx(l - 1, m));
+                }
+                const int eb = (int)((uint32_t)__double2hiint(bd * 1.03) >> 20) & 0x7ff;
+                tm[tid - 64] = make_double2(beta, __hiloint2double(0, max(eb - 1022, -1000)));
+            } else if (tid >= 128 && b.mb0 == 0 && b.n0 == 0) {
+                for (int k = tid - 128; k <= l + 1 && k < TC_LMAX; k += TC_OPT - 128) s_mx[(l % 3) * TC_LMAX + k] = 0u;
+            }
+            op_bar();
+            const int nq = (b.mcount + 3) >> 2, nu = nq + ((b.ncount + 7) >> 3);
+            const int at0 = (TC_DG * b.nb0 + 63) >> 6, natoms = at0 + ((TC_DG * b.nb1 + 63) >> 6);
+            // written and read in this kernel: no read-only loads
+            double *rw0 = a.rows + (size_t)(l & 1) * lset;  // Q_{l-2}, overwritten by Q_l
+            const double *rw1 = a.rows + (size_t)((l + 1) & 1) * lset;
+            const double2 *__restrict__ tab = LERP ? a.tab + (size_t)l * a.npts : nullptr;
+            const bool first = b.n0 == 0;  // this block advances the rows; later n-blocks read them
+            // The rows and phases of a warp's unit are loaded while the digits of its unit before are
+            // stored: the L2's latency (~1000 cycles) is a third of a unit otherwise.
+            double q[4], q2[4];
+            ulonglong2 ph[4];
+            auto load_next = [&](int t, int u) {  // this warp's unit after unit u of tile t (zeros if it is none of m)
+                u += TC_OPW;
+                while (u >= nu) {
+                    u -= nu;
+                    ++t;
+                }
+                const bool go = t < t1 && u < nq;
+                const int m0 = b.mb0 + 4 * u;
+                const uint32_t r0 = ((uint32_t)t * a.lmp + m0) * TC_KT + lane;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) ph[h] = ld_if(a.phase + r0 + h * TC_KT, go);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    // the first n-block reads Q_{l-1}, Q_{l-2}; later ones Q_l
+                    q[h] = ld_if(first ? rw1 + r0 + (m0 + h == l ? h - 1 : h) * TC_KT : rw0 + r0 + h * TC_KT,
+                                 go && m0 + h <= l && (l > 0 || !first));
+                    q2[h] = ld_if(rw0 + r0 + h * TC_KT, go && first && m0 + h <= l - 2);
+                }
+                if (go && t + 2 < t1) {
+                    // the same of the tile after next into L2: 32 lines, one per lane
+                    const uint32_t rp = r0 - lane + 2u * a.lmp * TC_KT;
+                    const char *pf = lane < 16   ? reinterpret_cast<const char *>(a.phase + rp) + lane * 128
+                                     : lane < 24 ? reinterpret_cast<const char *>(rw1 + rp) + (lane - 16) * 128
+                                                 : reinterpret_cast<const char *>(rw0 + rp) + (lane - 24) * 128;
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(pf));
+                }
+            };
+            {
+                int u = warp - ofs;
+                if (u < 0) u += TC_OPW;
+                load_next(t0, u - TC_OPW);
+            }
+            double2 xs = __ldg(a.xs + (size_t)t0 * TC_KT + lane);
+            uint64_t r = __ldg(a.rint + (size_t)t0 * TC_KT + lane);
+            for (int t = t0; t < t1; ++t) {
+                const uint32_t bf = use & 1u, it = use >> 1;
+                ++use;
+                int u = warp - ofs;
+                if (u < 0) u += TC_OPW;
+                ofs = (ofs + nu) % TC_OPW;
+                // every warp takes part in every tile, with or without a unit of it: none falls so far
+                // behind that a barrier's parity would mean another phase.  The buffer is waited for
+                // when a unit's digits are ready.
+                bool mine = it == 0;
+                const bool any = u < nu;
+                uint8_t *sy = sm + bf * TC_BUF, *sj = sy + TC_SY;
+                for (; u < nu; u += TC_OPW) {
+                    uint64_t v[8];
+                    if (u < nq) {
+                        // four complex m at this point: rows 8 u .. 8 u + 7
+                        const int m0 = b.mb0 + 4 * u;
+                        if (first) {
+                            const uint32_t r0 = ((uint32_t)t * a.lmp + m0) * TC_KT + lane;
+                            uint32_t mh[4];
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) {
+                                q[h] = fma(m0 + h == l ? xs.y : xs.x, q[h], -tm[4 * u + h].x * q2[h]);
+                                if (l == 0) q[h] = 1.0;
+                                if (m0 + h <= l) rw0[r0 + h * TC_KT] = q[h];
+                                mh[h] = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(q[h]) & 0x7fffffffu);
+                            }
+                            if (lane < 4 && m0 + lane <= l)
+                                atomicMax(&s_mx[(l % 3) * TC_LMAX + m0 + lane],
+                                          lane & 2 ? (lane & 1 ? mh[3] : mh[2]) : (lane & 1 ? mh[1] : mh[0]));
+                        }
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) {
+                            // |q| 2^(61 - EP), then times the 58-bit phase, upper 64 bits: < 2^55
+                            const uint32_t qh = (uint32_t)__double2hiint(q[h]), ql = (uint32_t)__double2loint(q[h]);
+                            const int s = __double2loint(tm[4 * u + h].y) + 1022 - (int)((qh >> 20) & 0x7ffu);
+                            const uint64_t p = shr64(((uint64_t)((qh & 0xfffffu) | 0x100000u) << 40) | ((uint64_t)ql << 8), s);
+                            // both factors as signed halves: three products, no sign to carry along
+                            const uint64_t ps = signed_halves(qh >> 31 ? -(int64_t)p : (int64_t)p);
+                            const int32_t p1 = (int32_t)(ps >> 32), p0 = (int32_t)ps;
+                            auto prod = [&](uint64_t c) {
+                                const int32_t c1 = (int32_t)(c >> 32), c0 = (int32_t)c;
+                                const int64_t t2 = (int64_t)p1 * c0 + ((int64_t)p0 * c1 + 0x80000000ll);  // rounded
+                                return (uint64_t)((int64_t)p1 * c1 + ((t2 >> 32) + (int64_t)TC_OFF_Y));
+                            };
+                            v[2 * h] = prod(ph[h].x);
+                            v[2 * h + 1] = prod(ph[h].y);
+                        }
+                    } else {
+                        // eight radial orders at this point
+                        const int o = u - nq;
+                        if (LERP) {
+                            const uint32_t rh = (uint32_t)(r >> 32), rl = (uint32_t)r;
+#pragma unroll
+                            for (int h0 = 0; h0 < 8; h0 += 4) {
+                                double2 y[4];
+                                double f[4];
+#pragma unroll
+                                for (int h = 0; h < 4; ++h) {
+                                    const uint4 kd = tn[8 * o + h0 + h];
+                                    const uint64_t tt = (uint64_t)rl * kd.x + (uint64_t)rh * kd.y;
+                                    const uint64_t res = (uint64_t)rh * kd.x + (tt >> 32);
+                                    const uint32_t i = min((uint32_t)(res >> 32) >> (32u - kd.z), (uint32_t)(a.npts - 1));
+                                    y[h] = __ldg(tab + i);
+                                    const uint32_t fh = __funnelshift_l((uint32_t)res, (uint32_t)(res >> 32), kd.z);
+                                    const uint32_t fl = __funnelshift_l((uint32_t)tt, (uint32_t)res, kd.z);
+                                    f[h] = __hiloint2double((int)(0x3ff00000u | (fh >> 12)), (int)__funnelshift_l(fl, fh, 20));
+                                }
+#pragma unroll
+                                for (int h = 0; h < 4; ++h)
+                                    v[h0 + h] = (uint64_t)__double_as_longlong(fma(y[h].y, f[h], y[h].x));
+                            }
+                        } else {
+                            const double *jp = a.jarr + (((size_t)(l - a.l0) * a.tiles + t) * a.nmax + b.n0 + 8 * o) * TC_KT + lane;
+#pragma unroll
+                            for (int h = 0; h < 8; ++h)
+                                v[h] = 8 * o + h < b.ncount ? (uint64_t)__double_as_longlong(__ldg(jp + h * TC_KT)) : 0ull;
+                        }
+#pragma unroll
+                        for (int h = 0; h < 8; ++h) {
+                            const uint32_t jh = (uint32_t)(v[h] >> 32), jl = (uint32_t)v[h];
+                            const int s = (int)(tn[8 * o + h].w - (jh & 0x7ff00000u)) >> 20;
+                            const uint64_t p = shr64(((uint64_t)((jh & 0xfffffu) | 0x100000u) << 42) | ((uint64_t)jl << 10), s);
+                            v[h] = jh >> 31 ? TC_OFF_J - p : TC_OFF_J + p;
+                        }
+                    }
+                    load_next(t, u);
+                    if (!mine) wait(&empty[bf], (it - 1) & 1, dead);
+                    mine = true;
+                    if (u < nq) {
+                        const uint32_t atom = (uint32_t)u >> 3, c = (uint32_t)u & 7u;
+                        uint8_t *dst = sy + (lk * 2 + atom) * 1024u + lr * 128u + ((c ^ lr) << 4);
+                        Digits<0, TC_DY>::each([&](int d) { return dst + d * TC_YD; }, v);
+                    } else {
+                        // digit d's columns of a half start at d nb: an octet lies in one atom of 64
+                        const int n = 8 * (u - nq), nbh = n < TC_NH ? b.nb0 : b.nb1;
+                        uint8_t *dst = sj + (lk * (uint32_t)natoms + (n < TC_NH ? 0u : (uint32_t)at0)) * 1024u + lr * 128u;
+                        uint32_t col = (uint32_t)(n & (TC_NH - 1));
+                        Digits<0, TC_DG>::each(
+                            [&](int) {
+                                uint8_t *q8 = dst + (col >> 6) * 1024u + ((((col & 63u) >> 3) ^ lr) << 4);
+                                col += (uint32_t)nbh;
+                                return q8;
+                            },
+                            v);
+                    }
+                }
+                if (t + 1 < t1) {  // the next tile's points
+                    xs = __ldg(a.xs + (size_t)(t + 1) * TC_KT + lane);
+                    r = __ldg(a.rint + (size_t)(t + 1) * TC_KT + lane);
+                }
+                if (any) {
+                    tc05::fence_proxy_async();
+                    __syncwarp();
+                } else if (!mine) {
+                    wait(&empty[bf], (it - 1) & 1, dead);
+                }
+                if (lane == 0) tc_arrive(&full[bf]);
+            }
+        });
+        op_bar();
+        for (int k = tid; k < 3 * TC_LMAX; k += TC_OPT) a.maxq[(size_t)slab * 3 * TC_LMAX + k] = s_mx[k];
+    } else if (warp < TC_FOLD0) {
+        uint32_t use = 0, groups = 0;  // tiles taken, groups issued
+        bool dead = false;
+        tc_blocks(a, [&](const TcBlock &b, int) {
+            const uint32_t at0 = (uint32_t)(TC_DG * b.nb0 + 63) >> 6, natoms = at0 + ((uint32_t)(TC_DG * b.nb1 + 63) >> 6);
+            for (int g = t0; g < t1; g += TC_GROUP) {
+                const int ge = min(t1, g + TC_GROUP);
+                for (int t = g; t < ge; ++t) {
+                    const uint32_t bf = use & 1u;
+                    wait(&full[bf], (use >> 1) & 1, dead);
+                    ++use;
+                    const uint32_t ya = tc05::smem_u32(sm + bf * TC_BUF), jb = ya + TC_SY;
+                    for (uint32_t h = 0; h < (alt ? 1u : 2u); ++h) {
+                        const uint32_t reg = alt ? groups & 1u : h, rn = alt ? groups >> 1 : groups;
+                        // the region's group before is folded
+                        if (t == g && rn > 0) wait(&dfree[reg], (rn - 1) & 1, dead);
+                        if (lane == 0 && !dead) {
+                            tc05::fence_after();
+                            const uint32_t nbh = (uint32_t)(h ? b.nb1 : b.nb0), dt = tmem + reg * TC_DREG;
+                            uint64_t da0 = tc05::desc_sw128(ya, 1024, 2048);
+                            uint64_t db = tc05::desc_sw128(jb + (h ? at0 * 1024u : 0u), 1024, natoms * 1024u);
+                            if (nbh) {
+#pragma unroll
+                                for (int ks = 0; ks < 2; ++ks) {
+                                    uint32_t idesc = tc05::idesc_f16_mn(128, 0) + ((TC_DG * nbh >> 3) << 17), dc = dt;
+#pragma unroll
+                                    for (int ad = 0; ad < TC_DY; ++ad) {
+                                        tc05::mma_f16(dc, da0 + (uint64_t)(ad * (TC_YD >> 4) + ks * 256), db, idesc,
+                                                      (t > g || ks > 0 || ad > 0) ? 1u : 0u);
+                                        dc += nbh;
+                                        idesc -= (nbh >> 3) << 17;
+                                    }
+                                    db += natoms * 128u;
+                                }
+                            }
+                            if (t + 1 == ge) tc05::commit(&gdone[reg]);
+                        }
+                        __syncwarp();
+                    }
+                    if (lane == 0 && !dead) tc05::commit(&empty[bf]);
+                    __syncwarp();
+                }
+                ++groups;
+            }
+        });
+        // MMAs still in flight land before the tensor memory is released
+        if (dead)
+            for (uint32_t bf = 0; bf < 2; ++bf) {
+                const uint32_t n = (use + 1 - bf) >> 1;
+                if (n > 0) tc05::mbar_wait(&empty[bf], (n - 1) & 1, TC_WAIT_NS);
+            }
+        if (dead && lane == 0) *a.err = CATANA_ERR_CUDA;
+    } else {
+        uint32_t groups = 0;  // groups folded
+        bool dead = false;
+        const int qd = warp & 3, row = qd * 32 + lane;
+        const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
+        // slab sums are kept in units of 2^(48 + sh): |sum| <= points * 2^118 <= 2^(62 + 48 + sh)
+        const int npt = 32 * (t1 - t0), sh = npt <= 256 ? 16 : npt <= 512 ? 17 : npt <= 1024 ? 18 : 19;
+        const int rnd = (1 << (sh - 16)) >> 1;
+        const int ew = a.slab[slab].ew;
+        const int set = warp >= TC_FOLD0 + 4 ? 1 : 0;
+        tc_blocks(a, [&](const TcBlock &b, int seq) {
+            const bool live = qd * 32 < 2 * b.mcount;  // warp-uniform: the quadrant holds rows of the block
+            // this warp's radial orders of the block, and their column in the region
+            const int nbh = !alt && set ? b.nb1 : b.nb0, ncol = alt ? nbh >> 1 : nbh, col0 = alt ? set * ncol : 0;
+            const int nb = alt ? col0 : set * TC_NH;
+            int64_t acc[TC_NH];
+#pragma unroll
+            for (int c = 0; c < TC_NH; ++c) acc[c] = 0;
+            for (int g = t0; g < t1; g += TC_GROUP) {
+                const uint32_t reg = alt ? groups & 1u : (uint32_t)set, rn = alt ? groups >> 1 : groups;
+                wait(&gdone[reg], rn & 1, dead);
+                ++groups;
+                if (!dead && live) {
+                    tc05::fence_after();
+                    const uint32_t dt = tmem + reg * TC_DREG + lane_off + (uint32_t)col0;
+#pragma unroll
+                    for (int c2 = 0; c2 < TC_NH; c2 += 2) {
+                        if (c2 < ncol) {
+                            uint32_t d[TC_DG][2];
+#pragma unroll
+                            for (int k = 0; k < TC_DG; ++k) tmem_ld2(dt + (uint32_t)(k * nbh + c2), d[k]);
+                            tc05::tmem_wait_ld();
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                int iv[TC_DG];
+#pragma unroll
+                                for (int ad = 0; ad < TC_DG; ++ad) iv[ad] = __float2int_rn(__uint_as_float(d[ad][k]));
+                                // sum_d iv_d 2^(56 - 8 d) in units of 2^16, the lowest digits rounded off
+                                const int low = iv[5] + ((iv[6] + ((iv[7] + 128) >> 8) + 128) >> 8);
+                                int64_t v = low + (int64_t)iv[4] * 256;
+                                v += (int64_t)iv[3] * 65536;
+                                v += (int64_t)iv[2] * 16777216;
+                                v += (int64_t)(iv[0] * 256 + iv[1]) << 32;
+                                acc[c2 + k] += (v + rnd) >> (sh - 16);
+                            }
+                        }
+                    }
+                }
+                tc05::fence_before();
+                tc_arrive(&dfree[reg]);
+            }
+            // the slab's sums: value = acc 2^(sh - 70 + EJ + EP + EW) A_lm
+            if (live && row < 2 * b.mcount) {
+                const int ring = seq & (int)(TC_RING - 1);
+                const uint4 *tn = s_n + ring * TC_NB + nb;
+                const int m = b.mb0 + (row >> 1);
+                const double am = scalbn(a.coef[(size_t)b.l * (b.l + 1) / 2 + m].y,
+                                         __double2loint(s_m[ring * TC_MB + (row >> 1)].y) + ew);
+                const int w2 = 2 * (b.l + 1);
+                double *out = a.partial + (size_t)slab * a.pslab +
+                              (size_t)a.nmax * ((size_t)b.l * (b.l + 1) - (size_t)a.l0 * (a.l0 + 1)) + 2 * b.mb0 + row +
+                              (size_t)(b.n0 + nb) * w2;
+#pragma unroll
+                for (int c4 = 0; c4 < TC_NH; c4 += 4)
+                    if (c4 < ncol) {
+                        double v[4];  // 2^(EJ + sh - 70) is a normal number: EJ >= -900
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            v[c] = (double)acc[c4 + c] * __hiloint2double((int)(tn[c4 + c].w + ((uint32_t)(sh - 69) << 20)), 0);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            if (nb + c4 + c < b.ncount) out[(size_t)(c4 + c) * w2] = v[c] * am;
+                    }
+            }
+        });
+        if (dead && lane == 0) *a.err = CATANA_ERR_CUDA;
+    }
+    tc05::fence_before();
+    __syncthreads();
+    tc05::fence_after();
+    if (warp == TC_FOLD0) tc05::tmem_dealloc(tmem, tcols);
+}
+
+// Per (slab, l, n): the table's step (k / dx as 62-bit mantissa and shift) and the exponent bound of
+// |j_l(k r)| over the slab's radii.  With the table, a slab that reaches past it is a domain error.
+__global__ void __launch_bounds__(128) k_ptc_ntab(const TcSlab *__restrict__ slab, const double *__restrict__ kln,
+                                                  const double *__restrict__ dxinv, const double *__restrict__ zmax, int l0,
+                                                  int nl, int nmax, int er, uint4 *__restrict__ out, int *err) {
+    const int e = blockIdx.y * 128 + threadIdx.x;
+    if (e >= nl * nmax) return;
+    const int l = l0 + e / nmax, n = e % nmax;
+    const TcSlab sl = slab[blockIdx.x];
+    const double k = kln[(size_t)l * nmax + n];
+    float z1 = (float)(k * sl.rmin), z2 = (float)(k * sl.rmax);
+    uint4 o = make_uint4(0u, 0u, 31u, 0u);
+    if (dxinv) {
+        const double kd = k * dxinv[l];
+        const float dx = 1.f / (float)dxinv[l];
+        z1 = fmaxf(z1 - 1.0001f * dx, 0.f);  // interpolated values lie between nodes up to dx away
+        z2 += 1.0001f * dx;
+        const uint64_t bits = (uint64_t)__double_as_longlong(kd);
+        const int ek = (int)(bits >> 52) - 1022;  // kd in [2^(ek - 1), 2^ek)
+        const uint64_t kdi = ((bits & 0xfffffffffffffull) | 0x10000000000000ull) << 9;  // kd 2^(62 - ek)
+        o.x = (uint32_t)(kdi >> 32);
+        o.y = (uint32_t)kdi;
+        o.z = (uint32_t)(4 + er + ek);  // k r / dx = (rint kdi / 2^64) / 2^(60 - er - ek)
+        if (n == nmax - 1 && k * sl.rmax >= zmax[l]) *err = CATANA_ERR_DOMAIN;
+    }
+    const float lb = jl_log2_bound(l, z1, z2 * 1.000001f) + 0.03f;
+    o.w = (uint32_t)(max(-900, (int)floorf(lb) + 1) + 1022) << 20;
+    out[(size_t)blockIdx.x * nl * nmax + e] = o;
+}
+
+// Sort keys: r / rmax on 65536 steps (radii past rmax share the last one).
+__global__ void k_ptc_keys(const double *__restrict__ pts, int pitch, int64_t n, double inv_rmax, uint32_t *keys,
+                           uint32_t *vals) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double q = fabs(pts[pitch * i]) * inv_rmax * 65536.0;
+    keys[i] = q >= 65535.0 ? 65535u : (q > 0.0 ? (uint32_t)q : 0u);
+    vals[i] = (uint32_t)i;
+}
+
+// Per slab: range of |r| and exponent of the largest |w|.  Values that are not finite are left out (they
+// poison the result, k_ptc_points); so are, with the table, radii outside it (a domain error).
+__global__ void __launch_bounds__(256) k_ptc_slabs(const double *__restrict__ pts, int pitch, const double *__restrict__ w,
+                                                   const uint32_t *__restrict__ perm, int64_t n, int64_t per, double rlim,
+                                                   TcSlab *__restrict__ out) {
+    const int64_t i0 = blockIdx.x * per, i1 = min(n, i0 + per);
+    double lo = INFINITY, hi = 0.0, mw = 0.0;
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const int64_t j = perm[i];
+        const double r = fabs(pts[pitch * j]);
+        if (r < rlim) {  // false for NaN
+            lo = fmin(lo, r);
+            hi = fmax(hi, r);
+        }
+        const double v = w ? fabs(w[j]) : 1.0;
+        if (isfinite(v)) mw = fmax(mw, v);
+    }
+    __shared__ double s[3][8];
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s[0][threadIdx.x >> 5] = lo;
+        s[1][threadIdx.x >> 5] = hi;
+        s[2][threadIdx.x >> 5] = mw;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) {
+            lo = fmin(lo, s[0][k]);
+            hi = fmax(hi, s[1][k]);
+            mw = fmax(mw, s[2][k]);
+        }
+        TcSlab o;
+        o.rmin = lo <= hi ? lo : 0.0;
+        o.rmax = hi;
+        o.ew = mw > 0.0 ? ilogb(mw) + 1 : 0;  // mw < 2^ew
+        o.pad = 0;
+        out[blockIdx.x] = o;
+    }
+}
+
+constexpr int TC_POISON_THETA = 1, TC_POISON_PHI = 2, TC_POISON_W = 4;
+
+// v = w cos or -w sin of m phi, times 2^(58 - ew), in signed halves
+__device__ __forceinline__ uint64_t phase_word(double v, double scale) { return signed_halves(__double2ll_rn(v * scale)); }
+
+// Point records and phase tables, in sorted order: a warp per (tile, run of 8 m), lane = point.  The
+// phase of the run's middle comes from the exactly reduced fraction frac(m phi / 2 pi) and is rotated
+// by e^{+-i phi} for the others (at most four times).
+__global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ pts, const double *__restrict__ w,
+                                                    const uint32_t *__restrict__ perm, int64_t n, int tiles, int tslab, int lmp,
+                                                    const TcSlab *__restrict__ slab, int er, int lerp, double rlim,
+                                                    uint64_t *__restrict__ rint, double *__restrict__ rabs, double2 *__restrict__ xs,
+                                                    ulonglong2 *__restrict__ phase, int *__restrict__ poison, int *__restrict__ err) {
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= tiles) return;
+    const int64_t i = (int64_t)t * TC_KT + lane;
+    const bool in = i < n;
+    const int64_t j = in ? perm[i] : perm[n - 1];  // padding takes the last point's radius and no weight
+    const double r = pts[3 * j], th = pts[3 * j + 1], ph = pts[3 * j + 2];
+    double wv = in ? (w ? w[j] : 1.0) : 0.0;
+    int bad = 0;
+    if (!isfinite(th)) bad |= TC_POISON_THETA;
+    if (!isfinite(ph)) bad |= TC_POISON_PHI;
+    if (!isfinite(wv)) bad |= TC_POISON_W;
+    const bool rbad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
+    if (rbad && !lerp) bad |= TC_POISON_W;
+    const double ct = cos(th);
+    const bool use = in && !bad && !rbad;
+    if (blockIdx.y == 0) {
+        if (in && bad) atomicOr(poison, bad);
+        if (in && rbad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
+        rint[i] = rbad ? 0ull : (uint64_t)(int64_t)ldexp(r < 0.0 ? 0.0 : r, 62 - er);
+        rabs[i] = r;
+        xs[i] = use ? make_double2(ct, sqrt((1.0 - ct) * (1.0 + ct))) : make_double2(0.0, 0.0);
+    }
+    const double scale = ldexp(1.0, 58 - slab[t / tslab].ew);
+    if (!use) wv = 0.0;
+    const double phi = use ? ph : 0.0;
+    // frac(phi / 2 pi) 2^64 (mod 2^64), 1 / 2 pi as a pair of doubles: rounded at 2^-64 of a turn
+    const double p = phi * 0.15915494309189535, pl = fma(phi, 0.15915494309189535, -p) - phi * 9.839338337591243e-18;
+    const double f = p - floor(p);
+    const unsigned long long u = (f < 1.0 ? (unsigned long long)ldexp(f, 64) : 0ull) +
+                                 (unsigned long long)__double2ll_rn(fabs(pl) < 0.25 ? ldexp(pl, 64) : 0.0);
+    double s1, c1;
+    sincos(phi, &s1, &c1);
+    const int m0 = blockIdx.y * 8, mc = m0 + 4;
+    double sn, cs;
+    sincospi((double)(long long)((unsigned long long)mc * u) * 1.0842021724855044340074528008699e-19, &sn, &cs);  // 2^-63
+    ulonglong2 *o = phase + ((size_t)t * lmp + m0) * TC_KT + lane;
+    double er_ = cs * wv, ei = -sn * wv;
+    double ur = er_, ui = ei;
+    for (int k = 4; k < 8 && m0 + k < lmp; ++k) {
+        o[k * TC_KT] = make_ulonglong2(phase_word(ur, scale), phase_word(ui, scale));
+        const double nr = ur * c1 + ui * s1, ni = ui * c1 - ur * s1;
+        ur = nr;
+        ui = ni;
+    }
+    for (int k = 3; k >= 0; --k) {
+        const double nr = er_ * c1 - ei * s1, ni = ei * c1 + er_ * s1;
+        er_ = nr;
+        ei = ni;
+        if (m0 + k < lmp) o[k * TC_KT] = make_ulonglong2(phase_word(er_, scale), phase_word(ei, scale));
+    }
+}
+
+// (y0 - dy, dy) per node of the linear tables; the last node is empty
+__global__ void k_ptc_pairs(const double *__restrict__ y, int npts, int64_t total, double2 *__restrict__ o) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    if ((int)(t % npts) == npts - 1) {
+        o[t] = make_double2(0.0, 0.0);
+        return;
+    }
+    const double d = y[t + 1] - y[t];
+    o[t] = make_double2(y[t] - d, d);
+}
+
+// f[l][m][n] += k_ln sum over slabs, in eight interleaved parts added in order; one CTA per 32 (m, n) of
+// a level.  Points that are not finite make their terms NaN: theta every l > 0, phi every m > 0, w all.
+__global__ void __launch_bounds__(256) k_ptc_reduce(const double *__restrict__ partial, int64_t pslab, int nslabs, int l0,
+                                                    int nmax, const double *__restrict__ kln, const int *__restrict__ poison,
+                                                    double2 *__restrict__ f) {
+    __shared__ double2 s[8][33];
+    const int l = l0 + blockIdx.y, cnt = (l + 1) * nmax;
+    const int64_t base = (int64_t)nmax * ((int64_t)l * (l + 1) - (int64_t)l0 * (l0 + 1));
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    for (int e0 = blockIdx.x * 32; e0 < cnt; e0 += gridDim.x * 32) {
+        const int e = e0 + lane;  // n (l + 1) + m
+        double sr = 0.0, si = 0.0;
+        if (e < cnt) {
+            const double2 *p = reinterpret_cast<const double2 *>(partial + base) + e;
+#pragma unroll 4
+            for (int k = part; k < nslabs; k += 8) {
+                const double2 v = p[(size_t)k * (pslab / 2)];
+                sr += v.x;
+                si += v.y;
+            }
+        }
+        s[part][lane] = make_double2(sr, si);
+        __syncthreads();
+        if (part == 0 && e < cnt) {
+#pragma unroll
+            for (int k = 1; k < 8; ++k) {
+                sr += s[k][lane].x;
+                si += s[k][lane].y;
+            }
+            const int n = e / (l + 1), m = e - n * (l + 1);
+            const double k = kln[(size_t)l * nmax + n];
+            double2 *o = f + (size_t)nmax * l * (l + 1) / 2 + (size_t)m * nmax + n;
+            const int bad = *poison;
+            double2 v = *o;
+            if ((bad & TC_POISON_W) || ((bad & TC_POISON_THETA) && l > 0) || ((bad & TC_POISON_PHI) && m > 0)) {
+                v = make_double2(NAN, NAN);
+            } else {
+                v.x += k * sr;
+                v.y += k * si;
+            }
+            *o = v;
+        }
+        __syncthreads();
+    }
+}
+
+// j_l(k_ln r) of every (l, n, point) of the launch's levels: the direct evaluation
+__global__ void k_ptc_jl_exact(const double *__restrict__ r, const double *__restrict__ kln, int l0, int nl, int nmax, int tiles,
+                               double *__restrict__ out) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // [l][tile][n][lane]
+    if (e >= (int64_t)nl * tiles * nmax * TC_KT) return;
+    const int lane = (int)(e & 31);
+    const int64_t q = e >> 5;
+    const int n = (int)(q % nmax);
+    const int64_t q2 = q / nmax;
+    const int t = (int)(q2 % tiles), l = l0 + (int)(q2 / tiles);
+    const double z = kln[(size_t)l * nmax + n] * r[(size_t)t * TC_KT + lane];
+    out[e] = isfinite(z) ? sbessel_jl(l, z) : 0.0;
+}
+
+// the same from the FP64 polynomials ([l][interval][12])
+__global__ void k_ptc_jl_poly(const double *__restrict__ r, const double *__restrict__ kln, int l0, int nl, int nmax, int tiles,
+                              const double *__restrict__ poly, int nint, double *__restrict__ out, int *err) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= (int64_t)nl * tiles * nmax * TC_KT) return;
+    const int lane = (int)(e & 31);
+    const int64_t q = e >> 5;
+    const int n = (int)(q % nmax);
+    const int64_t q2 = q / nmax;
+    const int t = (int)(q2 % tiles), l = l0 + (int)(q2 / tiles);
+    const double z = kln[(size_t)l * nmax + n] * r[(size_t)t * TC_KT + lane];
+    const double zr = rint(z);
+    int jj = (int)zr;
+    if (!(z >= 0.0) || jj >= nint) {  // the host sized the table from max r
+        *err = CATANA_ERR_DOMAIN;
+        jj = 0;
+    }
+    const double t2 = 2.0 * (z - zr);
+    const double2 *c2 = reinterpret_cast<const double2 *>(poly + ((size_t)l * nint + jj) * 12);
+    double2 c = c2[5];
+    double p = fma(c.y, t2, c.x);
+#pragma unroll
+    for (int k = 4; k >= 0; --k) {
+        c = c2[k];
+        p = fma(p, t2, c.y);
+        p = fma(p, t2, c.x);
+    }
+    out[e] = p;
+}
+
+size_t tc_al(size_t b) { return (b + 255) & ~size_t(255); }
+
+// (beta, A) per (l, m): Q_l = x Q_{l-1} - beta Q_{l-2}, P = A Q, Q_mm = sin^m
+catana_status_t ensure_tc_coefs(DeviceContext *ctx, int lmax, cudaStream_t st) {
+    if (ctx->tc_coef_lmax >= lmax) return CATANA_OK;
+    std::vector<double2> h((size_t)lmax * (lmax + 1) / 2);
+    long double amm = 0.28209479177387814347403972578038630L;  // 1 / sqrt(4 pi)
+    for (int m = 0; m < lmax; ++m) {
+        if (m > 0) amm *= -sqrtl((2.0L * m + 1.0L) / (2.0L * m));
+        long double A = amm;
+        for (int l = m; l < lmax; ++l) {
+            double beta = 0.0;
+            if (l > m) {
+                const long double dl = l, mm = (long double)m * m;
+                A *= sqrtl((4.0L * dl * dl - 1.0L) / (dl * dl - mm));
+            }
+            if (l > m + 1) {
+                const double d1 = l - 1;
+                beta = (d1 * d1 - (double)m * m) / (4.0 * d1 * d1 - 1.0);
+            }
+            h[(size_t)l * (l + 1) / 2 + m] = make_double2(beta, (double)A);
+        }
+    }
+    CG_CUDA_TRY(ctx->tc_coef.ensure(h.size() * sizeof(double2)));
+    CG_CUDA_TRY(cudaMemcpyAsync(ctx->tc_coef.ptr, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
+    CG_CUDA_TRY(cudaStreamSynchronize(st));
+    ctx->tc_coef_lmax = lmax;
+    return CATANA_OK;
+}
+
+// (y0 - dy, dy) tables, dx^-1 and z_max per l (cached like the tables that they are made from)
+catana_status_t ensure_tc_tables(DeviceContext *ctx, int lmax, int nmax, cudaStream_t st) {
+    catana_status_t s = ensure_lerp_tables(ctx, lmax, nmax, st);
+    if (s != CATANA_OK) return s;
+    if (ctx->tc_tab_lmax >= lmax && ctx->tc_tab_nmax == nmax) return CATANA_OK;
+    lmax = ctx->tab_lmax;
+    const int npts = 1000 * nmax;
+    const int64_t total = (int64_t)lmax * npts;
+    const size_t tb = tc_al((size_t)total * sizeof(double2));
+    CG_CUDA_TRY(ctx->tc_tab.ensure(tb + 2 * (size_t)lmax * sizeof(double)));
+    double *dz = reinterpret_cast<double *>(ctx->tc_tab.as<char>() + tb);
+    k_ptc_pairs<<<ceil_div(total, 256), 256, 0, st>>>(ctx->tables.as<double>(), npts, total, ctx->tc_tab.as<double2>());
+    count_launch();
+    CG_CUDA_TRY(cudaGetLastError());
+    CG_CUDA_TRY(cudaMemcpyAsync(dz, ctx->tab_dxinv.data(), lmax * sizeof(double), cudaMemcpyHostToDevice, st));
+    CG_CUDA_TRY(cudaMemcpyAsync(dz + lmax, ctx->tab_zmax.data(), lmax * sizeof(double), cudaMemcpyHostToDevice, st));
+    CG_CUDA_TRY(cudaStreamSynchronize(st));
+    ctx->tc_tab_off = tb;
+    ctx->tc_tab_lmax = lmax;
+    ctx->tc_tab_nmax = nmax;
+    return CATANA_OK;
+}
+
+}  // namespace
+
+// nmax: the table position k r / dx has at most 27 integer bits; rmax: k / dx stays inside FP64
+bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
+    return ctx->cc_major == 10 && ctx->cc_minor == 3 && lmax <= TC_LMAX && nmax >= 1 && nmax <= 4096 && rmax > 1e-100 &&
+           rmax < 1e100;
+}
+
+catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, int64_t npoints,
+                                    int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev, double *f_acc_dev,
+                                    int *err_dev, cudaStream_t st) {
+    const bool lerp = jl == JL_MODE_LERP;
+    catana_status_t s = ensure_tc_coefs(ctx, lmax, st);
+    if (s != CATANA_OK) return s;
+    if (lerp) {
+        s = ensure_tc_tables(ctx, lmax, nmax, st);
+        if (s != CATANA_OK) return s;
+    }
+    if (!ctx->attr_tc) {
+        CG_CUDA_TRY(cudaFuncSetAttribute(k_ptc_main<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+        CG_CUDA_TRY(cudaFuncSetAttribute(k_ptc_main<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+        ctx->attr_tc = true;
+    }
+    const int lmp = (lmax + 3) & ~3;
+    // 2^er > 4 rmax: radii at or past 4 rmax lie outside the table of l = 0 whatever nmax
+    const int er = ilogb(rmax) + 3;
+    const double rlim = lerp ? ldexp(1.0, er) : INFINITY;
+    // points per pass: rows and phases (32 B per point and m) stay under 12 GB
+    int64_t chunk = std::max<int64_t>(TC_KT, (int64_t)(12e9 / (32.0 * lmp)) / TC_KT * TC_KT);
+    chunk = std::min(chunk, npoints);
+    const int tiles_c = ceil_div(chunk, TC_KT);
+    const size_t np = (size_t)tiles_c * TC_KT;
+    // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
+    const size_t kb = tc_al(np * 4), hb = tc_al((size_t)256 * ((np + 4095) / 4096 + 1) * 4);
+    const size_t o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(np * 8), o_xs = o_rabs + tc_al(np * 8);
+    const size_t o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
+    // slabs: at most TC_SLAB_TILES tiles (the 64-bit sums' resolution), a whole number of waves
+    auto slab_tiles = [&](int tiles) {
+        const int waves = ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES);
+        return ceil_div(tiles, (int64_t)ctx->sm_count * waves);
+    };
+    const int max_slabs = ctx->sm_count * ceil_div(tiles_c, (int64_t)ctx->sm_count * TC_SLAB_TILES);
+    const size_t o_mx = o_sl + tc_al((size_t)max_slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)max_slabs * 3 * TC_LMAX * 4);
+    CG_CUDA_TRY(ctx->tc_ws.ensure(o_poi + 256));
+    char *ws = ctx->tc_ws.as<char>();
+    uint32_t *keys = reinterpret_cast<uint32_t *>(ws), *perm = reinterpret_cast<uint32_t *>(ws + kb);
+    uint32_t *tk = reinterpret_cast<uint32_t *>(ws + 2 * kb), *tv = reinterpret_cast<uint32_t *>(ws + 3 * kb);
+    uint32_t *hist = reinterpret_cast<uint32_t *>(ws + 4 * kb);
+    int *poison = reinterpret_cast<int *>(ws + o_poi);
+    TcSlab *slabs = reinterpret_cast<TcSlab *>(ws + o_sl);
+    CG_CUDA_TRY(cudaMemsetAsync(poison, 0, sizeof(int), st));
+    for (int64_t c0 = 0; c0 < npoints; c0 += chunk) {
+        const int64_t nc = std::min(chunk, npoints - c0);
+        const int tiles = ceil_div(nc, TC_KT);
+        const int tslab = slab_tiles(tiles), nslabs = ceil_div(tiles, tslab);
+        const double *pts = points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
+        k_ptc_keys<<<ceil_div(nc, 256), 256, 0, st>>>(pts, 3, nc, 1.0 / rmax, keys, perm);
+        count_launch();
+        s = radix_sort_pairs(keys, perm, tk, tv, nc, 16, hist, st);
+        if (s != CATANA_OK) return s;
+        k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, 3, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
+        k_ptc_points<<<dim3(ceil_div(tiles, 8), ceil_div(lmp, 8)), 256, 0, st>>>(
+            pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, reinterpret_cast<uint64_t *>(ws + o_rint),
+            reinterpret_cast<double *>(ws + o_rabs), reinterpret_cast<double2 *>(ws + o_xs),
+            reinterpret_cast<ulonglong2 *>(ws + o_ph), poison, err_dev);
+        count_launch(2);
+        CG_CUDA_TRY(cudaGetLastError());
+        TcArgs a;
+        a.nmax = nmax;
+        a.lmp = lmp;
+        a.tiles = tiles;
+        a.tslab = tslab;
+        a.phase = reinterpret_cast<const ulonglong2 *>(ws + o_ph);
+        a.rows = reinterpret_cast<double *>(ws + o_rows);
+        a.rint = reinterpret_cast<const uint64_t *>(ws + o_rint);
+        a.xs = reinterpret_cast<const double2 *>(ws + o_xs);
+        a.slab = slabs;
+        a.coef = ctx->tc_coef.as<double2>();
+        a.npts = 1000 * nmax;
+        a.maxq = reinterpret_cast<uint32_t *>(ws + o_mx);
+        a.err = err_dev;
+        a.tab = nullptr;
+        const double *dxinv = nullptr;
+        if (lerp) {
+            a.tab = ctx->tc_tab.as<double2>();
+            dxinv = reinterpret_cast<const double *>(ctx->tc_tab.as<char>() + ctx->tc_tab_off);
+        }
+        // levels per launch: the slabs' partial sums stay under 256 MB (they are read back at once and
+        // mostly hit L2), the j_l arrays of the other modes under 2 GB
+        for (int l0 = 0; l0 < lmax;) {
+            int l1 = l0 + 1;
+            auto pdoubles = [&](int e) { return (int64_t)nmax * ((int64_t)e * (e + 1) - (int64_t)l0 * (l0 + 1)); };
+            const double jbytes = lerp ? 0.0 : 8.0 * tiles * TC_KT * nmax;
+            while (l1 < lmax && pdoubles(l1 + 1) * 8.0 * nslabs < 256e6 && jbytes * (l1 + 1 - l0) < 2e9) ++l1;
+            a.l0 = l0;
+            a.l1 = l1;
+            a.pslab = pdoubles(l1);
+            const size_t pb = tc_al((size_t)a.pslab * nslabs * 8);
+            CG_CUDA_TRY(ctx->partial.ensure(pb + (size_t)nslabs * (l1 - l0) * nmax * sizeof(uint4)));
+            a.partial = ctx->partial.as<double>();
+            uint4 *ntab = reinterpret_cast<uint4 *>(ctx->partial.as<char>() + pb);
+            a.ntab = ntab;
+            k_ptc_ntab<<<dim3(nslabs, ceil_div((int64_t)(l1 - l0) * nmax, 128)), 128, 0, st>>>(
+                slabs, kln_dev, dxinv, dxinv ? dxinv + ctx->tc_tab_lmax : nullptr, l0, l1 - l0, nmax, er, ntab, err_dev);
+            count_launch();
+            a.jarr = nullptr;
+            if (!lerp) {
+                const int64_t cnt = (int64_t)(l1 - l0) * tiles * nmax * TC_KT;
+                CG_CUDA_TRY(ctx->tc_jarr.ensure((size_t)cnt * 8));
+                double *ja = ctx->tc_jarr.as<double>();
+                const double *r = reinterpret_cast<const double *>(ws + o_rabs);
+                if (jl == JL_MODE_POLY)
+                    k_ptc_jl_poly<<<ceil_div(cnt, 256), 256, 0, st>>>(r, kln_dev, l0, l1 - l0, nmax, tiles,
+                                                                      ctx->poly.as<double>(), ctx->poly_nint, ja, err_dev);
+                else
+                    k_ptc_jl_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(r, kln_dev, l0, l1 - l0, nmax, tiles, ja);
+                count_launch();
+                CG_CUDA_TRY(cudaGetLastError());
+                a.jarr = ja;
+            }
+            prof_begin(st);
+            if (lerp) k_ptc_main<true><<<nslabs, TC_THREADS, TC_SMEM, st>>>(a);
+            else k_ptc_main<false><<<nslabs, TC_THREADS, TC_SMEM, st>>>(a);
+            prof_end(st, 2.0 * (double)nc * (double)pdoubles(l1));
+            k_ptc_reduce<<<dim3(std::min(64, ceil_div((int64_t)l1 * nmax, 32)), l1 - l0), 256, 0, st>>>(
+                a.partial, a.pslab, nslabs, l0, nmax, kln_dev, poison, reinterpret_cast<double2 *>(f_acc_dev));
+            count_launch(2);
+            CG_CUDA_TRY(cudaGetLastError());
+            l0 = l1;
+        }
+    }
+    return CATANA_OK;
+}
+
+}  // namespace catana_gpu

@@ -473,7 +473,7 @@ catana_status_t ensure_poly_tables(DeviceContext *ctx, int lmax, int nint, cudaS
 }
 
 catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
-                                    int64_t npoints, int lmax, int nmax, JlMode jl, const double *kln_dev,
+                                    int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev,
                                     double *f_acc_dev, int *err_dev, cudaStream_t st) {
     const bool interpolated = (jl == JL_MODE_LERP);
     catana_status_t s = ensure_coefs(ctx, lmax, st);
@@ -513,6 +513,9 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
         s = ensure_poly_tables(ctx, lmax, (int)std::floor(zmax + 0.5) + 2, st);
         if (s != CATANA_OK) return s;
     }
+    if (plain_tc_takes(ctx, lmax, nmax, rmax))
+        return plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, kln_dev, f_acc_dev,
+                                   err_dev, st);
     // Chunk so that the three Legendre rows stay under ~1.5 GB.
     int64_t chunk = (int64_t)(1.5e9 / (3.0 * 8.0 * std::max(lmax, 1)));
     chunk = std::max<int64_t>(1024, std::min<int64_t>(chunk, npoints));

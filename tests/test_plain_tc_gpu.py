@@ -1,0 +1,82 @@
+"""The plain form's tensor-core contraction (k_ptc_main) at the sizes where its tiling can go wrong:
+point counts around a tile (32), a group (128) and a slab, multipoles around the 64-row blocks, radial
+orders around the 16-column steps, the 32-column halves and the 64-column blocks; weights that vary by
+many orders; points that are not finite.
+
+Tolerance, from the arithmetic: digits are cut at 2^-55 of a row's bound and sums at 2^-51 of a slab's
+largest term, ~1e-15; the oracle's own table position k r / dx carries a rounding of 1e5 * 2^-53 in a slope of
+~3e-3 (4e-14 of j_l's envelope), and both recurrences build up ~l 2^-53.  1e-12 of the level's largest
+|f| leaves a factor of ten over their sum."""
+import numpy as np
+import pytest
+
+import catana_gb300 as catana
+from oracle import oracle as O
+from conftest import uniform_ball
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def _check(pts, lmax, nmax, interp, weights=None, rmax=1000.0):
+    res = catana.sfb_decomposition(catana.PointContainer(pts), lmax, nmax, rmax, True, False, weights=weights,
+                                   interpolation=interp)
+    k, c, f = O.sfb_raw(pts, lmax, nmax, rmax, interpolated=(interp == "on"), weights=weights)
+    assert np.array_equal(res.k_ln, k)
+    for l, (a, b) in enumerate(zip(res.f_lmn, f)):
+        assert np.max(np.abs(a - b)) <= TOL * np.max(np.abs(b)), (l, np.max(np.abs(a - b)) / np.max(np.abs(b)))
+
+
+@pytest.mark.parametrize("n,lmax,nmax", [(1, 1, 1), (31, 2, 16), (32, 5, 17), (33, 33, 32), (129, 64, 33), (300, 65, 48),
+                                         (161, 66, 64), (700, 70, 65), (5000, 34, 130)])
+def test_tile_edges(cuda_device, n, lmax, nmax):
+    pts = uniform_ball(n, 1000.0, seed=n)
+    _check(pts, lmax, nmax, "on")
+    if n <= 200:
+        _check(pts, lmax, nmax, "off")
+        _check(pts, lmax, nmax, "poly", np.random.default_rng(1).uniform(0.5, 1.5, n))
+
+
+def test_many_slabs_and_groups(cuda_device):
+    """More than one slab per CTA slot is not needed here: 40k points give slabs of nine tiles, a last group
+    of one tile, and sixteen-column D regions that alternate."""
+    _check(uniform_ball(40000, 1000.0, seed=3), 7, 16, "on")
+
+
+def test_narrow_catalogs(cuda_device):
+    """Points in a polar cap and in a thin, distant shell: the row bounds follow the points (|P_lm| down to
+    sin(0.05)^m, j_l far below its first maximum) and the small values keep their digits."""
+    rng = np.random.default_rng(5)
+    n = 400
+    cap = np.stack([1000.0 * rng.random(n) ** (1 / 3), rng.uniform(0.01, 0.05, n), rng.uniform(0, 2 * np.pi, n)], 1)
+    _check(cap, 24, 12, "on")
+    near = cap.copy()
+    near[:, 0] = rng.uniform(20.0, 25.0, n)
+    near[:, 1] = np.arccos(rng.uniform(-1, 1, n))
+    _check(near, 24, 12, "off")
+    same = np.tile(np.array([[700.0, 1.1, 2.2]]), (n, 1))  # every digit the same: the sums' largest values
+    _check(same, 24, 12, "on")
+
+
+def test_weights_over_many_orders(cuda_device):
+    rng = np.random.default_rng(6)
+    pts = uniform_ball(3000, 1000.0, seed=8)
+    _check(pts, 12, 20, "on", 10.0 ** rng.uniform(-9, 3, 3000))
+    _check(pts, 12, 20, "on", rng.normal(size=3000))
+    _check(pts, 12, 20, "on", np.where(np.arange(3000) == 17, 1.0, 0.0))
+
+
+@pytest.mark.parametrize("column,bad", [(1, np.nan), (2, np.inf), (3, np.nan)])
+def test_points_that_are_not_finite(cuda_device, column, bad):
+    """theta enters every l > 0, phi every m > 0, a weight everything; the rest stays as without the flaw."""
+    pts = uniform_ball(200, 1000.0, seed=9)
+    w = np.ones(200)
+    if column < 3:
+        pts[50, column] = bad
+    else:
+        w[50] = bad
+    res = catana.sfb_decomposition(catana.PointContainer(pts), 4, 3, 1000.0, True, False, weights=w, interpolation="on")
+    for l, f in enumerate(res.f_lmn):
+        for m in range(l + 1):
+            nan = (column == 1 and l > 0) or (column == 2 and m > 0) or column == 3
+            assert np.all(np.isnan(f[m])) == nan and np.all(np.isfinite(f[m])) == (not nan), (l, m)
