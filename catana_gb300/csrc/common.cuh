@@ -97,6 +97,8 @@ struct DeviceContext {
     DevBuf tc_coef;    // (beta, A) of the monic recurrence
     DevBuf tc_tab;     // (y0 - dy, dy) lerp tables, dx^-1 and z_max per l
     DevBuf tc_jarr;    // j_l arrays of the modes without a table
+    DevBuf tc_poly;    // the polynomials of `poly` as integers
+    int tc_poly_lmax = -1, tc_poly_nint = -1;
     int tc_coef_lmax = -1, tc_tab_lmax = -1, tc_tab_nmax = -1;
     size_t tc_tab_off = 0;
     bool attr_tc = false;
@@ -130,11 +132,11 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
                                     int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev,
                                     double *f_acc_dev, int *err_dev, cudaStream_t st);
 // The same sum with its contraction on the tensor cores (plain_tc.cu), where the device has them and
-// lmax <= 512; with JL_MODE_POLY the caller has prepared ctx->poly.
+// lmax <= 512; with JL_MODE_POLY the caller has prepared ctx->poly and passes the largest radius (else rtop = 0).
 bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax);
 catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
-                                    int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev,
-                                    double *f_acc_dev, int *err_dev, cudaStream_t st);
+                                    int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, double rtop,
+                                    const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st);
 // f *= norm; c_ln from f (device).
 catana_status_t finish_flmn_cln(double *f_dev, double norm, int lmax, int nmax, double *c_ln_dev,
                                 cudaStream_t st);

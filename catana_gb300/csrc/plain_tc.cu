@@ -106,7 +106,7 @@ struct TcArgs {
     const uint4 *ntab;          // [slab][l - l0][n]: (kd hi, kd lo, shift, EJ)
     const double2 *tab;         // lerp tables [l][npts]: (y_i - dy_i, dy_i), or null
     int npts;
-    const double *jarr;         // [l - l0][tile][nmax][32] where tab is null
+    const uint64_t *jarr;       // J with its digit offset, [l - l0][tile][nmax][32], where tab is null
     uint32_t *maxq;             // [slab][3][TC_LMAX]: level maxima between launches
     double *partial;            // [slab][l - l0][n][2 (l + 1)]
     int64_t pslab;              // doubles per slab in partial
@@ -167,6 +167,14 @@ __device__ __forceinline__ ulonglong2 ld_if(const ulonglong2 *p, bool pred) {
                  : "=l"(v.x), "=l"(v.y)
                  : "l"(p), "r"((int)pred));
     return v;
+}
+
+// j 2^(63 - EJ) with the digit offset; w = (EJ + 1022) 2^20
+__device__ __forceinline__ uint64_t j_digits(double j, uint32_t w) {
+    const uint32_t jh = (uint32_t)__double2hiint(j), jl = (uint32_t)__double2loint(j);
+    const int s = (int)(w - (jh & 0x7ff00000u)) >> 20;
+    const uint64_t p = shr64(((uint64_t)((jh & 0xfffffu) | 0x100000u) << 42) | ((uint64_t)jl << 10), s);
+    return jh >> 31 ? TC_OFF_J - p : TC_OFF_J + p;
 }
 
 // log2 of a bound on |j_l| over [z1, z2] (FP32; checked to exceed log2 |j_l| up to 1e-6 for every l < 512):
@@ -413,20 +421,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                                 }
 #pragma unroll
                                 for (int h = 0; h < 4; ++h)
-                                    v[h0 + h] = (uint64_t)__double_as_longlong(fma(y[h].y, f[h], y[h].x));
+                                    v[h0 + h] = j_digits(fma(y[h].y, f[h], y[h].x), tn[8 * o + h0 + h].w);
                             }
                         } else {
-                            const double *jp = a.jarr + (((size_t)(l - a.l0) * a.tiles + t) * a.nmax + b.n0 + 8 * o) * TC_KT + lane;
+                            const uint64_t *jp = a.jarr + (((size_t)(l - a.l0) * a.tiles + t) * a.nmax + b.n0 + 8 * o) * TC_KT + lane;
 #pragma unroll
-                            for (int h = 0; h < 8; ++h)
-                                v[h] = 8 * o + h < b.ncount ? (uint64_t)__double_as_longlong(__ldg(jp + h * TC_KT)) : 0ull;
-                        }
-#pragma unroll
-                        for (int h = 0; h < 8; ++h) {
-                            const uint32_t jh = (uint32_t)(v[h] >> 32), jl = (uint32_t)v[h];
-                            const int s = (int)(tn[8 * o + h].w - (jh & 0x7ff00000u)) >> 20;
-                            const uint64_t p = shr64(((uint64_t)((jh & 0xfffffu) | 0x100000u) << 42) | ((uint64_t)jl << 10), s);
-                            v[h] = jh >> 31 ? TC_OFF_J - p : TC_OFF_J + p;
+                            for (int h = 0; h < 8; ++h) v[h] = 8 * o + h < b.ncount ? __ldg(jp + h * TC_KT) : TC_OFF_J;
                         }
                     }
                     load_next(t, u);
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
     if (blockIdx.y == 0) {
         if (in && bad) atomicOr(poison, bad);
         if (in && rbad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
-        rint[i] = rbad ? 0ull : (uint64_t)(int64_t)ldexp(r < 0.0 ? 0.0 : r, 62 - er);
+        rint[i] = rbad || !(fabs(r) < ldexp(1.0, er)) ? 0ull : (uint64_t)(int64_t)ldexp(fmax(r, 0.0), 62 - er);
         rabs[i] = r;
         xs[i] = use ? make_double2(ct, sqrt((1.0 - ct) * (1.0 + ct))) : make_double2(0.0, 0.0);
     }
@@ -807,48 +807,153 @@ __global__ void __launch_bounds__(256) k_ptc_reduce(const double *__restrict__ p
     }
 }
 
-// j_l(k_ln r) of every (l, n, point) of the launch's levels: the direct evaluation
-__global__ void k_ptc_jl_exact(const double *__restrict__ r, const double *__restrict__ kln, int l0, int nl, int nmax, int tiles,
-                               double *__restrict__ out) {
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // [l][tile][n][lane]
-    if (e >= (int64_t)nl * tiles * nmax * TC_KT) return;
-    const int lane = (int)(e & 31);
-    const int64_t q = e >> 5;
-    const int n = (int)(q % nmax);
-    const int64_t q2 = q / nmax;
-    const int t = (int)(q2 % tiles), l = l0 + (int)(q2 / tiles);
-    const double z = kln[(size_t)l * nmax + n] * r[(size_t)t * TC_KT + lane];
-    out[e] = isfinite(z) ? sbessel_jl(l, z) : 0.0;
+// j_l(z), z finite: the direct evaluation of sbessel_jl (same branches) with the recurrences' (2 k + 1) / z
+// from one reciprocal, corrected by an FMA to within an ulp of the quotient -- a division costs about
+// twelve FP64 operations at two per SM and cycle, and the recurrences take one per step.
+__device__ __forceinline__ double jl_direct(int l, double z) {
+    if (z == 0.0) return l == 0 ? 1.0 : 0.0;
+    const double sgn = z < 0.0 && (l & 1) ? -1.0 : 1.0, x = fabs(z);
+    if (x * x < 2.0 * l + 3.0) return sgn * jl_series(l, x);
+    const double ix = 1.0 / x;
+    auto quot = [&](double n) {
+        const double q = n * ix;
+        return fma(fma(-q, x, n), ix, q);
+    };
+    double sn, cs;
+    sincos(x, &sn, &cs);
+    const double t0 = quot(sn), t1 = quot(t0 - cs);
+    if (x >= (double)l) {
+        if (l == 0) return sgn * t0;
+        double j0 = t0, j1 = t1;
+        for (int k = 1; k < l; ++k) {
+            const double j2 = fma(quot(2.0 * k + 1.0), j1, -j0);
+            j0 = j1;
+            j1 = j2;
+        }
+        return sgn * j1;
+    }
+    const int nstart = (int)((double)l + 20.0 + 16.0 * cbrt((double)l + 1.0));
+    double jp1 = 0.0, jk = 1e-200, jl = 0.0;
+    for (int k = nstart; k > 0; --k) {
+        const double jm1 = fma(quot(2.0 * k + 1.0), jk, -jp1);
+        jp1 = jk;
+        jk = jm1;
+        if (k - 1 == l) jl = jk;
+        if (fabs(jk) > 1e200) {
+            jk *= 1e-200;
+            jp1 *= 1e-200;
+            jl *= 1e-200;
+        }
+    }
+    return sgn * (fabs(t0) >= fabs(t1) ? jl * (t0 / jk) : jl * (t1 / jp1));
 }
 
-// the same from the FP64 polynomials ([l][interval][12])
-__global__ void k_ptc_jl_poly(const double *__restrict__ r, const double *__restrict__ kln, int l0, int nl, int nmax, int tiles,
-                              const double *__restrict__ poly, int nint, double *__restrict__ out, int *err) {
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= (int64_t)nl * tiles * nmax * TC_KT) return;
-    const int lane = (int)(e & 31);
-    const int64_t q = e >> 5;
-    const int n = (int)(q % nmax);
-    const int64_t q2 = q / nmax;
-    const int t = (int)(q2 % tiles), l = l0 + (int)(q2 / tiles);
-    const double z = kln[(size_t)l * nmax + n] * r[(size_t)t * TC_KT + lane];
-    const double zr = rint(z);
-    int jj = (int)zr;
-    if (!(z >= 0.0) || jj >= nint) {  // the host sized the table from max r
+// J of every (l, n, point) of the launch's levels: a warp per (l, tile, n), lane = point
+struct TcJ {
+    const double *r, *kln;
+    const uint64_t *rint;
+    const uint4 *ntab;
+    int l0, nl, nmax, tiles, tslab, er;
+    uint64_t *out;
+};
+__device__ __forceinline__ bool tc_j_index(const TcJ &a, int &l, int &t, int &n, size_t &e) {
+    const int64_t q = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (q >= (int64_t)a.nl * a.tiles * a.nmax) return false;  // warp-uniform
+    n = (int)(q % a.nmax);
+    const int64_t q2 = q / a.nmax;
+    t = (int)(q2 % a.tiles);
+    l = a.l0 + (int)(q2 / a.tiles);
+    e = (size_t)q * TC_KT + (threadIdx.x & 31);
+    return true;
+}
+__global__ void __launch_bounds__(256) k_ptc_jl_exact(TcJ a) {
+    int l, t, n;
+    size_t e;
+    if (!tc_j_index(a, l, t, n, e)) return;
+    const double z = a.kln[(size_t)l * a.nmax + n] * a.r[(size_t)t * TC_KT + (threadIdx.x & 31)];
+    const uint32_t w = a.ntab[((size_t)(t / a.tslab) * a.nl + (l - a.l0)) * a.nmax + n].w;
+    a.out[e] = j_digits(isfinite(z) ? jl_direct(l, z) : 0.0, w);
+}
+
+// The FP64 polynomials (sfb_fp64.cu, sum_s a_s t^s on unit intervals, t in [-1, 1]) as integers: Horner's
+// steps are 64-bit integer products here (~10 instructions each; an FP64 FMA occupies its pipe for 16
+// cycles per warp).  With B_s = 4^s A_s K the step B_s = 4^s a_s K + t B_{s+1} / 4 is the upper half of
+// t 2^62 times B_{s+1}; K = 2^(59 - e), max_s |4^s a_s| < 2^e, keeps |B_s| < 2^60.  The terms s >= 9 (below
+// 1e-8 of the first) take 32-bit products at a scale of their own, and are shifted to the others' (up).
+struct TcPoly {
+    int64_t c[9];
+    int32_t h[3];
+    int32_t e, up, pad;
+};
+static_assert(sizeof(TcPoly) == 96, "TcPoly layout");
+
+__global__ void k_ptc_poly_int(const double *__restrict__ poly, int64_t total, TcPoly *__restrict__ out) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    double a[12], mx = 0.0;
+    for (int k = 0; k < 12; ++k) {
+        a[k] = ldexp(poly[t * 12 + k], 2 * k);
+        mx = fmax(mx, fabs(a[k]));
+    }
+    TcPoly o;
+    o.e = mx > 0.0 ? ilogb(mx) + 1 : -2000;
+    for (int k = 0; k < 9; ++k) o.c[k] = __double2ll_rn(ldexp(a[k], 59 - o.e));
+    double mh = 0.0;
+    for (int k = 9; k < 12; ++k) mh = fmax(mh, fabs(a[k]));
+    const int e9 = mh > 0.0 ? ilogb(mh) + 1 : -2000;  // |4^s a_s| < 2^e9
+    for (int k = 9; k < 12; ++k) o.h[k - 9] = __double2int_rn(ldexp(a[k], 29 - e9));
+    o.up = 30 - o.e + e9;
+    o.pad = 0;
+    out[t] = o;
+}
+
+__global__ void __launch_bounds__(256) k_ptc_jl_poly(TcJ a, const TcPoly *__restrict__ poly, int nint, int *err) {
+    int l, t, n;
+    size_t e;
+    if (!tc_j_index(a, l, t, n, e)) return;
+    const uint64_t kb = (uint64_t)__double_as_longlong(a.kln[(size_t)l * a.nmax + n]);
+    const uint64_t r = a.rint[(size_t)t * TC_KT + (threadIdx.x & 31)];
+    const uint32_t w = a.ntab[((size_t)(t / a.tslab) * a.nl + (l - a.l0)) * a.nmax + n].w;
+    // z = k r = (r kmant / 2^64) / 2^(60 - er - ek): integer and 64-bit fraction of z + 1/2
+    const int sh = 4 + a.er + (int)(kb >> 52) - 1022;
+    const uint64_t km = ((kb & 0xfffffffffffffull) | 0x10000000000000ull) << 9;
+    const uint32_t kh = (uint32_t)(km >> 32), kl = (uint32_t)km, rh = (uint32_t)(r >> 32), rl = (uint32_t)r;
+    const uint64_t tt = (uint64_t)rl * kh + (uint64_t)rh * kl, res = (uint64_t)rh * kh + (tt >> 32);
+    // 60 - er - ek bits of res are fraction (up to 64: k r < 1/16 when sh < 0)
+    uint64_t fr = sh >= 0 ? (res << sh) | ((uint64_t)(uint32_t)tt << 32 >> (64 - sh) & (sh ? ~0ull : 0ull)) : shr64(res, -sh);
+    uint32_t j = sh > 0 ? (uint32_t)(res >> (64 - sh)) : 0u;
+    fr += 0x8000000000000000ull;
+    j += fr < 0x8000000000000000ull ? 1u : 0u;
+    if (j >= (uint32_t)nint) {  // the host sized the table from max r
         *err = CATANA_ERR_DOMAIN;
-        jj = 0;
+        j = 0;
     }
-    const double t2 = 2.0 * (z - zr);
-    const double2 *c2 = reinterpret_cast<const double2 *>(poly + ((size_t)l * nint + jj) * 12);
-    double2 c = c2[5];
-    double p = fma(c.y, t2, c.x);
+    const uint64_t ts = signed_halves((int64_t)(fr - 0x8000000000000000ull) >> 1);  // t 2^62
+    const int32_t t1 = (int32_t)(ts >> 32), t0 = (int32_t)ts;
+    const int4 *q = reinterpret_cast<const int4 *>(poly + (size_t)l * nint + j);
+    const longlong2 c8 = __ldg(reinterpret_cast<const longlong2 *>(q + 4));  // c_8; h_9, h_10
+    const int4 he = __ldg(q + 5);                                              // h_11, e, up
+    int32_t b = he.x;
+    b = (int32_t)(c8.y >> 32) + __mulhi(b, t1);
+    b = (int32_t)c8.y + __mulhi(b, t1);
+    int64_t v = he.z >= 0 ? (int64_t)b << min(he.z, 32) : (int64_t)(b >> min(-he.z, 31));
+    auto step = [&](int64_t ck) {
+        const uint64_t h = signed_halves(v);
+        const int32_t h1 = (int32_t)(h >> 32), h0 = (int32_t)h;
+        const int64_t m = (int64_t)h1 * t0 + ((int64_t)h0 * t1 + 0x80000000ll);
+        v = (int64_t)h1 * t1 + ((m >> 32) + ck);
+    };
+    step(c8.x);
 #pragma unroll
-    for (int k = 4; k >= 0; --k) {
-        c = c2[k];
-        p = fma(p, t2, c.y);
-        p = fma(p, t2, c.x);
+    for (int k = 3; k >= 0; --k) {
+        const longlong2 c = __ldg(reinterpret_cast<const longlong2 *>(q + k));
+        step(c.y);
+        step(c.x);
     }
-    out[e] = p;
+    // j_l = v 2^(e - 59) -> 2^(63 - EJ) j_l
+    const int up = 4 + he.y - ((int)(w >> 20) - 1022);
+    v = up >= 0 ? (up > 63 ? 0 : v << up) : v >> min(63, -up);
+    a.out[e] = TC_OFF_J + (uint64_t)v;
 }
 
 size_t tc_al(size_t b) { return (b + 255) & ~size_t(255); }
@@ -904,6 +1009,20 @@ catana_status_t ensure_tc_tables(DeviceContext *ctx, int lmax, int nmax, cudaStr
     return CATANA_OK;
 }
 
+// the polynomials of ctx->poly as integers (rebuilt when those are)
+catana_status_t ensure_tc_poly(DeviceContext *ctx, cudaStream_t st) {
+    if (ctx->tc_poly_lmax == ctx->poly_lmax && ctx->tc_poly_nint == ctx->poly_nint) return CATANA_OK;
+    const int64_t total = (int64_t)ctx->poly_lmax * ctx->poly_nint;
+    CG_CUDA_TRY(ctx->tc_poly.ensure((size_t)total * sizeof(TcPoly)));
+    k_ptc_poly_int<<<ceil_div(total, 128), 128, 0, st>>>(ctx->poly.as<double>(), total, ctx->tc_poly.as<TcPoly>());
+    count_launch();
+    CG_CUDA_TRY(cudaGetLastError());
+    CG_CUDA_TRY(cudaStreamSynchronize(st));  // other streams' calls may read the table next
+    ctx->tc_poly_lmax = ctx->poly_lmax;
+    ctx->tc_poly_nint = ctx->poly_nint;
+    return CATANA_OK;
+}
+
 }  // namespace
 
 // nmax: the table position k r / dx has at most 27 integer bits; rmax: k / dx stays inside FP64
@@ -913,8 +1032,8 @@ bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
 }
 
 catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, int64_t npoints,
-                                    int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev, double *f_acc_dev,
-                                    int *err_dev, cudaStream_t st) {
+                                    int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
+                                    double *f_acc_dev, int *err_dev, cudaStream_t st) {
     const bool lerp = jl == JL_MODE_LERP;
     catana_status_t s = ensure_tc_coefs(ctx, lmax, st);
     if (s != CATANA_OK) return s;
@@ -928,8 +1047,13 @@ catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev
         ctx->attr_tc = true;
     }
     const int lmp = (lmax + 3) & ~3;
-    // 2^er > 4 rmax: radii at or past 4 rmax lie outside the table of l = 0 whatever nmax
-    const int er = ilogb(rmax) + 3;
+    if (jl == JL_MODE_POLY) {
+        s = ensure_tc_poly(ctx, st);
+        if (s != CATANA_OK) return s;
+    }
+    // 2^er > 4 rmax: radii at or past 4 rmax lie outside the table of l = 0 whatever nmax; rtop, the largest
+    // radius, where the caller knows it
+    const int er = std::max(ilogb(rmax) + 3, rtop > 0.0 ? ilogb(rtop) + 1 : -1000);
     const double rlim = lerp ? ldexp(1.0, er) : INFINITY;
     // points per pass: rows and phases (32 B per point and m) stay under 12 GB
     int64_t chunk = std::max<int64_t>(TC_KT, (int64_t)(12e9 / (32.0 * lmp)) / TC_KT * TC_KT);
@@ -1013,13 +1137,23 @@ catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev
             if (!lerp) {
                 const int64_t cnt = (int64_t)(l1 - l0) * tiles * nmax * TC_KT;
                 CG_CUDA_TRY(ctx->tc_jarr.ensure((size_t)cnt * 8));
-                double *ja = ctx->tc_jarr.as<double>();
-                const double *r = reinterpret_cast<const double *>(ws + o_rabs);
+                uint64_t *ja = ctx->tc_jarr.as<uint64_t>();
+                TcJ j;
+                j.r = reinterpret_cast<const double *>(ws + o_rabs);
+                j.kln = kln_dev;
+                j.rint = a.rint;
+                j.ntab = ntab;
+                j.l0 = l0;
+                j.nl = l1 - l0;
+                j.nmax = nmax;
+                j.tiles = tiles;
+                j.tslab = tslab;
+                j.er = er;
+                j.out = ja;
                 if (jl == JL_MODE_POLY)
-                    k_ptc_jl_poly<<<ceil_div(cnt, 256), 256, 0, st>>>(r, kln_dev, l0, l1 - l0, nmax, tiles,
-                                                                      ctx->poly.as<double>(), ctx->poly_nint, ja, err_dev);
+                    k_ptc_jl_poly<<<ceil_div(cnt, 256), 256, 0, st>>>(j, ctx->tc_poly.as<TcPoly>(), ctx->tc_poly_nint, err_dev);
                 else
-                    k_ptc_jl_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(r, kln_dev, l0, l1 - l0, nmax, tiles, ja);
+                    k_ptc_jl_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(j);
                 count_launch();
                 CG_CUDA_TRY(cudaGetLastError());
                 a.jarr = ja;

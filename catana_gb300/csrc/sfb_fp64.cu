@@ -483,6 +483,7 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
         if (s != CATANA_OK) return s;
     }
     if (npoints == 0 || lmax == 0 || nmax == 0) return CATANA_OK;
+    double rtop = 0.0;
     if (jl == JL_MODE_POLY) {
         // the table must reach max_l k_{l,nmax-1} * max r: one read-back of max r
         CG_CUDA_TRY(ctx->cat_scratch.ensure(16));
@@ -512,10 +513,11 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
         }
         s = ensure_poly_tables(ctx, lmax, (int)std::floor(zmax + 0.5) + 2, st);
         if (s != CATANA_OK) return s;
+        rtop = max_r;
     }
     if (plain_tc_takes(ctx, lmax, nmax, rmax))
-        return plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, kln_dev, f_acc_dev,
-                                   err_dev, st);
+        return plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, rtop, kln_dev,
+                                   f_acc_dev, err_dev, st);
     // Chunk so that the three Legendre rows stay under ~1.5 GB.
     int64_t chunk = (int64_t)(1.5e9 / (3.0 * 8.0 * std::max(lmax, 1)));
     chunk = std::max<int64_t>(1024, std::min<int64_t>(chunk, npoints));
