@@ -909,7 +909,7 @@ catana_status_t catana_gpu_sfb_healpix(int64_t nside, const int64_t *pix_offsets
         if (i == 0 || r < r_lo) r_lo = r;
         if (i == 0 || r > r_hi) r_hi = r;
     }
-    s = healpix_sfb_dev(ctx, nside, off_d, rs_d, npoints, lmax, nmax, resolve_interp(flags, npoints),
+    s = healpix_sfb_dev(ctx, nside, off_d, rs_d, npoints, lmax, nmax, rmax, resolve_interp(flags, npoints),
                         (flags & CATANA_HEALPIX_CONJ_FIX) != 0, kln_d, kh.data(), r_lo, r_hi, nf, f_d, cln_d, err_d,
                         st);
     if (s != CATANA_OK) return s;

@@ -80,7 +80,7 @@ struct DeviceContext {
     double split_last_waves = 0.0;
     int split_last_mblk = 0;
     cudaStream_t capture_stream = nullptr;      // stream the split level loop is captured on
-    cudaEvent_t split_ws_event = nullptr;       // end of the last split run (orders workspace reuse across streams)
+    cudaEvent_t split_ws_event = nullptr;       // end of the last split or plain run (orders workspace reuse across streams)
     DevBuf hp_ws;      // HEALPix workspace
     DevBuf ingest_ws;  // ingest: converted records, keep flags, block counts, window, mask
     // kernels whose shared-memory limit this device's context has raised (the
@@ -145,6 +145,23 @@ catana_status_t ensure_lerp_tables(DeviceContext *ctx, int lmax, int nmax, cudaS
 // Legendre coefficients for l < lmax, cached in ctx->coef.
 catana_status_t ensure_coefs(DeviceContext *ctx, int lmax, cudaStream_t st);
 
+// A catalog in RING pixels, with its ring tables (device pointers).
+struct PixelCatalog {
+    const double *r;            // radii grouped by pixel
+    const int64_t *offs;        // [npix + 1]
+    int64_t npix;
+    int nrings;
+    bool conj;                  // CATANA_HEALPIX_CONJ_FIX
+    const int64_t *ring_start;
+    const int *ring_pix;
+    const double *ring_x, *ring_phi;
+    const double2 *tw;          // e^{-2 pi i k / N} per ring length, at tw_off[ring]
+    const int64_t *tw_off;
+};
+// The pixelized sum (un-normalised, times k_ln) as a sum over points at their pixels' centres.
+catana_status_t plain_tc_pixels(DeviceContext *ctx, const PixelCatalog &pix, int64_t npoints, int lmax, int nmax, double rmax,
+                                JlMode jl, const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st);
+
 // One catalog of a split-form run (device pointers; f_acc zeroed by the caller).
 struct SplitCatInput {
     const double *pts = nullptr;  // n x 3 (r, theta, phi)
@@ -193,8 +210,8 @@ catana_status_t healpix_pix2ang_dev(int64_t nside, const int64_t *pix, int64_t n
 // kln_host (L x M, may be null) and the radii's range [r_min, r_max] (r_min NaN when a
 // radius is NaN) let levels that lie inside the j_l table skip the per-point range test
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
-                                const double *r_sorted_dev, int64_t npoints, int lmax, int nmax, bool interpolated,
-                                bool conj_fix, const double *kln_dev, const double *kln_host, double r_min,
+                                const double *r_sorted_dev, int64_t npoints, int lmax, int nmax, double rmax,
+                                bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host, double r_min,
                                 double r_max, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st);
 

@@ -8,6 +8,8 @@
 // gathered in point order within each pixel, as the reference's push_back does.
 //
 // SFB (sfb_reverse_fft.cpp:43-209), per multipole l:
+// Catalogs of up to some tens of points per pixel (and lmax <= 512) are summed point by point with the phase
+// of the pixel's centre (plain_tc.cu).  The others, level by level:
 //   k_hp_map    map[pix][n] = sum_{p in pix} j_l(k_ln r_p), points in order
 //   k_hp_ylm    Y_lm(ring) = P_lm(cos theta_ring) e^{-i m phi_0(ring)} (phi_0: the ring's
 //               first pixel centre, as the reference's RingInfo)
@@ -616,8 +618,8 @@ catana_status_t healpix_bin_dev(DeviceContext *ctx, int64_t nside, const double 
 }
 
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
-                                const double *r_sorted_dev, int64_t npoints, int lmax, int nmax, bool interpolated,
-                                bool conj_fix, const double *kln_dev, const double *kln_host, double r_min,
+                                const double *r_sorted_dev, int64_t npoints, int lmax, int nmax, double rmax,
+                                bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host, double r_min,
                                 double r_max, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st) {
     if (lmax == 0 || nmax == 0) return CATANA_OK;
@@ -625,13 +627,7 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
         set_error("HEALPix path supports nside <= 1024");
         return CATANA_ERR_ARG;
     }
-    catana_status_t s = ensure_coefs(ctx, lmax + 1, st);
-    if (s != CATANA_OK) return s;
-    if (interpolated) {
-        s = ensure_lerp_tables(ctx, lmax, nmax, st);
-        if (s != CATANA_OK) return s;
-    }
-    s = ensure_rings(nside, st);
+    catana_status_t s = ensure_rings(nside, st);
     if (s != CATANA_OK) return s;
     RingTables &R = g_rings;
     const int64_t npix = 12 * nside * nside;
@@ -644,6 +640,37 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     const int64_t *tw_off = reinterpret_cast<const int64_t *>(rb + R.off_twoff);
     const double2 *tw = reinterpret_cast<const double2 *>(rb + R.off_tw);
     const int *order = reinterpret_cast<const int *>(rb + R.off_order);
+    // As a sum over points on the tensor cores (plain_tc.cu) unless the pixels hold many points each, whose
+    // j_l the map below sums first: a point and level costs 0.35..1.3 ns there; here nmax x 0.015 ns plus the
+    // pixels' share (0.04 ns per pixel and radial order).  Measured, ms here / there: nside 64, 400k points,
+    // l 64: n 8 11.7 / 12.2, n 24 18.6 / 14.4; 1.6M points: n 8 22.6 / 47.6, n 24 45.9 / 55.4, n 40 70.0 / 71.5;
+    // nside 256, 1M points, l 128, n 64: 400 / 165.
+    if (plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (nmax < 16 ? 8 : 24) * npix) {
+        if (npoints > 0) {
+            PixelCatalog px;
+            px.r = r_sorted_dev;
+            px.offs = offsets_dev;
+            px.npix = npix;
+            px.nrings = nrings;
+            px.conj = conj_fix;
+            px.ring_start = ring_start;
+            px.ring_pix = ring_pix;
+            px.ring_x = ring_x;
+            px.ring_phi = ring_phi;
+            px.tw = tw;
+            px.tw_off = tw_off;
+            s = plain_tc_pixels(ctx, px, npoints, lmax, nmax, rmax, interpolated ? JL_MODE_LERP : JL_MODE_EXACT, kln_dev,
+                                f_dev, err_dev, st);
+            if (s != CATANA_OK) return s;
+        }
+        return finish_flmn_cln(f_dev, norm, lmax, nmax, c_ln_dev, st);
+    }
+    s = ensure_coefs(ctx, lmax + 1, st);
+    if (s != CATANA_OK) return s;
+    if (interpolated) {
+        s = ensure_lerp_tables(ctx, lmax, nmax, st);
+        if (s != CATANA_OK) return s;
+    }
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t mapb = al((size_t)npix * nmax * sizeof(double));
     const size_t ylmb = al((size_t)nrings * lmax * sizeof(double2));

@@ -14,7 +14,7 @@
 // FP32 sum is exact.  After 128 points the eight D_d are added, as integers with weights
 // 256^(7 - d), to one 64-bit register per (m, ri, n), which holds the slab's whole sum.
 // What is rounded: the operands (Y to 2^-55 of its row's bound, J to 2^-63), the products of digits
-// a + b > 7 (2^-64), and each group's sum (2^-54 to 2^-51 of the slab's largest term).  (With seven digits of J,
+// a + b > 7 (2^-64), and each group's sum (2^-54 of the slab's largest term).  (With seven digits of J,
 // 28 products, the sums erred by 30% more, at the same speed.)  The rows' bounds are kept close to
 // the values: points are sorted by radius, a CTA owns a contiguous slab of at most 2048 of them, EJ
 // bounds |j_l| over the slab's radii (Debye's and Watson's inequalities), EP bounds
@@ -66,7 +66,7 @@ constexpr int TC_OPW = 11;       // operand warps
 constexpr int TC_OPT = 32 * TC_OPW;
 constexpr int TC_FOLD0 = 12;     // first fold warp (warp 11 issues the MMAs)
 constexpr int TC_THREADS = 640;  // 12 + 8 warps
-constexpr int TC_SLAB_TILES = 64;  // most tiles per slab
+constexpr int TC_SLAB_TILES = 64;  // most tiles per slab (an exact sum's count has room for 240)
 constexpr int TC_LMAX = 512;     // |Q_lm| and A_lm stay inside FP64 up to here
 constexpr uint64_t TC_WAIT_NS = 1000000000ull;
 constexpr uint64_t TC_OFF_Y = 0x0080808080808080ull;  // 128 in every digit
@@ -522,9 +522,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
         bool dead = false;
         const int qd = warp & 3, row = qd * 32 + lane;
         const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-        // slab sums are kept in units of 2^(48 + sh): |sum| <= points * 2^118 <= 2^(62 + 48 + sh)
-        const int npt = 32 * (t1 - t0), sh = npt <= 256 ? 16 : npt <= 512 ? 17 : npt <= 1024 ? 18 : 19;
-        const int rnd = (1 << (sh - 16)) >> 1;
+        // Slab sums are kept in units of 2^64, 2^-54 of the largest term: a group adds at most 2^61, and what
+        // passes 2^60 goes to a count per sum (signed bytes, four to a word; at most two a group).
         const int ew = a.slab[slab].ew;
         const int set = warp >= TC_FOLD0 + 4 ? 1 : 0;
         tc_blocks(a, [&](const TcBlock &b, int seq) {
@@ -535,6 +534,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
             int64_t acc[TC_NH];
 #pragma unroll
             for (int c = 0; c < TC_NH; ++c) acc[c] = 0;
+            int top[TC_NH / 4];
+#pragma unroll
+            for (int c = 0; c < TC_NH / 4; ++c) top[c] = 0;
             for (int g = t0; g < t1; g += TC_GROUP) {
                 const uint32_t reg = alt ? groups & 1u : (uint32_t)set, rn = alt ? groups >> 1 : groups;
                 wait(&gdone[reg], rn & 1, dead);
@@ -560,7 +562,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                                 v += (int64_t)iv[3] * 65536;
                                 v += (int64_t)iv[2] * 16777216;
                                 v += (int64_t)(iv[0] * 256 + iv[1]) << 32;
-                                acc[c2 + k] += (v + rnd) >> (sh - 16);
+                                v += acc[c2 + k];
+                                const int hi = ((int)(v >> 32) + (1 << 27)) >> 28;  // multiples of 2^60, to nearest
+                                acc[c2 + k] = v - ((int64_t)hi << 60);
+                                top[(c2 + k) >> 2] += hi << (8 * ((c2 + k) & 3));
                             }
                         }
                     }
@@ -568,7 +573,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                 tc05::fence_before();
                 tc_arrive(&dfree[reg]);
             }
-            // the slab's sums: value = acc 2^(sh - 70 + EJ + EP + EW) A_lm
+            // the slab's sums: value = (acc + top 2^60) 2^(-54 + EJ + EP + EW) A_lm
             if (live && row < 2 * b.mcount) {
                 const int ring = seq & (int)(TC_RING - 1);
                 const uint4 *tn = s_n + ring * TC_NB + nb;
@@ -582,10 +587,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
 #pragma unroll
                 for (int c4 = 0; c4 < TC_NH; c4 += 4)
                     if (c4 < ncol) {
-                        double v[4];  // 2^(EJ + sh - 70) is a normal number: EJ >= -900
+                        double v[4];
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            v[c] = (double)acc[c4 + c] * __hiloint2double((int)(tn[c4 + c].w + ((uint32_t)(sh - 69) << 20)), 0);
+                        for (int c = 0; c < 4; ++c) v[c] = (double)acc[c4 + c];
+                        if (__any_sync(__activemask(), top[c4 >> 2] != 0)) {
+                            int x = top[c4 >> 2];
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) {
+                                const int y = (int)(int8_t)x;
+                                v[c] = fma((double)y, 0x1p60, v[c]);
+                                x = (x - y) >> 8;
+                            }
+                        }
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)  // 2^(EJ - 54) is a normal number: EJ >= -900
+                            v[c] *= __hiloint2double((int)(tn[c4 + c].w - (53u << 20)), 0);
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
                             if (nb + c4 + c < b.ncount) out[(size_t)(c4 + c) * w2] = v[c] * am;
@@ -684,6 +700,20 @@ __global__ void __launch_bounds__(256) k_ptc_slabs(const double *__restrict__ pt
     }
 }
 
+// A catalog in RING pixels (k_ptc_pixels)
+struct TcPixels {
+    const double *r;            // radii grouped by pixel
+    const int64_t *offs;        // [npix + 1]
+    int64_t npix;
+    int nrings, lmax, conj;
+    const int64_t *ring_start;  // first pixel
+    const int *ring_pix;        // pixels
+    const double *ring_x;       // cos theta
+    const double2 *ring_ph;     // [m][ring]: e^{-i m phi_0}
+    const double2 *tw;          // e^{-2 pi i k / N} per ring length, at tw_off[ring]
+    const int64_t *tw_off;
+};
+
 constexpr int TC_POISON_THETA = 1, TC_POISON_PHI = 2, TC_POISON_W = 4;
 
 // v = w cos or -w sin of m phi, times 2^(58 - ew), in signed halves
@@ -747,6 +777,70 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
         ei = ni;
         if (m0 + k < lmp) o[k * TC_KT] = make_ulonglong2(phase_word(er_, scale), phase_word(ei, scale));
     }
+}
+
+// The same for a catalog in RING pixels: a point stands at its pixel's centre, (ring's cos theta, phase
+// e^{-i m phi_0} e^{-2 pi i j s / N}) with phi_0 the ring's first centre, j the pixel's place among the ring's N
+// and s the frequency that the m-extraction reads (sfb_reverse_fft.cpp:192-207): m mod N up to N / 2, then
+// N - m mod N, conjugated only where `conj` says so.  Both factors come from tables (ring_ph, tw).
+__global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t *__restrict__ perm, int64_t n, int64_t q0, int tiles,
+                                                    int tslab, int lmp, const TcSlab *__restrict__ slab, int er, int lerp, double rlim,
+                                                    uint64_t *__restrict__ rint, double *__restrict__ rabs, double2 *__restrict__ xs,
+                                                    ulonglong2 *__restrict__ phase, int *__restrict__ poison, int *__restrict__ err) {
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= tiles) return;
+    const int64_t i = (int64_t)t * TC_KT + lane;
+    const bool in = i < n;
+    const int64_t q = q0 + (in ? perm[i] : perm[n - 1]);
+    const double r = px.r[q];
+    // last pixel with offs[p] <= q, then its ring
+    int64_t lo = 0, hi = px.npix;
+    while (hi - lo > 1) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (px.offs[mid] <= q) lo = mid;
+        else hi = mid;
+    }
+    int ra = 0, rb = px.nrings;
+    while (rb - ra > 1) {
+        const int mid = (ra + rb) >> 1;
+        if (px.ring_start[mid] <= lo) ra = mid;
+        else rb = mid;
+    }
+    const bool rbad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
+    const bool use = in && !rbad;
+    if (blockIdx.y == 0) {
+        if (in && rbad && !lerp) atomicOr(poison, TC_POISON_W);
+        if (in && rbad && lerp) *err = CATANA_ERR_DOMAIN;
+        rint[i] = rbad || !(fabs(r) < ldexp(1.0, er)) ? 0ull : (uint64_t)(int64_t)ldexp(fmax(r, 0.0), 62 - er);
+        rabs[i] = r;
+        const double x = px.ring_x[ra];
+        xs[i] = use ? make_double2(x, sqrt((1.0 - x) * (1.0 + x))) : make_double2(0.0, 0.0);
+    }
+    const double scale = use ? ldexp(1.0, 58 - slab[t / tslab].ew) : 0.0;
+    const int N = px.ring_pix[ra], j = (int)(lo - px.ring_start[ra]);
+    const double2 *tw = px.tw + px.tw_off[ra];
+    const int m0 = blockIdx.y * 8;
+    ulonglong2 *o = phase + ((size_t)t * lmp + m0) * TC_KT + lane;
+    for (int k = 0; k < 8 && m0 + k < lmp; ++k) {
+        const int m = m0 + k, mm = m % N, s = 2 * mm > N ? N - mm : mm;
+        double2 a = make_double2(0.0, 0.0), f = a;
+        if (m < px.lmax) {
+            a = px.ring_ph[(size_t)m * px.nrings + ra];
+            f = tw[(int)((int64_t)j * s % N)];
+            if (px.conj && 2 * mm > N) f.y = -f.y;
+        }
+        o[k * TC_KT] = make_ulonglong2(phase_word(a.x * f.x - a.y * f.y, scale), phase_word(a.x * f.y + a.y * f.x, scale));
+    }
+}
+
+// e^{-i m phi_0} per (m, ring)
+__global__ void k_ptc_ring_phases(const double *__restrict__ ring_phi, int nrings, int lmax, double2 *__restrict__ o) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nrings * lmax) return;
+    const int m = t / nrings;
+    double sn, cs;
+    sincos((double)m * ring_phi[t - m * nrings], &sn, &cs);
+    o[t] = make_double2(cs, -sn);
 }
 
 // (y0 - dy, dy) per node of the linear tables; the last node is empty
@@ -1031,9 +1125,12 @@ bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
            rmax < 1e100;
 }
 
-catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, int64_t npoints,
-                                    int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
-                                    double *f_acc_dev, int *err_dev, cudaStream_t st) {
+namespace {
+
+// pix == nullptr: points_dev are npoints x 3; otherwise the pixelized catalog
+catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, const PixelCatalog *pix,
+                              int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
+                              double *f_acc_dev, int *err_dev, cudaStream_t st) {
     const bool lerp = jl == JL_MODE_LERP;
     catana_status_t s = ensure_tc_coefs(ctx, lmax, st);
     if (s != CATANA_OK) return s;
@@ -1069,9 +1166,13 @@ catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev
         const int waves = ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES);
         return ceil_div(tiles, (int64_t)ctx->sm_count * waves);
     };
+    const size_t phb = pix ? tc_al((size_t)pix->nrings * lmax * sizeof(double2)) : 0;
     const int max_slabs = ctx->sm_count * ceil_div(tiles_c, (int64_t)ctx->sm_count * TC_SLAB_TILES);
     const size_t o_mx = o_sl + tc_al((size_t)max_slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)max_slabs * 3 * TC_LMAX * 4);
-    CG_CUDA_TRY(ctx->tc_ws.ensure(o_poi + 256));
+    CG_CUDA_TRY(ctx->tc_ws.ensure(o_poi + 256 + phb));
+    // the workspace is shared by every stream that runs the plain or the split form on this device
+    if (!ctx->split_ws_event) CG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->split_ws_event, cudaEventDisableTiming));
+    else CG_CUDA_TRY(cudaStreamWaitEvent(st, ctx->split_ws_event, 0));
     char *ws = ctx->tc_ws.as<char>();
     uint32_t *keys = reinterpret_cast<uint32_t *>(ws), *perm = reinterpret_cast<uint32_t *>(ws + kb);
     uint32_t *tk = reinterpret_cast<uint32_t *>(ws + 2 * kb), *tv = reinterpret_cast<uint32_t *>(ws + 3 * kb);
@@ -1079,20 +1180,46 @@ catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev
     int *poison = reinterpret_cast<int *>(ws + o_poi);
     TcSlab *slabs = reinterpret_cast<TcSlab *>(ws + o_sl);
     CG_CUDA_TRY(cudaMemsetAsync(poison, 0, sizeof(int), st));
+    TcPixels px = {};
+    if (pix) {
+        double2 *ph = reinterpret_cast<double2 *>(ws + o_poi + 256);
+        k_ptc_ring_phases<<<ceil_div((int64_t)pix->nrings * lmax, 128), 128, 0, st>>>(pix->ring_phi, pix->nrings, lmax, ph);
+        count_launch();
+        px.r = pix->r;
+        px.offs = pix->offs;
+        px.npix = pix->npix;
+        px.nrings = pix->nrings;
+        px.lmax = lmax;
+        px.conj = pix->conj ? 1 : 0;
+        px.ring_start = pix->ring_start;
+        px.ring_pix = pix->ring_pix;
+        px.ring_x = pix->ring_x;
+        px.ring_ph = ph;
+        px.tw = pix->tw;
+        px.tw_off = pix->tw_off;
+    }
     for (int64_t c0 = 0; c0 < npoints; c0 += chunk) {
         const int64_t nc = std::min(chunk, npoints - c0);
         const int tiles = ceil_div(nc, TC_KT);
         const int tslab = slab_tiles(tiles), nslabs = ceil_div(tiles, tslab);
-        const double *pts = points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
-        k_ptc_keys<<<ceil_div(nc, 256), 256, 0, st>>>(pts, 3, nc, 1.0 / rmax, keys, perm);
+        const double *pts = pix ? pix->r + c0 : points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
+        const int pitch = pix ? 1 : 3;
+        k_ptc_keys<<<ceil_div(nc, 256), 256, 0, st>>>(pts, pitch, nc, 1.0 / rmax, keys, perm);
         count_launch();
         s = radix_sort_pairs(keys, perm, tk, tv, nc, 16, hist, st);
         if (s != CATANA_OK) return s;
-        k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, 3, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
-        k_ptc_points<<<dim3(ceil_div(tiles, 8), ceil_div(lmp, 8)), 256, 0, st>>>(
-            pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, reinterpret_cast<uint64_t *>(ws + o_rint),
-            reinterpret_cast<double *>(ws + o_rabs), reinterpret_cast<double2 *>(ws + o_xs),
-            reinterpret_cast<ulonglong2 *>(ws + o_ph), poison, err_dev);
+        k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, pitch, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
+        const dim3 pg(ceil_div(tiles, 8), ceil_div(lmp, 8));
+        uint64_t *rint_d = reinterpret_cast<uint64_t *>(ws + o_rint);
+        double *rabs_d = reinterpret_cast<double *>(ws + o_rabs);
+        double2 *xs_d = reinterpret_cast<double2 *>(ws + o_xs);
+        ulonglong2 *ph_d = reinterpret_cast<ulonglong2 *>(ws + o_ph);
+        if (pix)
+            k_ptc_pixels<<<pg, 256, 0, st>>>(px, perm, nc, c0, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,
+                                             xs_d, ph_d, poison, err_dev);
+        else
+            k_ptc_points<<<pg, 256, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,
+                                             xs_d, ph_d, poison, err_dev);
         count_launch(2);
         CG_CUDA_TRY(cudaGetLastError());
         TcArgs a;
@@ -1169,7 +1296,22 @@ catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev
             l0 = l1;
         }
     }
+    CG_CUDA_TRY(cudaEventRecord(ctx->split_ws_event, st));
     return CATANA_OK;
+}
+
+}  // namespace
+
+catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, int64_t npoints,
+                                    int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
+                                    double *f_acc_dev, int *err_dev, cudaStream_t st) {
+    return tc_accumulate(ctx, points_dev, weights_dev, nullptr, npoints, lmax, nmax, rmax, jl, rtop, kln_dev, f_acc_dev,
+                         err_dev, st);
+}
+
+catana_status_t plain_tc_pixels(DeviceContext *ctx, const PixelCatalog &pix, int64_t npoints, int lmax, int nmax, double rmax,
+                                JlMode jl, const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st) {
+    return tc_accumulate(ctx, nullptr, nullptr, &pix, npoints, lmax, nmax, rmax, jl, 0.0, kln_dev, f_acc_dev, err_dev, st);
 }
 
 }  // namespace catana_gpu

@@ -80,3 +80,20 @@ def test_points_that_are_not_finite(cuda_device, column, bad):
         for m in range(l + 1):
             nan = (column == 1 and l > 0) or (column == 2 and m > 0) or column == 3
             assert np.all(np.isnan(f[m])) == nan and np.all(np.isfinite(f[m])) == (not nan), (l, m)
+
+
+@pytest.mark.parametrize("nside,n,lmax,nmax", [(1, 40, 12, 3), (2, 300, 20, 16), (8, 1500, 40, 33), (16, 30000, 8, 8), (4, 5000, 6, 5)])
+@pytest.mark.parametrize("dense", [False, True])
+def test_pixelized_points(cuda_device, nside, n, lmax, nmax, dense):
+    """The pixelized sum point by point at pixel centres, polar rings shorter than 2 l included (aliases with
+    and without the conjugate); nside 4 with 26 points per pixel takes the map form instead."""
+    pts = uniform_ball(n, 1000.0, seed=n + nside)
+    ppc = catana.PixelizedPointContainer(nside, catana.PointContainer(pts))
+    if dense:
+        res = catana.sfb_reverse(ppc, lmax, nmax, 1000.0, True, False, interpolated=True)
+        k, c, f = O.sfb_reverse(nside, ppc.offsets, ppc.r_sorted, lmax, nmax, 1000.0, interpolated=True)
+    else:
+        res = catana.sfb_decomposition(ppc, lmax, nmax, 1000.0, True, False, interpolation="on")
+        k, c, f = O.sfb_healpix(nside, ppc.offsets, ppc.r_sorted, lmax, nmax, 1000.0, interpolated=True)
+    for l, (a, b) in enumerate(zip(res.f_lmn, f)):
+        assert np.max(np.abs(a - b)) <= TOL * max(np.max(np.abs(b)), 1e-6 * np.max(np.abs(f[0]))), l
