@@ -3,21 +3,26 @@
 //
 //   I(k1, k2) = int_0^rmax w(r) j_l(k1 r) j_l(k2 r) dr      (sbessel_integrator.cpp:53-110)
 //
-// The reference integrates with GSL's adaptive Gauss-Kronrod (QAG, 21-point rule,
+// The reference integrates pair by pair with GSL's adaptive Gauss-Kronrod (QAG, 21-point rule,
 // epsrel 1e-7) over the sub-intervals between consecutive zeros of j_l(k1 r) and, inside
 // each, of j_l(k2 r) (SBesselIntegrationRangeGenerator, :113-133), stopping once an outer
-// interval adds less than 1e-10 of the total.  Here one warp integrates one (k1, k2) pair
-// over the same breakpoints -- the merged zero sets z_{l,i}/k1 and z_{l,j}/k2 inside
-// (0, rmax) -- plus the nodes of the w table, so that w is linear on every piece (w is a
-// FunctionInterpolator table, FunctionInterpolator.cpp:6-30: linear on equally spaced
-// nodes, domain error outside [x_min, x_max); its kinks would otherwise cost GL its
-// accuracy).  Between consecutive zeros the warp spreads the table segments over its
-// lanes with a Gauss-Legendre rule chosen by the segment length L: 2 points for
-// k2 L <= 0.02, 4 for <= 0.1, 8 for <= 0.25, else 32 (error below 1e-10 of the
-// segment's integral in every case); the whole range is summed.
+// interval adds less than 1e-10 of the total.  Here all pairs of a call share one quadrature:
+// w is a FunctionInterpolator table (FunctionInterpolator.cpp:6-30), linear between its nodes, so
+// the breakpoints are the table's nodes, and a fixed Gauss-Legendre rule per segment integrates the
+// product of the two Bessel functions -- an entire function of exponential type k1 + k2 -- to
+// 2^(2p+1) p!^4 / ((2p+1) (2p)!^3) (kappa / 2)^(2p), kappa = (k1 + k2) length: below 1e-14 for p = 2, 3, 4, 8 points
+// and kappa up to 0.002, 0.046, 0.23, 3.4 (longer segments are cut).  kappa takes the call's largest k, and at
+// least (l + 1) / rmax, the growth of j_l below its turning point.
+//   k_dsb_nodes   abscissae and weights (rule times w) of a chunk of the quadrature
+//   k_dsb_bessel  j_l(k x) for the call's distinct k: K x nodes evaluations instead of two per pair and node
+//                 (a matrix of n x n pairs has n distinct k) -- the FP64 recurrences bound the call
+//   k_dsb_pairs   a CTA per pair: the weighted product of two rows, added in a fixed order
+// Measured, GB300: l 16, 32 x 32 pairs, 10001 nodes, host arrays in and out: 58.2 ms one warp per pair with
+// both j_l evaluated at every node, 0.82 ms so.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -28,82 +33,54 @@ namespace catana_gpu {
 
 namespace {
 
+constexpr int DSB_MAXP = 8;
 
-// GL rules packed in one array: 2 points at [0, 2), 4 at [2, 6), 8 at [6, 14), 32 at [14, 46)
-constexpr int GL_OFF2 = 0, GL_OFF4 = 2, GL_OFF8 = 6, GL_OFF32 = 14, GL_TOT = 46;
+struct DsbRule {
+    double x[DSB_MAXP], w[DSB_MAXP];  // on [-1, 1]
+    int p, cuts;                      // points per piece, pieces per table segment
+    int64_t seg0, nseg;               // table segments [seg0, seg0 + nseg) meet (0, rmax)
+    double wmin, wdx, wdxinv, rmax;
+};
 
-__device__ __forceinline__ double dsb_w(const double *__restrict__ wt, int64_t wn, double wmin, double wdxinv,
-                                        double x) {
-    const double ia = (x - wmin) * wdxinv;  // FunctionInterpolator form; x may round onto wmax at the end
-    unsigned ii = (unsigned)ia;
-    if (ii > (unsigned)(wn - 2)) ii = (unsigned)(wn - 2);
-    return wt[ii] + (wt[ii + 1] - wt[ii]) * (ia - ii);
+// node q = (segment, piece, point)
+__global__ void k_dsb_nodes(DsbRule R, const double *__restrict__ wt, int64_t q0, int64_t nq, double *__restrict__ xo,
+                            double *__restrict__ wo) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= nq) return;
+    const int64_t q = q0 + i, piece = q / R.p, sg = R.seg0 + piece / R.cuts;
+    const int j = (int)(q - piece * R.p), c = (int)(piece % R.cuts);
+    const double sa = fmax(0.0, R.wmin + (double)sg * R.wdx), sb = fmin(R.rmax, R.wmin + (double)(sg + 1) * R.wdx);
+    const double len = (sb - sa) / R.cuts, half = 0.5 * len, x = sa + (double)c * len + half * (R.x[j] + 1.0);
+    const double f = (x - R.wmin) * R.wdxinv - (double)sg;  // place in the table segment
+    xo[i] = x;
+    wo[i] = sb > sa ? R.w[j] * half * (wt[sg] + (wt[sg + 1] - wt[sg]) * f) : 0.0;
 }
 
-__global__ void k_dsb_integrals(const double *__restrict__ zeros, int nz, const double *__restrict__ glx,
-                                const double *__restrict__ glw, const double *__restrict__ wt, int64_t wn,
-                                double wmin, double wmax, double wdx, double wdxinv, int l, double rmax,
-                                const double *__restrict__ k1v, const double *__restrict__ k2v, int64_t np,
-                                double *__restrict__ out, int *__restrict__ err) {
-    const int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (p >= np) return;  // warp-uniform
-    double a = k1v[p], b = k2v[p];
-    if (a > b) {
-        const double t = a;
-        a = b;
-        b = t;
-    }
+__global__ void k_dsb_bessel(const double *__restrict__ k, const double *__restrict__ x, int64_t nq, int l, double *__restrict__ o) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < nq) o[(size_t)blockIdx.y * nq + i] = jl_direct(l, k[blockIdx.y] * x[i]);
+}
+
+constexpr int DSB_T = 128;
+
+// out[p] (+)= sum_q w_q J[i1][q] J[i2][q]; first = 0 adds to the chunks before
+__global__ void __launch_bounds__(DSB_T) k_dsb_pairs(const double *__restrict__ J, const double *__restrict__ w, int64_t nq,
+                                                     const uint32_t *__restrict__ i1, const uint32_t *__restrict__ i2, int first,
+                                                     double *__restrict__ out) {
+    __shared__ double s[DSB_T / 32];
+    const int64_t p = blockIdx.x;
+    // the smaller index first: I(k1, k2) and I(k2, k1) are the same sum
+    const uint32_t a = min(i1[p], i2[p]), b = max(i1[p], i2[p]);
+    const double *ja = J + (size_t)a * nq, *jb = J + (size_t)b * nq;
     double acc = 0.0;
-    int i1 = 0, i2 = 0;
-    double lo = 0.0;
-    const int bad = (wmin > 0.0 || rmax > wmax) ? 1 : 0;
-    while (lo < rmax && !bad) {
-        // the next zero of either factor: the Bessel product keeps its sign up to there
-        const double z1 = (a > 0.0 && i1 < nz) ? zeros[i1] / a : INFINITY;
-        const double z2 = (b > 0.0 && i2 < nz) ? zeros[i2] / b : INFINITY;
-        const double hi = fmin(fmin(z1, z2), rmax);
-        if (hi > lo) {
-            // table nodes strictly inside (lo, hi) split it into segments on which w is linear
-            int64_t ilo = (int64_t)floor((lo - wmin) * wdxinv) + 1;
-            while (ilo > 0 && wmin + (double)(ilo - 1) * wdx > lo) --ilo;
-            while (wmin + (double)ilo * wdx <= lo) ++ilo;
-            int64_t ihi = ilo - 1;
-            {
-                int64_t c = (int64_t)ceil((hi - wmin) * wdxinv) - 1;
-                while (c >= ilo && wmin + (double)c * wdx >= hi) --c;
-                while (wmin + (double)(c + 1) * wdx < hi && c + 1 < wn) ++c;
-                ihi = c;
-            }
-            const int64_t nseg = (ihi >= ilo) ? ihi - ilo + 2 : 1;
-            const double seglen = (nseg > 1) ? wdx : (hi - lo);
-            // rule per segment length (k2 len: <= 0.02 -> 2 points, 0.1 -> 4, 0.25 -> 8, else 32)
-            const double kl = b * seglen;
-            const int npg = kl <= 0.02 ? 2 : (kl <= 0.1 ? 4 : (kl <= 0.25 ? 8 : 32));
-            const int goff = npg == 2 ? GL_OFF2 : (npg == 4 ? GL_OFF4 : (npg == 8 ? GL_OFF8 : GL_OFF32));
-            const int per = 32 / npg;  // segments per warp pass
-            const int j = lane % npg;
-            const double xg = glx[goff + j], wg = glw[goff + j];
-            for (int64_t s0 = 0; s0 < nseg; s0 += per) {
-                const int64_t sgi = s0 + lane / npg;
-                if (sgi < nseg) {
-                    const double sa = (sgi == 0) ? lo : wmin + (double)(ilo + sgi - 1) * wdx;
-                    const double sb = (sgi == nseg - 1) ? hi : wmin + (double)(ilo + sgi) * wdx;
-                    const double half = 0.5 * (sb - sa);
-                    const double x = sa + half * (xg + 1.0);
-                    acc += wg * half * dsb_w(wt, wn, wmin, wdxinv, x) * sbessel_jl(l, a * x) * sbessel_jl(l, b * x);
-                }
-            }
-        }
-        if (z1 <= hi) ++i1;
-        if (z2 <= hi) ++i2;
-        if (hi >= rmax || (!(z1 <= hi) && !(z2 <= hi))) break;
-        lo = hi;
-    }
+#pragma unroll 4
+    for (int64_t q = threadIdx.x; q < nq; q += DSB_T) acc = fma(w[q] * ja[q], jb[q], acc);
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-        out[p] = acc;
-        if (bad) atomicOr(err, 1);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < DSB_T / 32; ++k) acc += s[k];
+        out[p] = first ? acc : out[p] + acc;
     }
 }
 
@@ -155,54 +132,74 @@ catana_status_t catana_gpu_sbessel_integrals(const double *w_table, int64_t w_n,
         }
         kmax = std::max(kmax, std::max(k1[i], k2[i]));
     }
-    // zeros of j_l up to kmax rmax (plus one beyond)
-    int nz = 2;
-    const double *z = zeros_for(l, nz);
-    while (z[nz - 1] <= kmax * r_max) {
-        nz *= 2;
-        z = zeros_for(l, nz);
+    if (w_min > 0.0 || r_max > w_max) {
+        set_error("argument outside range for which this FunctionInterpolator is defined");
+        return CATANA_ERR_DOMAIN;
     }
+    // the distinct k and each pair's two places among them
+    std::vector<double> ks(k1, k1 + npairs);
+    ks.insert(ks.end(), k2, k2 + npairs);
+    std::sort(ks.begin(), ks.end());
+    ks.erase(std::unique(ks.begin(), ks.end()), ks.end());
+    std::vector<uint32_t> idx(2 * (size_t)npairs);
+    for (int64_t i = 0; i < npairs; ++i) {
+        idx[i] = (uint32_t)(std::lower_bound(ks.begin(), ks.end(), k1[i]) - ks.begin());
+        idx[npairs + i] = (uint32_t)(std::lower_bound(ks.begin(), ks.end(), k2[i]) - ks.begin());
+    }
+    const size_t nk = ks.size();
+    // the rule: table segments from that of 0 to that of r_max
+    DsbRule R;
+    R.wmin = w_min;
+    R.wdx = (w_max - w_min) / (double)(w_n - 1);
+    R.wdxinv = 1.0 / R.wdx;
+    R.rmax = r_max;
+    R.seg0 = std::min<int64_t>(w_n - 2, std::max<int64_t>(0, (int64_t)std::floor((0.0 - w_min) * R.wdxinv)));
+    const int64_t sl = std::min<int64_t>(w_n - 2, (int64_t)std::floor((r_max - w_min) * R.wdxinv));
+    R.nseg = std::max<int64_t>(1, sl - R.seg0 + 1);
+    const double kappa = 2.0 * std::max(kmax, (l + 1.0) / r_max) * R.wdx;
+    R.p = kappa <= 0.002 ? 2 : kappa <= 0.046 ? 3 : kappa <= 0.23 ? 4 : 8;
+    const double cuts = std::max(1.0, std::ceil(kappa / 3.4));
+    if (!(cuts < 1e8) || cuts * (double)R.nseg * R.p > 1e11) {
+        set_error("sbessel_integrals: k r_max too large");
+        return CATANA_ERR_ARG;
+    }
+    R.cuts = (int)cuts;
+    gauss_legendre(R.p, R.x, R.w);
+    const int64_t nodes = R.nseg * R.cuts * R.p;
     int cs;
     DeviceContext *ctx = get_context(&cs);
     if (!ctx) return (catana_status_t)cs;
     std::lock_guard<std::mutex> g(ctx->mu);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    std::vector<double> glx(GL_TOT), glw(GL_TOT);
-    gauss_legendre(2, glx.data() + GL_OFF2, glw.data() + GL_OFF2);
-    gauss_legendre(4, glx.data() + GL_OFF4, glw.data() + GL_OFF4);
-    gauss_legendre(8, glx.data() + GL_OFF8, glw.data() + GL_OFF8);
-    gauss_legendre(32, glx.data() + GL_OFF32, glw.data() + GL_OFF32);
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t zb = al((size_t)nz * 8), gb = al(2 * GL_TOT * 8), wb = al((size_t)w_n * 8), kb = al((size_t)npairs * 8);
-    CG_CUDA_TRY(ctx->io_points.ensure(zb + gb + wb + 3 * kb + 256));
+    // nodes per pass: the Bessel rows stay under 512 MB, the distinct k within a grid's second dimension
+    const int64_t chunk = std::max<int64_t>(1024, std::min<int64_t>(nodes, (int64_t)(512e6 / (8.0 * (double)nk))));
+    const size_t wb = al((size_t)w_n * 8), kb = al(nk * 8), ib = al((size_t)npairs * 8), ob = al((size_t)npairs * 8),
+                 cb = al((size_t)chunk * 8), jb = al(nk * (size_t)chunk * 8);
+    CG_CUDA_TRY(ctx->io_points.ensure(wb + kb + ib + ob + 2 * cb + jb + 256));
     char *d = ctx->io_points.as<char>();
-    double *zd = reinterpret_cast<double *>(d), *gd = reinterpret_cast<double *>(d + zb),
-           *wd = reinterpret_cast<double *>(d + zb + gb), *k1d = reinterpret_cast<double *>(d + zb + gb + wb),
-           *k2d = reinterpret_cast<double *>(d + zb + gb + wb + kb),
-           *od = reinterpret_cast<double *>(d + zb + gb + wb + 2 * kb);
-    CG_CUDA_TRY(cudaMemcpyAsync(zd, z, (size_t)nz * 8, cudaMemcpyHostToDevice, st));
-    CG_CUDA_TRY(cudaMemcpyAsync(gd, glx.data(), GL_TOT * 8, cudaMemcpyHostToDevice, st));
-    CG_CUDA_TRY(cudaMemcpyAsync(gd + GL_TOT, glw.data(), GL_TOT * 8, cudaMemcpyHostToDevice, st));
+    double *wd = reinterpret_cast<double *>(d), *kd = reinterpret_cast<double *>(d + wb),
+           *od = reinterpret_cast<double *>(d + wb + kb + ib), *xd = reinterpret_cast<double *>(d + wb + kb + ib + ob),
+           *qd = reinterpret_cast<double *>(d + wb + kb + ib + ob + cb),
+           *jd = reinterpret_cast<double *>(d + wb + kb + ib + ob + 2 * cb);
+    uint32_t *id = reinterpret_cast<uint32_t *>(d + wb + kb);
     CG_CUDA_TRY(cudaMemcpyAsync(wd, w_table, (size_t)w_n * 8, cudaMemcpyHostToDevice, st));
-    CG_CUDA_TRY(cudaMemcpyAsync(k1d, k1, (size_t)npairs * 8, cudaMemcpyHostToDevice, st));
-    CG_CUDA_TRY(cudaMemcpyAsync(k2d, k2, (size_t)npairs * 8, cudaMemcpyHostToDevice, st));
-    CG_CUDA_TRY(ctx->misc.ensure(256));
-    int *err = reinterpret_cast<int *>(ctx->misc.as<char>() + 160);
-    CG_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
-    const double wdx = (w_max - w_min) / (double)(w_n - 1), wdxinv = 1.0 / wdx;
-    const int64_t threads = npairs * 32;
-    k_dsb_integrals<<<ceil_div(threads, 256), 256, 0, st>>>(zd, nz, gd, gd + GL_TOT, wd, w_n, w_min, w_max, wdx,
-                                                            wdxinv, (int)l, r_max, k1d, k2d, npairs, od, err);
-    count_launch();
-    CG_CUDA_TRY(cudaGetLastError());
-    int err_h = 0;
-    CG_CUDA_TRY(cudaMemcpyAsync(out, od, (size_t)npairs * 8, cudaMemcpyDeviceToHost, st));
-    CG_CUDA_TRY(cudaMemcpyAsync(&err_h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CG_CUDA_TRY(cudaStreamSynchronize(st));
-    if (err_h) {
-        set_error("argument outside range for which this FunctionInterpolator is defined");
-        return CATANA_ERR_DOMAIN;
+    CG_CUDA_TRY(cudaMemcpyAsync(kd, ks.data(), nk * 8, cudaMemcpyHostToDevice, st));
+    CG_CUDA_TRY(cudaMemcpyAsync(id, idx.data(), idx.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    for (int64_t q0 = 0; q0 < nodes; q0 += chunk) {
+        const int64_t nq = std::min(chunk, nodes - q0);
+        k_dsb_nodes<<<ceil_div(nq, 256), 256, 0, st>>>(R, wd, q0, nq, xd, qd);
+        for (size_t k0 = 0; k0 < nk; k0 += 65535) {
+            k_dsb_bessel<<<dim3(ceil_div(nq, 256), (unsigned)std::min<size_t>(65535, nk - k0)), 256, 0, st>>>(
+                kd + k0, xd, nq, (int)l, jd + k0 * (size_t)nq);
+            count_launch();
+        }
+        k_dsb_pairs<<<(unsigned)npairs, DSB_T, 0, st>>>(jd, qd, nq, id, id + npairs, q0 == 0 ? 1 : 0, od);
+        count_launch(2);
+        CG_CUDA_TRY(cudaGetLastError());
     }
+    CG_CUDA_TRY(cudaMemcpyAsync(out, od, (size_t)npairs * 8, cudaMemcpyDeviceToHost, st));
+    CG_CUDA_TRY(cudaStreamSynchronize(st));
     return CATANA_OK;
 }
 

@@ -901,47 +901,6 @@ __global__ void __launch_bounds__(256) k_ptc_reduce(const double *__restrict__ p
     }
 }
 
-// j_l(z), z finite: the direct evaluation of sbessel_jl (same branches) with the recurrences' (2 k + 1) / z
-// from one reciprocal, corrected by an FMA to within an ulp of the quotient -- a division costs about
-// twelve FP64 operations at two per SM and cycle, and the recurrences take one per step.
-__device__ __forceinline__ double jl_direct(int l, double z) {
-    if (z == 0.0) return l == 0 ? 1.0 : 0.0;
-    const double sgn = z < 0.0 && (l & 1) ? -1.0 : 1.0, x = fabs(z);
-    if (x * x < 2.0 * l + 3.0) return sgn * jl_series(l, x);
-    const double ix = 1.0 / x;
-    auto quot = [&](double n) {
-        const double q = n * ix;
-        return fma(fma(-q, x, n), ix, q);
-    };
-    double sn, cs;
-    sincos(x, &sn, &cs);
-    const double t0 = quot(sn), t1 = quot(t0 - cs);
-    if (x >= (double)l) {
-        if (l == 0) return sgn * t0;
-        double j0 = t0, j1 = t1;
-        for (int k = 1; k < l; ++k) {
-            const double j2 = fma(quot(2.0 * k + 1.0), j1, -j0);
-            j0 = j1;
-            j1 = j2;
-        }
-        return sgn * j1;
-    }
-    const int nstart = (int)((double)l + 20.0 + 16.0 * cbrt((double)l + 1.0));
-    double jp1 = 0.0, jk = 1e-200, jl = 0.0;
-    for (int k = nstart; k > 0; --k) {
-        const double jm1 = fma(quot(2.0 * k + 1.0), jk, -jp1);
-        jp1 = jk;
-        jk = jm1;
-        if (k - 1 == l) jl = jk;
-        if (fabs(jk) > 1e200) {
-            jk *= 1e-200;
-            jp1 *= 1e-200;
-            jl *= 1e-200;
-        }
-    }
-    return sgn * (fabs(t0) >= fabs(t1) ? jl * (t0 / jk) : jl * (t1 / jp1));
-}
-
 // J of every (l, n, point) of the launch's levels: a warp per (l, tile, n), lane = point
 struct TcJ {
     const double *r, *kln;

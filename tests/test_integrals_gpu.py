@@ -40,3 +40,28 @@ def test_vs_oracle(cuda_device, l, rmax, nodes, nk):
         for j in range(nk):
             ref = O.dsb_integral(fi.y_values, (fi.x_min, fi.x_max), l, rmax, k1[i, j], k2[i, j])
             assert abs(got[i, j] - ref) <= 1e-10 * scale, (i, j, got[i, j], ref)
+
+
+@pytest.mark.parametrize("l,rmax,wmin,wmax,nodes", [(3, 100.0, 0.0, 100.0, 2), (3, 100.0, 0.0, 100.0, 7), (0, 37.3, -5.0, 60.0, 131),
+                                                  (12, 50.0, -1.0, 50.0, 1001), (0, 10.0, 0.0, 12.0, 4001)])
+def test_shared_quadrature_rules(cuda_device, l, rmax, wmin, wmax, nodes):
+    """Every rule of the shared quadrature: segments cut into pieces (few nodes), 8, 4, 3 and 2 points, a table
+    that reaches beyond [0, r_max) on both sides, k = 0 and equal k.  The rule errs below 1e-14, the oracle
+    is adaptive to 1e-13, j_l carries ~1e-14: 1e-12 of the largest integral."""
+    fi = catana.FunctionInterpolator(lambda r: 1.0 + np.cos(0.05 * r) * r, nodes, wmin, wmax)
+    k = np.array([0.0, 1.0, 1.0]) * (30.0 if nodes < 1000 else 3.0 + l) / rmax
+    k1, k2 = np.meshgrid(k, k)
+    got = besseltools.double_sbessel_integrator(fi, l, rmax, k1, k2)
+    ref = np.array([[O.dsb_integral(fi.y_values, (fi.x_min, fi.x_max), l, rmax, a, b) for a, b in zip(p, q)]
+                    for p, q in zip(k1, k2)])
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_many_distinct_k_in_passes(cuda_device):
+    """4000 distinct k: the Bessel rows exceed one pass, the pairs' sums run over several."""
+    rng = np.random.default_rng(2)
+    fi = catana.FunctionInterpolator(lambda r: np.exp(-(r / 30) ** 2), 12001, 0.0, 100.0)
+    k1, k2 = rng.uniform(0.05, 2.0, 2000), rng.uniform(0.05, 2.0, 2000)
+    got = besseltools.double_sbessel_integrator(fi, 5, 100.0, k1, k2)
+    one = np.array([besseltools.double_sbessel_integrator(fi, 5, 100.0, a, b) for a, b in zip(k1[:20], k2[:20])])
+    assert np.max(np.abs(got[:20] - one)) <= 1e-13 * np.max(np.abs(one))
