@@ -1805,8 +1805,10 @@ catana_status_t split_run(DeviceContext *ctx, std::vector<SplitCatInput> &cats_i
                     }
                 std::stable_sort(act.begin(), act.end(),
                                  [&](int x, int y) { return cats[x].ntiles > cats[y].ntiles; });
-                // slab length T: the largest for which the level still has at least
-                // waves x SMs items (small catalogs contribute one short item each)
+                // slab length T: the smallest for which the level's items fit `waves` rounds of
+                // the SMs (one CTA each).  A few items more would run as one more round, as long
+                // as the others and nearly empty: 20k points at lmax 512, nmax 256 gave 154 to 162
+                // items at l < 384 by the opposite rule (at least one round): 111 us a level, now 87.
                 const double slots = std::max(1.0, waves * ctx->sm_count);
                 auto nitems = [&](int64_t T) {
                     double k = 0.0;
@@ -1817,12 +1819,12 @@ catana_status_t split_run(DeviceContext *ctx, std::vector<SplitCatInput> &cats_i
                 };
                 int64_t T = 1;
                 if (nitems(1) > slots) {
-                    int64_t lo = 1, hi = tmax;  // nitems(lo) >= slots
-                    while (lo < hi) {
-                        const int64_t mid = lo + (hi - lo + 1) / 2;
-                        if (nitems(mid) >= slots) lo = mid; else hi = mid - 1;
+                    int64_t lo = 1, hi = tmax;  // nitems(lo) > slots; nitems(hi) the fewest there are
+                    while (hi - lo > 1) {
+                        const int64_t mid = lo + (hi - lo) / 2;
+                        if (nitems(mid) <= slots) hi = mid; else lo = mid;
                     }
-                    T = lo;
+                    T = hi;
                 }
                 for (int c : act) {
                     CatPlan &P = cats[c];
