@@ -386,6 +386,10 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
     __syncthreads();
     tc05::fence_after();
     const uint32_t tmem = tmem_base_sh;
+    // everything above reads only the plan and the tables, fixed before the level loop; from here
+    // on the rows and partials of the previous level's launches are read and written (20k points,
+    // lmax 512, nmax 256: this set-up and the gaps between launches were 8 us of a level's 131)
+    tc05::grid_dep_wait();
     const uint32_t d_tile = tmem, d_acc = tmem + half_cols;
 
     const int64_t t0 = item.t0, t1 = item.t1;
@@ -1172,6 +1176,7 @@ constexpr int RED_G = 4;
 __global__ void __launch_bounds__(32 * RED_G) k_split_reduce(const float *__restrict__ partial, int lp1,
                                                              const SplitRed *__restrict__ reds) {
     __shared__ Sum3 sh[2][RED_G][32];
+    tc05::grid_dep_launch();  // the next level's CTAs may set up meanwhile; they wait before they touch memory
     const SplitRed r = reds[blockIdx.y];
     const int nch = (r.nmax_l + 31) >> 5;  // groups of 32 radial orders
     const int m = blockIdx.x / nch, lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -1182,6 +1187,7 @@ __global__ void __launch_bounds__(32 * RED_G) k_split_reduce(const float *__rest
     const float *p = partial + (size_t)(r.item0 + (blk * r.nhalves + hf) * r.nslabs) * 256 * 128 +
                      (size_t)(2 * ml) * 128 + nl;
     double2 *o = r.fl + (size_t)m * r.kzw + n;
+    tc05::grid_dep_wait();
     double k = 0.0;
     double2 v = make_double2(0.0, 0.0);
     if (live && g == 0) {
@@ -1411,6 +1417,23 @@ struct CatPlan {
     std::vector<int> nmax_l;    // radial orders kept at each l (kmax cut)
     int64_t stride = 0, ntiles = 0;
 };
+
+// <<<grid, threads, smem, st>>>; `dep`: the launch may start before the one ahead of it on the
+// stream has finished, and waits for it inside (grid_dep_wait)
+template <typename... P, typename... A>
+cudaError_t launch_dep(void (*kern)(P...), dim3 grid, int threads, uint32_t smem, cudaStream_t st, bool dep, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = dep ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
 
 size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -2038,18 +2061,22 @@ catana_status_t split_run(DeviceContext *ctx, std::vector<SplitCatInput> &cats_i
         }
         // ---- the level loop (optionally captured as one CUDA graph) ----
         auto levels = [&](bool profile, cudaStream_t ls_st) -> catana_status_t {
+            bool first = true;
             for (int l = 0; l < lmax_g; ++l) {
                 const int ni = S.item0[l + 1] - S.item0[l];
                 const int nr = S.red0[l + 1] - S.red0[l];
                 if (ni == 0) continue;
                 if (profile) prof_begin(ls_st);
-                kern_for(S.fullj[l] != 0)<<<ni, NTOT, smem, ls_st>>>(level_args(S, l));
+                // programmatic launches, after the loop's first: each waits for the one before it
+                // to finish before it reads or writes what a level changes
+                CG_CUDA_TRY(launch_dep(kern_for(S.fullj[l] != 0), dim3(ni), NTOT, smem, ls_st, !first,
+                                       level_args(S, l)));
+                first = false;
                 if (profile) prof_end(ls_st, S.flops[l]);
                 const dim3 rg((l + 1) * ceil_div(S.maxn[l], 32), nr);
-                k_split_reduce<<<rg, 32 * RED_G, 0, ls_st>>>(
-                    partial, l + 1, reinterpret_cast<const SplitRed *>(pd + o_reds) + S.red0[l]);
+                CG_CUDA_TRY(launch_dep(k_split_reduce, rg, 32 * RED_G, 0, ls_st, true, (const float *)partial, l + 1,
+                                       reinterpret_cast<const SplitRed *>(pd + o_reds) + S.red0[l]));
                 count_launch(2);
-                CG_CUDA_TRY(cudaGetLastError());
             }
             return CATANA_OK;
         };
