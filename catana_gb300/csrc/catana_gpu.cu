@@ -232,19 +232,40 @@ catana_status_t check_args(int64_t npoints, uint16_t lmax, uint16_t nmax, double
     return CATANA_OK;
 }
 
-// Weighted sum on device for the normalisation (sum of weights).
-__global__ void k_wsum(const double *w, int64_t n, double *out) {
-    // single CTA, fixed-order tree: deterministic
+// Weighted sum on device for the normalisation (sum of weights), in a fixed order.  One CTA waits
+// for memory a few loads at a time (1M weights: 294 us), so more than WSUM_CHUNK weights are
+// summed by chunks of one CTA each first, and the chunks' sums by one CTA (9 + 6 us).
+constexpr int WSUM_CHUNK = 8192, WSUM_CTAS = 592;
+__global__ void __launch_bounds__(1024) k_wsum(const double *__restrict__ w, int64_t n, int64_t chunk,
+                                               double *__restrict__ out) {
     __shared__ double sh[1024];
+    const int64_t b = blockIdx.x * chunk, e = min(n, b + chunk);
     double s = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += w[i];
+#pragma unroll 4
+    for (int64_t i = b + threadIdx.x; i < e; i += 1024) s += w[i];
     sh[threadIdx.x] = s;
     __syncthreads();
-    for (int k = blockDim.x / 2; k > 0; k >>= 1) {
+    for (int k = 512; k > 0; k >>= 1) {
         if ((int)threadIdx.x < k) sh[threadIdx.x] += sh[threadIdx.x + k];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = sh[0];
+    if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
+}
+
+// *out = sum of n weights; scratch: WSUM_CTAS doubles
+catana_status_t weight_sum(const double *w, int64_t n, double *out, double *scratch, cudaStream_t st) {
+    if (n <= WSUM_CHUNK) {
+        k_wsum<<<1, 1024, 0, st>>>(w, n, n, out);
+        count_launch();
+    } else {
+        const int64_t chunk = std::max<int64_t>(WSUM_CHUNK, (n + WSUM_CTAS - 1) / WSUM_CTAS);
+        const int ctas = (int)((n + chunk - 1) / chunk);
+        k_wsum<<<ctas, 1024, 0, st>>>(w, n, chunk, scratch);
+        k_wsum<<<1, 1024, 0, st>>>(scratch, ctas, ctas, out);
+        count_launch(2);
+    }
+    CG_CUDA_TRY(cudaGetLastError());
+    return CATANA_OK;
 }
 
 // Core of both raw entry points: device inputs, device outputs.  `wsum_host` < 0
@@ -279,11 +300,10 @@ catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double
     if (s != CATANA_OK) return s;
     double wsum = (double)npoints;
     if (w_d && npoints > 0) {
-        CG_CUDA_TRY(ctx->misc.ensure(256));
-        double *ws = reinterpret_cast<double *>(ctx->misc.as<char>() + 64);
-        k_wsum<<<1, 1024, 0, st>>>(w_d, npoints, ws);
-        count_launch();
-        CG_CUDA_TRY(cudaGetLastError());
+        CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)8 * (1 + WSUM_CTAS)));
+        double *ws = ctx->cat_scratch.as<double>();
+        s = weight_sum(w_d, npoints, ws, ws + 1, st);
+        if (s != CATANA_OK) return s;
         CG_CUDA_TRY(cudaMemcpyAsync(&wsum, ws, sizeof(double), cudaMemcpyDeviceToHost, st));
         CG_CUDA_TRY(cudaStreamSynchronize(st));
     }
@@ -415,14 +435,13 @@ catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats,
         any_w |= (cats[c].weights && cats[c].npoints > 0);
     }
     if (any_w) {
-        CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)8 * ncat));
+        CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)8 * (ncat + WSUM_CTAS)));
         double *ws = ctx->cat_scratch.as<double>();
         for (int c = 0; c < ncat; ++c)
             if (cats[c].weights && cats[c].npoints > 0) {
-                k_wsum<<<1, 1024, 0, st>>>(cats[c].weights, cats[c].npoints, ws + c);
-                count_launch();
+                s = weight_sum(cats[c].weights, cats[c].npoints, ws + c, ws + ncat, st);
+                if (s != CATANA_OK) return s;
             }
-        CG_CUDA_TRY(cudaGetLastError());
         std::vector<double> wh(ncat);
         CG_CUDA_TRY(cudaMemcpyAsync(wh.data(), ws, (size_t)8 * ncat, cudaMemcpyDeviceToHost, st));
         CG_CUDA_TRY(cudaStreamSynchronize(st));

@@ -39,27 +39,72 @@ __global__ void k_radix_hist(const uint32_t *__restrict__ keys, int64_t n, int s
     hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// Single-CTA exclusive scan of count entries (1024 threads, contiguous segments).
-__global__ void k_radix_scan(uint32_t *__restrict__ data, int64_t count) {
-    __shared__ uint32_t part[1024];
-    const int t = threadIdx.x;
-    const int64_t seg = (count + 1023) / 1024;
-    const int64_t b = t * seg, e = min(count, b + seg);
-    uint32_t s = 0;
-    for (int64_t i = b; i < e; ++i) s += data[i];
-    part[t] = s;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {  // inclusive Hillis-Steele scan
-        uint32_t v = t >= off ? part[t - off] : 0u;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    uint32_t run = part[t] - s;  // exclusive prefix of this segment
-    for (int64_t i = b; i < e; ++i) {
-        const uint32_t v = data[i];
-        data[i] = run;
-        run += v;
+// Single-CTA exclusive scan of count entries: 1024 threads take 16384 consecutive words a round,
+// sixteen each as four 16-byte loads, and load the next round's words before they scan this one's,
+// so a round costs one scan and not a trip to memory (62.7k words, the histogram of 1M pairs: 16 us;
+// with a contiguous segment per thread, read word by word twice, 61).
+constexpr int SC_PER = 16;
+__global__ void __launch_bounds__(1024) k_radix_scan(uint32_t *__restrict__ data, int64_t count) {
+    __shared__ uint32_t part[2][32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const bool vec = (reinterpret_cast<uintptr_t>(data) & 15) == 0;
+    auto load = [&](int64_t base, uint32_t (&v)[SC_PER]) {
+        const int64_t i = base + (int64_t)SC_PER * t;
+        if (vec && i + SC_PER <= count) {
+#pragma unroll
+            for (int k = 0; k < SC_PER; k += 4) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(data + i + k);
+                v[k] = q.x;
+                v[k + 1] = q.y;
+                v[k + 2] = q.z;
+                v[k + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < SC_PER; ++k) v[k] = i + k < count ? data[i + k] : 0u;
+        }
+    };
+    uint32_t v[SC_PER], nx[SC_PER];
+    load(0, v);
+    uint32_t carry = 0;
+    int par = 0;
+    for (int64_t base = 0; base < count; base += 1024 * SC_PER, par ^= 1) {
+        load(base + 1024 * SC_PER, nx);  // words the others have not written yet: a later round's
+        uint32_t s = 0;
+#pragma unroll
+        for (int k = 0; k < SC_PER; ++k) {  // exclusive within the thread
+            const uint32_t x = v[k];
+            v[k] = s;
+            s += x;
+        }
+        uint32_t inc = s;  // inclusive over the warp's threads
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (lane == 31) part[par][warp] = inc;
+        __syncthreads();  // two buffers: the next round's writes come after the next barrier's reads
+        uint32_t wsum = part[par][lane];  // every warp scans the 32 warp sums
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, wsum, o);
+            if (lane >= o) wsum += y;
+        }
+        const uint32_t before = warp ? __shfl_sync(0xffffffffu, wsum, warp - 1) : 0u;
+        const uint32_t add = carry + before + inc - s;
+        carry += __shfl_sync(0xffffffffu, wsum, 31);
+        const int64_t i = base + (int64_t)SC_PER * t;
+        if (vec && i + SC_PER <= count) {
+#pragma unroll
+            for (int k = 0; k < SC_PER; k += 4)
+                *reinterpret_cast<uint4 *>(data + i + k) =
+                    make_uint4(v[k] + add, v[k + 1] + add, v[k + 2] + add, v[k + 3] + add);
+        } else {
+#pragma unroll
+            for (int k = 0; k < SC_PER; ++k)
+                if (i + k < count) data[i + k] = v[k] + add;
+        }
+#pragma unroll
+        for (int k = 0; k < SC_PER; ++k) v[k] = nx[k];
     }
 }
 
