@@ -44,10 +44,19 @@
 //   * e^{-i m phi}: one sincospif of the exact phase (64-bit fixed-point fraction of a
 //     turn) per warp-run of <= 8 m, then complex rotation by e^{i phi}.
 // Pipeline: two operand buffers and two row stages.  Warps 0..15 generate the operands
-// of tile t+1 while the tensor core multiplies tile t; warps 16..19 (one per TMEM lane
-// quadrant) fold D_tile into D_acc, flush, and issue each tile's MMAs, so the fold no
-// longer sits between a CTA barrier and the next MMA.  Hand-offs are mbarriers: operands
-// written, MMAs complete, row stage read.  Every wait is bounded (1 s); on timeout the
+// of tile t+1 while the tensor core multiplies tile t, in two column parts; warps 16..19 (one
+// per TMEM lane quadrant) fold each part of D_tile into D_acc while the other part is
+// multiplied, and flush; one thread stages the tiles and one issues the MMAs.  Hand-offs are
+// mbarriers: operands written, MMAs of a part complete, part folded, row stage read.  What
+// bounds it is the operand warps' instructions, ~550 a warp and tile in dependent chains
+// (clock stamps at 1M points, l = 200: 4.3k cycles a tile, of which J 1.1k, Y 1.7k, waits and
+// hand-offs 1.3k).  Staging by an operand warp (its copies and the proxy fence kept that warp
+// 1.3k cycles behind the others, and every tile waited for it), the fold of a whole tile between
+// two MMAs and the MMAs' issue by a fold warp had made it 4.8k.  1M points, lmax 256, nmax 128:
+// 200 -> 178 ms; 2 x 20k points, lmax 512, nmax 256: 114.6 -> 104.9.  Measured and dropped on this
+// layout: 16-column TMEM loads in flight two deep in the fold (+5%), Taylor coefficients of J by
+// two warps of their own (+2.5%: they wait for the stage, then every operand warp for them), waits
+// by one lane of a warp (+4%).  Every wait is bounded (1 s); on timeout the
 // kernel records CATANA_ERR_CUDA in the error word, stops issuing work and frees its
 // tensor memory.
 #include <cuda.h>
@@ -78,9 +87,12 @@ constexpr int QPW = (32 + NOPW - 1) / NOPW;   // most quads of complex m per ope
 constexpr int JPW = (64 + NOPW - 1) / NOPW;   // most J row pairs per operand warp (128 rows)
 static_assert(JPW <= 16, "k_split_l: one lane per J row in the Taylor coefficients");
 constexpr int NFOLDW = 4;           // fold / MMA warps, one per TMEM lane quadrant
-constexpr int NTOT = NTHR + 32 * NFOLDW;
+constexpr int NTOT = NTHR + 32 * NFOLDW + 128;  // and a warpgroup of which one thread stages the tiles, one issues the MMAs
+// registers a thread: at launch, and what the three kinds of warps give up or take for their work
+constexpr int REG_LAUNCH = 80, REG_OP = 88, REG_FOLD = 88, REG_STAGE = 40;
+static_assert(REG_OP >= REG_LAUNCH && REG_FOLD >= REG_LAUNCH && REG_STAGE <= REG_LAUNCH, "setmaxnreg: directions");
+static_assert(REG_OP * NTHR + REG_FOLD * 32 * NFOLDW + REG_STAGE * 128 <= REG_LAUNCH * NTOT, "setmaxnreg: the split");
 constexpr int MBLK = 128;           // complex m per CTA block (256 accumulator columns)
-constexpr int FOLD_TILES = 1;       // tiles accumulated by the tensor core before a fold into D_acc (2 doubles the C_l error)
 constexpr int FLUSH_FOLDS = 128;    // folds into the TMEM sum before it goes to global memory
 constexpr int NINT_MAX = 1664 - (NOPW * JPW - 64);  // table intervals resident in shared memory (lmax 512, nmax 256 at r <= rmax: 1522)
 constexpr double H = 1.0;           // table interval width in z (intervals centred on integers)
@@ -164,10 +176,16 @@ struct SplitCat {
     unsigned long long *rexp;  // extended range: exponent sets [tile][lrows] by the parity of l, set k at
                                // rexp + k * eset (one word per value serves P_l and X_l)
     int64_t eset;           // words per exponent set
-    const char *tmaps;      // TMA descriptors (128 B each): rows of sets 0..3, exponent words of sets 0, 1 at 4, 5
+    const char *tmaps;      // TMAPS TMA descriptors
     const float4 *kz;       // [l][kzw]: (k_ln / H as float-float, J scale 2^s_ln, 1 / (2^s_ln 2^12))
     const int *nmax_l;      // [l]: radial orders computed at l (kmax cut)
 };
+
+// the descriptors of a catalog (128 bytes each): rows of set k in boxes of 32 nb m (nb 1..4) x 32
+// points, and the exponent words of set k
+constexpr int TMAPS = 18;
+__host__ __device__ constexpr int tmap_rows(int k, int nb) { return 4 * k + nb - 1; }
+__host__ __device__ constexpr int tmap_exp(int k) { return 16 + k; }
 
 // One CTA of a level launch: a catalog, a block of complex m, a range of tiles.
 struct SplitItem {
@@ -240,19 +258,6 @@ __device__ __forceinline__ void phase_seed(unsigned long long u, int m, float &c
 __device__ __forceinline__ void ws_arrive(uint64_t *mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc05::smem_u32(mbar)) : "memory");
 }
-// named barrier 1 of the four fold warps (128 threads); fold_vote is the same barrier
-// returning the AND of every fold thread's flag, so the fold warps always agree
-__device__ __forceinline__ void fold_bar() { asm volatile("barrier.sync.aligned 1, 128;" ::: "memory"); }
-__device__ __forceinline__ bool fold_vote(bool v) {
-    int r;
-    asm volatile(
-        "{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbarrier.red.and.aligned.pred q, 1, 128, p;\nselp.s32 %0, 1, 0, q;\n}"
-        : "=r"(r)
-        : "r"((int)v)
-        : "memory");
-    return r != 0;
-}
-
 // A tt - B p2 rounded once (A = ah + al, B = bh + bl as float-float): TwoSum of the two
 // large products, plus their exact remainders.  The usual fma chain rounds a partial sum
 // that the large B p2 dominates, so the small A_lo tt term is absorbed -- and it has a
@@ -309,11 +314,13 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
     constexpr uint32_t STG = sm_stage(EXT, RS);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t mbar[2];  // MMA completion per operand buffer
+    __shared__ uint64_t mbar[2];   // MMA completion per operand buffer
+    __shared__ uint64_t hbar;      // MMA completion of a tile's first column part
+    __shared__ uint64_t dfree[2];  // the column part read by every fold warp (NFOLDW arrivals)
     __shared__ uint64_t sbar[NST];  // TMA completion per stage
     __shared__ uint32_t tmem_base_sh;
-    __shared__ uint64_t fbar[2];   // operands of buffer b written (NTHR arrivals)
-    __shared__ uint64_t gfree[NST];  // stage s read by every operand thread (NTHR arrivals)
+    __shared__ uint64_t fbar[2];   // operands of buffer b written (NOPW arrivals)
+    __shared__ uint64_t gfree[NST];  // stage s read by every operand warp (NOPW arrivals)
     __shared__ int abort_sh;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -366,9 +373,10 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
         tc05::mbar_init(&mbar[0], 1);
         tc05::mbar_init(&mbar[1], 1);
         for (int k = 0; k < NST; ++k) tc05::mbar_init(&sbar[k], 1);
-        tc05::mbar_init(&fbar[0], NTHR);
-        tc05::mbar_init(&fbar[1], NTHR);
-        for (int k = 0; k < NST; ++k) tc05::mbar_init(&gfree[k], NTHR);
+        tc05::mbar_init(&hbar, 1);
+        for (int k = 0; k < 2; ++k) tc05::mbar_init(&fbar[k], NOPW);
+        for (int k = 0; k < 2; ++k) tc05::mbar_init(&dfree[k], NFOLDW);
+        for (int k = 0; k < NST; ++k) tc05::mbar_init(&gfree[k], NOPW);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -399,7 +407,10 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
     const int nquads = (mcount + 3) >> 2;
     const int qb0 = (g * nquads) / NOPW, qb1 = ((g + 1) * nquads) / NOPW;
     const int mlo = 4 * qb0, mhi = min(4 * qb1, mcount);  // local m range of this warp
-    const uint32_t idesc = tc05::idesc_f16_mn(128, ncols_pad);
+    // The accumulator's columns in two parts, each a whole number of the operand layout's 64-column
+    // atoms (one part when there are no more than 64): the fold of one part runs while the
+    // tensor core multiplies the other.
+    const int cols_a = ncols_pad <= 64 ? ncols_pad : ((ncols_pad >> 1) + 32) & ~63, cols_b = ncols_pad - cols_a;
     const int stride = cat.stride;
     const size_t set = (size_t)stride * cat.lrp;
     // the rows this level writes: P_l (and, Reinsch-modified rows, X_l)
@@ -411,74 +422,42 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
     if (EXT) ex0 = cat.rexp + (size_t)(l & 1) * cat.eset;
     float *__restrict__ partial_cta = a.partial + (size_t)blockIdx.x * 256 * 128;
 
-    uint32_t uses0 = 0, uses1 = 0, waited0 = 0, waited1 = 0;  // commits / completed waits per buffer
-    int64_t iss = 0, wtd = 0;  // stage loads issued / waited (tiles of the item, counted from t0)
     bool acc_fresh = true;   // next fold overwrites D_acc
     bool first_flush = true; // partial rows not yet written by this CTA
     int folds = 0;
-    bool ok = true;
 
-    auto wait_buf = [&](int b, uint64_t limit) -> bool {
-        uint32_t &wt = b ? waited1 : waited0;
-        const uint32_t us = b ? uses1 : uses0;
-        while (wt < us) {
-            if (!tc05::mbar_wait(&mbar[b], wt & 1, limit)) return false;
-            ++wt;
-        }
-        return true;
+    // the MMAs of tile t0 + j are the (j / 2)-th completion of its buffer's barrier
+    auto wait_mma = [&](int64_t j, uint64_t limit) -> bool {
+        return tc05::mbar_wait(&mbar[j & 1], (uint32_t)((j >> 1) & 1), limit);
     };
 
-    // stage tile t0 + j into stage j % NST, all by one thread, completing on sbar[j % NST]: the point
+    // tile t0 + j goes into stage j % NST, loaded by the staging warp, completing on sbar[j % NST]: the point
     // records (one bulk copy), the rows P_{l-1}(m) and P_{l-2}(m) of this block's m in
     // 32-row TMA boxes (rows past the tensor's end arrive as zeros; slots the step does
     // not read -- the sectoral m = l of P_{l-1}, m > l-2 of P_{l-2} -- hold stale rows),
     // and (extended range) the exponent words of level l-1
-    // staged rows: P_{l-1} and P_{l-2} (three-term rows) or X_{l-1} (Reinsch-modified rows);
-    // descriptors 0..3 are the row sets, 4 and 5 the exponent sets
-    const char *tm_r1 = cat.tmaps + 128 * (RS ? (l + 1) & 1 : (l + 2) % 3);
-    const char *tm_r2 = cat.tmaps + 128 * (RS ? 2 + ((l + 1) & 1) : (l + 1) % 3);
-    const char *tm_e1 = cat.tmaps + 128 * (4 + ((l + 1) & 1));
+    // staged rows: P_{l-1} and P_{l-2} (three-term rows) or X_{l-1} (Reinsch-modified rows), nb
+    // times 32 m of each in one box (an empty one is not loaded)
     const int nb1 = l > 0 ? (mcount + 31) >> 5 : 0;
     const int nb2 = (max(0, min(mcount, RS ? l - mb0 : l - 1 - mb0)) + 31) >> 5;
+    const char *tm_r1 = cat.tmaps + 128 * tmap_rows(RS ? (l + 1) & 1 : (l + 2) % 3, max(nb1, 1));
+    const char *tm_r2 = cat.tmaps + 128 * tmap_rows(RS ? 2 + ((l + 1) & 1) : (l + 1) % 3, max(nb2, 1));
+    const char *tm_e1 = cat.tmaps + 128 * tmap_exp((l + 1) & 1);
     const uint32_t stage_bytes =
         SM_STPTS + 4096u * (uint32_t)(nb1 + nb2) + ((EXT && l > 0) ? SM_STEXP : 0u);
-    if (tid == 0) {  // descriptors rewritten by the host between launches: read them afresh
-        tc05::tmap_acquire(tm_r1);
-        tc05::tmap_acquire(tm_r2);
-        if (EXT) tc05::tmap_acquire(tm_e1);
-    }
-    auto prefetch = [&](int64_t j) {
-        const int64_t t = t0 + j;
-        if (t >= t1) return;
-        iss = j + 1;
-        if (tid != 0) return;
-        const int sidx = (int)(j % NST);
-        uint8_t *stg = sm + OFF_ST + (uint32_t)sidx * STG;
-        tc05::fence_proxy_async();  // earlier generic reads of this stage before the async writes
-        tc05::mbar_arrive_expect_tx(&sbar[sidx], stage_bytes);
-        tc05::bulk_g2s(stg + 2 * SM_STROW, cat.pts + t * KT, SM_STPTS, &sbar[sidx]);
-        // 32 m (16 interleaved pairs) x 32 points per box: 16 row segments of 256 B
-        for (int k = 0; k < nb1; ++k) tc05::tma_load_2d(stg + k * 4096, tm_r1, (int)(2 * KT * t), (mb0 >> 1) + 16 * k, &sbar[sidx]);
-        for (int k = 0; k < nb2; ++k)
-            tc05::tma_load_2d(stg + SM_STROW + k * 4096, tm_r2, (int)(2 * KT * t), (mb0 >> 1) + 16 * k, &sbar[sidx]);
-        if (EXT && l > 0) tc05::tma_load_2d(stg + 2 * SM_STROW + SM_STPTS, tm_e1, mb0, (int)t, &sbar[sidx]);
-    };
     // the load of tile t0 + j is the (j / NST)-th completion of its stage's barrier
     auto wait_stage = [&](int64_t j, uint64_t limit) -> bool {
-        if (!tc05::mbar_wait(&sbar[j % NST], (uint32_t)((j / NST) & 1), limit)) return false;
-        wtd = j + 1;
-        return true;
+        return tc05::mbar_wait(&sbar[j % NST], (uint32_t)((j / NST) & 1), limit);
     };
 
-    // D_acc (+)= D_tile, by the fold warps: each its lane quadrant (warp % 4), every column group
-    auto fold = [&]() {
+    // D_acc (+)= D_tile in columns [c0, c1), by the fold warps: each its lane quadrant (warp % 4)
+    auto fold = [&](int c0, int c1) {
         tc05::fence_after();
-        const int qd = warp & 3;
-        const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-        for (int gi = 0; gi < (ncols_pad >> 4); ++gi) {
+        const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+        for (int c = c0; c < c1; c += 16) {
             uint32_t vt[16], va[16];
-            tc05::tmem_ld16(d_tile + lane_off + gi * 16, vt);
-            if (!acc_fresh) tc05::tmem_ld16(d_acc + lane_off + gi * 16, va);
+            tc05::tmem_ld16(d_tile + lane_off + c, vt);
+            if (!acc_fresh) tc05::tmem_ld16(d_acc + lane_off + c, va);
             tc05::tmem_wait_ld();
             if (!acc_fresh) {
 #pragma unroll
@@ -489,11 +468,10 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
                     vt[j + 1] = __float_as_uint(sm2.y);
                 }
             }
-            tc05::tmem_st16(d_acc + lane_off + gi * 16, vt);
+            tc05::tmem_st16(d_acc + lane_off + c, vt);
         }
         tc05::tmem_wait_st();
-        acc_fresh = false;
-        ++folds;
+        tc05::fence_before();
     };
 
     // partial[cta] (+)= D_acc / (2^s_ln 2^12) (lane n), then the next fold restarts D_acc
@@ -532,34 +510,26 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
         folds = 0;
     };
 
-    // roles: warps 0..15 write each tile's operands (J, Y) into the two operand buffers;
-    // warps 16..19 (one per TMEM lane quadrant) fold the previous tile's tensor-core sum,
-    // flush, and issue the tile's MMAs.  Hand-offs: fbar[b] operands of buffer b written,
-    // mbar[b] the MMAs reading buffer b complete, gfree[s] stage s read by every operand
-    // thread (it may be refilled).  Every wait is bounded; a failed one raises abort_sh.
+    // Roles: warps 0..15 write each tile's operands (J, Y) into the two operand buffers; warps 16..19
+    // (one per TMEM lane quadrant) fold each tile's tensor-core sum and flush; one thread of warp 20
+    // stages the tiles and one of warp 21 issues the MMAs.  Hand-offs: fbar[b] operands of buffer b
+    // written, hbar / mbar[b] the first part's / all MMAs of a tile complete, dfree[] the column part
+    // folded (it may be overwritten), gfree[s] stage s read (it may be refilled).  Every wait is
+    // bounded; a failed one raises abort_sh, at which the others stop too.
     volatile int *abort_v = &abort_sh;
+    auto fail = [&]() {
+        *abort_v = 1;
+        *a.err = CATANA_ERR_CUDA;
+    };
     if (warp < NTHR / 32) {
-        for (int64_t jp = 0; jp + 1 < NST; ++jp) prefetch(jp);  // NST - 1 tiles ahead
+        tc05::reg_inc<REG_OP>();
         for (int64_t t = t0; t < t1; ++t) {
             const int64_t j = t - t0;
-            if (*abort_v) {
-                ok = false;
-                break;
-            }
             const int b = (int)(j & 1);
-            bool okp = true;
-            if (tid == 0 && j >= 1 && t + NST - 1 < t1) {  // stage (j-1) % NST last held tile j-1
-                okp = tc05::mbar_wait(&gfree[(j - 1) % NST], (uint32_t)(((j - 1) / NST) & 1), a.wait_ns);
-            }
-            if (!okp) {
-                *abort_v = 1;
-                ok = false;
-                break;
-            }
-            prefetch(j + NST - 1);
-            if (!(wait_buf(b, a.wait_ns) && wait_stage(j, a.wait_ns))) {
-                *abort_v = 1;
-                ok = false;
+            // the buffer's last reader (tile j - 2), this tile's stage
+            if (!__all_sync(0xffffffffu, (j < 2 || wait_mma(j - 2, a.wait_ns)) && wait_stage(j, a.wait_ns) &&
+                                             !*abort_v)) {
+                if (lane == 0) fail();
                 break;
             }
             const int sidx = (int)(j % NST);
@@ -1008,79 +978,117 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
                 }
             }
             tc05::fence_proxy_async();
-            ws_arrive(&gfree[sidx]);
-            if (!(a.stall && t == t0)) ws_arrive(&fbar[b]);  // the test hook withholds the first hand-off
-            if (b) ++uses1; else ++uses0;
-        }
-        // stage loads still in flight (a loop that stopped early) land before the CTA exits
-        while (wtd < iss && wait_stage(wtd, WAIT_NS)) {
-        }
-    } else {
-        uint32_t fw0 = 0, fw1 = 0;  // fbar phases waited
-        for (int64_t t = t0; t < t1; ++t) {
-            const int b = (int)((t - t0) & 1);
-            uint32_t &fw = b ? fw1 : fw0;
-            bool okw = tc05::mbar_wait(&fbar[b], fw & 1, a.wait_ns);
-            ++fw;
-            if (okw && t > t0) okw = wait_buf(b ^ 1, a.wait_ns);  // the MMAs of tile t-1 (D_tile) complete
-            if (!fold_vote(okw && !*abort_v)) {        // the fold warps decide together
-                *abort_v = 1;
-                ok = false;
-                break;
+            __syncwarp();
+            if (lane == 0) {
+                ws_arrive(&gfree[sidx]);
+                if (!(a.stall && t == t0)) ws_arrive(&fbar[b]);  // the test hook withholds the first hand-off
             }
-            if (t > t0) {
-                fold();
-                if (folds == FLUSH_FOLDS) flush();
-            }
-            tc05::fence_before();
-            fold_bar();
-            tc05::fence_after();
-            uint8_t *bufp = sm + b * SM_BUF;
-            uint8_t *jhi = bufp, *jlo = bufp + SM_J, *yhi = bufp + 2 * SM_J, *ylo = bufp + 2 * SM_J + SM_Y;
-            const bool fresh_tile = ((t - t0) % FOLD_TILES == 0);  // D_tile was folded (or never used)
-            if (tid == NTHR) {
-                const uint32_t sj_hi = tc05::smem_u32(jhi), sj_lo = tc05::smem_u32(jlo);
-                const uint32_t sy_hi = tc05::smem_u32(yhi), sy_lo = tc05::smem_u32(ylo);
-                // the four small hi x lo / lo x hi products first, the two hi x hi last: the
-                // tensor core rounds each MMA's sum into the FP32 accumulator, and the
-                // small terms then round at their own magnitude (2^-11 of the sum), so
-                // only two roundings per tile fall at the full magnitude instead of five
-                uint64_t ah[2], al[2], bh[2], bl[2];
-    #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) {
-                    ah[ks] = tc05::desc_sw128(sj_hi + ks * 4096, 1024, 2048);
-                    al[ks] = tc05::desc_sw128(sj_lo + ks * 4096, 1024, 2048);
-                    bh[ks] = tc05::desc_sw128(sy_hi + ks * 8192, 1024, 4096);
-                    bl[ks] = tc05::desc_sw128(sy_lo + ks * 8192, 1024, 4096);
+        }
+        __syncwarp();
+        tc05::reg_dec<REG_LAUNCH>();
+    } else if (warp >= NTHR / 32 + NFOLDW) {
+        tc05::reg_dec<REG_STAGE>();
+        // one thread stages the tiles, up to NST ahead
+        if (tid == NTHR + 32 * NFOLDW && t0 < t1) {
+            tc05::tmap_acquire(tm_r1);  // descriptors rewritten by the host between launches: read them afresh
+            tc05::tmap_acquire(tm_r2);
+            if (EXT) tc05::tmap_acquire(tm_e1);
+            int64_t j = 0;
+            for (; t0 + j < t1; ++j) {
+                const int64_t t = t0 + j;
+                const int sidx = (int)(j % NST);
+                if (*abort_v) break;
+                // the stage's last tile, j - NST, read by every operand thread
+                if (j >= NST && !tc05::mbar_wait(&gfree[sidx], (uint32_t)((j / NST - 1) & 1), a.wait_ns)) {
+                    fail();
+                    break;
                 }
-                tc05::mma_f16(d_tile, ah[0], bl[0], idesc, fresh_tile ? 0u : 1u);
-                tc05::mma_f16(d_tile, al[0], bh[0], idesc, 1u);
-                tc05::mma_f16(d_tile, ah[1], bl[1], idesc, 1u);
-                tc05::mma_f16(d_tile, al[1], bh[1], idesc, 1u);
-                tc05::mma_f16(d_tile, ah[0], bh[0], idesc, 1u);
-                tc05::mma_f16(d_tile, ah[1], bh[1], idesc, 1u);
+                uint8_t *stg = sm + OFF_ST + (uint32_t)sidx * STG;
+                tc05::fence_proxy_async();  // earlier generic reads of this stage before the async writes
+                tc05::mbar_arrive_expect_tx(&sbar[sidx], stage_bytes);
+                tc05::bulk_g2s(stg + 2 * SM_STROW, cat.pts + t * KT, SM_STPTS, &sbar[sidx]);
+                if (nb1) tc05::tma_load_2d(stg, tm_r1, (int)(2 * KT * t), mb0 >> 1, &sbar[sidx]);
+                if (nb2) tc05::tma_load_2d(stg + SM_STROW, tm_r2, (int)(2 * KT * t), mb0 >> 1, &sbar[sidx]);
+                if (EXT && l > 0)
+                    tc05::tma_load_2d(stg + 2 * SM_STROW + SM_STPTS, tm_e1, mb0, (int)t, &sbar[sidx]);
+            }
+            // loads still in flight (a loop that stopped early) land before the CTA exits
+            for (int64_t k = j > NST ? j - NST : 0; k < j; ++k) wait_stage(k, WAIT_NS);
+        }
+        if (tid == NTHR + 32 * NFOLDW + 32) {
+            const uint32_t idesc_a = tc05::idesc_f16_mn(128, cols_a), idesc_b = tc05::idesc_f16_mn(128, cols_b);
+            int64_t j = 0;    // tiles issued in full
+            bool half = false;  // and the first part of one more
+            for (; t0 + j < t1; ++j) {
+                const int b = (int)(j & 1);
+                // one part's MMAs: the four small hi x lo / lo x hi products first, the two hi x hi
+                // last: the tensor core rounds each MMA's sum into the FP32 accumulator, and the
+                // small terms then round at their own magnitude (2^-11 of the sum), so only two
+                // roundings per tile fall at the full magnitude instead of five.  c0: the part's
+                // first column (1024 bytes an atom of 64 columns in the operand)
+                auto mmas = [&](int c0, uint32_t idesc) {
+                    const uint32_t sj = tc05::smem_u32(sm + b * SM_BUF), sy = sj + 2 * SM_J + (c0 >> 6) * 1024;
+                    const uint32_t d = d_tile + c0;
+#pragma unroll
+                    for (int p = 0; p < 6; ++p) {
+                        const int ks = p < 4 ? p >> 1 : p - 4;  // the K = 16 step
+                        const bool jlo = p < 4 && (p & 1), ylo = p < 4 && !(p & 1);
+                        tc05::mma_f16(d, tc05::desc_sw128(sj + (jlo ? SM_J : 0) + ks * 4096, 1024, 2048),
+                                      tc05::desc_sw128(sy + (ylo ? SM_Y : 0) + ks * 8192, 1024, 4096), idesc,
+                                      p ? 1u : 0u);
+                    }
+                };
+                const uint32_t pj = (uint32_t)((j - 1) & 1);
+                if (!tc05::mbar_wait(&fbar[b], (uint32_t)((j >> 1) & 1), a.wait_ns) ||
+                    (j > 0 && !tc05::mbar_wait(&dfree[0], pj, a.wait_ns)) || *abort_v) {
+                    fail();
+                    break;
+                }
+                tc05::fence_after();
+                mmas(0, idesc_a);
+                tc05::commit(&hbar);
+                if (cols_b) {
+                    if (j > 0 && !tc05::mbar_wait(&dfree[1], pj, a.wait_ns)) {
+                        half = true;
+                        fail();
+                        break;
+                    }
+                    tc05::fence_after();
+                    mmas(cols_a, idesc_b);
+                }
                 tc05::commit(&mbar[b]);
             }
-            if (b) ++uses1; else ++uses0;
+            // what was issued lands before the block's memory goes (bounded by the drain limit, not by
+            // the possibly shortened pipeline limit)
+            if (j > 0) wait_mma(j - 1, WAIT_NS);
+            if (j > 0 || half) tc05::mbar_wait(&hbar, (uint32_t)((half ? j : j - 1) & 1), WAIT_NS);
         }
-        if (ok && t1 > t0) {
-            const int lb = (int)((t1 - 1 - t0) & 1);
-            ok = fold_vote(wait_buf(lb, a.wait_ns));
-            if (ok) {
-                fold();
-                flush();
+        __syncwarp();
+        tc05::reg_inc<REG_LAUNCH>();  // once the others have given theirs back
+    } else {
+        tc05::reg_inc<REG_FOLD>();
+        for (int64_t t = t0; t < t1; ++t) {
+            const int64_t j = t - t0;
+            if (!__all_sync(0xffffffffu, tc05::mbar_wait(&hbar, (uint32_t)(j & 1), a.wait_ns) && !*abort_v)) {
+                if (lane == 0) fail();
+                break;
             }
+            fold(0, cols_a);
+            __syncwarp();
+            if (lane == 0) ws_arrive(&dfree[0]);
+            if (!__all_sync(0xffffffffu, wait_mma(j, a.wait_ns) && !*abort_v)) {
+                if (lane == 0) fail();
+                break;
+            }
+            fold(cols_a, ncols_pad);
+            __syncwarp();
+            if (lane == 0) ws_arrive(&dfree[1]);
+            acc_fresh = false;
+            if (++folds == FLUSH_FOLDS || t + 1 == t1) flush();
         }
-        if (ok) ok = fold_vote(wait_buf(0, a.wait_ns) && wait_buf(1, a.wait_ns));
-        if (!ok) {
-            // MMAs already issued land before TMEM is released (bounded by the 1 s
-            // drain limit, not by the possibly shortened pipeline limit)
-            wait_buf(0, WAIT_NS);
-            wait_buf(1, WAIT_NS);
-            *abort_v = 1;
-        }
+        __syncwarp();
+        tc05::reg_dec<REG_LAUNCH>();
     }
-    if (!ok && (tid == 0 || tid == NTHR)) *a.err = CATANA_ERR_CUDA;
     // an empty slab still owns partial rows: write zeros so the reduction sees them
     if (t0 >= t1) {
         for (int t = tid; t < ncols * 128; t += NTOT) partial_cta[t] = 0.f;
@@ -1775,26 +1783,28 @@ catana_status_t split_run(DeviceContext *ctx, std::vector<SplitCatInput> &cats_i
         };
         std::vector<size_t> o_kz(gn), o_nl(gn), o_tm(gn);
         for (int c = c0; c < c1; ++c) {
-            // TMA descriptors 0..3: the Legendre row sets (m pairs interleaved per point:
-            // [lrp / 2][2 stride] FP32, 64 x 16 boxes = 32 m x 32 points); 4, 5, extended
-            // range: the exponent sets by the parity of l ([tile][epitch] words, 128 x 1 boxes)
+            // TMA descriptors: the Legendre row sets (m pairs interleaved per point:
+            // [lrp / 2][2 stride] FP32, boxes of 64 x 16 nb = 32 nb m x 32 points) and, extended
+            // range, the exponent sets by the parity of l ([tile][epitch] words, 128 x 1 boxes)
             CatPlan &P = cats[c];
-            CUtensorMap tm[8];
+            CUtensorMap tm[TMAPS];
             memset(tm, 0, sizeof(tm));
             char *rows = ws + off_rows[c - c0];
             const uint64_t lrp = (uint64_t)((P.in.lmax + 1) & ~1);
             const size_t set_bytes = (size_t)P.stride * lrp * sizeof(float);
             for (int k = 0; k < nsets; ++k)
-                if (!tmap_2d(&tm[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rows + k * set_bytes, 2 * (uint64_t)P.stride,
-                             lrp / 2, 2 * (uint64_t)P.stride * sizeof(float), 2 * KT, 16)) {
-                    set_error("cuTensorMapEncodeTiled failed for the Legendre rows");
-                    return CATANA_ERR_CUDA;
-                }
+                for (int nb = 1; nb <= MBLK / 32; ++nb)
+                    if (!tmap_2d(&tm[tmap_rows(k, nb)], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rows + k * set_bytes,
+                                 2 * (uint64_t)P.stride, lrp / 2, 2 * (uint64_t)P.stride * sizeof(float), 2 * KT,
+                                 16 * nb)) {
+                        set_error("cuTensorMapEncodeTiled failed for the Legendre rows");
+                        return CATANA_ERR_CUDA;
+                    }
             if (ext) {
                 const int ep = (P.in.lmax + 1) & ~1;
                 char *ex = ws + off_exp[c - c0];
                 for (int k = 0; k < 2; ++k)
-                    if (!tmap_2d(&tm[4 + k], CU_TENSOR_MAP_DATA_TYPE_UINT64, ex + (size_t)k * exp_set_words(P) * 8,
+                    if (!tmap_2d(&tm[tmap_exp(k)], CU_TENSOR_MAP_DATA_TYPE_UINT64, ex + (size_t)k * exp_set_words(P) * 8,
                                  (uint64_t)ep, (uint64_t)P.ntiles, (uint64_t)ep * 8, 128, 1)) {
                         set_error("cuTensorMapEncodeTiled failed for the row exponents");
                         return CATANA_ERR_CUDA;
