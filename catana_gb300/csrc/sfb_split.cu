@@ -389,6 +389,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
             *reinterpret_cast<uint4 *>(sm + SM_BUF + t * 16) = make_uint4(0u, 0u, 0u, 0u);  // buffer 1
         }
     }
+    __syncwarp();  // the allocation is one instruction of a converged warp
     if (warp == 0) tc05::tmem_alloc(&tmem_base_sh, tcols);
     tc05::fence_before();
     __syncthreads();
@@ -481,6 +482,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
         const int lane_n = qd * 32 + lane;
         for (int gi = 0; gi < (ncols_pad >> 4); ++gi) {
             uint32_t v[16];
+            __syncwarp();
             tc05::tmem_ld16(d_acc + ((uint32_t)(qd * 32) << 16) + gi * 16, v);
             tc05::tmem_wait_ld();
             if (lane_n < nmax) {
@@ -1096,6 +1098,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
     tc05::fence_before();
     __syncthreads();
     tc05::fence_after();
+    __syncwarp();
     if (warp == 0) tc05::tmem_dealloc(tmem, tcols);
 }
 
