@@ -4,12 +4,11 @@
 // published algorithm of Gorski et al. 2005, ApJ 622:759, sec. 4, evaluated in the
 // same operation order as the CPU restatement with every product and sum rounded
 // separately -- no FMA contraction -- so both give the same pixel), then a stable
-// radix sort of (pixel, point index) and a histogram scan give CSR offsets; radii are
+// radix sort of (pixel, point index); CSR offsets by bisection of the sorted keys; radii are
 // gathered in point order within each pixel, as the reference's push_back does.
 //
 // SFB (sfb_reverse_fft.cpp:43-209), per multipole l:
-// Catalogs of up to some tens of points per pixel (and lmax <= 512) are summed point by point with the phase
-// of the pixel's centre (plain_tc.cu).  The others, level by level:
+// Up to lmax 512 the points are summed at their pixels' centres (plain_tc.cu).  Beyond, level by level:
 //   k_hp_map    map[pix][n] = sum_{p in pix} j_l(k_ln r_p), points in order
 //   k_hp_ylm    Y_lm(ring) = P_lm(cos theta_ring) e^{-i m phi_0(ring)} (phi_0: the ring's
 //               first pixel centre, as the reference's RingInfo)
@@ -644,12 +643,12 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     const int64_t *tw_off = reinterpret_cast<const int64_t *>(rb + R.off_twoff);
     const double2 *tw = reinterpret_cast<const double2 *>(rb + R.off_tw);
     const int *order = reinterpret_cast<const int *>(rb + R.off_order);
-    // As a sum over points on the tensor cores (plain_tc.cu) unless the pixels hold many points each, whose
-    // j_l the map below sums first: a point and level costs 0.35..1.3 ns there; here nmax x 0.015 ns plus the
-    // pixels' share (0.04 ns per pixel and radial order).  Measured, ms here / there: nside 64, 400k points,
-    // l 64: n 8 11.7 / 12.2, n 24 18.6 / 14.4; 1.6M points: n 8 22.6 / 47.6, n 24 45.9 / 55.4, n 40 70.0 / 71.5;
-    // nside 256, 1M points, l 128, n 64: 400 / 165.
-    if (plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (nmax < 16 ? 8 : 24) * npix) {
+    // As a sum over points at their pixels' centres on the tensor cores (plain_tc.cu) wherever that takes the
+    // sizes: it sums the j_l of a pixel's points first, and was faster at every density measured, ms there / by the
+    // maps and FFTs below: nside 256, 1M points, l 128, n 64: 116 / 400; nside 64, 1.6M points, l 24: n 4 2.9 / 6.7,
+    // n 48 8.2 / 30; nside 16, 3M points (977 a pixel), l 10: n 4 4.0 / 8.7, n 48 8.0 / 24; nside 1, 20k points
+    // (1667 a pixel), l 24, n 4: 0.44 / 12.
+    if (plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (int64_t)0xFFFFFFFEll) {
         if (npoints > 0) {
             PixelCatalog px;
             px.r = r_sorted_dev;

@@ -89,7 +89,7 @@ static_assert(TC_SMEM <= 232448 - 1024, "k_ptc_main shared memory");
 struct TcSlab {
     double rmin, rmax;  // of |r|
     int ew;             // |w| < 2^ew
-    int pad;
+    int ec;             // at most 2^ec points in an entry of a pixelized catalog (0 otherwise)
 };
 
 struct TcArgs {
@@ -175,6 +175,17 @@ __device__ __forceinline__ uint64_t j_digits(double j, uint32_t w) {
     const int s = (int)(w - (jh & 0x7ff00000u)) >> 20;
     const uint64_t p = shr64(((uint64_t)((jh & 0xfffffu) | 0x100000u) << 42) | ((uint64_t)jl << 10), s);
     return jh >> 31 ? TC_OFF_J - p : TC_OFF_J + p;
+}
+
+// The position of k r in the linear tables from a radius and an entry of k_ptc_ntab: node and FP64 fraction
+__device__ __forceinline__ uint32_t lerp_at(uint64_t r, const uint4 &kd, int npts, double &f) {
+    const uint32_t rh = (uint32_t)(r >> 32), rl = (uint32_t)r;
+    const uint64_t tt = (uint64_t)rl * kd.x + (uint64_t)rh * kd.y;
+    const uint64_t res = (uint64_t)rh * kd.x + (tt >> 32);
+    const uint32_t fh = __funnelshift_l((uint32_t)res, (uint32_t)(res >> 32), kd.z);
+    const uint32_t fl = __funnelshift_l((uint32_t)tt, (uint32_t)res, kd.z);
+    f = __hiloint2double((int)(0x3ff00000u | (fh >> 12)), (int)__funnelshift_l(fl, fh, 20));
+    return min((uint32_t)(res >> 32) >> (32u - kd.z), (uint32_t)(npts - 1));
 }
 
 // log2 of a bound on |j_l| over [z1, z2] (FP32; checked to exceed log2 |j_l| up to 1e-6 for every l < 512):
@@ -403,7 +414,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                         // eight radial orders at this point
                         const int o = u - nq;
                         if (LERP) {
-                            const uint32_t rh = (uint32_t)(r >> 32), rl = (uint32_t)r;
 #pragma unroll
                             for (int h0 = 0; h0 < 8; h0 += 4) {
                                 double2 y[4];
@@ -411,13 +421,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
 #pragma unroll
                                 for (int h = 0; h < 4; ++h) {
                                     const uint4 kd = tn[8 * o + h0 + h];
-                                    const uint64_t tt = (uint64_t)rl * kd.x + (uint64_t)rh * kd.y;
-                                    const uint64_t res = (uint64_t)rh * kd.x + (tt >> 32);
-                                    const uint32_t i = min((uint32_t)(res >> 32) >> (32u - kd.z), (uint32_t)(a.npts - 1));
-                                    y[h] = __ldg(tab + i);
-                                    const uint32_t fh = __funnelshift_l((uint32_t)res, (uint32_t)(res >> 32), kd.z);
-                                    const uint32_t fl = __funnelshift_l((uint32_t)tt, (uint32_t)res, kd.z);
-                                    f[h] = __hiloint2double((int)(0x3ff00000u | (fh >> 12)), (int)__funnelshift_l(fl, fh, 20));
+                                    y[h] = __ldg(tab + lerp_at(r, kd, a.npts, f[h]));
                                 }
 #pragma unroll
                                 for (int h = 0; h < 4; ++h)
@@ -642,30 +646,30 @@ __global__ void __launch_bounds__(128) k_ptc_ntab(const TcSlab *__restrict__ sla
         if (n == nmax - 1 && k * sl.rmax >= zmax[l]) *err = CATANA_ERR_DOMAIN;
     }
     const float lb = jl_log2_bound(l, z1, z2 * 1.000001f) + 0.03f;
-    o.w = (uint32_t)(max(-900, (int)floorf(lb) + 1) + 1022) << 20;
+    o.w = (uint32_t)(max(-900, (int)floorf(lb) + 1 + sl.ec) + 1022) << 20;
     out[(size_t)blockIdx.x * nl * nmax + e] = o;
 }
 
 // Sort keys: r / rmax on 65536 steps (radii past rmax share the last one).
-__global__ void k_ptc_keys(const double *__restrict__ pts, int pitch, int64_t n, double inv_rmax, uint32_t *keys,
+__global__ void k_ptc_keys(const double *__restrict__ pts, int64_t n, double inv_rmax, uint32_t *keys,
                            uint32_t *vals) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double q = fabs(pts[pitch * i]) * inv_rmax * 65536.0;
+    const double q = fabs(pts[3 * i]) * inv_rmax * 65536.0;
     keys[i] = q >= 65535.0 ? 65535u : (q > 0.0 ? (uint32_t)q : 0u);
     vals[i] = (uint32_t)i;
 }
 
 // Per slab: range of |r| and exponent of the largest |w|.  Values that are not finite are left out (they
 // poison the result, k_ptc_points); so are, with the table, radii outside it (a domain error).
-__global__ void __launch_bounds__(256) k_ptc_slabs(const double *__restrict__ pts, int pitch, const double *__restrict__ w,
+__global__ void __launch_bounds__(256) k_ptc_slabs(const double *__restrict__ pts, const double *__restrict__ w,
                                                    const uint32_t *__restrict__ perm, int64_t n, int64_t per, double rlim,
                                                    TcSlab *__restrict__ out) {
     const int64_t i0 = blockIdx.x * per, i1 = min(n, i0 + per);
     double lo = INFINITY, hi = 0.0, mw = 0.0;
     for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
         const int64_t j = perm[i];
-        const double r = fabs(pts[pitch * j]);
+        const double r = fabs(pts[3 * j]);
         if (r < rlim) {  // false for NaN
             lo = fmin(lo, r);
             hi = fmax(hi, r);
@@ -695,12 +699,14 @@ __global__ void __launch_bounds__(256) k_ptc_slabs(const double *__restrict__ pt
         o.rmin = lo <= hi ? lo : 0.0;
         o.rmax = hi;
         o.ew = mw > 0.0 ? ilogb(mw) + 1 : 0;  // mw < 2^ew
-        o.pad = 0;
+        o.ec = 0;
         out[blockIdx.x] = o;
     }
 }
 
-// A catalog in RING pixels (k_ptc_pixels)
+// A catalog in RING pixels (k_ptc_pixels).  Its points share their pixels' centres, so what the main kernel
+// takes as a point is an entry: up to TC_CELL points of one pixel, whose j_l are summed first (k_ptc_jl_cells).
+constexpr int TC_CELL = 64;
 struct TcPixels {
     const double *r;            // radii grouped by pixel
     const int64_t *offs;        // [npix + 1]
@@ -779,44 +785,100 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
     }
 }
 
-// The same for a catalog in RING pixels: a point stands at its pixel's centre, (ring's cos theta, phase
-// e^{-i m phi_0} e^{-2 pi i j s / N}) with phi_0 the ring's first centre, j the pixel's place among the ring's N
-// and s the frequency that the m-extraction reads (sfb_reverse_fft.cpp:192-207): m mod N up to N / 2, then
-// N - m mod N, conjugated only where `conj` says so.  Both factors come from tables (ring_ph, tw).
-__global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t *__restrict__ perm, int64_t n, int64_t q0, int tiles,
-                                                    int tslab, int lmp, const TcSlab *__restrict__ slab, int er, int lerp, double rlim,
-                                                    uint64_t *__restrict__ rint, double *__restrict__ rabs, double2 *__restrict__ xs,
-                                                    ulonglong2 *__restrict__ phase, int *__restrict__ poison, int *__restrict__ err) {
-    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (t >= tiles) return;
-    const int64_t i = (int64_t)t * TC_KT + lane;
-    const bool in = i < n;
-    const int64_t q = q0 + (in ? perm[i] : perm[n - 1]);
-    const double r = px.r[q];
-    // last pixel with offs[p] <= q, then its ring
+// last pixel with offs[p] <= q
+__device__ __forceinline__ int64_t pixel_of(const TcPixels &px, int64_t q) {
     int64_t lo = 0, hi = px.npix;
     while (hi - lo > 1) {
         const int64_t mid = (lo + hi) >> 1;
         if (px.offs[mid] <= q) lo = mid;
         else hi = mid;
     }
+    return lo;
+}
+
+// Sort keys of a pixelized catalog: every TC_CELL-th point of a pixel heads an entry, the fullest entries
+// first (a warp sums as long as its longest); the other points come last.  Also each radius in the table's units.
+__global__ void k_ptc_cells(TcPixels px, int64_t n, int er, int lerp, double rlim, uint32_t *__restrict__ keys,
+                            uint32_t *__restrict__ vals, uint64_t *__restrict__ rint, int *__restrict__ poison,
+                            unsigned long long *__restrict__ count, int *__restrict__ err) {
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const int64_t p = pixel_of(px, q), k = q - px.offs[p];
+    const unsigned act = __activemask(), heads = __ballot_sync(act, k % TC_CELL == 0);
+    if ((threadIdx.x & 31) == 0 && heads) atomicAdd(count, (unsigned long long)__popc(heads));
+    keys[q] = k % TC_CELL == 0 ? (uint32_t)(TC_CELL - min((int64_t)TC_CELL, px.offs[p + 1] - q)) : (uint32_t)TC_CELL;
+    vals[q] = (uint32_t)q;
+    const double r = px.r[q];
+    const bool bad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
+    if (bad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
+    if (bad && !lerp) atomicOr(poison, TC_POISON_W);
+    rint[q] = bad || !(fabs(r) < ldexp(1.0, er)) ? 0ull : (uint64_t)(int64_t)ldexp(fmax(r, 0.0), 62 - er);
+}
+
+// Per slab of entries what k_ptc_slabs finds for points (weights are 1)
+__global__ void __launch_bounds__(256) k_ptc_cell_slabs(TcPixels px, const uint2 *__restrict__ cell, int64_t n, int64_t per,
+                                                        double rlim, TcSlab *__restrict__ out) {
+    const int64_t i0 = blockIdx.x * per, i1 = min(n, i0 + per);
+    double lo = INFINITY, hi = 0.0;
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const uint2 c = cell[i];
+        for (uint32_t k = 0; k < c.y; ++k) {
+            const double r = fabs(px.r[(int64_t)c.x + k]);
+            if (r < rlim) {  // false for NaN
+                lo = fmin(lo, r);
+                hi = fmax(hi, r);
+            }
+        }
+    }
+    __shared__ double s[2][8];
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s[0][threadIdx.x >> 5] = lo;
+        s[1][threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) {
+            lo = fmin(lo, s[0][k]);
+            hi = fmax(hi, s[1][k]);
+        }
+        TcSlab o;
+        o.rmin = lo <= hi ? lo : 0.0;
+        o.rmax = hi;
+        o.ew = 1;
+        o.ec = 32 - __clz((int)cell[i0].y - 1);  // the slab's first entry is its fullest
+        out[blockIdx.x] = o;
+    }
+}
+
+// The same as k_ptc_points for the entries of a catalog in RING pixels, at their pixels' centres: (ring's cos
+// theta, phase e^{-i m phi_0} e^{-2 pi i j s / N}) with phi_0 the ring's first centre, j the pixel's place among
+// the ring's N and s the frequency that the m-extraction reads (sfb_reverse_fft.cpp:192-207): m mod N up to
+// N / 2, then N - m mod N, conjugated only where `conj` says so.  Both factors come from tables (ring_ph, tw).
+__global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t *__restrict__ perm, int64_t n, int tiles, int lmp,
+                                                    uint2 *__restrict__ cell, double2 *__restrict__ xs,
+                                                    ulonglong2 *__restrict__ phase) {
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= tiles) return;
+    const int64_t i = (int64_t)t * TC_KT + lane;
+    const bool use = i < n;
+    const int64_t q = use ? perm[i] : perm[n - 1];
+    const int64_t lo = pixel_of(px, q);
     int ra = 0, rb = px.nrings;
     while (rb - ra > 1) {
         const int mid = (ra + rb) >> 1;
         if (px.ring_start[mid] <= lo) ra = mid;
         else rb = mid;
     }
-    const bool rbad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
-    const bool use = in && !rbad;
     if (blockIdx.y == 0) {
-        if (in && rbad && !lerp) atomicOr(poison, TC_POISON_W);
-        if (in && rbad && lerp) *err = CATANA_ERR_DOMAIN;
-        rint[i] = rbad || !(fabs(r) < ldexp(1.0, er)) ? 0ull : (uint64_t)(int64_t)ldexp(fmax(r, 0.0), 62 - er);
-        rabs[i] = r;
         const double x = px.ring_x[ra];
+        cell[i] = make_uint2((uint32_t)q, use ? (uint32_t)min((int64_t)TC_CELL, px.offs[lo + 1] - q) : 0u);
         xs[i] = use ? make_double2(x, sqrt((1.0 - x) * (1.0 + x))) : make_double2(0.0, 0.0);
     }
-    const double scale = use ? ldexp(1.0, 58 - slab[t / tslab].ew) : 0.0;
+    const double scale = use ? ldexp(1.0, 58 - 1) : 0.0;  // unit weights: ew = 1
     const int N = px.ring_pix[ra], j = (int)(lo - px.ring_start[ra]);
     const double2 *tw = px.tw + px.tw_off[ra];
     const int m0 = blockIdx.y * 8;
@@ -908,6 +970,9 @@ struct TcJ {
     const uint4 *ntab;
     int l0, nl, nmax, tiles, tslab, er;
     uint64_t *out;
+    const uint2 *cell;   // pixelized catalogs: (first point, points) of each entry
+    const double2 *tab;  // and the linear tables [l][npts], or null
+    int npts;
 };
 __device__ __forceinline__ bool tc_j_index(const TcJ &a, int &l, int &t, int &n, size_t &e) {
     const int64_t q = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -926,6 +991,60 @@ __global__ void __launch_bounds__(256) k_ptc_jl_exact(TcJ a) {
     const double z = a.kln[(size_t)l * a.nmax + n] * a.r[(size_t)t * TC_KT + (threadIdx.x & 31)];
     const uint32_t w = a.ntab[((size_t)(t / a.tslab) * a.nl + (l - a.l0)) * a.nmax + n].w;
     a.out[e] = j_digits(isfinite(z) ? jl_direct(l, z) : 0.0, w);
+}
+
+// J of a pixelized catalog's entries, the sums over their points, exact in units of 2^-63 of the bound (which
+// leaves room for the count).  With the tables a warp takes eight radial orders of a tile, so a radius is read
+// once for eight values; what bounds it is the table's gathers, whose radii are unsorted (32 sectors a warp, 7.6 TB/s
+// from L2), and the FP64 pipe (one operation a value).  1M points on nside 256, l 128, n 64: 34 ms, and the main
+// kernel over 0.57M entries 78 ms; over 1M points with their j_l 165.
+__global__ void __launch_bounds__(256, 3) k_ptc_jl_cells(TcJ a) {
+    const int lane = threadIdx.x & 31, noct = (a.nmax + 7) >> 3;
+    const int64_t q = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (q >= (int64_t)a.nl * a.tiles * noct) return;  // warp-uniform
+    const int o = (int)(q % noct);
+    const int64_t q2 = q / noct;
+    const int t = (int)(q2 % a.tiles), lv = (int)(q2 / a.tiles), nc = min(8, a.nmax - 8 * o);
+    const uint4 *kd = a.ntab + ((size_t)(t / a.tslab) * a.nl + lv) * a.nmax + 8 * o;
+    const double2 *__restrict__ tab = a.tab + (size_t)(a.l0 + lv) * a.npts;
+    const uint2 c = a.cell[(size_t)t * TC_KT + lane];
+    uint64_t v[8];
+#pragma unroll
+    for (int h = 0; h < 8; ++h) v[h] = TC_OFF_J;
+    for (uint32_t k = 0; k < c.y; ++k) {
+        const uint64_t r = __ldg(a.rint + (size_t)c.x + k);
+#pragma unroll
+        for (int h0 = 0; h0 < 8; h0 += 4) {
+            double2 y[4];
+            double f[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const uint4 e = __ldg(kd + min(h0 + h, nc - 1));
+                y[h] = __ldg(tab + lerp_at(r, e, a.npts, f[h]));
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+                v[h0 + h] += j_digits(fma(y[h].y, f[h], y[h].x), __ldg(&kd[min(h0 + h, nc - 1)].w)) - TC_OFF_J;
+        }
+    }
+    uint64_t *out = a.out + (((size_t)lv * a.tiles + t) * a.nmax + 8 * o) * TC_KT + lane;
+#pragma unroll
+    for (int h = 0; h < 8; ++h)
+        if (h < nc) out[h * TC_KT] = v[h];
+}
+__global__ void __launch_bounds__(256) k_ptc_jl_cells_exact(TcJ a) {
+    int l, t, n;
+    size_t e;
+    if (!tc_j_index(a, l, t, n, e)) return;
+    const uint32_t w = a.ntab[((size_t)(t / a.tslab) * a.nl + (l - a.l0)) * a.nmax + n].w;
+    const double kl = a.kln[(size_t)l * a.nmax + n];
+    const uint2 c = a.cell[(size_t)t * TC_KT + (threadIdx.x & 31)];
+    uint64_t v = TC_OFF_J;
+    for (uint32_t k = 0; k < c.y; ++k) {
+        const double z = kl * a.r[(size_t)c.x + k];
+        v += j_digits(isfinite(z) ? jl_direct(l, z) : 0.0, w) - TC_OFF_J;
+    }
+    a.out[e] = v;
 }
 
 // The FP64 polynomials (sfb_fp64.cu, sum_s a_s t^s on unit intervals, t in [-1, 1]) as integers: Horner's
@@ -1086,11 +1205,13 @@ bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
 
 namespace {
 
-// pix == nullptr: points_dev are npoints x 3; otherwise the pixelized catalog
+// pix == nullptr: points_dev are npoints x 3; otherwise the pixelized catalog.  "Points" below are what the main
+// kernel takes as such: the catalog's points, or a pixelized one's entries.
 catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, const PixelCatalog *pix,
-                              int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
+                              int64_t nall, int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
                               double *f_acc_dev, int *err_dev, cudaStream_t st) {
-    const bool lerp = jl == JL_MODE_LERP;
+    const bool lerp = jl == JL_MODE_LERP, fused = lerp && !pix;  // fused: the main kernel evaluates j_l itself
+    int64_t npoints = nall;  // an upper bound of a pixelized catalog's entries, until they are counted
     catana_status_t s = ensure_tc_coefs(ctx, lmax, st);
     if (s != CATANA_OK) return s;
     if (lerp) {
@@ -1117,8 +1238,10 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     const int tiles_c = ceil_div(chunk, TC_KT);
     const size_t np = (size_t)tiles_c * TC_KT;
     // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
-    const size_t kb = tc_al(np * 4), hb = tc_al((size_t)256 * ((np + 4095) / 4096 + 1) * 4);
-    const size_t o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(np * 8), o_xs = o_rabs + tc_al(np * 8);
+    // (a pixelized catalog's points are sorted at once, its entries then taken in passes)
+    const size_t ns = pix ? (size_t)nall : np;
+    const size_t kb = tc_al(ns * 4), hb = tc_al((size_t)256 * ((ns + 4095) / 4096 + 1) * 4);
+    const size_t o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(std::max(ns, np) * 8), o_xs = o_rabs + tc_al(np * 8);
     const size_t o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
     // slabs: at most TC_SLAB_TILES tiles (the 64-bit sums' resolution), a whole number of waves
     auto slab_tiles = [&](int tiles) {
@@ -1138,7 +1261,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     uint32_t *hist = reinterpret_cast<uint32_t *>(ws + 4 * kb);
     int *poison = reinterpret_cast<int *>(ws + o_poi);
     TcSlab *slabs = reinterpret_cast<TcSlab *>(ws + o_sl);
-    CG_CUDA_TRY(cudaMemsetAsync(poison, 0, sizeof(int), st));
+    CG_CUDA_TRY(cudaMemsetAsync(poison, 0, 16, st));  // and the entries' count
     TcPixels px = {};
     if (pix) {
         double2 *ph = reinterpret_cast<double2 *>(ws + o_poi + 256);
@@ -1156,29 +1279,41 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         px.ring_ph = ph;
         px.tw = pix->tw;
         px.tw_off = pix->tw_off;
+        k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, er, lerp ? 1 : 0, rlim, keys, perm,
+                                                         reinterpret_cast<uint64_t *>(ws + o_rint), poison,
+                                                         reinterpret_cast<unsigned long long *>(poison) + 1, err_dev);
+        count_launch();
+        unsigned long long cells = 0;
+        CG_CUDA_TRY(cudaMemcpyAsync(&cells, reinterpret_cast<unsigned long long *>(poison) + 1, sizeof(cells),
+                                    cudaMemcpyDeviceToHost, st));
+        s = radix_sort_pairs(keys, perm, tk, tv, nall, 8, hist, st);
+        if (s != CATANA_OK) return s;
+        CG_CUDA_TRY(cudaStreamSynchronize(st));
+        npoints = (int64_t)cells;
     }
     for (int64_t c0 = 0; c0 < npoints; c0 += chunk) {
         const int64_t nc = std::min(chunk, npoints - c0);
         const int tiles = ceil_div(nc, TC_KT);
         const int tslab = slab_tiles(tiles), nslabs = ceil_div(tiles, tslab);
-        const double *pts = pix ? pix->r + c0 : points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
-        const int pitch = pix ? 1 : 3;
-        k_ptc_keys<<<ceil_div(nc, 256), 256, 0, st>>>(pts, pitch, nc, 1.0 / rmax, keys, perm);
-        count_launch();
-        s = radix_sort_pairs(keys, perm, tk, tv, nc, 16, hist, st);
-        if (s != CATANA_OK) return s;
-        k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, pitch, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
         const dim3 pg(ceil_div(tiles, 8), ceil_div(lmp, 8));
         uint64_t *rint_d = reinterpret_cast<uint64_t *>(ws + o_rint);
         double *rabs_d = reinterpret_cast<double *>(ws + o_rabs);
         double2 *xs_d = reinterpret_cast<double2 *>(ws + o_xs);
         ulonglong2 *ph_d = reinterpret_cast<ulonglong2 *>(ws + o_ph);
-        if (pix)
-            k_ptc_pixels<<<pg, 256, 0, st>>>(px, perm, nc, c0, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,
-                                             xs_d, ph_d, poison, err_dev);
-        else
+        uint2 *cell = reinterpret_cast<uint2 *>(ws + o_rabs);
+        if (pix) {
+            k_ptc_pixels<<<pg, 256, 0, st>>>(px, perm + c0, nc, tiles, lmp, cell, xs_d, ph_d);
+            k_ptc_cell_slabs<<<nslabs, 256, 0, st>>>(px, cell, nc, (int64_t)tslab * TC_KT, rlim, slabs);
+        } else {
+            const double *pts = points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
+            k_ptc_keys<<<ceil_div(nc, 256), 256, 0, st>>>(pts, nc, 1.0 / rmax, keys, perm);
+            count_launch();
+            s = radix_sort_pairs(keys, perm, tk, tv, nc, 16, hist, st);
+            if (s != CATANA_OK) return s;
+            k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
             k_ptc_points<<<pg, 256, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,
                                              xs_d, ph_d, poison, err_dev);
+        }
         count_launch(2);
         CG_CUDA_TRY(cudaGetLastError());
         TcArgs a;
@@ -1198,7 +1333,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         a.tab = nullptr;
         const double *dxinv = nullptr;
         if (lerp) {
-            a.tab = ctx->tc_tab.as<double2>();
+            if (fused) a.tab = ctx->tc_tab.as<double2>();
             dxinv = reinterpret_cast<const double *>(ctx->tc_tab.as<char>() + ctx->tc_tab_off);
         }
         // levels per launch: the slabs' partial sums stay under 256 MB (they are read back at once and
@@ -1206,7 +1341,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         for (int l0 = 0; l0 < lmax;) {
             int l1 = l0 + 1;
             auto pdoubles = [&](int e) { return (int64_t)nmax * ((int64_t)e * (e + 1) - (int64_t)l0 * (l0 + 1)); };
-            const double jbytes = lerp ? 0.0 : 8.0 * tiles * TC_KT * nmax;
+            const double jbytes = fused ? 0.0 : 8.0 * tiles * TC_KT * nmax;
             while (l1 < lmax && pdoubles(l1 + 1) * 8.0 * nslabs < 256e6 && jbytes * (l1 + 1 - l0) < 2e9) ++l1;
             a.l0 = l0;
             a.l1 = l1;
@@ -1220,12 +1355,15 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
                 slabs, kln_dev, dxinv, dxinv ? dxinv + ctx->tc_tab_lmax : nullptr, l0, l1 - l0, nmax, er, ntab, err_dev);
             count_launch();
             a.jarr = nullptr;
-            if (!lerp) {
+            if (!fused) {
                 const int64_t cnt = (int64_t)(l1 - l0) * tiles * nmax * TC_KT;
                 CG_CUDA_TRY(ctx->tc_jarr.ensure((size_t)cnt * 8));
                 uint64_t *ja = ctx->tc_jarr.as<uint64_t>();
                 TcJ j;
-                j.r = reinterpret_cast<const double *>(ws + o_rabs);
+                j.r = pix ? pix->r : reinterpret_cast<const double *>(ws + o_rabs);
+                j.cell = cell;
+                j.tab = ctx->tc_tab.as<double2>();
+                j.npts = a.npts;
                 j.kln = kln_dev;
                 j.rint = a.rint;
                 j.ntab = ntab;
@@ -1236,7 +1374,11 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
                 j.tslab = tslab;
                 j.er = er;
                 j.out = ja;
-                if (jl == JL_MODE_POLY)
+                if (pix && lerp)
+                    k_ptc_jl_cells<<<ceil_div((int64_t)(l1 - l0) * tiles * ((nmax + 7) / 8), 8), 256, 0, st>>>(j);
+                else if (pix)
+                    k_ptc_jl_cells_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(j);
+                else if (jl == JL_MODE_POLY)
                     k_ptc_jl_poly<<<ceil_div(cnt, 256), 256, 0, st>>>(j, ctx->tc_poly.as<TcPoly>(), ctx->tc_poly_nint, err_dev);
                 else
                     k_ptc_jl_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(j);
@@ -1245,7 +1387,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
                 a.jarr = ja;
             }
             prof_begin(st);
-            if (lerp) k_ptc_main<true><<<nslabs, TC_THREADS, TC_SMEM, st>>>(a);
+            if (fused) k_ptc_main<true><<<nslabs, TC_THREADS, TC_SMEM, st>>>(a);
             else k_ptc_main<false><<<nslabs, TC_THREADS, TC_SMEM, st>>>(a);
             prof_end(st, 2.0 * (double)nc * (double)pdoubles(l1));
             k_ptc_reduce<<<dim3(std::min(64, ceil_div((int64_t)l1 * nmax, 32)), l1 - l0), 256, 0, st>>>(

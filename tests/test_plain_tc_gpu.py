@@ -86,7 +86,7 @@ def test_points_that_are_not_finite(cuda_device, column, bad):
 @pytest.mark.parametrize("dense", [False, True])
 def test_pixelized_points(cuda_device, nside, n, lmax, nmax, dense):
     """The pixelized sum point by point at pixel centres, polar rings shorter than 2 l included (aliases with
-    and without the conjugate); nside 4 with 26 points per pixel takes the map form instead."""
+    and without the conjugate)."""
     pts = uniform_ball(n, 1000.0, seed=n + nside)
     ppc = catana.PixelizedPointContainer(nside, catana.PointContainer(pts))
     if dense:
@@ -95,5 +95,22 @@ def test_pixelized_points(cuda_device, nside, n, lmax, nmax, dense):
     else:
         res = catana.sfb_decomposition(ppc, lmax, nmax, 1000.0, True, False, interpolation="on")
         k, c, f = O.sfb_healpix(nside, ppc.offsets, ppc.r_sorted, lmax, nmax, 1000.0, interpolated=True)
+    for l, (a, b) in enumerate(zip(res.f_lmn, f)):
+        assert np.max(np.abs(a - b)) <= TOL * max(np.max(np.abs(b)), 1e-6 * np.max(np.abs(f[0]))), l
+
+
+@pytest.mark.parametrize("nside,counts", [(1, (64,)), (1, (65, 1)), (2, (129, 63, 64, 1)), (2, (3000,)), (4, (1,) * 33 + (200,))])
+@pytest.mark.parametrize("interpolated", [True, False])
+def test_pixelized_cells(cuda_device, nside, counts, interpolated):
+    """Pixels with less, just as many and more points than are summed at once; entries of unlike counts in a tile."""
+    npix = 12 * nside * nside
+    offs = np.zeros(npix + 1, dtype=np.int64)
+    offs[1:] = np.cumsum(np.bincount((7 * np.arange(len(counts)) + 3) % npix, weights=counts, minlength=npix))
+    n = int(offs[-1])
+    r = 1000.0 * np.random.default_rng(n).uniform(0.0, 1.0, n) ** (1.0 / 3.0)
+    ppc = catana.PixelizedPointContainer(nside)
+    ppc.offsets, ppc.r_sorted = offs, r
+    res = catana.sfb_decomposition(ppc, 9, 11, 1000.0, True, False, interpolation="on" if interpolated else "off")
+    k, c, f = O.sfb_healpix(nside, offs, r, 9, 11, 1000.0, interpolated=interpolated)
     for l, (a, b) in enumerate(zip(res.f_lmn, f)):
         assert np.max(np.abs(a - b)) <= TOL * max(np.max(np.abs(b)), 1e-6 * np.max(np.abs(f[0]))), l
