@@ -128,14 +128,54 @@ CG_HD void sbessel_jl_all(int lcount, double x, double *out) {
 }
 
 #if defined(__CUDACC__)
-// sbessel_jl on the device, for kernels that evaluate it at every point (z finite): the same branches, the
-// recurrences' (2 k + 1) / z from one reciprocal, corrected by an FMA to within an ulp of the quotient -- a
-// division costs about twelve FP64 operations at two per SM and cycle, and the recurrences take one
-// per step (445 points, l 10, n 10: 88 -> 57 us).
+// sbessel_jl on the device, for kernels that evaluate it at every point (z finite): the same three forms with
+// fewer FP64 operations, of which an SM takes two a cycle -- a division costs about twelve.  Against 80-bit
+// values (l 0 to 4000) the errors are those of sbessel_jl or smaller.
+//   * series, x^2 < 2 l + 3: 17 terms (the next is below 2^-56 of the first) over a common denominator, and
+//     x^l / (2l + 1)!! in blocks of 16 factors, x^16 as a float-float so that its rounding does not add up;
+//   * upward and downward recurrences: (2 k + 1) / z from one reciprocal, corrected by an FMA to within an ulp of
+//     the quotient;
+//   * downward: from 8 + 9 cbrt(l + 1) above l, where what the start leaves out is below 2^-55 (at x = l it
+//     falls as exp(-1.9 d^1.5 l^-0.5) with the distance d).
+// 445 points, l 10, n 10: 66 -> 33 us; the rows of a shot-noise matrix, l 16, 32 wave numbers: 575 -> 380 us.
+__device__ __forceinline__ double jl_series_direct(int l, double x) {
+    const double y = -0.5 * x * x;
+    double p = 1.0, q = 1.0;
+#pragma unroll 1
+    for (int k = 17; k > 0; --k) {
+        const double t = (double)(k * (2 * l + 2 * k + 1)) * q;
+        p = fma(y, p, t);
+        q = t;
+    }
+    double r = p / q, c = 1.0;
+    const int nb = l >> 4;
+    if (nb) {
+        double h = x, e = 0.0;  // x^16 = h + e
+        for (int k = 0; k < 4; ++k) {
+            const double t = h * h;
+            e = fma(2.0 * h, e, fma(h, h, -t));
+            h = t;
+        }
+        for (int b = 0; b < nb; ++b) {
+            double den = 1.0;
+#pragma unroll 1
+            for (int k = 0; k < 16; ++k) den *= (c += 2.0);
+            r *= h / den;
+        }
+        if (h > 1e-280) r = fma(r, nb * (e / h), r);
+    }
+    double num = 1.0, den = 1.0;
+#pragma unroll 1
+    for (int k = l & 15; k > 0; --k) {
+        num *= x;
+        den *= (c += 2.0);
+    }
+    return r * (num / den);
+}
 __device__ __forceinline__ double jl_direct(int l, double z) {
     if (z == 0.0) return l == 0 ? 1.0 : 0.0;
     const double sgn = z < 0.0 && (l & 1) ? -1.0 : 1.0, x = fabs(z);
-    if (x * x < 2.0 * l + 3.0) return sgn * jl_series(l, x);
+    if (x * x < 2.0 * l + 3.0) return sgn * jl_series_direct(l, x);
     const double ix = 1.0 / x;
     auto quot = [&](double n) {
         const double q = n * ix;
@@ -146,22 +186,25 @@ __device__ __forceinline__ double jl_direct(int l, double z) {
     const double t0 = quot(sn), t1 = quot(t0 - cs);
     if (x >= (double)l) {
         if (l == 0) return sgn * t0;
-        double j0 = t0, j1 = t1;
+        double j0 = t0, j1 = t1, c = 1.0;
+#pragma unroll 1
         for (int k = 1; k < l; ++k) {
-            const double j2 = fma(quot(2.0 * k + 1.0), j1, -j0);
+            const double j2 = fma(quot(c += 2.0), j1, -j0);
             j0 = j1;
             j1 = j2;
         }
         return sgn * j1;
     }
-    const int nstart = (int)((double)l + 20.0 + 16.0 * cbrt((double)l + 1.0));
-    double jp1 = 0.0, jk = 1e-200, jl = 0.0;
+    const int nstart = l + 8 + (int)(9.f * cbrtf((float)(l + 1)));
+    double jp1 = 0.0, jk = 1e-200, jl = 0.0, c = 2.0 * nstart + 1.0;
+#pragma unroll 1
     for (int k = nstart; k > 0; --k) {
-        const double jm1 = fma(quot(2.0 * k + 1.0), jk, -jp1);
+        const double jm1 = fma(quot(c), jk, -jp1);
+        c -= 2.0;
         jp1 = jk;
         jk = jm1;
         if (k - 1 == l) jl = jk;
-        if (fabs(jk) > 1e200) {
+        if ((__double2hiint(jk) & 0x7fffffff) > 0x6974e718) {  // above 1e200
             jk *= 1e-200;
             jp1 *= 1e-200;
             jl *= 1e-200;
