@@ -193,7 +193,9 @@ catana_status_t split_raw_accumulate(DeviceContext *ctx, const double *points_de
                                      int64_t npoints, int lmax, int nmax, double rmax, const double *kln_dev,
                                      double *f_acc_dev, int *err_dev, cudaStream_t st, bool accurate);
 
-// Stable radix sort of (key, index) pairs by the low key_bits bits (sort.cu).
+// Stable radix sort of (key, index) pairs by the low key_bits bits (sort.cu); hist_scratch:
+// radix_hist_words(n) words, which does not fall as n grows.
+size_t radix_hist_words(int64_t n);
 catana_status_t radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *tmp_keys, uint32_t *tmp_vals, int64_t n,
                                  int key_bits, uint32_t *hist_scratch, cudaStream_t st);
 

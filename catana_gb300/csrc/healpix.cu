@@ -597,7 +597,7 @@ catana_status_t healpix_bin_dev(DeviceContext *ctx, int64_t nside, const double 
     }
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t nb = al((size_t)std::max<int64_t>(npoints, 1) * sizeof(uint32_t));
-    const size_t hb = al((size_t)256 * ((npoints + 4095) / 4096 + 1) * sizeof(uint32_t));
+    const size_t hb = al(radix_hist_words(npoints) * sizeof(uint32_t));
     CG_CUDA_TRY(ctx->hp_ws.ensure(4 * nb + hb));
     char *w = ctx->hp_ws.as<char>();
     uint32_t *keys = reinterpret_cast<uint32_t *>(w), *vals = reinterpret_cast<uint32_t *>(w + nb);

@@ -650,13 +650,14 @@ __global__ void __launch_bounds__(128) k_ptc_ntab(const TcSlab *__restrict__ sla
     out[(size_t)blockIdx.x * nl * nmax + e] = o;
 }
 
-// Sort keys: r / rmax on 65536 steps (radii past rmax share the last one).
-__global__ void k_ptc_keys(const double *__restrict__ pts, int64_t n, double inv_rmax, uint32_t *keys,
-                           uint32_t *vals) {
+// Sort keys: r / rmax on 2^bits steps (radii past rmax share the last one).
+__global__ void k_ptc_keys(const double *__restrict__ pts, int64_t n, double inv_rmax, int bits,
+                           uint32_t *keys, uint32_t *vals) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double q = fabs(pts[3 * i]) * inv_rmax * 65536.0;
-    keys[i] = q >= 65535.0 ? 65535u : (q > 0.0 ? (uint32_t)q : 0u);
+    const double top = (double)(1 << bits);
+    const double q = fabs(pts[3 * i]) * inv_rmax * top;
+    keys[i] = q >= top - 1.0 ? (1u << bits) - 1u : (q > 0.0 ? (uint32_t)q : 0u);
     vals[i] = (uint32_t)i;
 }
 
@@ -1240,7 +1241,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
     // (a pixelized catalog's points are sorted at once, its entries then taken in passes)
     const size_t ns = pix ? (size_t)nall : np;
-    const size_t kb = tc_al(ns * 4), hb = tc_al((size_t)256 * ((ns + 4095) / 4096 + 1) * 4);
+    const size_t kb = tc_al(ns * 4), hb = tc_al(radix_hist_words((int64_t)ns) * 4);
     const size_t o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(std::max(ns, np) * 8), o_xs = o_rabs + tc_al(np * 8);
     const size_t o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
     // slabs: at most TC_SLAB_TILES tiles (the 64-bit sums' resolution), a whole number of waves
@@ -1306,9 +1307,12 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             k_ptc_cell_slabs<<<nslabs, 256, 0, st>>>(px, cell, nc, (int64_t)tslab * TC_KT, rlim, slabs);
         } else {
             const double *pts = points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
-            k_ptc_keys<<<ceil_div(nc, 256), 256, 0, st>>>(pts, nc, 1.0 / rmax, keys, perm);
+            // Neighbours share cells of the j_l table and slabs take a bound each.  A tile of 32 of few points
+            // spans more than one of 256 steps anyway: one pass of the sort instead of two.
+            const int bits = nc <= 8192 ? 8 : 16;
+            k_ptc_keys<<<ceil_div(nc, 256), 256, 0, st>>>(pts, nc, 1.0 / rmax, bits, keys, perm);
             count_launch();
-            s = radix_sort_pairs(keys, perm, tk, tv, nc, 16, hist, st);
+            s = radix_sort_pairs(keys, perm, tk, tv, nc, bits, hist, st);
             if (s != CATANA_OK) return s;
             k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
             k_ptc_points<<<pg, 256, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,

@@ -1737,7 +1737,7 @@ catana_status_t split_run(DeviceContext *ctx, std::vector<SplitCatInput> &cats_i
         size_t ws_bytes = 0;
         std::vector<size_t> off_pts(gn), off_rows(gn), off_exp(gn);
         for (int c = c0; c < c1; ++c) smax = std::max(smax, cats[c].stride);
-        const size_t keyb = al256((size_t)smax * 4), histb = al256((size_t)256 * ((smax + 4095) / 4096 + 1) * 4);
+        const size_t keyb = al256((size_t)smax * 4), histb = al256(radix_hist_words(smax) * 4);
         ws_bytes = 4 * keyb + histb;
         for (int c = c0; c < c1; ++c) {
             off_pts[c - c0] = ws_bytes;

@@ -7,13 +7,15 @@
 // reads into broadcasts).
 //
 // One pass per 8-bit digit:
-//   k_radix_hist     per-tile digit histogram (tile = 4096 consecutive pairs)
+//   k_radix_hist     per-tile digit histogram (tile = up to 4096 consecutive pairs)
 //   k_radix_scan     exclusive scan of the (digit-major, tile-minor) histogram
 //   k_radix_scatter  each tile re-reads its pairs in order, 256 at a time, ranks equal
 //                    digits with __match_any_sync within a warp and with per-warp
 //                    counts across warps, and scatters -- a stable, deterministic order.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -22,16 +24,16 @@ namespace catana_gpu {
 namespace {
 
 constexpr int RS_THREADS = 256;
-constexpr int RS_TILE = 4096;  // pairs per tile (16 rounds of 256)
+constexpr int RS_ROUNDS = 16;  // most rounds of 256 pairs per tile
 constexpr int RS_WARPS = RS_THREADS / 32;
 
 __global__ void k_radix_hist(const uint32_t *__restrict__ keys, int64_t n, int shift, uint32_t *__restrict__ hist,
-                             int ntiles) {
+                             int ntiles, int tile) {
     __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RS_TILE;
-    for (int k = threadIdx.x; k < RS_TILE; k += RS_THREADS) {
+    const int64_t base = (int64_t)blockIdx.x * tile;
+    for (int k = threadIdx.x; k < tile; k += RS_THREADS) {
         const int64_t i = base + k;
         if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
     }
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(1024) k_radix_scan(uint32_t *__restrict__ data
 
 __global__ void k_radix_scatter(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals, int64_t n,
                                 int shift, const uint32_t *__restrict__ offs, int ntiles,
-                                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out) {
+                                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int tile) {
     __shared__ uint32_t base[256];
     __shared__ uint32_t wcnt[RS_WARPS][256];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -118,8 +120,8 @@ __global__ void k_radix_scatter(const uint32_t *__restrict__ keys, const uint32_
     for (int w = 0; w < RS_WARPS; ++w) wcnt[w][t] = 0;
     __syncthreads();
     const uint32_t lt_mask = (1u << lane) - 1u;
-    const int64_t tile0 = (int64_t)blockIdx.x * RS_TILE;
-    for (int r = 0; r < RS_TILE / RS_THREADS; ++r) {
+    const int64_t tile0 = (int64_t)blockIdx.x * tile;
+    for (int r = 0; r < tile / RS_THREADS; ++r) {
         const int64_t i = tile0 + (int64_t)r * RS_THREADS + t;
         const bool valid = i < n;
         uint32_t key = 0, val = 0, d = 0xFFFFFFFFu;  // invalid lanes form their own group
@@ -162,19 +164,32 @@ catana_status_t scan_u32(uint32_t *data, int64_t count, cudaStream_t st) {
     return CATANA_OK;
 }
 
+namespace {
+// Pairs per tile: a tile's rounds run one after the other (1.3 us each in the scatter), so fewer than
+// 262144 pairs take as few rounds as leave at most 64 tiles, whose histogram the scan takes in one round.
+// 5000 pairs, a pass: 35 us by tiles of 4096, 12 so.
+int radix_tile(int64_t n) {
+    return RS_THREADS * (int)std::min<int64_t>(RS_ROUNDS, std::max<int64_t>(1, (n + 64 * RS_THREADS - 1) / (64 * RS_THREADS)));
+}
+}  // namespace
+
+size_t radix_hist_words(int64_t n) {
+    return (size_t)256 * (size_t)std::max<int64_t>(64, (n + RS_ROUNDS * RS_THREADS - 1) / (RS_ROUNDS * RS_THREADS));
+}
+
 // Sorts (keys, vals) by the low `key_bits` bits of the keys, stably.  The result
 // ends in (keys, vals); tmp_keys / tmp_vals are scratch of n entries; hist_scratch
-// holds 256 * ceil(n / 4096) words.
+// holds radix_hist_words(n) words.
 catana_status_t radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *tmp_keys, uint32_t *tmp_vals, int64_t n,
                                  int key_bits, uint32_t *hist_scratch, cudaStream_t st) {
     if (n <= 1) return CATANA_OK;
-    const int ntiles = (int)((n + RS_TILE - 1) / RS_TILE);
+    const int tile = radix_tile(n), ntiles = (int)((n + tile - 1) / tile);
     uint32_t *ka = keys, *va = vals, *kb = tmp_keys, *vb = tmp_vals;
     int passes = 0;
     for (int shift = 0; shift < key_bits; shift += 8, ++passes) {
-        k_radix_hist<<<ntiles, RS_THREADS, 0, st>>>(ka, n, shift, hist_scratch, ntiles);
+        k_radix_hist<<<ntiles, RS_THREADS, 0, st>>>(ka, n, shift, hist_scratch, ntiles, tile);
         k_radix_scan<<<1, 1024, 0, st>>>(hist_scratch, (int64_t)256 * ntiles);
-        k_radix_scatter<<<ntiles, RS_THREADS, 0, st>>>(ka, va, n, shift, hist_scratch, ntiles, kb, vb);
+        k_radix_scatter<<<ntiles, RS_THREADS, 0, st>>>(ka, va, n, shift, hist_scratch, ntiles, kb, vb, tile);
         count_launch(3);
         CG_CUDA_TRY(cudaGetLastError());
         uint32_t *t;
