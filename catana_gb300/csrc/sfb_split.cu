@@ -88,7 +88,8 @@ constexpr int JPW = (64 + NOPW - 1) / NOPW;   // most J row pairs per operand wa
 static_assert(JPW <= 16, "k_split_l: one lane per J row in the Taylor coefficients");
 constexpr int NFOLDW = 4;           // fold / MMA warps, one per TMEM lane quadrant
 constexpr int NTOT = NTHR + 32 * NFOLDW + 128;  // and a warpgroup of which one thread stages the tiles, one issues the MMAs
-// registers a thread: at launch, and what the three kinds of warps give up or take for their work
+// registers a thread: at launch, and what the three kinds of warps give up or take for their work (the
+// increases are taken from the staging warps' decrease; every warp ends with the staging warps' count)
 constexpr int REG_LAUNCH = 80, REG_OP = 88, REG_FOLD = 88, REG_STAGE = 40;
 static_assert(REG_OP >= REG_LAUNCH && REG_FOLD >= REG_LAUNCH && REG_STAGE <= REG_LAUNCH, "setmaxnreg: directions");
 static_assert(REG_OP * NTHR + REG_FOLD * 32 * NFOLDW + REG_STAGE * 128 <= REG_LAUNCH * NTOT, "setmaxnreg: the split");
@@ -254,6 +255,11 @@ __device__ __forceinline__ void phase_seed(unsigned long long u, int m, float &c
 // FULLJ: every item of the launch has 128 radial orders in its half (no kmax cut):
 // with 16 operand warps each evaluates 8 J rows; otherwise the items' live row pairs
 // are spread over the warps and the rest of J stays zero.
+// the end of a role's work: every warp of the block (named barrier 1)
+__device__ __forceinline__ void role_end() {
+    __syncwarp();
+    asm volatile("barrier.sync 1, %0;" ::"n"(NTOT) : "memory");
+}
 // one arrival (release, CTA scope) on an mbarrier
 __device__ __forceinline__ void ws_arrive(uint64_t *mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc05::smem_u32(mbar)) : "memory");
@@ -986,8 +992,8 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
                 if (!(a.stall && t == t0)) ws_arrive(&fbar[b]);  // the test hook withholds the first hand-off
             }
         }
-        __syncwarp();
-        tc05::reg_dec<REG_LAUNCH>();
+        role_end();
+        tc05::reg_dec<REG_STAGE>();
     } else if (warp >= NTHR / 32 + NFOLDW) {
         tc05::reg_dec<REG_STAGE>();
         // one thread stages the tiles, up to NST ahead
@@ -1065,8 +1071,9 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
             if (j > 0) wait_mma(j - 1, WAIT_NS);
             if (j > 0 || half) tc05::mbar_wait(&hbar, (uint32_t)((half ? j : j - 1) & 1), WAIT_NS);
         }
-        __syncwarp();
-        tc05::reg_inc<REG_LAUNCH>();  // once the others have given theirs back
+        // No increase here: a warp that took back what it gave up, before the operand warps of its
+        // quarter of the SM had taken it, would leave them waiting for it for good.
+        role_end();
     } else {
         tc05::reg_inc<REG_FOLD>();
         for (int64_t t = t0; t < t1; ++t) {
@@ -1088,8 +1095,8 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
             acc_fresh = false;
             if (++folds == FLUSH_FOLDS || t + 1 == t1) flush();
         }
-        __syncwarp();
-        tc05::reg_dec<REG_LAUNCH>();
+        role_end();
+        tc05::reg_dec<REG_STAGE>();
     }
     // an empty slab still owns partial rows: write zeros so the reduction sees them
     if (t0 >= t1) {
