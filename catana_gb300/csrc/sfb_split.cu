@@ -83,6 +83,7 @@ namespace {
 constexpr int KT = 32;              // points per tile (two K=16 MMA steps)
 constexpr int NOPW = 16;            // operand warps
 constexpr int NTHR = 32 * NOPW;
+static_assert((NOPW & (NOPW - 1)) == 0, "the runs of m move on modulo a power of two");
 constexpr int QPW = (32 + NOPW - 1) / NOPW;   // most quads of complex m per operand warp (128 m = 32 quads)
 constexpr int JPW = (64 + NOPW - 1) / NOPW;   // most J row pairs per operand warp (128 rows)
 static_assert(JPW <= 16, "k_split_l: one lane per J row in the Taylor coefficients");
@@ -409,11 +410,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
 
     const int64_t t0 = item.t0, t1 = item.t1;
     const int q = lane, g = warp;
-    // this warp's m: quads [qb0, qb1) of the block's ceil(mcount / 4) quads of complex m, spread
-    // evenly (a quad fills one 16-byte column group of each Y half: whole-chunk stores)
     const int nquads = (mcount + 3) >> 2;
-    const int qb0 = (g * nquads) / NOPW, qb1 = ((g + 1) * nquads) / NOPW;
-    const int mlo = 4 * qb0, mhi = min(4 * qb1, mcount);  // local m range of this warp
     // The accumulator's columns in two parts, each a whole number of the operand layout's 64-column
     // atoms (one part when there are no more than 64): the fold of one part runs while the
     // tensor core multiplies the other.
@@ -758,6 +755,12 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
                 }
             }
             // ---- Y tile: local m = mlo .. mhi-1 of this block, in pairs (m, m+1), stored by quads ----
+            // The block's ceil(mcount / 4) quads of complex m are spread over the warps (a quad fills one
+            // 16-byte column group of each Y half: whole-chunk stores), a run each; the runs move on by a
+            // warp per tile, so that with a count that the warps do not divide no warp has the longer run
+            // in every tile (the operand buffers let it fall back and catch up).
+            const int gt = (g + (int)j) & (NOPW - 1);
+            const int mlo = 4 * ((gt * nquads) / NOPW), mhi = min(4 * (((gt + 1) * nquads) / NOPW), mcount);
             if (mlo < mhi) {
                 // x = cos(theta) (Reinsch-modified rows: |cos(theta)|) and eps = 1 - |cos(theta)|
                 const float xh = pt.x_hi, xl = pt.x_lo, eh = pt.s_hi, el = pt.s_lo, c1 = pt.cphi, s1 = pt.sphi;
