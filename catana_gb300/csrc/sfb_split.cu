@@ -49,14 +49,16 @@
 // multiplied, and flush; one thread stages the tiles and one issues the MMAs.  Hand-offs are
 // mbarriers: operands written, MMAs of a part complete, part folded, row stage read.  What
 // bounds it is the operand warps' instructions, ~550 a warp and tile in dependent chains
-// (clock stamps at 1M points, l = 200: 4.3k cycles a tile, of which J 1.1k, Y 1.7k, waits and
-// hand-offs 1.3k).  Staging by an operand warp (its copies and the proxy fence kept that warp
-// 1.3k cycles behind the others, and every tile waited for it), the fold of a whole tile between
-// two MMAs and the MMAs' issue by a fold warp had made it 4.8k.  1M points, lmax 256, nmax 128:
-// 200 -> 178 ms; 2 x 20k points, lmax 512, nmax 256: 114.6 -> 104.9.  Measured and dropped on this
-// layout: 16-column TMEM loads in flight two deep in the fold (+5%), Taylor coefficients of J by
-// two warps of their own (+2.5%: they wait for the stage, then every operand warp for them), waits
-// by one lane of a warp (+4%).  Every wait is bounded (1 s); on timeout the
+// (clock stamps at 1M points, l = 200: J 1.1k cycles a tile, Y 1.7k, waits and hand-offs 1.3k).
+// What had held it up before: staging by an operand warp (its copies and the proxy fence kept that
+// warp 1.3k cycles behind the others, and every tile waited for it), the fold of a whole tile
+// between two MMAs with their issue by a fold warp, two barriers to wait for and two to arrive at
+// per tile and operand warp, the longer runs of m always on the same warps.  1M points, lmax 256,
+// nmax 128: 200 -> 172 ms; 8 catalogs with k <= 0.2: 43.5 -> 36.9; 2 x 20k points, lmax 512,
+// nmax 256: 114.6 -> 104.  Measured and dropped on this layout: 16-column TMEM loads in flight
+// two deep in the fold (+5%), Taylor coefficients of J by two warps of their own (+2.5%: they wait
+// for the stage, then every operand warp for them), waits by one lane of a warp (+4%), e^{i m phi}
+// from memory instead of a sincospif per warp and tile (-1%, +2% at lmax 512).  Every wait is bounded (1 s); on timeout the
 // kernel records CATANA_ERR_CUDA in the error word, stops issuing work and frees its
 // tensor memory.
 #include <cuda.h>
@@ -324,10 +326,10 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
     __shared__ uint64_t mbar[2];   // MMA completion per operand buffer
     __shared__ uint64_t hbar;      // MMA completion of a tile's first column part
     __shared__ uint64_t dfree[2];  // the column part read by every fold warp (NFOLDW arrivals)
-    __shared__ uint64_t sbar[NST];  // TMA completion per stage
+    __shared__ uint64_t sbar[NST];  // tile staged, and its operand buffer free (2 arrivals and the copies' bytes)
     __shared__ uint32_t tmem_base_sh;
     __shared__ uint64_t fbar[2];   // operands of buffer b written (NOPW arrivals)
-    __shared__ uint64_t gfree[NST];  // stage s read by every operand warp (NOPW arrivals)
+    __shared__ uint64_t gfree[NST];  // stage s read by every operand warp (NOPW arrivals; two stages: fbar says so too)
     __shared__ int abort_sh;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
     if (tid == 0) {
         tc05::mbar_init(&mbar[0], 1);
         tc05::mbar_init(&mbar[1], 1);
-        for (int k = 0; k < NST; ++k) tc05::mbar_init(&sbar[k], 1);
+        for (int k = 0; k < NST; ++k) tc05::mbar_init(&sbar[k], 2);
         tc05::mbar_init(&hbar, 1);
         for (int k = 0; k < 2; ++k) tc05::mbar_init(&fbar[k], NOPW);
         for (int k = 0; k < 2; ++k) tc05::mbar_init(&dfree[k], NFOLDW);
@@ -531,9 +533,9 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
         for (int64_t t = t0; t < t1; ++t) {
             const int64_t j = t - t0;
             const int b = (int)(j & 1);
-            // the buffer's last reader (tile j - 2), this tile's stage
-            if (!__all_sync(0xffffffffu, (j < 2 || wait_mma(j - 2, a.wait_ns)) && wait_stage(j, a.wait_ns) &&
-                                             !*abort_v)) {
+            // this tile's stage, and the buffer's last reader (tile j - 2)
+            if (!__all_sync(0xffffffffu, tc05::mbar_try(&sbar[j % NST], (uint32_t)((j / NST) & 1))) &&
+                !__all_sync(0xffffffffu, !*abort_v && wait_stage(j, a.wait_ns) && !*abort_v)) {
                 if (lane == 0) fail();
                 break;
             }
@@ -991,7 +993,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
             tc05::fence_proxy_async();
             __syncwarp();
             if (lane == 0) {
-                ws_arrive(&gfree[sidx]);
+                if (NST != 2) ws_arrive(&gfree[sidx]);
                 if (!(a.stall && t == t0)) ws_arrive(&fbar[b]);  // the test hook withholds the first hand-off
             }
         }
@@ -1010,7 +1012,8 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
                 const int sidx = (int)(j % NST);
                 if (*abort_v) break;
                 // the stage's last tile, j - NST, read by every operand thread
-                if (j >= NST && !tc05::mbar_wait(&gfree[sidx], (uint32_t)((j / NST - 1) & 1), a.wait_ns)) {
+                if (j >= NST && !tc05::mbar_wait(NST == 2 ? &fbar[sidx] : &gfree[sidx], (uint32_t)((j / NST - 1) & 1),
+                                                 a.wait_ns)) {
                     fail();
                     break;
                 }
@@ -1022,6 +1025,14 @@ __global__ void __launch_bounds__(NTOT, 1) k_split_l(SplitArgs a) {
                 if (nb2) tc05::tma_load_2d(stg + SM_STROW, tm_r2, (int)(2 * KT * t), mb0 >> 1, &sbar[sidx]);
                 if (EXT && l > 0)
                     tc05::tma_load_2d(stg + 2 * SM_STROW + SM_STPTS, tm_e1, mb0, (int)t, &sbar[sidx]);
+                // the operand warps then have one barrier to wait for, not two
+                const bool okm = j < 2 || wait_mma(j - 2, a.wait_ns);
+                ws_arrive(&sbar[sidx]);
+                if (!okm) {
+                    fail();
+                    ++j;
+                    break;
+                }
             }
             // loads still in flight (a loop that stopped early) land before the CTA exits
             for (int64_t k = j > NST ? j - NST : 0; k < j; ++k) wait_stage(k, WAIT_NS);
