@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
                                                     const TcSlab *__restrict__ slab, int er, int lerp, double rlim,
                                                     uint64_t *__restrict__ rint, double *__restrict__ rabs, double2 *__restrict__ xs,
                                                     ulonglong2 *__restrict__ phase, int *__restrict__ poison, int *__restrict__ err) {
-    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= tiles) return;
     const int64_t i = (int64_t)t * TC_KT + lane;
     const bool in = i < n;
@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(256) k_ptc_cell_slabs(TcPixels px, const uint2
 __global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t *__restrict__ perm, int64_t n, int tiles, int lmp,
                                                     uint2 *__restrict__ cell, double2 *__restrict__ xs,
                                                     ulonglong2 *__restrict__ phase) {
-    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= tiles) return;
     const int64_t i = (int64_t)t * TC_KT + lane;
     const bool use = i < n;
@@ -1296,14 +1296,17 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         const int64_t nc = std::min(chunk, npoints - c0);
         const int tiles = ceil_div(nc, TC_KT);
         const int tslab = slab_tiles(tiles), nslabs = ceil_div(tiles, tslab);
-        const dim3 pg(ceil_div(tiles, 8), ceil_div(lmp, 8));
+        // warps per CTA: eight, or as few as still give every SM one (the FP64 pipe, one an SM, bounds both
+        // kernels: 445 points, l 10: 17 us by eight, 11 so)
+        const int pw = std::max(1, std::min(8, tiles * ceil_div(lmp, 8) / ctx->sm_count));
+        const dim3 pg(ceil_div(tiles, pw), ceil_div(lmp, 8));
         uint64_t *rint_d = reinterpret_cast<uint64_t *>(ws + o_rint);
         double *rabs_d = reinterpret_cast<double *>(ws + o_rabs);
         double2 *xs_d = reinterpret_cast<double2 *>(ws + o_xs);
         ulonglong2 *ph_d = reinterpret_cast<ulonglong2 *>(ws + o_ph);
         uint2 *cell = reinterpret_cast<uint2 *>(ws + o_rabs);
         if (pix) {
-            k_ptc_pixels<<<pg, 256, 0, st>>>(px, perm + c0, nc, tiles, lmp, cell, xs_d, ph_d);
+            k_ptc_pixels<<<pg, 32 * pw, 0, st>>>(px, perm + c0, nc, tiles, lmp, cell, xs_d, ph_d);
             k_ptc_cell_slabs<<<nslabs, 256, 0, st>>>(px, cell, nc, (int64_t)tslab * TC_KT, rlim, slabs);
         } else {
             const double *pts = points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
@@ -1315,7 +1318,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             s = radix_sort_pairs(keys, perm, tk, tv, nc, bits, hist, st);
             if (s != CATANA_OK) return s;
             k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
-            k_ptc_points<<<pg, 256, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,
+            k_ptc_points<<<pg, 32 * pw, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,
                                              xs_d, ph_d, poison, err_dev);
         }
         count_launch(2);
