@@ -229,12 +229,16 @@ def side_workloads(torch, _lib, catana, sp, fp64_peak=None):
     _lib.check(_lib.lib.catana_gpu_profile_report(ctypes.byref(kms), ctypes.byref(kn), ctypes.byref(kfl)))
     ms = e0.elapsed_time(e1) / 5
     ktf = kfl.value / (kms.value / 1e3) / 1e12
-    pk = fp64_peak["tflops"] if fp64_peak else None
+    # the contraction runs on the tensor cores as 35 exact products of 8-bit digits per MAC
+    bf16, _, _, src = peaks()
+    pk = bf16 / 35.0
     res["plain_fp64_100k_l32_n32"] = {"value": 100000 * modes(L, M) / (ms / 1e3), "unit": UNIT, "ms_per_step": ms,
-                                     "roofline": {"bound": "fp64", "kernel": "k_fp64_raw_l", "achieved": ktf,
+                                     "roofline": {"bound": "tensor", "kernel": "k_ptc_main", "achieved": ktf,
                                                   "peak": pk, "unit": "TFLOP/s",
                                                   "frac": (ktf / pk) if pk else None,
-                                                  "peak_source": "measured in this run (catana_gpu_fp64_peak)"}}
+                                                  "peak_source": "bf16_tflops / 35 (exact products of 8-bit digits per "
+                                                                 "MAC), of %s" % src,
+                                                  "fp64_peak": fp64_peak["tflops"] if fp64_peak else None}}
     # the same case with exact j_l per (point, l, n) (the reference's branch for N <= 1000)
     run(_lib.JL_EXACT)
     torch.cuda.synchronize()
@@ -262,10 +266,9 @@ def side_workloads(torch, _lib, catana, sp, fp64_peak=None):
     ts = time.perf_counter() - t0
     _lib.lib.catana_gpu_profile_enable(0)
     _lib.check(_lib.lib.catana_gpu_profile_report(ctypes.byref(kms), ctypes.byref(kn), ctypes.byref(kfl)))
-    res["healpix_nside256_1M_l128_n64"] = {"binning_s": tb, "sfb_s": ts, "ring_transform_s": kms.value / 1e3,
-                                           "note": "host API incl. copies; FP64; ring transform: batched FFT "
-                                                   "for the power-of-two rings (the 513 equatorial rings of "
-                                                   "1024 pixels and 16 polar ones), direct sums over quarter-orbits for the rest"}
+    res["healpix_nside256_1M_l128_n64"] = {"binning_s": tb, "sfb_s": ts, "contraction_s": kms.value / 1e3,
+                                           "note": "host API incl. copies; to FP64 accuracy; contraction: k_ptc_main "
+                                                   "over the pixels' summed j_l (k_ptc_jl_cells)"}
     return res
 
 
@@ -775,10 +778,10 @@ def main():
         bound = "tensor"
         kernel = "k_split_l (tcgen05 kind::f16 contraction + operand generation)"
     else:
-        peak = fp64_peak["tflops"]
-        peak_note = "FP64 FMA throughput measured by catana_gpu_fp64_peak in this run"
-        bound = "fp64"
-        kernel = "k_fp64_raw_l"
+        peak = bf16_sus / 35.0
+        peak_note = "bf16_tflops_sustained / 35 (exact products of 8-bit digits per MAC), of %s" % src
+        bound = "tensor"
+        kernel = "k_ptc_main (tcgen05 kind::f16 digit products + operand generation)"
     achieved = (kfl.value / (kms.value / 1e3)) / 1e12 if kms.value > 0 else None
     # DRAM bytes of an average k_split_l launch: the ncu capture of l = 200 on 300k points
     # (profiles/k_split_l_l200_300k_full.md) read+wrote 756.0 MB = 1.024 x the algorithmic

@@ -236,9 +236,12 @@ __device__ __forceinline__ void tc_blocks(const TcArgs &a, F &&body) {
             }
 }
 
-// What bounds it at 64 m x 64 n: the FP64 pipe (2 operations per (point, m), 1 per (point, n), 16 cycles
-// each per warp: ~3.1k cycles per tile), the issue slots (~9k warp instructions per tile) and the tensor
-// core (70 MMAs of 128 x 64 x 16 per tile, ~2.2k cycles) are of one size.
+// What bounds it: the operand warps' dependent instructions.  A unit (4 complex m or 8 radial orders at 32
+// points) is ~450 instructions of one warp and takes it 4.5k cycles, with eleven such warps an SM; measured on
+// 200k points, lmax 96, nmax 48 (ncu): 1.57 instructions a cycle, FP64 pipe 32%, ALU 40%, tensor pipe 26%, DRAM
+// 13.8 + 3.7 GB; 20 ms against 281 with FP64 FMAs on CUDA cores.  More operand warps spill at the registers that
+// are left (15 of them: +25%), fewer are slower, and J from a kernel of its own (which takes 60% off the units of
+// n) made it 22.7 ms.
 template <bool LERP>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
     extern __shared__ uint8_t tc_smem[];

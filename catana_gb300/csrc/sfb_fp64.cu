@@ -1,4 +1,6 @@
-// sfb_fp64.cu -- the plain FP64 raw SFB path on CUDA cores (the drop-in form).
+// sfb_fp64.cu -- the plain raw SFB in FP64 on CUDA cores: the sizes that the tensor-core kernel does not take
+// (plain_tc.cu; lmax > 512, nmax > 4096, extreme rmax), other devices and the allocation-free entry.  Also the
+// j_l tables of both, and the normalisation.
 //
 // Reference: _sfb_raw, sfb_raw.cpp:13-108.  The reference loops l outermost and,
 // per point, evaluates j_l(k_ln r) for every n (:67-69), P_lm by gsl_sf_legendre_sphPlm

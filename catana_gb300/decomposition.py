@@ -9,7 +9,8 @@ HEALPix method (py_decomposition.cpp:135-153, sfb_decomposition.cpp:22-26).
 
 Keyword extensions (absent in the reference, defaults reproduce it):
   weights=None         per-point weights; f is normalised by V/sum(w)
-  precision='plain'    'plain': FP64 on CUDA cores (the drop-in);
+  precision='plain'    'plain': to FP64 accuracy, the contraction as exact products of
+                       8-bit digits on the tensor cores (the drop-in);
                        'split': tcgen05 tensor cores, 3-term FP16 hi+lo products;
                        'split_accurate': the same with Reinsch-modified Legendre
                        rows: half the f_lmn error at high l (ten times less near

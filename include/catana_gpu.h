@@ -59,7 +59,8 @@ typedef enum {
  * radii are CATANA_ERR_DOMAIN. */
 #define CATANA_JL_POLY 3u
 #define CATANA_JL_MASK 3u
-/* Contraction form.  PLAIN: FP64 on CUDA cores, the drop-in.  SPLIT: tensor-core
+/* Contraction form.  PLAIN: to FP64 accuracy, the drop-in (tensor-core products of
+ * 8-bit digits that are exact; FP64 on CUDA cores past lmax 512).  SPLIT: tensor-core
  * tcgen05 contraction of 3-term FP16 hi+lo products with FP32 accumulation,
  * folded per 32-point tile and reduced in FP64; j_l from piecewise degree-6
  * polynomials on unit intervals with FP32 coefficients, accurate to ~1e-7 of its
