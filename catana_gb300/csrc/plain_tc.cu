@@ -801,8 +801,10 @@ __device__ __forceinline__ int64_t pixel_of(const TcPixels &px, int64_t q) {
 }
 
 // Sort keys of a pixelized catalog: every TC_CELL-th point of a pixel heads an entry, the fullest entries
-// first (a warp sums as long as its longest); the other points come last.  Also each radius in the table's units.
-__global__ void k_ptc_cells(TcPixels px, int64_t n, int er, int lerp, double rlim, uint32_t *__restrict__ keys,
+// first (a warp sums as long as its longest), of like ones by the head's radius in 256 steps (the lanes of a
+// warp then share cells of the j_l table where entries hold few points: 34 -> 32 ms below); the other points
+// come last.  Also each radius in the table's units.
+__global__ void k_ptc_cells(TcPixels px, int64_t n, double inv_rmax, int er, int lerp, double rlim, uint32_t *__restrict__ keys,
                             uint32_t *__restrict__ vals, uint64_t *__restrict__ rint, int *__restrict__ poison,
                             unsigned long long *__restrict__ count, int *__restrict__ err) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -810,9 +812,10 @@ __global__ void k_ptc_cells(TcPixels px, int64_t n, int er, int lerp, double rli
     const int64_t p = pixel_of(px, q), k = q - px.offs[p];
     const unsigned act = __activemask(), heads = __ballot_sync(act, k % TC_CELL == 0);
     if ((threadIdx.x & 31) == 0 && heads) atomicAdd(count, (unsigned long long)__popc(heads));
-    keys[q] = k % TC_CELL == 0 ? (uint32_t)(TC_CELL - min((int64_t)TC_CELL, px.offs[p + 1] - q)) : (uint32_t)TC_CELL;
+    const double r = px.r[q], rs = r * inv_rmax * 256.0;
+    const uint32_t rb = rs >= 255.0 ? 255u : (rs > 0.0 ? (uint32_t)rs : 0u);
+    keys[q] = (k % TC_CELL == 0 ? (uint32_t)(TC_CELL - min((int64_t)TC_CELL, px.offs[p + 1] - q)) : (uint32_t)TC_CELL) << 8 | rb;
     vals[q] = (uint32_t)q;
-    const double r = px.r[q];
     const bool bad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
     if (bad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
     if (bad && !lerp) atomicOr(poison, TC_POISON_W);
@@ -998,42 +1001,40 @@ __global__ void __launch_bounds__(256) k_ptc_jl_exact(TcJ a) {
 }
 
 // J of a pixelized catalog's entries, the sums over their points, exact in units of 2^-63 of the bound (which
-// leaves room for the count).  With the tables a warp takes eight radial orders of a tile, so a radius is read
-// once for eight values; what bounds it is the table's gathers, whose radii are unsorted (32 sectors a warp, 7.6 TB/s
-// from L2), and the FP64 pipe (one operation a value).  1M points on nside 256, l 128, n 64: 34 ms, and the main
-// kernel over 0.57M entries 78 ms; over 1M points with their j_l 165.
-__global__ void __launch_bounds__(256, 3) k_ptc_jl_cells(TcJ a) {
-    const int lane = threadIdx.x & 31, noct = (a.nmax + 7) >> 3;
+// leaves room for the count).  With the tables a warp takes four radial orders of a tile (with eight, or two, the
+// registers and the radii read again cost as much: 114.3 and 120.4 ms a call against 113.4).  What bounds it are
+// the table's gathers from L2, most of them of unsorted radii, and ~60 instructions a value.  1M points on nside
+// 256, l 128, n 64: 31 ms, and the main kernel over 0.57M entries 78 ms; over 1M points with their j_l 165.
+constexpr int JC_N = 4;
+__global__ void __launch_bounds__(256, 4) k_ptc_jl_cells(TcJ a) {
+    const int lane = threadIdx.x & 31, noct = (a.nmax + JC_N - 1) / JC_N;
     const int64_t q = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (q >= (int64_t)a.nl * a.tiles * noct) return;  // warp-uniform
     const int o = (int)(q % noct);
     const int64_t q2 = q / noct;
-    const int t = (int)(q2 % a.tiles), lv = (int)(q2 / a.tiles), nc = min(8, a.nmax - 8 * o);
-    const uint4 *kd = a.ntab + ((size_t)(t / a.tslab) * a.nl + lv) * a.nmax + 8 * o;
+    const int t = (int)(q2 % a.tiles), lv = (int)(q2 / a.tiles), nc = min(JC_N, a.nmax - JC_N * o);
+    const uint4 *kp = a.ntab + ((size_t)(t / a.tslab) * a.nl + lv) * a.nmax + JC_N * o;
     const double2 *__restrict__ tab = a.tab + (size_t)(a.l0 + lv) * a.npts;
     const uint2 c = a.cell[(size_t)t * TC_KT + lane];
-    uint64_t v[8];
+    uint64_t v[JC_N];
+    uint4 kd[JC_N];
 #pragma unroll
-    for (int h = 0; h < 8; ++h) v[h] = TC_OFF_J;
+    for (int h = 0; h < JC_N; ++h) {
+        v[h] = TC_OFF_J;
+        kd[h] = __ldg(kp + min(h, nc - 1));
+    }
     for (uint32_t k = 0; k < c.y; ++k) {
         const uint64_t r = __ldg(a.rint + (size_t)c.x + k);
+        double2 y[JC_N];
+        double f[JC_N];
 #pragma unroll
-        for (int h0 = 0; h0 < 8; h0 += 4) {
-            double2 y[4];
-            double f[4];
+        for (int h = 0; h < JC_N; ++h) y[h] = __ldg(tab + lerp_at(r, kd[h], a.npts, f[h]));
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const uint4 e = __ldg(kd + min(h0 + h, nc - 1));
-                y[h] = __ldg(tab + lerp_at(r, e, a.npts, f[h]));
-            }
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-                v[h0 + h] += j_digits(fma(y[h].y, f[h], y[h].x), __ldg(&kd[min(h0 + h, nc - 1)].w)) - TC_OFF_J;
-        }
+        for (int h = 0; h < JC_N; ++h) v[h] += j_digits(fma(y[h].y, f[h], y[h].x), kd[h].w) - TC_OFF_J;
     }
-    uint64_t *out = a.out + (((size_t)lv * a.tiles + t) * a.nmax + 8 * o) * TC_KT + lane;
+    uint64_t *out = a.out + (((size_t)lv * a.tiles + t) * a.nmax + JC_N * o) * TC_KT + lane;
 #pragma unroll
-    for (int h = 0; h < 8; ++h)
+    for (int h = 0; h < JC_N; ++h)
         if (h < nc) out[h * TC_KT] = v[h];
 }
 __global__ void __launch_bounds__(256) k_ptc_jl_cells_exact(TcJ a) {
@@ -1283,14 +1284,14 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         px.ring_ph = ph;
         px.tw = pix->tw;
         px.tw_off = pix->tw_off;
-        k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, er, lerp ? 1 : 0, rlim, keys, perm,
+        k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, 1.0 / rmax, er, lerp ? 1 : 0, rlim, keys, perm,
                                                          reinterpret_cast<uint64_t *>(ws + o_rint), poison,
                                                          reinterpret_cast<unsigned long long *>(poison) + 1, err_dev);
         count_launch();
         unsigned long long cells = 0;
         CG_CUDA_TRY(cudaMemcpyAsync(&cells, reinterpret_cast<unsigned long long *>(poison) + 1, sizeof(cells),
                                     cudaMemcpyDeviceToHost, st));
-        s = radix_sort_pairs(keys, perm, tk, tv, nall, 8, hist, st);
+        s = radix_sort_pairs(keys, perm, tk, tv, nall, 16, hist, st);
         if (s != CATANA_OK) return s;
         CG_CUDA_TRY(cudaStreamSynchronize(st));
         npoints = (int64_t)cells;
@@ -1385,7 +1386,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
                 j.er = er;
                 j.out = ja;
                 if (pix && lerp)
-                    k_ptc_jl_cells<<<ceil_div((int64_t)(l1 - l0) * tiles * ((nmax + 7) / 8), 8), 256, 0, st>>>(j);
+                    k_ptc_jl_cells<<<ceil_div((int64_t)(l1 - l0) * tiles * ((nmax + JC_N - 1) / JC_N), 8), 256, 0, st>>>(j);
                 else if (pix)
                     k_ptc_jl_cells_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(j);
                 else if (jl == JL_MODE_POLY)
