@@ -63,7 +63,7 @@ __global__ void k_bin_keys(int64_t nside, const double *pts, int64_t n, uint32_t
                            int *err) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int64_t p = ang2pix_ring_dev(nside, pts[3 * i + 1], pts[3 * i + 2]);
+    int64_t p = ang2pix_ring_any(nside, pts[3 * i + 1], pts[3 * i + 2]);
     if (p < 0) {
         *err = CATANA_ERR_ARG;
         p = 0;

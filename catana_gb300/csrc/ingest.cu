@@ -69,29 +69,40 @@ __device__ inline void load_record(const void *rec, uint32_t layout, int64_t i, 
     }
 }
 
-// convert + filter; keep flag per record, kept count per block (flags: 1 window domain, 2 mask theta)
+// a Cartesian record's angles (Point.cpp:5-10)
+__device__ __forceinline__ void record_angles(double a, double b, double c, double &th, double &ph) {
+    th = atan2(sqrt(a * a + b * b), c);
+    ph = (a == 0.0 && b == 0.0) ? 0.0 : atan2(b, a);
+    if (ph < 0.0) ph += 2.0 * kPi;
+    if (ph >= 2.0 * kPi) ph = fmod(ph, 2.0 * kPi);
+}
+__device__ __forceinline__ double record_radius(uint32_t layout, double a, double b, double c) {
+    return (layout & CATANA_REC_CARTESIAN) ? sqrt(a * a + b * b + c * c) : a;
+}
+
+// filter; keep flag per record, kept count per block (flags: 1 window domain, 2 mask theta).  With every record's
+// angles in FP64 here that pipe bounded the ingest (83%; 4M records 1.26 ms), so they are left to k_ingest_scatter,
+// which forms them for the records that are kept, and the tophat and the mask's pixel are decided in FP32 where that
+// settles them: 0.21 ms here and 0.53 there.
 __global__ void __launch_bounds__(IG_BLOCK) k_ingest_mark(const void *__restrict__ rec, int64_t n, IngestDev sp,
-                                                           double *__restrict__ tmp, uint8_t *__restrict__ keepv,
-                                                           uint32_t *__restrict__ bcount, int *__restrict__ err) {
+                                                           uint8_t *__restrict__ keepv, uint32_t *__restrict__ bcount,
+                                                           int *__restrict__ err) {
     const int64_t i = blockIdx.x * (int64_t)IG_BLOCK + threadIdx.x;
     int keep = 0;
     if (i < n) {
-        double r, th, ph;
         double a, b, c;
         load_record(rec, sp.layout, i, a, b, c);
-        if (sp.layout & CATANA_REC_CARTESIAN) {
-            r = sqrt(a * a + b * b + c * c);
-            th = atan2(sqrt(a * a + b * b), c);
-            ph = (a == 0.0 && b == 0.0) ? 0.0 : atan2(b, a);
-            if (ph < 0.0) ph += 2.0 * kPi;
-            if (ph >= 2.0 * kPi) ph = fmod(ph, 2.0 * kPi);
-        } else {
-            r = a;
-            th = b;
-            ph = c;
-        }
+        const bool cart = (sp.layout & CATANA_REC_CARTESIAN) != 0;
+        const float rf = cart ? sqrtf((float)a * (float)a + (float)b * (float)b + (float)c * (float)c) : 0.f;
+        const bool small = rf > 1e-15f && rf < 1e18f;  // rf stands for r to within 3e-7 of it
+        double r = 0.0;
         keep = 1;
-        if (sp.has_tophat && !(r < sp.tophat_r0)) keep = 0;
+        if (small && !sp.has_gauss && !sp.has_window && sp.has_tophat && fabs((double)rf - sp.tophat_r0) > 1e-5 * (double)rf) {
+            keep = (double)rf < sp.tophat_r0;
+        } else {
+            r = record_radius(sp.layout, a, b, c);
+            if (sp.has_tophat && !(r < sp.tophat_r0)) keep = 0;
+        }
         if (keep && (sp.has_gauss || sp.has_window)) {
             const double u = ingest_uniform(sp.seed, sp.index0 + (uint64_t)i);
             if (sp.has_gauss) {
@@ -112,7 +123,22 @@ __global__ void __launch_bounds__(IG_BLOCK) k_ingest_mark(const void *__restrict
             }
         }
         if (keep && sp.has_mask) {
-            const int64_t pix = ang2pix_ring_dev(sp.mask_nside, th, ph);
+            int64_t pix = -1;
+            if (cart) {
+                if (small) {
+                    float t = atan2f((float)b, (float)a) * 0.63661977f;
+                    if (t < 0.f) t += 4.f;
+                    const float rho = sqrtf((float)a * (float)a + (float)b * (float)b);
+                    pix = ang2pix_ring_fast(sp.mask_nside, (float)c / rf, rho / rf, t);
+                }
+                if (pix < 0) {
+                    double th, ph;
+                    record_angles(a, b, c, th, ph);
+                    pix = ang2pix_ring_dev(sp.mask_nside, th, ph);
+                }
+            } else {
+                pix = ang2pix_ring_any(sp.mask_nside, b, c);
+            }
             if (pix < 0) {
                 atomicOr(err, 2);
                 keep = 0;
@@ -120,27 +146,25 @@ __global__ void __launch_bounds__(IG_BLOCK) k_ingest_mark(const void *__restrict
                 keep = 0;
             }
         }
-        tmp[3 * i] = r;
-        tmp[3 * i + 1] = th;
-        tmp[3 * i + 2] = ph;
         keepv[i] = (uint8_t)keep;
     }
     const int cnt = __syncthreads_count(keep);
     if (threadIdx.x == 0) bcount[blockIdx.x] = (uint32_t)cnt;
 }
 
-// kept records to out[boff[block] + rank within the block], input order
-__global__ void __launch_bounds__(IG_BLOCK) k_ingest_scatter(const double *__restrict__ tmp,
+// kept records, converted, to out[boff[block] + rank within the block], input order: a thread per kept record
+__global__ void __launch_bounds__(IG_BLOCK) k_ingest_scatter(const void *__restrict__ rec, uint32_t layout,
                                                               const uint8_t *__restrict__ keepv, int64_t n,
                                                               const uint32_t *__restrict__ boff,
                                                               double *__restrict__ out) {
     __shared__ uint32_t wsum[IG_BLOCK / 32];
-    const int64_t i = blockIdx.x * (int64_t)IG_BLOCK + threadIdx.x;
-    const int keep = (i < n) ? keepv[i] : 0;
+    __shared__ uint16_t kept[IG_BLOCK];
+    const int64_t i0 = blockIdx.x * (int64_t)IG_BLOCK;
+    const int keep = (i0 + threadIdx.x < n) ? keepv[i0 + threadIdx.x] : 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned bal = __ballot_sync(0xffffffffu, keep);
     if (lane == 0) wsum[warp] = __popc(bal);
-    __syncthreads();
+    const int cnt = __syncthreads_count(keep);
     if (warp == 0) {  // exclusive scan of the 32 warp counts
         const uint32_t v = wsum[lane];
         uint32_t s = v;
@@ -151,13 +175,18 @@ __global__ void __launch_bounds__(IG_BLOCK) k_ingest_scatter(const double *__res
         wsum[lane] = s - v;
     }
     __syncthreads();
-    if (keep) {
-        const uint64_t dst = (uint64_t)boff[blockIdx.x] + wsum[warp] + __popc(bal & ((1u << lane) - 1u));
-        out[3 * dst] = tmp[3 * i];
-        out[3 * dst + 1] = tmp[3 * i + 1];
-        out[3 * dst + 2] = tmp[3 * i + 2];
-    }
+    if (keep) kept[wsum[warp] + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)threadIdx.x;
+    __syncthreads();
+    if ((int)threadIdx.x >= cnt) return;
+    double a, b, c;
+    load_record(rec, layout, i0 + kept[threadIdx.x], a, b, c);
+    double *o = out + 3 * ((uint64_t)boff[blockIdx.x] + threadIdx.x);
+    o[0] = record_radius(layout, a, b, c);
+    if (layout & CATANA_REC_CARTESIAN) record_angles(a, b, c, b, c);
+    o[1] = b;
+    o[2] = c;
 }
+static_assert(IG_BLOCK / 32 == 32, "k_ingest_scatter: one warp scans the warps' counts");
 
 bool spec_valid(const catana_ingest_t &s, std::string &why) {
     if (s.layout & ~(CATANA_REC_FLOAT32 | CATANA_REC_CARTESIAN)) {
@@ -195,16 +224,15 @@ catana_status_t ingest_dev(DeviceContext *ctx, const void *rec_dev, int64_t n, c
     if (n <= 0) return CATANA_OK;
     const int64_t nb = (n + IG_BLOCK - 1) / IG_BLOCK;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t tb = al((size_t)n * 3 * sizeof(double)), kb = al((size_t)n), cb = al((size_t)(nb + 1) * 4),
+    const size_t kb = al((size_t)n), cb = al((size_t)(nb + 1) * 4),
                  wb = spec.window ? al((size_t)spec.window_n * sizeof(double)) : 0,
                  mb = spec.mask ? al((size_t)12 * spec.mask_nside * spec.mask_nside * sizeof(float)) : 0;
-    CG_CUDA_TRY(ctx->ingest_ws.ensure(tb + kb + cb + wb + mb + 256));
+    CG_CUDA_TRY(ctx->ingest_ws.ensure(kb + cb + wb + mb + 256));
     char *w = ctx->ingest_ws.as<char>();
-    double *tmp = reinterpret_cast<double *>(w);
-    uint8_t *keepv = reinterpret_cast<uint8_t *>(w + tb);
-    uint32_t *cnt = reinterpret_cast<uint32_t *>(w + tb + kb);
-    double *win = reinterpret_cast<double *>(w + tb + kb + cb);
-    float *msk = reinterpret_cast<float *>(w + tb + kb + cb + wb);
+    uint8_t *keepv = reinterpret_cast<uint8_t *>(w);
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(w + kb);
+    double *win = reinterpret_cast<double *>(w + kb + cb);
+    float *msk = reinterpret_cast<float *>(w + kb + cb + wb);
     IngestDev sp;
     memset(&sp, 0, sizeof(sp));
     sp.layout = spec.layout;
@@ -235,12 +263,12 @@ catana_status_t ingest_dev(DeviceContext *ctx, const void *rec_dev, int64_t n, c
     int *err = reinterpret_cast<int *>(ctx->misc.as<char>() + 128);
     CG_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
     CG_CUDA_TRY(cudaMemsetAsync(cnt + nb, 0, sizeof(uint32_t), st));
-    k_ingest_mark<<<(unsigned)nb, IG_BLOCK, 0, st>>>(rec_dev, n, sp, tmp, keepv, cnt, err);
+    k_ingest_mark<<<(unsigned)nb, IG_BLOCK, 0, st>>>(rec_dev, n, sp, keepv, cnt, err);
     count_launch();
     CG_CUDA_TRY(cudaGetLastError());
     catana_status_t s = scan_u32(cnt, nb + 1, st);
     if (s != CATANA_OK) return s;
-    k_ingest_scatter<<<(unsigned)nb, IG_BLOCK, 0, st>>>(tmp, keepv, n, cnt, out_dev);
+    k_ingest_scatter<<<(unsigned)nb, IG_BLOCK, 0, st>>>(rec_dev, sp.layout, keepv, n, cnt, out_dev);
     count_launch();
     CG_CUDA_TRY(cudaGetLastError());
     uint32_t tot = 0;

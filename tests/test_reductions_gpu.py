@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import catana_gb300 as catana
+from catana_gb300 import _lib
 from oracle import oracle as O
 from conftest import uniform_ball
 
@@ -62,3 +63,48 @@ def test_bin_offsets(cuda_device, nside, n, spread):
     offs, rs = O.bin_points(nside, pts)
     assert np.array_equal(ppc.offsets, offs)
     assert np.array_equal(ppc.r_sorted, rs)
+
+
+def _pixels(nside, pts):
+    """The FP64 form on the device."""
+    pix = np.zeros(len(pts), dtype=np.int64)
+    th, ph = np.ascontiguousarray(pts[:, 1]), np.ascontiguousarray(pts[:, 2])
+    _lib.check(_lib.lib.catana_gpu_ang2pix_ring(nside, _lib.ptr(th), _lib.ptr(ph), len(pts), _lib.ptr(pix), None))
+    return pix
+
+
+# pixels by FP32 where that settles them: the smallest nside, ordinary ones, the largest it takes and one past
+@pytest.mark.parametrize("nside", [1, 2, 64, 1024])
+def test_pixels_settled_in_fp32(cuda_device, nside):
+    n = 200000
+    rng = np.random.default_rng(nside)
+    pts = uniform_ball(n, 1000.0, seed=nside)
+    k = n // 8
+    pts[:k, 1] = np.arccos(np.clip(rng.integers(-3, 4, k) / 3.0 + rng.choice([0, 1e-9, -1e-7, 3e-6], k), -1, 1))
+    pts[k:2 * k, 2] = (np.pi / 2) * rng.integers(-4, 9, k) / 2.0 ** rng.integers(0, 7, k)
+    pts[2 * k:3 * k, 2] += rng.choice([-4 * np.pi, 2 * np.pi, 100.0], k)
+    pix = _pixels(nside, pts)
+    ppc = catana.PixelizedPointContainer(nside, catana.PointContainer(pts))
+    assert np.array_equal(np.diff(ppc.offsets), np.bincount(pix, minlength=12 * nside * nside))
+    assert np.array_equal(ppc.r_sorted, pts[np.argsort(pix, kind="stable"), 0])
+
+
+@pytest.mark.parametrize("nside,cartesian,f32", [(4, True, True), (64, True, False), (64, False, True), (512, True, True),
+                                                 (2048, True, False)])
+def test_ingest_mask_settled_in_fp32(cuda_device, nside, cartesian, f32):
+    n = 150000
+    rng = np.random.default_rng(nside)
+    pts = uniform_ball(n, 1000.0, seed=nside + 1)
+    rec = pts
+    if cartesian:
+        st = np.sin(pts[:, 1])
+        rec = pts[:, :1] * np.stack([st * np.cos(pts[:, 2]), st * np.sin(pts[:, 2]), np.cos(pts[:, 1])], 1)
+        rec[:1000, rng.integers(0, 3)] = 0.0
+        rec[1000:1100] *= 1e-25
+        rec[0] = 0.0
+    rec = rec.astype(np.float32) if f32 else np.ascontiguousarray(rec)
+    mask = rng.integers(0, 2, 12 * nside * nside).astype(np.float32)
+    kind = "cartesian" if cartesian else "spherical"
+    got = np.asarray(catana.ingest(rec, kind, mask=mask, tophat_r0=900.0))
+    ref = np.asarray(catana.ingest(rec, kind, tophat_r0=900.0))
+    assert np.array_equal(got, ref[mask[_pixels(nside, ref)] == 1.0])
