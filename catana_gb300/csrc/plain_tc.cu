@@ -27,7 +27,7 @@
 //     Y = the upper half of a 64 x 64-bit integer product;
 //   * j_l from the reference's linear table (SBesselInterpolator.cpp:10-26): the table position
 //     k r / dx is a 64 x 64-bit integer product, the interpolation one FP64 FMA on (y0 - dy, dy);
-//     or, in the other j_l modes, read from an array that another kernel filled.
+//     or, in the other j_l modes and for pixelized catalogs, read from an array that another kernel filled.
 // FP64 work: 3 operations per (point, m) and (point, n) instead of 2 nmax (l + 1).
 //
 // Schedule: one CTA per slab walks every level of the launch (its Legendre rows are its own, so

@@ -17,7 +17,7 @@
 // FP32 round-to-nearest adds on the CUDA cores (the tensor core's own FP32
 // accumulation drifts measurably over long chains), and every FLUSH_FOLDS tiles adds
 // D_acc into the CTA's FP32 partial in global memory.  k_split_reduce sums the slab
-// partials in FP64 in fixed order and applies k_ln.
+// partials as three FP32 words each (closer than FP64), in fixed order, and applies k_ln.
 //
 // Operand generation (CUDA cores, FP32 with float-float inputs):
 //   * j_l from a per-l piecewise degree-6 polynomial on unit intervals of z = k r
