@@ -533,7 +533,7 @@ def next_rows_workload(torch, _lib, catana):
     dt = time.perf_counter() - t0
     res["ingest_8M_float32_cartesian"] = {"records_per_s": n / dt, "seconds": dt, "kept": len(kept),
                                           "note": "host API incl. 96 MB H2D and the kept points D2H",
-                                          "device_bytes_per_record": 12 + 24 + 1 + 24 + 1}
+                                          "device_bytes_per_record": 12 + 1 + 1 + 12 + 24}
     # integrals
     rmax = 1000.0
     fi = catana.FunctionInterpolator(lambda r: np.exp(-(r / 400.0) ** 2) * r ** 2, 10001, 0.0, rmax)
@@ -548,8 +548,8 @@ def next_rows_workload(torch, _lib, catana):
         total += k1.size
     dt = time.perf_counter() - t0
     res["shot_noise_integrals_l32_n32"] = {"integrals": total, "seconds": dt, "integrals_per_s": total / dt,
-                                           "note": "one warp per pair, 32/8-point Gauss-Legendre between the zeros "
-                                                   "and the window's nodes; host API incl. copies"}
+                                           "note": "one quadrature for all pairs of a call, j_l once per distinct k "
+                                                   "and node; host API incl. copies"}
     return res
 
 
