@@ -134,6 +134,7 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
 // The same sum with its contraction on the tensor cores (plain_tc.cu), where the device has them and
 // lmax <= 512; with JL_MODE_POLY the caller has prepared ctx->poly and passes the largest radius (else rtop = 0).
 bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax);
+bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl);  // and whether it is the faster one
 catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
                                     int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, double rtop,
                                     const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st);

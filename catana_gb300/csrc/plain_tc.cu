@@ -1208,6 +1208,19 @@ bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
            rmax < 1e100;
 }
 
+// Few points with many radial orders, or one or two levels: a CTA of the tensor-core kernel walks its blocks of 64
+// radial orders one after the other, 13 to 15 us each, where the FP64 path has a CTA for each and takes 40 us a
+// level (80 without the linear table, of 64 radial orders and more) and its FP64 work.  Microseconds a call, FP64 path / here:
+// 500 points, l 16: n 64 over 600 / 290, n 200 646 / 765, n 1000 955 / 3849; 2000 points, l 8: n 200 faster here,
+// n 400 728 / 750, n 1000 1266 / 1819; 1 point, l 1, n 1 79 / 94; 8000 points, l 1, n 64 139 / 151, l 2 faster here.
+bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl) {
+    if (npoints > 8192 || lmax > 64) return true;
+    const bool lerp = jl == JL_MODE_LERP;
+    const double nb = (nmax + 63) / 64, work = (double)npoints * 64.0 * nb;
+    const double fp64 = lmax * ((lerp ? 40.0 : 40.0 + 0.625 * std::min(nmax, 64)) + work * (2.8e-5 + 3.4e-6 * (lmax + 1)));
+    return (lerp ? 60.0 : 100.0) + (13.0 + 1e-3 * (double)npoints) * nb * lmax < fp64;
+}
+
 namespace {
 
 // pix == nullptr: points_dev are npoints x 3; otherwise the pixelized catalog.  "Points" below are what the main

@@ -114,3 +114,16 @@ def test_pixelized_cells(cuda_device, nside, counts, interpolated):
     k, c, f = O.sfb_healpix(nside, offs, r, 9, 11, 1000.0, interpolated=interpolated)
     for l, (a, b) in enumerate(zip(res.f_lmn, f)):
         assert np.max(np.abs(a - b)) <= TOL * max(np.max(np.abs(b)), 1e-6 * np.max(np.abs(f[0]))), l
+
+
+@pytest.mark.parametrize("n,lmax,nmax", [(1, 1, 1), (40, 2, 1), (500, 8, 64), (500, 8, 193), (2000, 4, 300), (8192, 1, 64), (8193, 1, 64),
+                                         (100, 64, 200), (100, 65, 200)])
+@pytest.mark.parametrize("interp", ["on", "off"])
+def test_small_catalogs_either_path(cuda_device, n, lmax, nmax, interp):
+    """Both sides of the rule that leaves few points with many radial orders to the FP64 path."""
+    pts = uniform_ball(n, 1000.0, seed=n + nmax)
+    res = catana.sfb_decomposition(catana.PointContainer(pts), lmax, nmax, 1000.0, True, False, interpolation=interp)
+    keep = min(lmax, 6)  # the oracle's levels
+    k, c, f = O.sfb_raw(pts, keep, nmax, 1000.0, interpolated=interp == "on")
+    for l in range(keep):
+        assert np.max(np.abs(res.f_lmn[l] - f[l])) <= 1e-10 * max(np.max(np.abs(f[0])), np.max(np.abs(f[l])))
