@@ -750,18 +750,20 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
     if (!isfinite(wv)) bad |= TC_POISON_W;
     const bool rbad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
     if (rbad && !lerp) bad |= TC_POISON_W;
+    // An angle that is not finite spoils the modes that it enters (k_ptc_reduce makes them NaN); the others, l = 0
+    // for theta and m = 0 for phi, keep the point.
+    const bool use = in && !(bad & TC_POISON_W) && !rbad;
     const double ct = cos(th);
-    const bool use = in && !bad && !rbad;
     if (blockIdx.y == 0) {
         if (in && bad) atomicOr(poison, bad);
         if (in && rbad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
         rint[i] = rbad || !(fabs(r) < ldexp(1.0, er)) ? 0ull : (uint64_t)(int64_t)ldexp(fmax(r, 0.0), 62 - er);
         rabs[i] = r;
-        xs[i] = use ? make_double2(ct, sqrt((1.0 - ct) * (1.0 + ct))) : make_double2(0.0, 0.0);
+        xs[i] = use && !(bad & TC_POISON_THETA) ? make_double2(ct, sqrt((1.0 - ct) * (1.0 + ct))) : make_double2(0.0, 0.0);
     }
     const double scale = ldexp(1.0, 58 - slab[t / tslab].ew);
     if (!use) wv = 0.0;
-    const double phi = use ? ph : 0.0;
+    const double phi = use && !(bad & TC_POISON_PHI) ? ph : 0.0;
     // frac(phi / 2 pi) 2^64 (mod 2^64), 1 / 2 pi as a pair of doubles: rounded at 2^-64 of a turn
     const double p = phi * 0.15915494309189535, pl = fma(phi, 0.15915494309189535, -p) - phi * 9.839338337591243e-18;
     const double f = p - floor(p);
