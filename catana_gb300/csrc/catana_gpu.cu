@@ -627,7 +627,7 @@ catana_status_t catana_gpu_sfb_raw(const double *points, const double *weights, 
         return CATANA_ERR_DOMAIN;
     }
     if (err_h != 0) {
-        set_error("split kernel reported a timed-out wait");
+        set_error("a kernel reported a timed-out wait");
         return CATANA_ERR_CUDA;
     }
     return CATANA_OK;
@@ -716,7 +716,7 @@ catana_status_t catana_gpu_sfb_raw_batched(const catana_catalog_t *cats, int32_t
         return CATANA_ERR_DOMAIN;
     }
     if (err_h != 0) {
-        set_error("split kernel reported a timed-out wait");
+        set_error("a kernel reported a timed-out wait");
         return CATANA_ERR_CUDA;
     }
     return CATANA_OK;

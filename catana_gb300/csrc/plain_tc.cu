@@ -44,6 +44,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -110,6 +111,8 @@ struct TcArgs {
     uint32_t *maxq;             // [slab][3][TC_LMAX]: level maxima between launches
     double *partial;            // [slab][l - l0][n][2 (l + 1)]
     int64_t pslab;              // doubles per slab in partial
+    uint64_t wait_ns;           // limit of every wait
+    int stall;                  // test hook: withhold the first tile's hand-off of every CTA
     int *err;
 };
 
@@ -246,7 +249,7 @@ template <bool LERP>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
     extern __shared__ uint8_t tc_smem[];
     uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(tc_smem) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t full[2], empty[2], gdone[2], dfree[2];
+    __shared__ uint64_t full[2], empty[2], gdone[2], dfree[2], drain;
     __shared__ uint32_t tmem_sh;
     __shared__ int abort_sh;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -265,6 +268,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
             tc05::mbar_init(&gdone[b], 1);
             tc05::mbar_init(&dfree[b], alt ? 256 : 128);
         }
+        tc05::mbar_init(&drain, 1);
         abort_sh = 0;
     }
     // level maxima carried over from the launch before (levels l0 - 1, l0 - 2)
@@ -275,10 +279,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
     __syncthreads();
     tc05::fence_after();
     const uint32_t tmem = tmem_sh;
-    // a bounded wait; once one ran out every later wait of the CTA returns at once
+    // a bounded wait; once one ran out every later wait of the warp returns at once, those of the others once
+    // they have to wait at all, and the roles walk on to their ends.  Each warp whose wait ran out reports it.
     auto wait = [&](uint64_t *bar, uint32_t parity, bool &dead) {
         if (dead || __all_sync(0xffffffffu, tc05::mbar_try(bar, parity))) return;
-        dead = __any_sync(0xffffffffu, *abort_v || !tc05::mbar_wait(bar, parity, TC_WAIT_NS));
+        dead = __any_sync(0xffffffffu, *abort_v || !tc05::mbar_wait(bar, parity, a.wait_ns));
         if (dead) *abort_v = 1;
     };
 
@@ -467,9 +472,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                 } else if (!mine) {
                     wait(&empty[bf], (it - 1) & 1, dead);
                 }
-                if (lane == 0) tc_arrive(&full[bf]);
+                if (lane == 0 && !(a.stall && warp == 0 && use == 1)) tc_arrive(&full[bf]);
             }
         });
+        if (dead && lane == 0) *a.err = CATANA_ERR_CUDA;
         op_bar();
         for (int k = tid; k < 3 * TC_LMAX; k += TC_OPT) a.maxq[(size_t)slab * 3 * TC_LMAX + k] = s_mx[k];
     } else if (warp < TC_FOLD0) {
@@ -517,13 +523,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                 ++groups;
             }
         });
-        // MMAs still in flight land before the tensor memory is released
-        if (dead)
-            for (uint32_t bf = 0; bf < 2; ++bf) {
-                const uint32_t n = (use + 1 - bf) >> 1;
-                if (n > 0) tc05::mbar_wait(&empty[bf], (n - 1) & 1, TC_WAIT_NS);
-            }
-        if (dead && lane == 0) *a.err = CATANA_ERR_CUDA;
+        // Whatever was issued lands before the block's memory goes, also where a role gave up (bounded by the
+        // drain limit, not by the possibly shortened limit of the waits above).
+        if (lane == 0) {
+            tc05::commit(&drain);
+            tc05::mbar_wait(&drain, 0, TC_WAIT_NS);
+            if (dead) *a.err = CATANA_ERR_CUDA;
+        }
+        __syncwarp();
     } else {
         uint32_t groups = 0;  // groups folded
         bool dead = false;
@@ -1223,6 +1230,8 @@ bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl) {
     return (lerp ? 60.0 : 100.0) + (13.0 + 1e-3 * (double)npoints) * nb * lmax < fp64;
 }
 
+std::atomic<uint64_t> g_plain_stall_ns{0};
+
 namespace {
 
 // pix == nullptr: points_dev are npoints x 3; otherwise the pixelized catalog.  "Points" below are what the main
@@ -1230,6 +1239,8 @@ namespace {
 catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, const PixelCatalog *pix,
                               int64_t nall, int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
                               double *f_acc_dev, int *err_dev, cudaStream_t st) {
+    // the test hook (catana_gpu_test_plain_stall) arms one run
+    const uint64_t stall_ns = g_plain_stall_ns.exchange(0);
     const bool lerp = jl == JL_MODE_LERP, fused = lerp && !pix;  // fused: the main kernel evaluates j_l itself
     int64_t npoints = nall;  // an upper bound of a pixelized catalog's entries, until they are counted
     catana_status_t s = ensure_tc_coefs(ctx, lmax, st);
@@ -1356,6 +1367,8 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         a.npts = 1000 * nmax;
         a.maxq = reinterpret_cast<uint32_t *>(ws + o_mx);
         a.err = err_dev;
+        a.wait_ns = stall_ns ? stall_ns : TC_WAIT_NS;
+        a.stall = stall_ns ? 1 : 0;
         a.tab = nullptr;
         const double *dxinv = nullptr;
         if (lerp) {
@@ -1442,3 +1455,12 @@ catana_status_t plain_tc_pixels(DeviceContext *ctx, const PixelCatalog &pix, int
 }
 
 }  // namespace catana_gpu
+
+extern "C" catana_status_t catana_gpu_test_plain_stall(uint32_t wait_us) {
+    if (wait_us < 1 || wait_us > 1000000) {
+        catana_gpu::set_error("test_plain_stall: wait_us must be in [1, 1000000]");
+        return CATANA_ERR_ARG;
+    }
+    catana_gpu::g_plain_stall_ns.store((uint64_t)wait_us * 1000ull);
+    return CATANA_OK;
+}

@@ -442,7 +442,7 @@ catana_status_t catana_gpu_accum_finish(catana_gpu_accum_t acc, double *k_ln, do
         return CATANA_ERR_DOMAIN;
     }
     if (err_h != 0) {
-        set_error("split kernel reported a timed-out wait");
+        set_error("a kernel reported a timed-out wait");
         return CATANA_ERR_CUDA;
     }
     return CATANA_OK;

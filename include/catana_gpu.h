@@ -346,6 +346,10 @@ catana_status_t catana_gpu_fp64_peak(int32_t ms, double *tflops);
  * which the entry point returns; the context stays usable.  wait_us in [1, 1e6]. */
 catana_status_t catana_gpu_test_split_stall(uint32_t wait_us);
 
+/* The same for the plain form's tensor-core kernel (raw, batched, streamed and HEALPix
+ * calls): arms the next run that takes it. */
+catana_status_t catana_gpu_test_plain_stall(uint32_t wait_us);
+
 /* Message of the last failing call on this thread ("" if none). */
 const char *catana_gpu_last_error(void);
 
