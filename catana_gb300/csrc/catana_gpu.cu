@@ -944,6 +944,10 @@ catana_status_t catana_gpu_sfb_healpix(int64_t nside, const int64_t *pix_offsets
         set_error("argument (z) outside of defined range.");
         return CATANA_ERR_DOMAIN;
     }
+    if (err_h != 0) {
+        set_error("a kernel reported a timed-out wait");
+        return CATANA_ERR_CUDA;
+    }
     return CATANA_OK;
 }
 

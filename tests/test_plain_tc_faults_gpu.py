@@ -38,6 +38,13 @@ def _raw(**kw):
     return lambda: catana.sfb_decomposition(catana.PointContainer(pts), 12, 20, 1000.0, True, False, interpolation="on", **kw)
 
 
+def _healpix(reverse):
+    ppc = catana.PixelizedPointContainer(8, catana.PointContainer(uniform_ball(3000, 1000.0, seed=5)))
+    if reverse:
+        return lambda: catana.sfb_reverse(ppc, 12, 20, 1000.0, True, False, interpolated=True)
+    return lambda: catana.sfb_decomposition(ppc, 12, 20, 1000.0, True, False)
+
+
 def _accumulator():
     pts = uniform_ball(3000, 1000.0, seed=5)
 
@@ -55,7 +62,8 @@ def _batched():
                                                     precision="plain")[0]
 
 
-@pytest.mark.parametrize("make", [_raw, _accumulator, _batched], ids=["raw", "accumulator", "batched"])
+@pytest.mark.parametrize("make", [_raw, lambda: _healpix(False), lambda: _healpix(True), _accumulator, _batched],
+                         ids=["raw", "healpix", "reverse", "accumulator", "batched"])
 def test_a_wait_that_runs_out_is_an_error(cuda_device, make):
     """The hook withholds one hand-off of the tensor-core kernel and cuts its waits to 3 ms: the call says so
     instead of returning what the kernel left, and the same call again is as before."""
