@@ -192,6 +192,18 @@ DeviceContext *get_context(int *status) {
     return p.get();
 }
 
+WsOrder::WsOrder(DeviceContext *ctx, cudaStream_t st) : ctx_(ctx), st_(st) {
+    err = ctx->ws_event ? cudaStreamWaitEvent(st, ctx->ws_event, 0)
+                        : cudaEventCreateWithFlags(&ctx->ws_event, cudaEventDisableTiming);
+}
+
+WsOrder::~WsOrder() {
+    // not into a capture: an event recorded there cannot be waited for outside it (such a call has failed anyway)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st_, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+        cudaEventRecord(ctx_->ws_event, st_);
+}
+
 }  // namespace catana_gpu
 
 using namespace catana_gpu;
@@ -274,6 +286,8 @@ catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double
                            int nmax, double rmax, uint32_t flags, double *kln_d, double *cln_d, double *f_d,
                            int *err_d, cudaStream_t st) {
     const bool split = (flags & CATANA_FORM_MASK) == CATANA_FORM_SPLIT;
+    WsOrder ws_order(ctx, st);
+    CG_CUDA_TRY(ws_order.err);
     // k_ln on the host (cached zeros), then to the device
     std::vector<double> kh((size_t)lmax * nmax);
     kln_table(lmax, nmax, rmax, kh.data());
@@ -366,6 +380,8 @@ catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats,
         set_error("the split (tcgen05) form needs an sm_103 device");
         return CATANA_ERR_UNSUPPORTED;
     }
+    WsOrder ws_order(ctx, st);
+    CG_CUDA_TRY(ws_order.err);
     // k_ln (host, cached zeros) and zeroed accumulators; internal f where none is given
     size_t fin = 0;
     for (int c = 0; c < ncat; ++c)

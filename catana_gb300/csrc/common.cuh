@@ -80,7 +80,7 @@ struct DeviceContext {
     double split_last_waves = 0.0;
     int split_last_mblk = 0;
     cudaStream_t capture_stream = nullptr;      // stream the split level loop is captured on
-    cudaEvent_t split_ws_event = nullptr;       // end of the last split or plain run (orders workspace reuse across streams)
+    cudaEvent_t ws_event = nullptr;             // end of the last call's work (WsOrder)
     DevBuf hp_ws;      // HEALPix workspace
     DevBuf ingest_ws;  // ingest: converted records, keep flags, block counts, window, mask
     // kernels whose shared-memory limit this device's context has raised (the
@@ -105,6 +105,24 @@ struct DeviceContext {
 };
 
 DeviceContext *get_context(int *status);
+
+// The workspaces and the cached tables of a context serve every stream that computes on its device, and calls on
+// device arrays return before their work is done.  An entry point holds one of these, under the context's mutex,
+// from before it touches any of them -- a table that is built for another nmax overwrites the one that an earlier
+// call still reads -- until all of its work is enqueued: its stream then waits for the work of the call before
+// it, and the next one's for its own.
+class WsOrder {
+public:
+    WsOrder(DeviceContext *ctx, cudaStream_t st);
+    ~WsOrder();
+    WsOrder(const WsOrder &) = delete;
+    WsOrder &operator=(const WsOrder &) = delete;
+    cudaError_t err;  // of the wait
+
+private:
+    DeviceContext *ctx_;
+    cudaStream_t st_;
+};
 
 // Bessel zeros (host, cached): z[l][n] for n < count.  Thread-safe.
 const double *zeros_for(unsigned l, int count);

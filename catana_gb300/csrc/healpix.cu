@@ -630,6 +630,8 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
         set_error("HEALPix path supports nside <= 1024");
         return CATANA_ERR_ARG;
     }
+    WsOrder ws_order(ctx, st);
+    CG_CUDA_TRY(ws_order.err);
     catana_status_t s = ensure_rings(nside, st);
     if (s != CATANA_OK) return s;
     RingTables &R = g_rings;

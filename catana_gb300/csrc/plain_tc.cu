@@ -1283,9 +1283,6 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     const int max_slabs = ctx->sm_count * ceil_div(tiles_c, (int64_t)ctx->sm_count * TC_SLAB_TILES);
     const size_t o_mx = o_sl + tc_al((size_t)max_slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)max_slabs * 3 * TC_LMAX * 4);
     CG_CUDA_TRY(ctx->tc_ws.ensure(o_poi + 256 + phb));
-    // the workspace is shared by every stream that runs the plain or the split form on this device
-    if (!ctx->split_ws_event) CG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->split_ws_event, cudaEventDisableTiming));
-    else CG_CUDA_TRY(cudaStreamWaitEvent(st, ctx->split_ws_event, 0));
     char *ws = ctx->tc_ws.as<char>();
     uint32_t *keys = reinterpret_cast<uint32_t *>(ws), *perm = reinterpret_cast<uint32_t *>(ws + kb);
     uint32_t *tk = reinterpret_cast<uint32_t *>(ws + 2 * kb), *tv = reinterpret_cast<uint32_t *>(ws + 3 * kb);
@@ -1436,7 +1433,6 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             l0 = l1;
         }
     }
-    CG_CUDA_TRY(cudaEventRecord(ctx->split_ws_event, st));
     return CATANA_OK;
 }
 

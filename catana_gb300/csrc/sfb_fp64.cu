@@ -532,9 +532,6 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
     if (plain_tc_takes(ctx, lmax, nmax, rmax) && plain_tc_pays(npoints, lmax, nmax, jl))
         return plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, rtop, kln_dev,
                                    f_acc_dev, err_dev, st);
-    // the workspaces are shared by every stream that runs a raw form on this device
-    if (!ctx->split_ws_event) CG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->split_ws_event, cudaEventDisableTiming));
-    else CG_CUDA_TRY(cudaStreamWaitEvent(st, ctx->split_ws_event, 0));
     // Chunk so that the three Legendre rows stay under ~1.5 GB.
     int64_t chunk = (int64_t)(1.5e9 / (3.0 * 8.0 * std::max(lmax, 1)));
     chunk = std::max<int64_t>(1024, std::min<int64_t>(chunk, npoints));
@@ -625,7 +622,6 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
             st0 = t;
         }
     }
-    CG_CUDA_TRY(cudaEventRecord(ctx->split_ws_event, st));
     return CATANA_OK;
 }
 

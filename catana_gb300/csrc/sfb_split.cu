@@ -1649,9 +1649,6 @@ catana_status_t split_run(DeviceContext *ctx, std::vector<SplitCatInput> &cats_i
     const int nc = (int)cats.size();
     CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)16 * nc));
     unsigned long long *mx = ctx->cat_scratch.as<unsigned long long>();
-    // the workspace is shared by every stream that runs the split form on this device
-    if (!ctx->split_ws_event) CG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->split_ws_event, cudaEventDisableTiming));
-    else CG_CUDA_TRY(cudaStreamWaitEvent(st, ctx->split_ws_event, 0));
     bool need = false;
     for (auto &P : cats) need |= (P.in.max_r < 0.0 || P.in.max_w < 0.0);
     std::vector<unsigned long long> mxh(2 * nc, 0ull);
@@ -2141,7 +2138,6 @@ catana_status_t split_run(DeviceContext *ctx, std::vector<SplitCatInput> &cats_i
         }
         // the next group reuses the workspace: stream order on `st` keeps them apart
     }
-    CG_CUDA_TRY(cudaEventRecord(ctx->split_ws_event, st));
     return CATANA_OK;
 }
 

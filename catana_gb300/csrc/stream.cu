@@ -116,6 +116,8 @@ catana_status_t accum_add(Accum *A, const T *points, const T *weights, int64_t n
     const T *pd = reinterpret_cast<const T *>(dst);
     const T *wd = weights ? reinterpret_cast<const T *>(dst + ((pb + 255) & ~size_t(255))) : nullptr;
     int *err_d = A->err.as<int>();
+    WsOrder ws_order(ctx, A->comp_st);
+    CG_CUDA_TRY(ws_order.err);
     catana_status_t s = CATANA_OK;
     if (A->split) {
         if (ctx->cc_major != 10 || ctx->cc_minor != 3) {
@@ -205,6 +207,8 @@ catana_status_t accum_add_records(Accum *A, const void *records, int64_t n, cons
     CG_CUDA_TRY(cudaMemcpyAsync(A->slot[k].ptr, records, rb, cudaMemcpyHostToDevice, A->copy_st));
     CG_CUDA_TRY(cudaEventRecord(A->copied[k], A->copy_st));
     CG_CUDA_TRY(cudaStreamWaitEvent(A->comp_st, A->copied[k], 0));
+    WsOrder ws_order(ctx, A->comp_st);
+    CG_CUDA_TRY(ws_order.err);
     int64_t kept = 0;
     double *pts = A->slot64[k].as<double>();
     catana_status_t s = ingest_dev(ctx, A->slot[k].ptr, n, spec, pts, &kept, A->comp_st);

@@ -81,3 +81,55 @@ def test_a_wait_that_runs_out_is_an_error(cuda_device, make):
 def test_stall_hook_validates_its_argument():
     assert _lib.lib.catana_gpu_test_plain_stall(0) == _lib.ERR_ARG
     assert _lib.lib.catana_gpu_test_plain_stall(2000000) == _lib.ERR_ARG
+
+
+def _interleaved(shapes, chunks, interp):
+    """Accumulators of unlike nmax fed in turn: each one's table replaces the others' in the shared cache."""
+    accs = [catana.SFBAccumulator(lmax, nmax, rmax, precision="plain", interpolation=interp) for lmax, nmax, rmax in shapes]
+    for c in chunks:
+        for a in accs:
+            a.add(c)
+    out = [a.finish(store_flmn=True) for a in accs]
+    for a in accs:
+        a.close()
+    return out
+
+
+@pytest.mark.parametrize("interp,shapes", [("on", [(24, 64, 1000.0), (24, 32, 1000.0), (9, 48, 1000.0)]),
+                                           ("poly", [(24, 40, 1000.0), (40, 64, 700.0), (30, 90, 500.0)])])
+def test_calls_on_different_streams_share_the_tables(cuda_device, interp, shapes):
+    """Each accumulator computes on a stream of its own and returns from add() before its work is done; a
+    table built for the next one must wait for that work.  Against the same points in one call, the sums in another
+    order: 1e-12 of the level's largest |f|."""
+    chunks = [uniform_ball(30000, 500.0, seed=k) for k in range(3)]
+    for (lmax, nmax, rmax), got in zip(shapes, _interleaved(shapes, chunks, interp)):
+        one = catana.sfb_decomposition(catana.PointContainer(np.concatenate(chunks)), lmax, nmax, rmax, True, False,
+                                       interpolation=interp)
+        for l in range(lmax):
+            assert np.max(np.abs(got.f_lmn[l] - one.f_lmn[l])) <= 1e-12 * np.max(np.abs(one.f_lmn[l])), (nmax, l)
+
+
+def test_raw_calls_on_two_streams(cuda_device):
+    """catana_gpu_sfb_raw_dev without weights returns at once: two streams with unlike nmax, in turn, without a
+    place for f_lmn of their own."""
+    torch = pytest.importorskip("torch")
+    pts = torch.from_numpy(uniform_ball(60000, 1000.0, seed=1)).cuda()
+    shapes = [(32, 64), (32, 20)]
+    streams = [torch.cuda.Stream() for _ in shapes]
+
+    def call(lmax, nmax, st):
+        k, c = (torch.zeros(lmax * nmax, dtype=torch.float64, device="cuda") for _ in range(2))
+        torch.cuda.current_stream().synchronize()  # zeroed on the default stream
+        p = [t.data_ptr() for t in (pts, k, c)]
+        _lib.check(_lib.lib.catana_gpu_sfb_raw_dev(p[0], None, 60000, lmax, nmax, 1000.0, _lib.JL_INTERP, p[1], p[2], None, None,
+                                                   st.cuda_stream))
+        return k, c  # both are held until the work is done
+
+    ref = []
+    for s, st in zip(shapes, streams):
+        ref.append(call(*s, st))
+        torch.cuda.synchronize()
+    for _ in range(3):
+        got = [call(*s, st) for s, st in zip(shapes, streams)]
+        torch.cuda.synchronize()
+        assert all(torch.equal(a[1], b[1]) for a, b in zip(got, ref))
