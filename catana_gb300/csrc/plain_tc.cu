@@ -817,10 +817,11 @@ __global__ void k_ptc_cells(TcPixels px, int64_t n, double inv_rmax, int er, int
                             uint32_t *__restrict__ vals, uint64_t *__restrict__ rint, int *__restrict__ poison,
                             unsigned long long *__restrict__ count, int *__restrict__ err) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t p = q < n ? pixel_of(px, q) : 0, k = q < n ? q - px.offs[p] : 1;
+    // every thread of the block takes part, whatever its bisection took
+    const int heads = __syncthreads_count(k % TC_CELL == 0);
+    if (threadIdx.x == 0 && heads) atomicAdd(count, (unsigned long long)heads);
     if (q >= n) return;
-    const int64_t p = pixel_of(px, q), k = q - px.offs[p];
-    const unsigned act = __activemask(), heads = __ballot_sync(act, k % TC_CELL == 0);
-    if ((threadIdx.x & 31) == 0 && heads) atomicAdd(count, (unsigned long long)__popc(heads));
     const double r = px.r[q], rs = r * inv_rmax * 256.0;
     const uint32_t rb = rs >= 255.0 ? 255u : (rs > 0.0 ? (uint32_t)rs : 0u);
     keys[q] = (k % TC_CELL == 0 ? (uint32_t)(TC_CELL - min((int64_t)TC_CELL, px.offs[p + 1] - q)) : (uint32_t)TC_CELL) << 8 | rb;

@@ -133,3 +133,16 @@ def test_raw_calls_on_two_streams(cuda_device):
         got = [call(*s, st) for s, st in zip(shapes, streams)]
         torch.cuda.synchronize()
         assert all(torch.equal(a[1], b[1]) for a, b in zip(got, ref))
+
+
+@pytest.mark.parametrize("nside,n", [(1, 31), (2, 257), (16, 1000), (64, 20000), (128, 3000)])
+def test_every_entry_of_a_pixelized_catalog_is_counted(cuda_device, nside, n):
+    """l = 0 holds every point with the same angular factor: its sums over pixels are those over the points, however
+    the lanes of a warp part in the bisection for their pixels (clumped and empty pixels, partial warps).  Only
+    the order of the sums differs: 1e-12."""
+    pts = uniform_ball(n, 1000.0, seed=nside)
+    pts[: n // 3, 1:] = [0.3, 1.0]  # a third of the points in one pixel
+    raw = catana.sfb_decomposition(catana.PointContainer(pts), 1, 8, 1000.0, True, False, interpolation="off")
+    ppc = catana.PixelizedPointContainer(nside, catana.PointContainer(pts))
+    hpx = catana.sfb_decomposition(ppc, 1, 8, 1000.0, True, False, interpolation="off")
+    assert np.max(np.abs(hpx.f_lmn[0] - raw.f_lmn[0])) <= 1e-12 * np.max(np.abs(raw.f_lmn[0]))
