@@ -587,13 +587,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                 tc05::fence_before();
                 tc_arrive(&dfree[reg]);
             }
-            // the slab's sums: value = (acc + top 2^60) 2^(-54 + EJ + EP + EW) A_lm
+            // the slab's sums: value = (acc + top 2^60) 2^(-54 + EJ + EP + EW) A_lm, the powers in two factors that
+            // FP64 holds for weights of any size
             if (live && row < 2 * b.mcount) {
                 const int ring = seq & (int)(TC_RING - 1);
                 const uint4 *tn = s_n + ring * TC_NB + nb;
-                const int m = b.mb0 + (row >> 1);
+                const int m = b.mb0 + (row >> 1), esh = ew > 0 ? 32 : 0;
                 const double am = scalbn(a.coef[(size_t)b.l * (b.l + 1) / 2 + m].y,
-                                         __double2loint(s_m[ring * TC_MB + (row >> 1)].y) + ew);
+                                         __double2loint(s_m[ring * TC_MB + (row >> 1)].y) + ew - esh);
                 const int w2 = 2 * (b.l + 1);
                 double *out = a.partial + (size_t)slab * a.pslab +
                               (size_t)a.nmax * ((size_t)b.l * (b.l + 1) - (size_t)a.l0 * (a.l0 + 1)) + 2 * b.mb0 + row +
@@ -614,8 +615,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                             }
                         }
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)  // 2^(EJ - 54) is a normal number: EJ >= -900
-                            v[c] *= __hiloint2double((int)(tn[c4 + c].w - (53u << 20)), 0);
+                        for (int c = 0; c < 4; ++c)  // 2^(EJ - 54 + esh) is a normal number: EJ >= -900
+                            v[c] *= __hiloint2double((int)tn[c4 + c].w - ((53 - esh) << 20), 0);
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
                             if (nb + c4 + c < b.ncount) out[(size_t)(c4 + c) * w2] = v[c] * am;
@@ -733,8 +734,8 @@ struct TcPixels {
 
 constexpr int TC_POISON_THETA = 1, TC_POISON_PHI = 2, TC_POISON_W = 4;
 
-// v = w cos or -w sin of m phi, times 2^(58 - ew), in signed halves
-__device__ __forceinline__ uint64_t phase_word(double v, double scale) { return signed_halves(__double2ll_rn(v * scale)); }
+// v = w 2^-ew cos or -w 2^-ew sin of m phi, times 2^58, in signed halves
+__device__ __forceinline__ uint64_t phase_word(double v) { return signed_halves(__double2ll_rn(v * 0x1p58)); }
 
 // Point records and phase tables, in sorted order: a warp per (tile, run of 8 m), lane = point.  The
 // phase of the run's middle comes from the exactly reduced fraction frac(m phi / 2 pi) and is rotated
@@ -768,8 +769,7 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
         rabs[i] = r;
         xs[i] = use && !(bad & TC_POISON_THETA) ? make_double2(ct, sqrt((1.0 - ct) * (1.0 + ct))) : make_double2(0.0, 0.0);
     }
-    const double scale = ldexp(1.0, 58 - slab[t / tslab].ew);
-    if (!use) wv = 0.0;
+    wv = use ? ldexp(wv, -slab[t / tslab].ew) : 0.0;  // in [-1, 1], exact for weights of any size
     const double phi = use && !(bad & TC_POISON_PHI) ? ph : 0.0;
     // frac(phi / 2 pi) 2^64 (mod 2^64), 1 / 2 pi as a pair of doubles: rounded at 2^-64 of a turn
     const double p = phi * 0.15915494309189535, pl = fma(phi, 0.15915494309189535, -p) - phi * 9.839338337591243e-18;
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
     double er_ = cs * wv, ei = -sn * wv;
     double ur = er_, ui = ei;
     for (int k = 4; k < 8 && m0 + k < lmp; ++k) {
-        o[k * TC_KT] = make_ulonglong2(phase_word(ur, scale), phase_word(ui, scale));
+        o[k * TC_KT] = make_ulonglong2(phase_word(ur), phase_word(ui));
         const double nr = ur * c1 + ui * s1, ni = ui * c1 - ur * s1;
         ur = nr;
         ui = ni;
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
         const double nr = er_ * c1 - ei * s1, ni = ei * c1 + er_ * s1;
         er_ = nr;
         ei = ni;
-        if (m0 + k < lmp) o[k * TC_KT] = make_ulonglong2(phase_word(er_, scale), phase_word(ei, scale));
+        if (m0 + k < lmp) o[k * TC_KT] = make_ulonglong2(phase_word(er_), phase_word(ei));
     }
 }
 
@@ -895,7 +895,7 @@ __global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t 
         cell[i] = make_uint2((uint32_t)q, use ? (uint32_t)min((int64_t)TC_CELL, px.offs[lo + 1] - q) : 0u);
         xs[i] = use ? make_double2(x, sqrt((1.0 - x) * (1.0 + x))) : make_double2(0.0, 0.0);
     }
-    const double scale = use ? ldexp(1.0, 58 - 1) : 0.0;  // unit weights: ew = 1
+    const double w = use ? 0.5 : 0.0;  // unit weights: ew = 1
     const int N = px.ring_pix[ra], j = (int)(lo - px.ring_start[ra]);
     const double2 *tw = px.tw + px.tw_off[ra];
     const int m0 = blockIdx.y * 8;
@@ -908,7 +908,7 @@ __global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t 
             f = tw[(int)((int64_t)j * s % N)];
             if (px.conj && 2 * mm > N) f.y = -f.y;
         }
-        o[k * TC_KT] = make_ulonglong2(phase_word(a.x * f.x - a.y * f.y, scale), phase_word(a.x * f.y + a.y * f.x, scale));
+        o[k * TC_KT] = make_ulonglong2(phase_word(w * (a.x * f.x - a.y * f.y)), phase_word(w * (a.x * f.y + a.y * f.x)));
     }
 }
 

@@ -146,3 +146,17 @@ def test_every_entry_of_a_pixelized_catalog_is_counted(cuda_device, nside, n):
     ppc = catana.PixelizedPointContainer(nside, catana.PointContainer(pts))
     hpx = catana.sfb_decomposition(ppc, 1, 8, 1000.0, True, False, interpolation="off")
     assert np.max(np.abs(hpx.f_lmn[0] - raw.f_lmn[0])) <= 1e-12 * np.max(np.abs(raw.f_lmn[0]))
+
+
+@pytest.mark.parametrize("n,power", [(300, -966), (300, -980), (40, -1000), (3, 1020), (2, 1022)])
+def test_weights_at_the_ends_of_the_double_range(cuda_device, n, power):
+    """f is normalised by the weights' sum, so weights times a power of two change it by the rounding of numbers near
+    the end of FP64's range only: sums of ~2^-1000 times products of ~2^-20 keep 2^-1074 + 1020 of their own, 1e-12
+    of the level's largest |f|."""
+    pts = uniform_ball(n, 1.0, seed=n)
+    w = np.random.default_rng(n).uniform(0.5, 1.0, n)
+    args = (11, 4, 1.0, True, False)
+    a = catana.sfb_decomposition(catana.PointContainer(pts), *args, weights=w, interpolation="on")
+    b = catana.sfb_decomposition(catana.PointContainer(pts), *args, weights=np.ldexp(w, power), interpolation="on")
+    for l, (f, g) in enumerate(zip(a.f_lmn, b.f_lmn)):
+        assert np.max(np.abs(f - g)) <= 1e-12 * np.max(np.abs(f)), l
