@@ -280,10 +280,54 @@ catana_status_t weight_sum(const double *w, int64_t n, double *out, double *scra
     return CATANA_OK;
 }
 
-// Core of both raw entry points: device inputs, device outputs.  `wsum_host` < 0
-// means "compute the weight sum on the device".
-catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double *w_d, int64_t npoints, int lmax,
-                           int nmax, double rmax, uint32_t flags, double *kln_d, double *cln_d, double *f_d,
+// WeightRange of device weights: bits of positive doubles in their order, out[0] from ~0 down, out[1] from 0 up
+__global__ void __launch_bounds__(256) k_weight_range(const double *__restrict__ w, int64_t n, unsigned long long *out) {
+    unsigned long long lo = ~0ull, hi = 0ull;
+    for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(w[i]));
+        if (b == 0ull || b >= 0x7ff0000000000000ull) continue;
+        lo = min(lo, b);
+        hi = max(hi, b);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&out[0], lo);
+        atomicMax(&out[1], hi);
+    }
+}
+
+// The ranges of the catalogs' weights (null: none) by one read-back
+catana_status_t weight_ranges(DeviceContext *ctx, const catana_catalog_t *cats, int ncat, WeightRange *out, cudaStream_t st) {
+    CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)16 * ncat));
+    unsigned long long *d = ctx->cat_scratch.as<unsigned long long>();
+    std::vector<unsigned long long> h(2 * (size_t)ncat);
+    for (int c = 0; c < ncat; ++c) h[2 * c] = ~0ull;
+    CG_CUDA_TRY(cudaMemcpyAsync(d, h.data(), (size_t)16 * ncat, cudaMemcpyHostToDevice, st));
+    for (int c = 0; c < ncat; ++c)
+        if (cats[c].weights && cats[c].npoints > 0) {
+            k_weight_range<<<std::min(4 * ctx->sm_count, ceil_div(cats[c].npoints, 256)), 256, 0, st>>>(cats[c].weights,
+                                                                                                       cats[c].npoints, d + 2 * c);
+            count_launch();
+        }
+    CG_CUDA_TRY(cudaGetLastError());
+    CG_CUDA_TRY(cudaMemcpyAsync(h.data(), d, (size_t)16 * ncat, cudaMemcpyDeviceToHost, st));
+    CG_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int c = 0; c < ncat; ++c) {
+        out[c] = WeightRange();
+        if (h[2 * c + 1] == 0ull) continue;
+        memcpy(&out[c].lo, &h[2 * c], 8);
+        memcpy(&out[c].hi, &h[2 * c + 1], 8);
+    }
+    return CATANA_OK;
+}
+
+// Core of both raw entry points: device inputs, device outputs; wr: of the weights where the caller has them on
+// the host, or null.
+catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double *w_d, const WeightRange *wr, int64_t npoints,
+                           int lmax, int nmax, double rmax, uint32_t flags, double *kln_d, double *cln_d, double *f_d,
                            int *err_d, cudaStream_t st) {
     const bool split = (flags & CATANA_FORM_MASK) == CATANA_FORM_SPLIT;
     WsOrder ws_order(ctx, st);
@@ -308,7 +352,17 @@ catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double
         s = split_raw_accumulate(ctx, pts_d, w_d, npoints, lmax, nmax, rmax, kln_d, facc, err_d, st,
                                  (flags & CATANA_SPLIT_ACCURATE) != 0);
     } else {
-        s = fp64_raw_accumulate(ctx, pts_d, w_d, npoints, lmax, nmax, rmax, resolve_jl(flags, npoints), kln_d, facc,
+        WeightRange w;
+        if (wr) {
+            w = *wr;
+        } else if (w_d && npoints > 0) {
+            catana_catalog_t c = {};
+            c.weights = w_d;
+            c.npoints = npoints;
+            s = weight_ranges(ctx, &c, 1, &w, st);
+            if (s != CATANA_OK) return s;
+        }
+        s = fp64_raw_accumulate(ctx, pts_d, w_d, w, npoints, lmax, nmax, rmax, resolve_jl(flags, npoints), kln_d, facc,
                                 err_d, st);
     }
     if (s != CATANA_OK) return s;
@@ -372,8 +426,8 @@ catana_status_t check_catalogs(const catana_catalog_t *cats, int32_t ncat) {
     return CATANA_OK;
 }
 
-// Core of both batched entry points: device pointers in the records.
-catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats, int ncat, uint32_t flags,
+// Core of both batched entry points: device pointers in the records; wr as in raw_device, one per catalog.
+catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats, const WeightRange *wr, int ncat, uint32_t flags,
                                double waves, int *err_d, cudaStream_t st) {
     const bool split = (flags & CATANA_FORM_MASK) == CATANA_FORM_SPLIT;
     if (split && (ctx->cc_major != 10 || ctx->cc_minor != 3)) {
@@ -430,9 +484,16 @@ catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats,
                       err_d, st);
         if (s != CATANA_OK) return s;
     } else {
+        std::vector<WeightRange> w(ncat);
+        bool ask = false;
+        for (int c = 0; c < ncat; ++c) ask |= (!wr && cats[c].weights && cats[c].npoints > 0);
+        if (ask) {
+            s = weight_ranges(ctx, cats, ncat, w.data(), st);
+            if (s != CATANA_OK) return s;
+        }
         for (int c = 0; c < ncat; ++c) {
             const catana_catalog_t &C = cats[c];
-            s = fp64_raw_accumulate(ctx, C.points, C.weights, C.npoints, C.lmax, C.nmax, C.rmax,
+            s = fp64_raw_accumulate(ctx, C.points, C.weights, wr ? wr[c] : w[c], C.npoints, C.lmax, C.nmax, C.rmax,
                                     resolve_jl(flags, C.npoints), C.k_ln, facc[c], err_d, st);
             if (s != CATANA_OK) return s;
             if (C.kmax > 0.0 && C.lmax > 0 && C.nmax > 0) {
@@ -595,7 +656,7 @@ catana_status_t catana_gpu_sfb_raw_dev(const double *points_dev, const double *w
         err_d = ctx->misc.as<int>();
         CG_CUDA_TRY(cudaMemsetAsync(err_d, 0, sizeof(int), st));
     }
-    return raw_device(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, flags, k_ln_dev, c_ln_dev, f_lmn_dev,
+    return raw_device(ctx, points_dev, weights_dev, nullptr, npoints, lmax, nmax, rmax, flags, k_ln_dev, c_ln_dev, f_lmn_dev,
                       err_d, st);
 }
 
@@ -630,7 +691,9 @@ catana_status_t catana_gpu_sfb_raw(const double *points, const double *weights, 
         CG_CUDA_TRY(cudaMemcpyAsync(pts_d, points, (size_t)npoints * 3 * sizeof(double), cudaMemcpyHostToDevice, st));
     if (weights && npoints > 0)
         CG_CUDA_TRY(cudaMemcpyAsync(w_d, weights, (size_t)npoints * sizeof(double), cudaMemcpyHostToDevice, st));
-    s = raw_device(ctx, pts_d, w_d, npoints, lmax, nmax, rmax, flags, kln_d, cln_d, f_d, err_d, st);
+    WeightRange wr;
+    if (weights && (flags & CATANA_FORM_MASK) != CATANA_FORM_SPLIT) wr.add(weights, npoints);
+    s = raw_device(ctx, pts_d, w_d, &wr, npoints, lmax, nmax, rmax, flags, kln_d, cln_d, f_d, err_d, st);
     if (s != CATANA_OK) return s;
     int err_h = 0;
     CG_CUDA_TRY(cudaMemcpyAsync(&err_h, err_d, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -664,7 +727,7 @@ catana_status_t catana_gpu_sfb_raw_batched_dev(const catana_catalog_t *cats, int
         err_d = ctx->misc.as<int>();
         CG_CUDA_TRY(cudaMemsetAsync(err_d, 0, sizeof(int), st));
     }
-    return batched_device(ctx, cats, ncat, flags, waves, err_d, st);
+    return batched_device(ctx, cats, nullptr, ncat, flags, waves, err_d, st);
 }
 
 catana_status_t catana_gpu_sfb_raw_batched(const catana_catalog_t *cats, int32_t ncat, uint32_t flags, double waves,
@@ -711,7 +774,11 @@ catana_status_t catana_gpu_sfb_raw_batched(const catana_catalog_t *cats, int32_t
         dc[c].f_lmn = reinterpret_cast<double *>(op);
         op += al(catana_gpu_flmn_size(C.lmax, C.nmax) * 2 * sizeof(double));
     }
-    s = batched_device(ctx, dc.data(), ncat, flags, waves, err_d, st);
+    std::vector<WeightRange> wr(ncat);
+    if ((flags & CATANA_FORM_MASK) != CATANA_FORM_SPLIT)
+        for (int c = 0; c < ncat; ++c)
+            if (cats[c].weights) wr[c].add(cats[c].weights, cats[c].npoints);
+    s = batched_device(ctx, dc.data(), wr.data(), ncat, flags, waves, err_d, st);
     if (s != CATANA_OK) return s;
     int err_h = 0;
     CG_CUDA_TRY(cudaMemcpyAsync(&err_h, err_d, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <string>
@@ -144,15 +145,30 @@ inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 // evaluation, or the piecewise FP64 polynomials (CATANA_JL_POLY).
 enum JlMode { JL_MODE_LERP = 0, JL_MODE_EXACT = 1, JL_MODE_POLY = 2 };
 
-// FP64 plain raw path (sfb_fp64.cu).  All pointers device.  Accumulates into
-// f_acc (complex, packed by l, un-normalised); the caller normalises.
+// The smallest and the largest |w| of a catalog that are neither 0 nor infinite nor NaN (none: lo > hi).
+struct WeightRange {
+    double lo = HUGE_VAL, hi = 0.0;
+    void add(double w) {
+        const double a = std::fabs(w);
+        if (!(a > 0.0 && a < HUGE_VAL)) return;
+        if (a < lo) lo = a;
+        if (a > hi) hi = a;
+    }
+    void add(const double *w, int64_t n) {
+        for (int64_t i = 0; i < n; ++i) add(w[i]);
+    }
+};
+
+// Plain raw form (sfb_fp64.cu).  All pointers device.  Accumulates into f_acc (complex, packed by l,
+// un-normalised); the caller normalises.  wr: of weights_dev, unused without weights.
 catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
-                                    int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, const double *kln_dev,
-                                    double *f_acc_dev, int *err_dev, cudaStream_t st);
+                                    const WeightRange &wr, int64_t npoints, int lmax, int nmax, double rmax, JlMode jl,
+                                    const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st);
 // The same sum with its contraction on the tensor cores (plain_tc.cu), where the device has them and
 // lmax <= 512; with JL_MODE_POLY the caller has prepared ctx->poly and passes the largest radius (else rtop = 0).
 bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax);
 bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl);  // and whether it is the faster one
+bool plain_tc_holds(const WeightRange &wr);  // and whether its fixed-point terms hold weights of this range
 catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
                                     int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, double rtop,
                                     const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st);

@@ -1218,6 +1218,13 @@ bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
            rmax < 1e100;
 }
 
+// A term is held to 2^-55 of its slab's bound, which goes with the slab's heaviest weight.  Where the heavy points add little
+// to a mode -- they lie near a pole and m is high, or where j_l is still small -- a mode has only the light
+// ones' terms, with as many bits less as they are lighter; FP64 held them all.  Up to eight bits, 2^-47 of such a mode's terms
+// (7e-15), stay inside the errors that both paths have from their recurrences (5e-15 to 1e-14 of f); a catalog whose
+// weights differ by more takes the FP64 path.
+bool plain_tc_holds(const WeightRange &wr) { return !(wr.hi > 256.0 * wr.lo); }
+
 // Few points with many radial orders, or one or two levels: a CTA of the tensor-core kernel walks its blocks of 64
 // radial orders one after the other, 13 to 15 us each, where the FP64 path has a CTA for each and takes 40 us a
 // level (80 without the linear table, of 64 radial orders and more) and its FP64 work.  Microseconds a call, FP64 path / here:

@@ -86,6 +86,7 @@ catana_status_t accum_add(Accum *A, const T *points, const T *weights, int64_t n
     (weights ? A->weighted : A->unweighted) = true;
     // extents and weight sum on the host (the chunk is in host memory already)
     double max_r = 0.0, max_w = weights ? 0.0 : 1.0, ws = 0.0;
+    WeightRange wr;
     for (int64_t i = 0; i < n; ++i) {
         const double r = (double)points[3 * i];
         if (!(r >= 0.0) || !std::isfinite(r)) {
@@ -97,6 +98,7 @@ catana_status_t accum_add(Accum *A, const T *points, const T *weights, int64_t n
             const double w = (double)weights[i];
             ws += w;
             if (std::fabs(w) > max_w) max_w = std::fabs(w);
+            wr.add(w);
         }
     }
     DeviceContext *ctx = A->ctx;
@@ -169,7 +171,7 @@ catana_status_t accum_add(Accum *A, const T *points, const T *weights, int64_t n
         // JL_AUTO picks the table form here (streamed catalogs are large)
         const uint32_t jl = A->flags & CATANA_JL_MASK;
         const JlMode mode = jl == CATANA_JL_POLY ? JL_MODE_POLY : jl == CATANA_JL_EXACT ? JL_MODE_EXACT : JL_MODE_LERP;
-        s = fp64_raw_accumulate(ctx, p64, w64, n, A->lmax, A->nmax, A->rmax, mode, A->kln.as<double>(),
+        s = fp64_raw_accumulate(ctx, p64, w64, wr, n, A->lmax, A->nmax, A->rmax, mode, A->kln.as<double>(),
                                 A->facc.as<double>(), err_d, A->comp_st);
     }
     if (s != CATANA_OK) return s;
@@ -240,7 +242,7 @@ catana_status_t accum_add_records(Accum *A, const void *records, int64_t n, cons
             const uint32_t jl = A->flags & CATANA_JL_MASK;
             const JlMode mode =
                 jl == CATANA_JL_POLY ? JL_MODE_POLY : jl == CATANA_JL_EXACT ? JL_MODE_EXACT : JL_MODE_LERP;
-            s = fp64_raw_accumulate(ctx, pts, nullptr, kept, A->lmax, A->nmax, A->rmax, mode,
+            s = fp64_raw_accumulate(ctx, pts, nullptr, WeightRange(), kept, A->lmax, A->nmax, A->rmax, mode,
                                     A->kln.as<double>(), A->facc.as<double>(), err_d, A->comp_st);
         }
         if (s != CATANA_OK) return s;

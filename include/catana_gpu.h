@@ -60,7 +60,8 @@ typedef enum {
 #define CATANA_JL_POLY 3u
 #define CATANA_JL_MASK 3u
 /* Contraction form.  PLAIN: to FP64 accuracy, the drop-in (tensor-core products of
- * 8-bit digits that are exact; FP64 on CUDA cores past lmax 512).  SPLIT: tensor-core
+ * 8-bit digits that are exact; FP64 on CUDA cores past lmax 512, for weights
+ * that differ by more than 2^8, and where that is faster).  SPLIT: tensor-core
  * tcgen05 contraction of 3-term FP16 hi+lo products with FP32 accumulation,
  * folded per 32-point tile and reduced in FP64; j_l from piecewise degree-6
  * polynomials on unit intervals with FP32 coefficients, accurate to ~1e-7 of its
@@ -110,7 +111,8 @@ catana_status_t catana_gpu_sfb_raw(const double *points, const double *weights, 
 
 /* Same computation on device-resident data: all pointers are device pointers,
  * the work is enqueued on `stream` and the call returns without synchronising
- * except where a domain check needs the host (JL_INTERP); *status_dev (device
+ * except where the host needs a value (the weights' range and sum, max r with
+ * JL_POLY, a table that is not cached yet); *status_dev (device
  * int, may be NULL) receives CATANA_ERR_DOMAIN when an argument left the table. */
 catana_status_t catana_gpu_sfb_raw_dev(const double *points_dev, const double *weights_dev, int64_t npoints,
                                        uint16_t lmax, uint16_t nmax, double rmax, uint32_t flags,

@@ -160,3 +160,43 @@ def test_weights_at_the_ends_of_the_double_range(cuda_device, n, power):
     b = catana.sfb_decomposition(catana.PointContainer(pts), *args, weights=np.ldexp(w, power), interpolation="on")
     for l, (f, g) in enumerate(zip(a.f_lmn, b.f_lmn)):
         assert np.max(np.abs(f - g)) <= 1e-12 * np.max(np.abs(f)), l
+
+
+def _entries(pts, w, lmax, nmax):
+    """f_lmn of the weighted catalog by every entry that takes weights."""
+    torch = pytest.importorskip("torch")
+    pc = catana.PointContainer(pts)
+    yield catana.sfb_decomposition(pc, lmax, nmax, 1.0, True, False, weights=w, interpolation="on").f_lmn
+    yield catana.sfb_decomposition_batched([pc, pc], lmax, nmax, 1.0, weights=[None, w], store_flmn=True, verbose=False,
+                                           precision="plain", interpolation="on")[1].f_lmn
+    with catana.SFBAccumulator(lmax, nmax, 1.0, precision="plain", interpolation="on") as acc:
+        acc.add(pts, w)
+        yield acc.finish(store_flmn=True).f_lmn
+    d = [torch.from_numpy(a).cuda() for a in (pts, w)]
+    k, c = (torch.zeros(lmax * nmax, dtype=torch.float64, device="cuda") for _ in range(2))
+    f = torch.zeros(nmax * lmax * (lmax + 1) // 2, dtype=torch.complex128, device="cuda")
+    _lib.check(_lib.lib.catana_gpu_sfb_raw_dev(d[0].data_ptr(), d[1].data_ptr(), len(pts), lmax, nmax, 1.0, _lib.JL_INTERP,
+                                               k.data_ptr(), c.data_ptr(), f.data_ptr(), None, None))
+    f = f.cpu().numpy()
+    yield [f[nmax * l * (l + 1) // 2: nmax * (l + 1) * (l + 2) // 2].reshape(l + 1, nmax) for l in range(lmax)]
+
+
+@pytest.mark.parametrize("power", [0, 7, 8, 9, 20, 45, 70])
+def test_light_points_beside_a_heavy_one(cuda_device, power):
+    """A heavy point at a pole adds nothing to m > 0: those modes are the light points' alone, and as accurate as
+    without it.  Fixed-point terms are cut at 2^-55 of the heaviest weight's bound, so up to the 2^8 that they are taken for
+    a mode errs by sqrt(33) 2^(8 - 55), times what the bound exceeds a mode's largest term by (below 2^5 here): 2e-12
+    of the mode's largest order."""
+    lmax, nmax = 8, 4
+    pts = uniform_ball(33, 1.0, seed=4)
+    pts[5, 1] = 0.0
+    w = np.random.default_rng(2).uniform(0.75, 1.0, 33)
+    light = w.copy()
+    light[5] = 0.0
+    w[5] = 0.75 * 2.0 ** power
+    ref = catana.sfb_decomposition(catana.PointContainer(pts), lmax, nmax, 1.0, True, False, weights=light, interpolation="on")
+    for f in _entries(pts, w, lmax, nmax):
+        for l in range(1, lmax):
+            g = ref.f_lmn[l] * (light.sum() / w.sum())
+            for m in range(1, l + 1):
+                assert np.max(np.abs(f[l][m] - g[m])) <= 2e-12 * np.max(np.abs(g[m])), (l, m)
