@@ -83,6 +83,7 @@ SIGNATURES = {
     "catana_gpu_fp64_peak": (ctypes.c_int, [ctypes.c_int32, _P]),
     "catana_gpu_test_split_stall": (ctypes.c_int, [_U32]),
     "catana_gpu_test_plain_stall": (ctypes.c_int, [_U32]),
+    "catana_gpu_test_alloc_limit": (None, [ctypes.c_size_t]),
     "catana_gpu_profile_enable": (None, [ctypes.c_int]),
     "catana_gpu_profile_report": (ctypes.c_int, [_P, _P, _P]),
     "catana_gpu_launch_count": (ctypes.c_uint64, []),

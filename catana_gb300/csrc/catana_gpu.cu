@@ -22,6 +22,7 @@ namespace catana_gpu {
 
 std::atomic<uint64_t> g_launches{0};
 static thread_local std::string t_last_error;
+thread_local size_t t_alloc_limit = 0;
 
 void set_error(const std::string &msg) { t_last_error = msg; }
 
@@ -544,6 +545,8 @@ size_t catana_gpu_flmn_size(uint16_t lmax, uint16_t nmax) {
 const char *catana_gpu_last_error(void) { return t_last_error.c_str(); }
 
 uint64_t catana_gpu_launch_count(void) { return g_launches.load(); }
+
+void catana_gpu_test_alloc_limit(size_t bytes) { t_alloc_limit = bytes; }
 
 void catana_gpu_profile_enable(int enable) { g_prof_on.store(enable ? 1 : 0); }
 

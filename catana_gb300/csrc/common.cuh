@@ -25,18 +25,30 @@ void set_error(const std::string &msg);
 void prof_begin(cudaStream_t st);
 void prof_end(cudaStream_t st, double algo_flops);
 
-// Grow-only device buffer.
+// Test hook (catana_gpu_test_alloc_limit): larger buffers than this cannot be had by this thread's calls (0: no limit)
+extern thread_local size_t t_alloc_limit;
+
+// Grow-only device buffer, allocated a quarter larger than asked for where that can be had.  A failed ensure() leaves
+// it empty, so whoever caches something in it forgets that before the call.
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
     cudaError_t ensure(size_t need) {
-        if (need <= bytes) return cudaSuccess;
-        if (ptr) cudaFree(ptr);
-        ptr = nullptr;
-        bytes = 0;
+        const bool refuse = t_alloc_limit && need > t_alloc_limit;
+        if (need <= bytes && !refuse) return cudaSuccess;
+        release();
         size_t cap = need + need / 4;
-        cudaError_t e = cudaMalloc(&ptr, cap);
-        if (e == cudaSuccess) bytes = cap;
+        cudaError_t e = refuse ? cudaErrorMemoryAllocation : cudaMalloc(&ptr, cap);
+        if (e == cudaErrorMemoryAllocation && !refuse) {
+            cudaGetLastError();
+            e = cudaMalloc(&ptr, cap = need);
+        }
+        if (e == cudaSuccess) {
+            bytes = cap;
+        } else {
+            ptr = nullptr;
+            cudaGetLastError();  // reported here, not by the next launch
+        }
         return e;
     }
     template <class T> T *as() const { return reinterpret_cast<T *>(ptr); }

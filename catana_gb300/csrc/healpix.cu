@@ -553,6 +553,7 @@ catana_status_t ensure_rings(int64_t nside, cudaStream_t st) {
     R.off_order = al(R.off_twoff + nrings * sizeof(int64_t));
     R.off_tw = al(R.off_order + nrings * sizeof(int));
     const size_t total = R.off_tw + tw.size() * sizeof(double2);
+    R.nside = 0;
     CG_CUDA_TRY(R.buf.ensure(total));
     char *b = R.buf.as<char>();
     CG_CUDA_TRY(cudaMemcpyAsync(b + R.off_start, start.data(), nrings * sizeof(int64_t), cudaMemcpyHostToDevice, st));

@@ -1166,6 +1166,7 @@ catana_status_t ensure_tc_coefs(DeviceContext *ctx, int lmax, cudaStream_t st) {
             h[(size_t)l * (l + 1) / 2 + m] = make_double2(beta, (double)A);
         }
     }
+    ctx->tc_coef_lmax = -1;
     CG_CUDA_TRY(ctx->tc_coef.ensure(h.size() * sizeof(double2)));
     CG_CUDA_TRY(cudaMemcpyAsync(ctx->tc_coef.ptr, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
     CG_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1182,6 +1183,7 @@ catana_status_t ensure_tc_tables(DeviceContext *ctx, int lmax, int nmax, cudaStr
     const int npts = 1000 * nmax;
     const int64_t total = (int64_t)lmax * npts;
     const size_t tb = tc_al((size_t)total * sizeof(double2));
+    ctx->tc_tab_lmax = ctx->tc_tab_nmax = -1;
     CG_CUDA_TRY(ctx->tc_tab.ensure(tb + 2 * (size_t)lmax * sizeof(double)));
     double *dz = reinterpret_cast<double *>(ctx->tc_tab.as<char>() + tb);
     k_ptc_pairs<<<ceil_div(total, 256), 256, 0, st>>>(ctx->tables.as<double>(), npts, total, ctx->tc_tab.as<double2>());
@@ -1200,6 +1202,7 @@ catana_status_t ensure_tc_tables(DeviceContext *ctx, int lmax, int nmax, cudaStr
 catana_status_t ensure_tc_poly(DeviceContext *ctx, cudaStream_t st) {
     if (ctx->tc_poly_lmax == ctx->poly_lmax && ctx->tc_poly_nint == ctx->poly_nint) return CATANA_OK;
     const int64_t total = (int64_t)ctx->poly_lmax * ctx->poly_nint;
+    ctx->tc_poly_lmax = ctx->tc_poly_nint = -1;
     CG_CUDA_TRY(ctx->tc_poly.ensure((size_t)total * sizeof(TcPoly)));
     k_ptc_poly_int<<<ceil_div(total, 128), 128, 0, st>>>(ctx->poly.as<double>(), total, ctx->tc_poly.as<TcPoly>());
     count_launch();

@@ -415,6 +415,7 @@ catana_status_t ensure_coefs(DeviceContext *ctx, int lmax, cudaStream_t st) {
             row[2 * m + 1] = cb;
         }
     }
+    ctx->coef_lmax = -1;
     CG_CUDA_TRY(ctx->coef.ensure(h.size() * sizeof(double)));
     CG_CUDA_TRY(cudaMemcpyAsync(ctx->coef.ptr, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     CG_CUDA_TRY(cudaStreamSynchronize(st));
@@ -426,6 +427,7 @@ catana_status_t ensure_lerp_tables(DeviceContext *ctx, int lmax, int nmax, cudaS
     if (ctx->tab_lmax >= lmax && ctx->tab_nmax == nmax) return CATANA_OK;
     const int npts = 1000 * nmax;  // BESSELINTERPOLATIONPOINTS_PER_ZERO * nmax
     std::vector<double> dx(lmax);
+    ctx->tab_lmax = ctx->tab_nmax = -1;
     ctx->tab_dxinv.assign(lmax, 0.0);
     ctx->tab_zmax.assign(lmax, 0.0);
     for (int l = 0; l < lmax; ++l) {
@@ -466,6 +468,7 @@ catana_status_t ensure_poly_tables(DeviceContext *ctx, int lmax, int nint, cudaS
     for (int s2 = 0; s2 < kPolyNC; ++s2)
         for (int r = 0; r < kPolyNC; ++r) m2[(size_t)s2 * kPolyNC + r] = T[(size_t)r * kPolyNC + s2];
     const size_t tab_bytes = (size_t)lmax * nint * kPolyNC * sizeof(double);
+    ctx->poly_lmax = ctx->poly_nint = -1;
     CG_CUDA_TRY(ctx->poly.ensure(tab_bytes));
     DevBuf tmp;
     const size_t vbytes = (size_t)nint * kPolyNC * lmax * sizeof(double);

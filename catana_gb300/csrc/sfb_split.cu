@@ -1478,6 +1478,7 @@ catana_status_t ensure_split_tables(DeviceContext *ctx, int lmax, int nint, cuda
     const size_t tab_bytes = (size_t)lmax * nint * 2 * sizeof(float4);
     const size_t coef_bytes = (size_t)lmax * (lmax + 1) / 2 * sizeof(float4);
     // [j_l tables][(A, B) per (l, m)][(c1, rho) per (l, m): the Reinsch-modified step]
+    C.lmax = C.nint = -1;
     CG_CUDA_TRY(ctx->split_tab.ensure(tab_bytes + 2 * coef_bytes + 1024));
     constexpr int NC = TDEG + 1;
     const size_t vbytes = (size_t)nint * NC * lmax * sizeof(double);

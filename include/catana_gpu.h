@@ -352,6 +352,10 @@ catana_status_t catana_gpu_test_split_stall(uint32_t wait_us);
  * calls): arms the next run that takes it. */
 catana_status_t catana_gpu_test_plain_stall(uint32_t wait_us);
 
+/* Test hook for device memory that cannot be had: until it is called with 0, this thread's calls
+ * fail to get any internal buffer of more than `bytes`, as if cudaMalloc had. */
+void catana_gpu_test_alloc_limit(size_t bytes);
+
 /* Message of the last failing call on this thread ("" if none). */
 const char *catana_gpu_last_error(void);
 

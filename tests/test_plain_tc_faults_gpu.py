@@ -200,3 +200,38 @@ def test_light_points_beside_a_heavy_one(cuda_device, power):
             g = ref.f_lmn[l] * (light.sum() / w.sum())
             for m in range(1, l + 1):
                 assert np.max(np.abs(f[l][m] - g[m])) <= 2e-12 * np.max(np.abs(g[m])), (l, m)
+
+
+class _AllocLimit:
+    """Within it, no internal buffer of more than `bytes` can be had."""
+
+    def __init__(self, nbytes):
+        self.nbytes = nbytes
+
+    def __enter__(self):
+        _lib.lib.catana_gpu_test_alloc_limit(self.nbytes)
+
+    def __exit__(self, *exc):
+        _lib.lib.catana_gpu_test_alloc_limit(0)
+
+
+@pytest.mark.parametrize("interp,precision,lmax,nmax,limit", [("on", "plain", 90, 30, 4 << 20), ("poly", "plain", 200, 4, 4 << 20),
+                                                              ("auto", "split", 200, 4, 2 << 20)])
+def test_a_table_that_could_not_be_had_is_not_taken_for_cached(cuda_device, interp, precision, lmax, nmax, limit):
+    """A failed growth frees the buffer that a table was cached in: the next call of the old size builds it again.
+    The limits lie between the catalog's and the results' buffers (at most 2.0, 1.3, 1.3 MB) and the tables (21.6, 4.4,
+    2.1 MB).  Tables for other l ranges are rounded otherwise (j_l of all l by one recurrence): to ~1e-14 the
+    polynomials in FP64, to ~1e-7 those of the split form."""
+    pts = uniform_ball(2000, 1000.0, seed=3)
+
+    def call(lmax, nmax):
+        return catana.sfb_decomposition(catana.PointContainer(pts), lmax, nmax, 1000.0, True, False, interpolation=interp,
+                                        precision=precision)
+
+    call(lmax, nmax)  # what this and the next call share is there
+    before = call(6, 5)
+    with _AllocLimit(limit):
+        with pytest.raises(MemoryError):
+            call(lmax + 20, nmax + 1)
+    after = call(6, 5)
+    assert np.allclose(before.c_ln, after.c_ln, rtol=1e-5 if precision == "split" else 1e-12, atol=0.0)
