@@ -1253,7 +1253,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     // the test hook (catana_gpu_test_plain_stall) arms one run
     const uint64_t stall_ns = g_plain_stall_ns.exchange(0);
     const bool lerp = jl == JL_MODE_LERP, fused = lerp && !pix;  // fused: the main kernel evaluates j_l itself
-    int64_t npoints = nall;  // an upper bound of a pixelized catalog's entries, until they are counted
+    int64_t npoints = nall;  // a pixelized catalog's entries, once they are counted
     catana_status_t s = ensure_tc_coefs(ctx, lmax, st);
     if (s != CATANA_OK) return s;
     if (lerp) {
@@ -1274,38 +1274,24 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     // radius, where the caller knows it
     const int er = std::max(ilogb(rmax) + 3, rtop > 0.0 ? ilogb(rtop) + 1 : -1000);
     const double rlim = lerp ? ldexp(1.0, er) : INFINITY;
-    // points per pass: rows and phases (32 B per point and m) stay under 12 GB
-    int64_t chunk = std::max<int64_t>(TC_KT, (int64_t)(12e9 / (32.0 * lmp)) / TC_KT * TC_KT);
-    chunk = std::min(chunk, npoints);
-    const int tiles_c = ceil_div(chunk, TC_KT);
-    const size_t np = (size_t)tiles_c * TC_KT;
-    // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
-    // (a pixelized catalog's points are sorted at once, its entries then taken in passes)
-    const size_t ns = pix ? (size_t)nall : np;
-    const size_t kb = tc_al(ns * 4), hb = tc_al(radix_hist_words((int64_t)ns) * 4);
-    const size_t o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(std::max(ns, np) * 8), o_xs = o_rabs + tc_al(np * 8);
-    const size_t o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
-    // slabs: at most TC_SLAB_TILES tiles (the 64-bit sums' resolution), a whole number of waves
-    auto slab_tiles = [&](int tiles) {
-        const int waves = ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES);
-        return ceil_div(tiles, (int64_t)ctx->sm_count * waves);
-    };
-    const size_t phb = pix ? tc_al((size_t)pix->nrings * lmax * sizeof(double2)) : 0;
-    const int max_slabs = ctx->sm_count * ceil_div(tiles_c, (int64_t)ctx->sm_count * TC_SLAB_TILES);
-    const size_t o_mx = o_sl + tc_al((size_t)max_slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)max_slabs * 3 * TC_LMAX * 4);
-    CG_CUDA_TRY(ctx->tc_ws.ensure(o_poi + 256 + phb));
-    char *ws = ctx->tc_ws.as<char>();
-    uint32_t *keys = reinterpret_cast<uint32_t *>(ws), *perm = reinterpret_cast<uint32_t *>(ws + kb);
-    uint32_t *tk = reinterpret_cast<uint32_t *>(ws + 2 * kb), *tv = reinterpret_cast<uint32_t *>(ws + 3 * kb);
-    uint32_t *hist = reinterpret_cast<uint32_t *>(ws + 4 * kb);
-    int *poison = reinterpret_cast<int *>(ws + o_poi);
-    TcSlab *slabs = reinterpret_cast<TcSlab *>(ws + o_sl);
-    CG_CUDA_TRY(cudaMemsetAsync(poison, 0, 16, st));  // and the entries' count
+    // A pixelized catalog is sorted into entries first, in the workspace of the HEALPix calls (which end before they
+    // return): [sort scratch][radii][ring phases][poison, count]
     TcPixels px = {};
+    const uint32_t *entries = nullptr;
+    const uint64_t *entry_r = nullptr;
+    int *poison = nullptr;
     if (pix) {
-        double2 *ph = reinterpret_cast<double2 *>(ws + o_poi + 256);
+        const size_t kb = tc_al((size_t)nall * 4), hb = tc_al(radix_hist_words(nall) * 4), rb = tc_al((size_t)nall * 8);
+        const size_t phb = tc_al((size_t)pix->nrings * lmax * sizeof(double2));
+        CG_CUDA_TRY(ctx->hp_ws.ensure(4 * kb + hb + rb + phb + 256));
+        char *hs = ctx->hp_ws.as<char>();
+        uint32_t *keys = reinterpret_cast<uint32_t *>(hs), *perm = reinterpret_cast<uint32_t *>(hs + kb);
+        uint64_t *rint = reinterpret_cast<uint64_t *>(hs + 4 * kb + hb);
+        double2 *ph = reinterpret_cast<double2 *>(hs + 4 * kb + hb + rb);
+        poison = reinterpret_cast<int *>(hs + 4 * kb + hb + rb + phb);
+        unsigned long long *count = reinterpret_cast<unsigned long long *>(poison) + 1;
+        CG_CUDA_TRY(cudaMemsetAsync(poison, 0, 16, st));  // and the entries' count
         k_ptc_ring_phases<<<ceil_div((int64_t)pix->nrings * lmax, 128), 128, 0, st>>>(pix->ring_phi, pix->nrings, lmax, ph);
-        count_launch();
         px.r = pix->r;
         px.offs = pix->offs;
         px.npix = pix->npix;
@@ -1318,17 +1304,45 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         px.ring_ph = ph;
         px.tw = pix->tw;
         px.tw_off = pix->tw_off;
-        k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, 1.0 / rmax, er, lerp ? 1 : 0, rlim, keys, perm,
-                                                         reinterpret_cast<uint64_t *>(ws + o_rint), poison,
-                                                         reinterpret_cast<unsigned long long *>(poison) + 1, err_dev);
-        count_launch();
+        k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, 1.0 / rmax, er, lerp ? 1 : 0, rlim, keys, perm, rint, poison,
+                                                         count, err_dev);
+        count_launch(2);
+        CG_CUDA_TRY(cudaGetLastError());
         unsigned long long cells = 0;
-        CG_CUDA_TRY(cudaMemcpyAsync(&cells, reinterpret_cast<unsigned long long *>(poison) + 1, sizeof(cells),
-                                    cudaMemcpyDeviceToHost, st));
-        s = radix_sort_pairs(keys, perm, tk, tv, nall, 16, hist, st);
+        CG_CUDA_TRY(cudaMemcpyAsync(&cells, count, sizeof(cells), cudaMemcpyDeviceToHost, st));
+        s = radix_sort_pairs(keys, perm, reinterpret_cast<uint32_t *>(hs + 2 * kb), reinterpret_cast<uint32_t *>(hs + 3 * kb), nall,
+                             16, reinterpret_cast<uint32_t *>(hs + 4 * kb), st);
         if (s != CATANA_OK) return s;
         CG_CUDA_TRY(cudaStreamSynchronize(st));
         npoints = (int64_t)cells;
+        entries = perm;
+        entry_r = rint;
+    }
+    // points per pass: rows and phases (32 B per point and m) stay under 12 GB
+    int64_t chunk = std::max<int64_t>(TC_KT, (int64_t)(12e9 / (32.0 * lmp)) / TC_KT * TC_KT);
+    chunk = std::min(chunk, npoints);
+    const int tiles_c = ceil_div(chunk, TC_KT);
+    const size_t np = (size_t)tiles_c * TC_KT;
+    // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
+    const size_t kb = pix ? 0 : tc_al(np * 4), hb = pix ? 0 : tc_al(radix_hist_words((int64_t)np) * 4);
+    const size_t o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(np * 8), o_xs = o_rabs + tc_al(np * 8);
+    const size_t o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
+    // slabs: at most TC_SLAB_TILES tiles (the 64-bit sums' resolution), a whole number of waves
+    auto slab_tiles = [&](int tiles) {
+        const int waves = ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES);
+        return ceil_div(tiles, (int64_t)ctx->sm_count * waves);
+    };
+    const int max_slabs = ctx->sm_count * ceil_div(tiles_c, (int64_t)ctx->sm_count * TC_SLAB_TILES);
+    const size_t o_mx = o_sl + tc_al((size_t)max_slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)max_slabs * 3 * TC_LMAX * 4);
+    CG_CUDA_TRY(ctx->tc_ws.ensure(o_poi + 256));
+    char *ws = ctx->tc_ws.as<char>();
+    uint32_t *keys = reinterpret_cast<uint32_t *>(ws), *perm = reinterpret_cast<uint32_t *>(ws + kb);
+    uint32_t *tk = reinterpret_cast<uint32_t *>(ws + 2 * kb), *tv = reinterpret_cast<uint32_t *>(ws + 3 * kb);
+    uint32_t *hist = reinterpret_cast<uint32_t *>(ws + 4 * kb);
+    TcSlab *slabs = reinterpret_cast<TcSlab *>(ws + o_sl);
+    if (!pix) {
+        poison = reinterpret_cast<int *>(ws + o_poi);
+        CG_CUDA_TRY(cudaMemsetAsync(poison, 0, 16, st));
     }
     for (int64_t c0 = 0; c0 < npoints; c0 += chunk) {
         const int64_t nc = std::min(chunk, npoints - c0);
@@ -1344,7 +1358,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         ulonglong2 *ph_d = reinterpret_cast<ulonglong2 *>(ws + o_ph);
         uint2 *cell = reinterpret_cast<uint2 *>(ws + o_rabs);
         if (pix) {
-            k_ptc_pixels<<<pg, 32 * pw, 0, st>>>(px, perm + c0, nc, tiles, lmp, cell, xs_d, ph_d);
+            k_ptc_pixels<<<pg, 32 * pw, 0, st>>>(px, entries + c0, nc, tiles, lmp, cell, xs_d, ph_d);
             k_ptc_cell_slabs<<<nslabs, 256, 0, st>>>(px, cell, nc, (int64_t)tslab * TC_KT, rlim, slabs);
         } else {
             const double *pts = points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
@@ -1368,7 +1382,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         a.tslab = tslab;
         a.phase = reinterpret_cast<const ulonglong2 *>(ws + o_ph);
         a.rows = reinterpret_cast<double *>(ws + o_rows);
-        a.rint = reinterpret_cast<const uint64_t *>(ws + o_rint);
+        a.rint = pix ? entry_r : reinterpret_cast<const uint64_t *>(ws + o_rint);
         a.xs = reinterpret_cast<const double2 *>(ws + o_xs);
         a.slab = slabs;
         a.coef = ctx->tc_coef.as<double2>();

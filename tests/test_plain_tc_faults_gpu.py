@@ -235,3 +235,18 @@ def test_a_table_that_could_not_be_had_is_not_taken_for_cached(cuda_device, inte
             call(lmax + 20, nmax + 1)
     after = call(6, 5)
     assert np.allclose(before.c_ln, after.c_ln, rtol=1e-5 if precision == "split" else 1e-12, atol=0.0)
+
+
+def test_a_pixelized_workspace_goes_by_the_entries(cuda_device):
+    """200k points in the 12 pixels of nside 1 are 3.1k entries: the sort takes 6.5 MB, rows and phases 3 MB (by the points
+    they took 154), so 16 MB are enough, to the same bits."""
+    pts = uniform_ball(200000, 1000.0, seed=1)
+    ppc = catana.PixelizedPointContainer(1, catana.PointContainer(pts))
+
+    def call():
+        return catana.sfb_decomposition(ppc, 24, 4, 1000.0, True, False)
+
+    ref = call()
+    with _AllocLimit(16 << 20):
+        got = call()
+    assert np.array_equal(got.c_ln, ref.c_ln)
