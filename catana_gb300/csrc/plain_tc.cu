@@ -1318,9 +1318,13 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         entries = perm;
         entry_r = rint;
     }
-    // points per pass: rows and phases (32 B per point and m) stay under 12 GB
-    int64_t chunk = std::max<int64_t>(TC_KT, (int64_t)(12e9 / (32.0 * lmp)) / TC_KT * TC_KT);
-    chunk = std::min(chunk, npoints);
+    // Points per pass: the rows and phases (32 B per point and m) stay under 4 GB, the J of one level (8 B per point
+    // and radial order) under 2 GB, and so do the sums of more slabs than there are SMs.
+    const double slab_bytes = 16.0 * lmax * nmax;  // of the largest level
+    const int64_t slabs_c = std::max<int64_t>(ctx->sm_count, (int64_t)(2e9 / slab_bytes));
+    double fit = std::min(4e9 / (32.0 * lmp), (double)slabs_c * TC_SLAB_TILES * TC_KT);
+    if (!fused) fit = std::min(fit, 2e9 / (8.0 * nmax));
+    const int64_t chunk = std::min(npoints, std::max<int64_t>(TC_KT, (int64_t)fit / TC_KT * TC_KT));
     const int tiles_c = ceil_div(chunk, TC_KT);
     const size_t np = (size_t)tiles_c * TC_KT;
     // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]

@@ -250,3 +250,20 @@ def test_a_pixelized_workspace_goes_by_the_entries(cuda_device):
     with _AllocLimit(16 << 20):
         got = call()
     assert np.array_equal(got.c_ln, ref.c_ln)
+
+
+def test_one_level_of_many_radial_orders_is_cut_too(cuda_device):
+    """300k points with 1000 radial orders have 2.4 GB of j_l in one level; a pass takes as many points as keep it under
+    2 GB.  The catalog's sums are those of its halves, in another order: 1e-12 of the level's largest |f|."""
+    n, lmax, nmax = 300000, 2, 1000
+    pts = uniform_ball(n, 1000.0, seed=2)
+
+    def call(p):
+        return catana.sfb_decomposition(catana.PointContainer(p), lmax, nmax, 1000.0, True, False, interpolation="poly").f_lmn
+
+    with _AllocLimit(2100 << 20):
+        whole = call(pts)
+    halves = [call(pts[: n // 2]), call(pts[n // 2:])]
+    for l in range(lmax):
+        both = 0.5 * (halves[0][l] + halves[1][l])
+        assert np.max(np.abs(whole[l] - both)) <= 1e-12 * np.max(np.abs(both)), l
