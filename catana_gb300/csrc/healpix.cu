@@ -667,9 +667,10 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
             px.tw_off = tw_off;
             s = plain_tc_pixels(ctx, px, npoints, lmax, nmax, rmax, interpolated ? JL_MODE_LERP : JL_MODE_EXACT, kln_dev,
                                 f_dev, err_dev, st);
-            if (s != CATANA_OK) return s;
+            if (s != CATANA_OK && s != CATANA_ERR_NOMEM) return s;
         }
-        return finish_flmn_cln(f_dev, norm, lmax, nmax, c_ln_dev, st);
+        if (s == CATANA_OK) return finish_flmn_cln(f_dev, norm, lmax, nmax, c_ln_dev, st);
+        set_error("");  // the maps may fit
     }
     s = ensure_coefs(ctx, lmax + 1, st);
     if (s != CATANA_OK) return s;

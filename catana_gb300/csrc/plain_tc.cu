@@ -1245,6 +1245,7 @@ std::atomic<uint64_t> g_plain_stall_ns{0};
 
 namespace {
 
+// CATANA_ERR_NOMEM: nothing has been added, and the caller has another path.
 // pix == nullptr: points_dev are npoints x 3; otherwise the pixelized catalog.  "Points" below are what the main
 // kernel takes as such: the catalog's points, or a pixelized one's entries.
 catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, const PixelCatalog *pix,
@@ -1319,26 +1320,42 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         entry_r = rint;
     }
     // Points per pass: the rows and phases (32 B per point and m) stay under 4 GB, the J of one level (8 B per point
-    // and radial order) under 2 GB, and so do the sums of more slabs than there are SMs.
+    // and radial order) under 2 GB, and so do the sums of more slabs than there are SMs.  The levels of a launch go by
+    // their sums, 256 MB (they are read back at once and mostly hit L2), and their J, 2 GB.  Where that cannot be had
+    // everything is cut to a quarter, and again, as long as a pass gives every SM a tile; nothing is allocated after.
     const double slab_bytes = 16.0 * lmax * nmax;  // of the largest level
-    const int64_t slabs_c = std::max<int64_t>(ctx->sm_count, (int64_t)(2e9 / slab_bytes));
-    double fit = std::min(4e9 / (32.0 * lmp), (double)slabs_c * TC_SLAB_TILES * TC_KT);
-    if (!fused) fit = std::min(fit, 2e9 / (8.0 * nmax));
-    const int64_t chunk = std::min(npoints, std::max<int64_t>(TC_KT, (int64_t)fit / TC_KT * TC_KT));
-    const int tiles_c = ceil_div(chunk, TC_KT);
-    const size_t np = (size_t)tiles_c * TC_KT;
-    // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
-    const size_t kb = pix ? 0 : tc_al(np * 4), hb = pix ? 0 : tc_al(radix_hist_words((int64_t)np) * 4);
-    const size_t o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(np * 8), o_xs = o_rabs + tc_al(np * 8);
-    const size_t o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
+    double scale = 1.0;
+    int64_t chunk;
     // slabs: at most TC_SLAB_TILES tiles (the 64-bit sums' resolution), a whole number of waves
     auto slab_tiles = [&](int tiles) {
         const int waves = ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES);
         return ceil_div(tiles, (int64_t)ctx->sm_count * waves);
     };
-    const int max_slabs = ctx->sm_count * ceil_div(tiles_c, (int64_t)ctx->sm_count * TC_SLAB_TILES);
-    const size_t o_mx = o_sl + tc_al((size_t)max_slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)max_slabs * 3 * TC_LMAX * 4);
-    CG_CUDA_TRY(ctx->tc_ws.ensure(o_poi + 256));
+    // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
+    size_t kb, hb, o_rint, o_rabs, o_xs, o_rows, o_ph, o_sl, o_mx, o_poi;
+    for (;; scale *= 0.25) {
+        const double slabs_c = std::max((double)ctx->sm_count, scale * 2e9 / slab_bytes);
+        double fit = std::min(scale * 4e9 / (32.0 * lmp), slabs_c * TC_SLAB_TILES * TC_KT);
+        if (!fused) fit = std::min(fit, scale * 2e9 / (8.0 * nmax));
+        chunk = std::min(npoints, std::max<int64_t>(TC_KT, (int64_t)fit / TC_KT * TC_KT));
+        const int tiles = ceil_div(chunk, TC_KT);
+        const size_t np = (size_t)tiles * TC_KT;
+        kb = pix ? 0 : tc_al(np * 4), hb = pix ? 0 : tc_al(radix_hist_words((int64_t)np) * 4);
+        o_rint = 4 * kb + hb, o_rabs = o_rint + tc_al(np * 8), o_xs = o_rabs + tc_al(np * 8);
+        o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
+        // a last pass of fewer points may have more slabs, up to this many
+        const int slabs = std::min(tiles, ctx->sm_count * ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES));
+        o_mx = o_sl + tc_al((size_t)slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)slabs * 3 * TC_LMAX * 4);
+        const double sums = std::max(slab_bytes * slabs, std::min(scale * 256e6, 0.5 * (lmax + 1) * slab_bytes * slabs));
+        const double ntab = std::min(sums, slab_bytes * slabs);
+        const double jl = fused ? 0.0 : 8.0 * np * nmax;
+        cudaError_t e = ctx->tc_ws.ensure(o_poi + 256);
+        if (e == cudaSuccess) e = ctx->partial.ensure((size_t)(sums + ntab) + 512);
+        if (e == cudaSuccess) e = ctx->tc_jarr.ensure((size_t)std::max(jl, std::min(scale * 2e9, jl * lmax)));
+        if (e == cudaSuccess) break;
+        const bool again = e == cudaErrorMemoryAllocation && (chunk > (int64_t)ctx->sm_count * TC_KT || scale == 1.0);
+        if (!again) CG_CUDA_TRY(e);
+    }
     char *ws = ctx->tc_ws.as<char>();
     uint32_t *keys = reinterpret_cast<uint32_t *>(ws), *perm = reinterpret_cast<uint32_t *>(ws + kb);
     uint32_t *tk = reinterpret_cast<uint32_t *>(ws + 2 * kb), *tv = reinterpret_cast<uint32_t *>(ws + 3 * kb);
@@ -1401,18 +1418,15 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             if (fused) a.tab = ctx->tc_tab.as<double2>();
             dxinv = reinterpret_cast<const double *>(ctx->tc_tab.as<char>() + ctx->tc_tab_off);
         }
-        // levels per launch: the slabs' partial sums stay under 256 MB (they are read back at once and
-        // mostly hit L2), the j_l arrays of the other modes under 2 GB
         for (int l0 = 0; l0 < lmax;) {
             int l1 = l0 + 1;
             auto pdoubles = [&](int e) { return (int64_t)nmax * ((int64_t)e * (e + 1) - (int64_t)l0 * (l0 + 1)); };
             const double jbytes = fused ? 0.0 : 8.0 * tiles * TC_KT * nmax;
-            while (l1 < lmax && pdoubles(l1 + 1) * 8.0 * nslabs < 256e6 && jbytes * (l1 + 1 - l0) < 2e9) ++l1;
+            while (l1 < lmax && pdoubles(l1 + 1) * 8.0 * nslabs < scale * 256e6 && jbytes * (l1 + 1 - l0) < scale * 2e9) ++l1;
             a.l0 = l0;
             a.l1 = l1;
             a.pslab = pdoubles(l1);
             const size_t pb = tc_al((size_t)a.pslab * nslabs * 8);
-            CG_CUDA_TRY(ctx->partial.ensure(pb + (size_t)nslabs * (l1 - l0) * nmax * sizeof(uint4)));
             a.partial = ctx->partial.as<double>();
             uint4 *ntab = reinterpret_cast<uint4 *>(ctx->partial.as<char>() + pb);
             a.ntab = ntab;
@@ -1422,7 +1436,6 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             a.jarr = nullptr;
             if (!fused) {
                 const int64_t cnt = (int64_t)(l1 - l0) * tiles * nmax * TC_KT;
-                CG_CUDA_TRY(ctx->tc_jarr.ensure((size_t)cnt * 8));
                 uint64_t *ja = ctx->tc_jarr.as<uint64_t>();
                 TcJ j;
                 j.r = pix ? pix->r : reinterpret_cast<const double *>(ws + o_rabs);

@@ -532,9 +532,12 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
         if (s != CATANA_OK) return s;
         rtop = max_r;
     }
-    if (plain_tc_takes(ctx, lmax, nmax, rmax) && plain_tc_pays(npoints, lmax, nmax, jl) && (!weights_dev || plain_tc_holds(wr)))
-        return plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, rtop, kln_dev,
-                                   f_acc_dev, err_dev, st);
+    if (plain_tc_takes(ctx, lmax, nmax, rmax) && plain_tc_pays(npoints, lmax, nmax, jl) && (!weights_dev || plain_tc_holds(wr))) {
+        s = plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, rtop, kln_dev, f_acc_dev,
+                                err_dev, st);
+        if (s != CATANA_ERR_NOMEM) return s;
+        set_error("");  // the buffers here are smaller
+    }
     // Chunk so that the three Legendre rows stay under ~1.5 GB.
     int64_t chunk = (int64_t)(1.5e9 / (3.0 * 8.0 * std::max(lmax, 1)));
     chunk = std::max<int64_t>(1024, std::min<int64_t>(chunk, npoints));

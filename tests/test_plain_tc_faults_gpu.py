@@ -267,3 +267,53 @@ def test_one_level_of_many_radial_orders_is_cut_too(cuda_device):
     for l in range(lmax):
         both = 0.5 * (halves[0][l] + halves[1][l])
         assert np.max(np.abs(whole[l] - both)) <= 1e-12 * np.max(np.abs(both)), l
+
+
+def _launches(call):
+    n = _lib.lib.catana_gpu_launch_count()
+    return call(), _lib.lib.catana_gpu_launch_count() - n
+
+
+@pytest.mark.parametrize("n,lmax,nmax,limit,interp", [
+    # 17 MB of rows and phases: passes of 5208 points
+    (20000, 24, 4, 5 << 20, "on"), (20000, 24, 4, 5 << 20, "off"), (20000, 24, 4, 5 << 20, "poly"),
+    # tables of 3.8 MB fit, their pair form of 7.7 does not: the FP64 path
+    (600, 24, 20, 6 << 20, "on")])
+def test_memory_that_cannot_be_had(cuda_device, n, lmax, nmax, limit, interp):
+    """Smaller passes, and past them the FP64 path, whose buffers are smaller: the sums in another order, and with the
+    FP64 path another table position (4e-14 of j_l's envelope) and recurrence: 1e-12 of the level's largest |f|."""
+    pts = uniform_ball(n, 1000.0, seed=n)
+    w = np.random.default_rng(n).uniform(0.5, 1.5, n)
+
+    def call(nmax=nmax):
+        return catana.sfb_decomposition(catana.PointContainer(pts), lmax, nmax, 1000.0, True, False, weights=w,
+                                        interpolation=interp).f_lmn
+
+    call(nmax - 1)  # tables of another nmax: both calls build their own
+    ref, few = _launches(call)
+    call(nmax - 1)
+    with _AllocLimit(limit):
+        got, more = _launches(call)
+    assert more > few  # more passes, or a launch per level
+    for l in range(lmax):
+        assert np.max(np.abs(got[l] - ref[l])) <= 1e-12 * np.max(np.abs(ref[l])), l
+
+
+@pytest.mark.parametrize("nside,n,lmax,nmax,limit", [(32, 40000, 24, 4, 5 << 20), (4, 3000, 10, 6, 800 << 10)])
+def test_memory_that_cannot_be_had_pixelized(cuda_device, nside, n, lmax, nmax, limit):
+    """The same for the pixelized sum: 12k entries in passes; room for the tables
+    (0.5 MB) but not for their pair form, so the maps."""
+    ppc = catana.PixelizedPointContainer(nside, catana.PointContainer(uniform_ball(n, 1000.0, seed=n)))
+
+    def call(nmax=nmax):
+        return catana.sfb_decomposition(ppc, lmax, nmax, 1000.0, True, False).f_lmn
+
+    call(nmax - 1)
+    ref, few = _launches(call)
+    call(nmax - 1)
+    with _AllocLimit(limit):
+        got, more = _launches(call)
+    assert more > few  # more passes, or a launch per level
+    fmax = max(np.max(np.abs(f)) for f in ref)
+    for l in range(lmax):
+        assert np.max(np.abs(got[l] - ref[l])) <= 1e-12 * fmax, l
