@@ -11,8 +11,9 @@
 // the breakpoints are the table's nodes, and a fixed Gauss-Legendre rule per segment integrates the
 // product of the two Bessel functions -- an entire function of exponential type k1 + k2 -- to
 // 2^(2p+1) p!^4 / ((2p+1) (2p)!^3) (kappa / 2)^(2p), kappa = (k1 + k2) length: below 1e-14 for p = 2, 3, 4, 8 points
-// and kappa up to 0.002, 0.046, 0.23, 3.4 (longer segments are cut).  kappa takes the call's largest k, and at
-// least (l + 1) / rmax, the growth of j_l below its turning point.
+// and kappa up to 0.002, 0.046, 0.23, 3.4 (longer segments are cut).  kappa takes the largest k of pairs whose
+// segments are cut into like numbers (within a factor of eight), and at least (l + 1) / rmax, the growth of j_l below
+// its turning point.
 //   k_dsb_nodes   abscissae and weights (rule times w) of a chunk of the quadrature
 //   k_dsb_bessel  j_l(k x) for the call's distinct k: K x nodes evaluations instead of two per pair and node
 //                 (a matrix of n x n pairs has n distinct k) -- the FP64 recurrences bound the call
@@ -20,6 +21,7 @@
 // Measured, GB300: l 16, 32 x 32 pairs, 10001 nodes, host arrays in and out: 58.2 ms one warp per pair with
 // both j_l evaluated at every node, 0.54 ms so.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -113,6 +115,82 @@ void gauss_legendre(int n, double *x, double *w) {
     }
 }
 
+// One call's weight table and range
+struct DsbCall {
+    int l;
+    const double *w;
+    int64_t wn;
+    double wmin, wdx, rmax;
+    // (k1 + k2) length of a piece of the segments inside (0, rmax), uncut
+    double kappa(double kmax) const { return 2.0 * std::max(kmax, (l + 1.0) / rmax) * std::min(wdx, rmax); }
+    double cuts(double kmax) const { return std::max(1.0, std::ceil(kappa(kmax) / 3.4)); }
+};
+
+// The integrals of pairs with k <= kmax (host arrays), by one rule
+catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, const double *k1, const double *k2, int64_t npairs,
+                          double *out, cudaStream_t st) {
+    std::vector<double> ks(k1, k1 + npairs);
+    ks.insert(ks.end(), k2, k2 + npairs);
+    std::sort(ks.begin(), ks.end());
+    ks.erase(std::unique(ks.begin(), ks.end()), ks.end());
+    // each pair's two places among the distinct k
+    std::vector<uint32_t> idx(2 * (size_t)npairs);
+    for (int64_t i = 0; i < npairs; ++i) {
+        idx[i] = (uint32_t)(std::lower_bound(ks.begin(), ks.end(), k1[i]) - ks.begin());
+        idx[npairs + i] = (uint32_t)(std::lower_bound(ks.begin(), ks.end(), k2[i]) - ks.begin());
+    }
+    const size_t nk = ks.size();
+    // the rule: table segments from that of 0 to that of r_max
+    DsbRule R;
+    R.wmin = C.wmin;
+    R.wdx = C.wdx;
+    R.wdxinv = 1.0 / R.wdx;
+    R.rmax = C.rmax;
+    R.seg0 = std::min<int64_t>(C.wn - 2, std::max<int64_t>(0, (int64_t)std::floor((0.0 - C.wmin) * R.wdxinv)));
+    const int64_t sl = std::min<int64_t>(C.wn - 2, (int64_t)std::floor((C.rmax - C.wmin) * R.wdxinv));
+    R.nseg = std::max<int64_t>(1, sl - R.seg0 + 1);
+    const double kappa = C.kappa(kmax), cuts = C.cuts(kmax);
+    R.p = kappa <= 0.002 ? 2 : kappa <= 0.046 ? 3 : kappa <= 0.23 ? 4 : 8;
+    if (!(cuts < 2e9) || cuts * (double)R.nseg * R.p > 1e11) {
+        set_error("sbessel_integrals: k r_max too large");
+        return CATANA_ERR_ARG;
+    }
+    R.cuts = (int)cuts;
+    gauss_legendre(R.p, R.x, R.w);
+    const int64_t nodes = R.nseg * R.cuts * R.p;
+    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+    // nodes per pass: the Bessel rows and the weighted ones stay under 512 MB
+    const int64_t chunk = std::max<int64_t>(1024, std::min<int64_t>(nodes, (int64_t)(512e6 / (16.0 * (double)nk))));
+    const size_t wb = al((size_t)C.wn * 8), kb = al(nk * 8), ib = al((size_t)npairs * 8), ob = al((size_t)npairs * 8),
+                 cb = al((size_t)chunk * 8), jb = al(nk * (size_t)chunk * 8);
+    CG_CUDA_TRY(ctx->io_points.ensure(wb + kb + ib + ob + 2 * cb + 2 * jb + 256));
+    char *d = ctx->io_points.as<char>();
+    double *wd = reinterpret_cast<double *>(d), *kd = reinterpret_cast<double *>(d + wb),
+           *od = reinterpret_cast<double *>(d + wb + kb + ib), *xd = reinterpret_cast<double *>(d + wb + kb + ib + ob),
+           *qd = reinterpret_cast<double *>(d + wb + kb + ib + ob + cb),
+           *jd = reinterpret_cast<double *>(d + wb + kb + ib + ob + 2 * cb),
+           *jw = reinterpret_cast<double *>(d + wb + kb + ib + ob + 2 * cb + jb);
+    uint32_t *id = reinterpret_cast<uint32_t *>(d + wb + kb);
+    CG_CUDA_TRY(cudaMemcpyAsync(wd, C.w, (size_t)C.wn * 8, cudaMemcpyHostToDevice, st));
+    CG_CUDA_TRY(cudaMemcpyAsync(kd, ks.data(), nk * 8, cudaMemcpyHostToDevice, st));
+    CG_CUDA_TRY(cudaMemcpyAsync(id, idx.data(), idx.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    for (int64_t q0 = 0; q0 < nodes; q0 += chunk) {
+        const int64_t nq = std::min(chunk, nodes - q0);
+        k_dsb_nodes<<<ceil_div(nq, 256), 256, 0, st>>>(R, wd, q0, nq, xd, qd);
+        for (size_t k0 = 0; k0 < nk; k0 += 65535) {
+            k_dsb_bessel<<<dim3(ceil_div(nq, 256), (unsigned)std::min<size_t>(65535, nk - k0)), 256, 0, st>>>(
+                kd + k0, xd, qd, nq, C.l, jd + k0 * (size_t)nq, jw + k0 * (size_t)nq);
+            count_launch();
+        }
+        k_dsb_pairs<<<(unsigned)npairs, DSB_T, 0, st>>>(jd, jw, nq, id, id + npairs, q0 == 0 ? 1 : 0, od);
+        count_launch(2);
+        CG_CUDA_TRY(cudaGetLastError());
+    }
+    CG_CUDA_TRY(cudaMemcpyAsync(out, od, (size_t)npairs * 8, cudaMemcpyDeviceToHost, st));
+    CG_CUDA_TRY(cudaStreamSynchronize(st));
+    return CATANA_OK;
+}
+
 }  // namespace
 
 }  // namespace catana_gpu
@@ -142,71 +220,46 @@ catana_status_t catana_gpu_sbessel_integrals(const double *w_table, int64_t w_n,
         set_error("argument outside range for which this FunctionInterpolator is defined");
         return CATANA_ERR_DOMAIN;
     }
-    // the distinct k and each pair's two places among them
-    std::vector<double> ks(k1, k1 + npairs);
-    ks.insert(ks.end(), k2, k2 + npairs);
-    std::sort(ks.begin(), ks.end());
-    ks.erase(std::unique(ks.begin(), ks.end()), ks.end());
-    std::vector<uint32_t> idx(2 * (size_t)npairs);
-    for (int64_t i = 0; i < npairs; ++i) {
-        idx[i] = (uint32_t)(std::lower_bound(ks.begin(), ks.end(), k1[i]) - ks.begin());
-        idx[npairs + i] = (uint32_t)(std::lower_bound(ks.begin(), ks.end(), k2[i]) - ks.begin());
-    }
-    const size_t nk = ks.size();
-    // the rule: table segments from that of 0 to that of r_max
-    DsbRule R;
-    R.wmin = w_min;
-    R.wdx = (w_max - w_min) / (double)(w_n - 1);
-    R.wdxinv = 1.0 / R.wdx;
-    R.rmax = r_max;
-    R.seg0 = std::min<int64_t>(w_n - 2, std::max<int64_t>(0, (int64_t)std::floor((0.0 - w_min) * R.wdxinv)));
-    const int64_t sl = std::min<int64_t>(w_n - 2, (int64_t)std::floor((r_max - w_min) * R.wdxinv));
-    R.nseg = std::max<int64_t>(1, sl - R.seg0 + 1);
-    const double kappa = 2.0 * std::max(kmax, (l + 1.0) / r_max) * R.wdx;
-    R.p = kappa <= 0.002 ? 2 : kappa <= 0.046 ? 3 : kappa <= 0.23 ? 4 : 8;
-    const double cuts = std::max(1.0, std::ceil(kappa / 3.4));
-    if (!(cuts < 1e8) || cuts * (double)R.nseg * R.p > 1e11) {
-        set_error("sbessel_integrals: k r_max too large");
-        return CATANA_ERR_ARG;
-    }
-    R.cuts = (int)cuts;
-    gauss_legendre(R.p, R.x, R.w);
-    const int64_t nodes = R.nseg * R.cuts * R.p;
     int cs;
     DeviceContext *ctx = get_context(&cs);
     if (!ctx) return (catana_status_t)cs;
     std::lock_guard<std::mutex> g(ctx->mu);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    // nodes per pass: the Bessel rows and the weighted ones stay under 512 MB, the distinct k within a grid's second dimension
-    const int64_t chunk = std::max<int64_t>(1024, std::min<int64_t>(nodes, (int64_t)(512e6 / (16.0 * (double)nk))));
-    const size_t wb = al((size_t)w_n * 8), kb = al(nk * 8), ib = al((size_t)npairs * 8), ob = al((size_t)npairs * 8),
-                 cb = al((size_t)chunk * 8), jb = al(nk * (size_t)chunk * 8);
-    CG_CUDA_TRY(ctx->io_points.ensure(wb + kb + ib + ob + 2 * cb + 2 * jb + 256));
-    char *d = ctx->io_points.as<char>();
-    double *wd = reinterpret_cast<double *>(d), *kd = reinterpret_cast<double *>(d + wb),
-           *od = reinterpret_cast<double *>(d + wb + kb + ib), *xd = reinterpret_cast<double *>(d + wb + kb + ib + ob),
-           *qd = reinterpret_cast<double *>(d + wb + kb + ib + ob + cb),
-           *jd = reinterpret_cast<double *>(d + wb + kb + ib + ob + 2 * cb),
-           *jw = reinterpret_cast<double *>(d + wb + kb + ib + ob + 2 * cb + jb);
-    uint32_t *id = reinterpret_cast<uint32_t *>(d + wb + kb);
-    CG_CUDA_TRY(cudaMemcpyAsync(wd, w_table, (size_t)w_n * 8, cudaMemcpyHostToDevice, st));
-    CG_CUDA_TRY(cudaMemcpyAsync(kd, ks.data(), nk * 8, cudaMemcpyHostToDevice, st));
-    CG_CUDA_TRY(cudaMemcpyAsync(id, idx.data(), idx.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    for (int64_t q0 = 0; q0 < nodes; q0 += chunk) {
-        const int64_t nq = std::min(chunk, nodes - q0);
-        k_dsb_nodes<<<ceil_div(nq, 256), 256, 0, st>>>(R, wd, q0, nq, xd, qd);
-        for (size_t k0 = 0; k0 < nk; k0 += 65535) {
-            k_dsb_bessel<<<dim3(ceil_div(nq, 256), (unsigned)std::min<size_t>(65535, nk - k0)), 256, 0, st>>>(
-                kd + k0, xd, qd, nq, (int)l, jd + k0 * (size_t)nq, jw + k0 * (size_t)nq);
-            count_launch();
-        }
-        k_dsb_pairs<<<(unsigned)npairs, DSB_T, 0, st>>>(jd, jw, nq, id, id + npairs, q0 == 0 ? 1 : 0, od);
-        count_launch(2);
-        CG_CUDA_TRY(cudaGetLastError());
+    DsbCall C;
+    C.l = (int)l;
+    C.w = w_table;
+    C.wn = w_n;
+    C.wmin = w_min;
+    C.wdx = (w_max - w_min) / (double)(w_n - 1);
+    C.rmax = r_max;
+    if (C.cuts(kmax) < 8.0) return dsb_group(ctx, C, kmax, k1, k2, npairs, out, st);
+    // The pairs by the octal order of their pieces per segment: a pair is not integrated on pieces that only a much larger k
+    // of the call asks for.
+    std::vector<int> order(npairs);
+    int lo = INT_MAX, hi = 0;
+    for (int64_t i = 0; i < npairs; ++i) {
+        order[i] = (int)(std::log2(C.cuts(std::max(k1[i], k2[i]))) / 3.0);
+        lo = std::min(lo, order[i]);
+        hi = std::max(hi, order[i]);
     }
-    CG_CUDA_TRY(cudaMemcpyAsync(out, od, (size_t)npairs * 8, cudaMemcpyDeviceToHost, st));
-    CG_CUDA_TRY(cudaStreamSynchronize(st));
+    if (lo == hi) return dsb_group(ctx, C, kmax, k1, k2, npairs, out, st);
+    for (int o = lo; o <= hi; ++o) {
+        std::vector<int64_t> at;
+        std::vector<double> a, b;
+        double km = 0.0;
+        for (int64_t i = 0; i < npairs; ++i)
+            if (order[i] == o) {
+                at.push_back(i);
+                a.push_back(k1[i]);
+                b.push_back(k2[i]);
+                km = std::max(km, std::max(k1[i], k2[i]));
+            }
+        if (at.empty()) continue;
+        std::vector<double> v(at.size());
+        const catana_status_t s = dsb_group(ctx, C, km, a.data(), b.data(), (int64_t)at.size(), v.data(), st);
+        if (s != CATANA_OK) return s;
+        for (size_t i = 0; i < at.size(); ++i) out[at[i]] = v[i];
+    }
     return CATANA_OK;
 }
 

@@ -65,3 +65,20 @@ def test_many_distinct_k_in_passes(cuda_device):
     got = besseltools.double_sbessel_integrator(fi, 5, 100.0, k1, k2)
     one = np.array([besseltools.double_sbessel_integrator(fi, 5, 100.0, a, b) for a, b in zip(k1[:20], k2[:20])])
     assert np.max(np.abs(got[:20] - one)) <= 1e-13 * np.max(np.abs(one))
+
+
+def test_one_large_k_does_not_set_the_others_rule(cuda_device):
+    """200 pairs of small k and one whose segments take some 200 pieces each: two rules, a pass each (by one rule 3.2M nodes
+    for 402 wave numbers, 41 passes), and each pair as by itself."""
+    from catana_gb300 import _lib
+    rng = np.random.default_rng(3)
+    fi = catana.FunctionInterpolator(lambda r: np.exp(-(r / 30) ** 2), 2001, 0.0, 100.0)
+    k1, k2 = rng.uniform(0.05, 2.0, 201), rng.uniform(0.05, 2.0, 201)
+    k1[77], k2[77] = 6400.0, 6000.0
+    n0 = _lib.lib.catana_gpu_launch_count()
+    got = besseltools.double_sbessel_integrator(fi, 3, 100.0, k1, k2)
+    assert _lib.lib.catana_gpu_launch_count() - n0 <= 6
+    one = np.array([besseltools.double_sbessel_integrator(fi, 3, 100.0, a, b) for a, b in zip(k1, k2)])
+    rest = np.arange(201) != 77
+    assert np.max(np.abs(got - one)[rest]) <= 1e-13 * np.max(np.abs(one[rest]))
+    assert abs(got[77] - one[77]) <= 1e-13 * abs(one[77])
