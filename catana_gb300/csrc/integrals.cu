@@ -126,13 +126,12 @@ struct DsbCall {
     double cuts(double kmax) const { return std::max(1.0, std::ceil(kappa(kmax) / 3.4)); }
 };
 
+// distinct k of a pass: their Bessel rows and the weighted ones, of 1024 nodes, take 512 MB
+constexpr size_t DSB_MAXK = 31250;
+
 // The integrals of pairs with k <= kmax (host arrays), by one rule
 catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, const double *k1, const double *k2, int64_t npairs,
-                          double *out, cudaStream_t st) {
-    std::vector<double> ks(k1, k1 + npairs);
-    ks.insert(ks.end(), k2, k2 + npairs);
-    std::sort(ks.begin(), ks.end());
-    ks.erase(std::unique(ks.begin(), ks.end()), ks.end());
+                          const std::vector<double> &ks, double *out, cudaStream_t st) {
     // each pair's two places among the distinct k
     std::vector<uint32_t> idx(2 * (size_t)npairs);
     for (int64_t i = 0; i < npairs; ++i) {
@@ -159,7 +158,7 @@ catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, con
     gauss_legendre(R.p, R.x, R.w);
     const int64_t nodes = R.nseg * R.cuts * R.p;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    // nodes per pass: the Bessel rows and the weighted ones stay under 512 MB
+    // nodes per pass: the Bessel rows and the weighted ones stay under 512 MB (up to DSB_MAXK distinct k)
     const int64_t chunk = std::max<int64_t>(1024, std::min<int64_t>(nodes, (int64_t)(512e6 / (16.0 * (double)nk))));
     const size_t wb = al((size_t)C.wn * 8), kb = al(nk * 8), ib = al((size_t)npairs * 8), ob = al((size_t)npairs * 8),
                  cb = al((size_t)chunk * 8), jb = al(nk * (size_t)chunk * 8);
@@ -177,17 +176,34 @@ catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, con
     for (int64_t q0 = 0; q0 < nodes; q0 += chunk) {
         const int64_t nq = std::min(chunk, nodes - q0);
         k_dsb_nodes<<<ceil_div(nq, 256), 256, 0, st>>>(R, wd, q0, nq, xd, qd);
-        for (size_t k0 = 0; k0 < nk; k0 += 65535) {
-            k_dsb_bessel<<<dim3(ceil_div(nq, 256), (unsigned)std::min<size_t>(65535, nk - k0)), 256, 0, st>>>(
-                kd + k0, xd, qd, nq, C.l, jd + k0 * (size_t)nq, jw + k0 * (size_t)nq);
-            count_launch();
-        }
+        k_dsb_bessel<<<dim3(ceil_div(nq, 256), (unsigned)nk), 256, 0, st>>>(kd, xd, qd, nq, C.l, jd, jw);
         k_dsb_pairs<<<(unsigned)npairs, DSB_T, 0, st>>>(jd, jw, nq, id, id + npairs, q0 == 0 ? 1 : 0, od);
-        count_launch(2);
+        count_launch(3);
         CG_CUDA_TRY(cudaGetLastError());
     }
     CG_CUDA_TRY(cudaMemcpyAsync(out, od, (size_t)npairs * 8, cudaMemcpyDeviceToHost, st));
     CG_CUDA_TRY(cudaStreamSynchronize(st));
+    return CATANA_OK;
+}
+
+// The same for any number of distinct k: in runs of pairs where they are too many for a pass
+catana_status_t dsb_pairs(DeviceContext *ctx, const DsbCall &C, double kmax, const double *k1, const double *k2, int64_t npairs,
+                          double *out, cudaStream_t st) {
+    auto distinct = [&](int64_t b, int64_t e) {
+        std::vector<double> ks(k1 + b, k1 + e);
+        ks.insert(ks.end(), k2 + b, k2 + e);
+        std::sort(ks.begin(), ks.end());
+        ks.erase(std::unique(ks.begin(), ks.end()), ks.end());
+        return ks;
+    };
+    std::vector<double> ks = distinct(0, npairs);
+    if (ks.size() <= DSB_MAXK) return dsb_group(ctx, C, kmax, k1, k2, npairs, ks, out, st);
+    const int64_t run = DSB_MAXK / 2;
+    for (int64_t b = 0; b < npairs; b += run) {
+        const int64_t e = std::min(npairs, b + run);
+        const catana_status_t s = dsb_group(ctx, C, kmax, k1 + b, k2 + b, e - b, distinct(b, e), out + b, st);
+        if (s != CATANA_OK) return s;
+    }
     return CATANA_OK;
 }
 
@@ -232,7 +248,7 @@ catana_status_t catana_gpu_sbessel_integrals(const double *w_table, int64_t w_n,
     C.wmin = w_min;
     C.wdx = (w_max - w_min) / (double)(w_n - 1);
     C.rmax = r_max;
-    if (C.cuts(kmax) < 8.0) return dsb_group(ctx, C, kmax, k1, k2, npairs, out, st);
+    if (C.cuts(kmax) < 8.0) return dsb_pairs(ctx, C, kmax, k1, k2, npairs, out, st);
     // The pairs by the octal order of their pieces per segment: a pair is not integrated on pieces that only a much larger k
     // of the call asks for.
     std::vector<int> order(npairs);
@@ -242,7 +258,7 @@ catana_status_t catana_gpu_sbessel_integrals(const double *w_table, int64_t w_n,
         lo = std::min(lo, order[i]);
         hi = std::max(hi, order[i]);
     }
-    if (lo == hi) return dsb_group(ctx, C, kmax, k1, k2, npairs, out, st);
+    if (lo == hi) return dsb_pairs(ctx, C, kmax, k1, k2, npairs, out, st);
     for (int o = lo; o <= hi; ++o) {
         std::vector<int64_t> at;
         std::vector<double> a, b;
@@ -256,7 +272,7 @@ catana_status_t catana_gpu_sbessel_integrals(const double *w_table, int64_t w_n,
             }
         if (at.empty()) continue;
         std::vector<double> v(at.size());
-        const catana_status_t s = dsb_group(ctx, C, km, a.data(), b.data(), (int64_t)at.size(), v.data(), st);
+        const catana_status_t s = dsb_pairs(ctx, C, km, a.data(), b.data(), (int64_t)at.size(), v.data(), st);
         if (s != CATANA_OK) return s;
         for (size_t i = 0; i < at.size(); ++i) out[at[i]] = v[i];
     }

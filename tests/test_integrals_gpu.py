@@ -82,3 +82,19 @@ def test_one_large_k_does_not_set_the_others_rule(cuda_device):
     rest = np.arange(201) != 77
     assert np.max(np.abs(got - one)[rest]) <= 1e-13 * np.max(np.abs(one[rest]))
     assert abs(got[77] - one[77]) <= 1e-13 * abs(one[77])
+
+
+def test_distinct_k_beyond_a_pass_memory(cuda_device):
+    """100k distinct k: runs of pairs under 512 MB of Bessel rows (1.6 GB by one)."""
+    from catana_gb300 import _lib
+    rng = np.random.default_rng(4)
+    fi = catana.FunctionInterpolator(lambda r: np.exp(-(r / 30) ** 2), 401, 0.0, 100.0)
+    k1, k2 = rng.uniform(0.05, 2.0, 50000), rng.uniform(0.05, 2.0, 50000)
+    _lib.lib.catana_gpu_test_alloc_limit(600 << 20)
+    try:
+        got = besseltools.double_sbessel_integrator(fi, 2, 100.0, k1, k2)
+    finally:
+        _lib.lib.catana_gpu_test_alloc_limit(0)
+    some = np.concatenate([np.arange(0, 50000, 2500), [15624, 15625, 49999]])
+    one = np.array([besseltools.double_sbessel_integrator(fi, 2, 100.0, k1[i], k2[i]) for i in some])
+    assert np.max(np.abs(got[some] - one)) <= 1e-13 * np.max(np.abs(one))
