@@ -180,6 +180,7 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
 // lmax <= 512; with JL_MODE_POLY the caller has prepared ctx->poly and passes the largest radius (else rtop = 0).
 bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax);
 bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl);  // and whether it is the faster one
+double plain_tc_blocks(int lmax, int nmax);  // blocks that a CTA of it walks
 bool plain_tc_holds(const WeightRange &wr);  // and whether its fixed-point terms hold weights of this range
 catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
                                     int64_t npoints, int lmax, int nmax, double rmax, JlMode jl, double rtop,

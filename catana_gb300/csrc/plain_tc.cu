@@ -1228,17 +1228,28 @@ bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
 // weights differ by more takes the FP64 path.
 bool plain_tc_holds(const WeightRange &wr) { return !(wr.hi > 256.0 * wr.lo); }
 
-// Few points with many radial orders, or one or two levels: a CTA of the tensor-core kernel walks its blocks of 64
-// radial orders one after the other, 13 to 15 us each, where the FP64 path has a CTA for each and takes 40 us a
-// level (80 without the linear table, of 64 radial orders and more) and its FP64 work.  Microseconds a call, FP64 path / here:
-// 500 points, l 16: n 64 over 600 / 290, n 200 646 / 765, n 1000 955 / 3849; 2000 points, l 8: n 200 faster here,
-// n 400 728 / 750, n 1000 1266 / 1819; 1 point, l 1, n 1 79 / 94; 8000 points, l 1, n 64 139 / 151, l 2 faster here.
+double plain_tc_blocks(int lmax, int nmax) {
+    const double full = lmax / 64, rest = lmax - 64.0 * full;
+    return (32.0 * full * (full + 1.0) + rest * (full + 1.0)) * ((nmax + 63) / 64);
+}
+
+// Few points with many radial orders, and catalogs of a few levels, are the FP64 path's: a CTA of the tensor-core
+// kernel walks its blocks of 64 complex m and 64 radial orders one after the other, 11 to 15 us each (5 to 7 with one
+// or two column steps), where the FP64 path has a CTA for each, and takes 35 us a level below l = 32 and 89 above it, or its
+// FP64 work.  Microseconds, fitted to 742 calls (l 1 to 512, n 1 to 3000, 1 to 8192 points, the three j_l modes): the
+// path chosen is at most 1.2 times slower than the other, in all but 13 of them within 5%.  For instance, tensor
+// cores / FP64: 100 points, n 200: l 8 404 / 269, l 100 7405 / 7334, l 300 43400 / 26200; n 1000: l 24 6340 / 1070, l 128
+// 48300 / 10300, with 4000 points 70100 / 178000; n 64, l 512 33400 / 44900; l 1, n 16 81 / 44, l 8 120 / 184.
 bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl) {
-    if (npoints > 8192 || lmax > 64) return true;
-    const bool lerp = jl == JL_MODE_LERP;
-    const double nb = (nmax + 63) / 64, work = (double)npoints * 64.0 * nb;
-    const double fp64 = lmax * ((lerp ? 40.0 : 40.0 + 0.625 * std::min(nmax, 64)) + work * (2.8e-5 + 3.4e-6 * (lmax + 1)));
-    return (lerp ? 60.0 : 100.0) + (13.0 + 1e-3 * (double)npoints) * nb * lmax < fp64;
+    const bool few = nmax <= 32, exact = jl == JL_MODE_EXACT;
+    const double n = (double)npoints, l = lmax, values = n * nmax * l;
+    const double tc = 68.0 + plain_tc_blocks(lmax, nmax) * ((few ? 5.4 : 11.0) + (npoints >= 32 ? 1.5 : 0.0) + 4.9e-4 * n) +
+                      (exact ? values * (5.6e-5 + 6.1e-6 * l) : 0.0);
+    double base = (few ? 22.0 : 35.0) * std::min(lmax, 32) + (few ? 80.0 : 89.0) * std::max(lmax - 32, 0);
+    if (jl == JL_MODE_POLY) base += 6.0 * l;
+    if (exact) base += 13.0 * l * l * std::min(nmax, 64) / 64.0 * (npoints < 32 ? 0.28 : 1.0);
+    const double work = n * 64.0 * ((nmax + 63) / 64) * l * (6.2e-5 + 2.4e-6 * (l + 1.0)) + (exact ? values * 3.4e-5 * l : 0.0);
+    return tc < 23.0 + std::sqrt(std::sqrt(base * base * base * base + work * work * work * work));
 }
 
 std::atomic<uint64_t> g_plain_stall_ns{0};

@@ -317,3 +317,23 @@ def test_memory_that_cannot_be_had_pixelized(cuda_device, nside, n, lmax, nmax, 
     fmax = max(np.max(np.abs(f)) for f in ref)
     for l in range(lmax):
         assert np.max(np.abs(got[l] - ref[l])) <= 1e-12 * fmax, l
+
+
+@pytest.mark.parametrize("n,lmax,nmax,fp64", [(100, 80, 600, True), (2, 300, 200, True), (20, 1, 16, True), (300, 100, 64, False),
+                                              (100, 512, 64, False), (4000, 70, 300, False), (300, 6, 64, False)])
+def test_the_faster_path_for_few_points(cuda_device, n, lmax, nmax, fp64):
+    """The FP64 path launches two kernels a level, the tensor-core path at most three dozen for these in all; levels
+    below 4 agree with the other side's oracle in either."""
+    from oracle import oracle as O
+    pts = uniform_ball(n, 1000.0, seed=n)
+
+    def call():
+        return catana.sfb_decomposition(catana.PointContainer(pts), lmax, nmax, 1000.0, True, False, interpolation="on")
+
+    call()
+    res, launches = _launches(call)
+    assert (launches >= 2 * lmax + 1 and launches < 2 * lmax + 5) == fp64, launches
+    keep = min(lmax, 4)
+    f = O.sfb_raw(pts, keep, nmax, 1000.0, interpolated=True)[2]
+    for l in range(keep):
+        assert np.max(np.abs(res.f_lmn[l] - f[l])) <= 1e-10 * np.max(np.abs(f[l])), l
