@@ -621,8 +621,26 @@ catana_status_t healpix_bin_dev(DeviceContext *ctx, int64_t nside, const double 
     return CATANA_OK;
 }
 
+// Against the maps and FFTs below, the pixel sum on the tensor cores: ms 114 / 400 at nside 256, 1M points, l 128, n 64;
+// nside 64, 1.6M points, l 24: n 4 2.9 / 6.7, n 48 8.2 / 30; nside 16, 3M points (977 a pixel), l 10: n 4 4.0 / 8.7, n 48 8.0 /
+// 24; nside 1, 20k points, l 24, n 4: 0.44 / 12.  The maps win where little is summed: one or two levels (nside 16, 300
+// points, l 2, n 8: 171 us / 132), and many radial orders of few points, whose blocks of 64 a CTA of the tensor-core
+// kernel walks in turn (nside 1, 3 points, l 24, n 1500: 5820 / 940).  Microseconds, fitted to 595 calls (nside 1 to 256, 3 to
+// 10000 points, l 1 to 500, n 1 to 1500, both j_l modes), all but five of them within 5% of the faster path; max_pix, the points
+// of the fullest pixel, which the maps sum one after the other.  With more points the maps were ahead at l <= 2 only, by a
+// quarter at most (nside 16, 30000 points, l 2, n 8: 253 / 193; 1M points: 1365 / 1510).
+bool pixel_sum_pays(int64_t nside, int64_t npoints, int64_t max_pix, int lmax, int nmax, bool interpolated) {
+    if (npoints > 16384) return true;
+    const double ns = (double)nside, npix = 12.0 * ns * ns, n = (double)npoints, l = lmax, m = nmax;
+    const double tc = 200.0 + plain_tc_blocks(lmax, nmax) * ((nmax <= 32 ? 6.5 : 12.0) + 3e-4 * std::min(n, npix + n / 64.0)) +
+                      n * m * l * (interpolated ? 3.3e-6 : 4.7e-5 * l) + 4.4e-4 * npix;
+    const double level = 21.0 + 0.8 * std::min(l, 40.0) + max_pix * (interpolated ? 0.34 : 0.34 + 0.36 * (l + 7.0)) +
+                         npix * m * 1.6e-5 + n * m * (interpolated ? 1.4e-5 : 3.3e-5 * l) + ns * l * m * 3.1e-4;
+    return tc < 67.0 + l * level + 1.7e-3 * npix;
+}
+
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
-                                const double *r_sorted_dev, int64_t npoints, int lmax, int nmax, double rmax,
+                                const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax, double rmax,
                                 bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host, double r_min,
                                 double r_max, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st) {
@@ -646,12 +664,9 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     const int64_t *tw_off = reinterpret_cast<const int64_t *>(rb + R.off_twoff);
     const double2 *tw = reinterpret_cast<const double2 *>(rb + R.off_tw);
     const int *order = reinterpret_cast<const int *>(rb + R.off_order);
-    // As a sum over points at their pixels' centres on the tensor cores (plain_tc.cu) wherever that takes the
-    // sizes: it sums the j_l of a pixel's points first, and was faster at every density measured, ms there / by the
-    // maps and FFTs below: nside 256, 1M points, l 128, n 64: 116 / 400; nside 64, 1.6M points, l 24: n 4 2.9 / 6.7,
-    // n 48 8.2 / 30; nside 16, 3M points (977 a pixel), l 10: n 4 4.0 / 8.7, n 48 8.0 / 24; nside 1, 20k points
-    // (1667 a pixel), l 24, n 4: 0.44 / 12.
-    if (plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (int64_t)0xFFFFFFFEll) {
+    // As a sum over points at their pixels' centres on the tensor cores (plain_tc.cu) where that takes the sizes and is
+    // the faster one: it sums the j_l of a pixel's points first.
+    if (plain_tc_takes(ctx, lmax, nmax, rmax) && pixel_sum_pays(nside, npoints, max_pix, lmax, nmax, interpolated) && npoints <= (int64_t)0xFFFFFFFEll) {
         if (npoints > 0) {
             PixelCatalog px;
             px.r = r_sorted_dev;

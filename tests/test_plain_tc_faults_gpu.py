@@ -337,3 +337,25 @@ def test_the_faster_path_for_few_points(cuda_device, n, lmax, nmax, fp64):
     f = O.sfb_raw(pts, keep, nmax, 1000.0, interpolated=True)[2]
     for l in range(keep):
         assert np.max(np.abs(res.f_lmn[l] - f[l])) <= 1e-10 * np.max(np.abs(f[l])), l
+
+
+@pytest.mark.parametrize("nside,n,lmax,nmax,maps", [(1, 3, 24, 1500, True), (4, 300, 24, 1500, True), (1, 300, 24, 8, False),
+                                                    (32, 2000, 24, 8, False), (16, 20000, 12, 300, False)])
+@pytest.mark.parametrize("interp", ["on", "off"])
+def test_the_faster_path_for_few_pixelized_points(cuda_device, nside, n, lmax, nmax, maps, interp):
+    """The maps launch at least four kernels a level, the sum over entries at most three dozen for these in all; the lowest
+    levels agree with the oracle in either."""
+    from oracle import oracle as O
+    if interp == "off" and (maps and n > 3 or nmax == 300):
+        return  # exact j_l: another crossing point
+    ppc = catana.PixelizedPointContainer(nside, catana.PointContainer(uniform_ball(n, 1000.0, seed=n)))
+
+    def call():
+        return catana.sfb_decomposition(ppc, lmax, nmax, 1000.0, True, False, interpolation=interp)
+
+    call()
+    res, launches = _launches(call)
+    assert (launches >= 4 * lmax) == maps, launches
+    f = O.sfb_healpix(nside, ppc.offsets, ppc.r_sorted, 2, nmax, 1000.0, interpolated=interp == "on")[2]
+    for l in range(2):
+        assert np.max(np.abs(res.f_lmn[l] - f[l])) <= 1e-10 * np.max(np.abs(f[l])), l
