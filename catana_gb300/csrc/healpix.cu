@@ -641,8 +641,8 @@ bool pixel_sum_pays(int64_t nside, int64_t npoints, int64_t max_pix, int lmax, i
 
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
                                 const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax, double rmax,
-                                bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host, double r_min,
-                                double r_max, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
+                                bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
+                                const double *r_host, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st) {
     if (lmax == 0 || nmax == 0) return CATANA_OK;
     if (4 * nside > HP_MAXPIX) {
@@ -703,7 +703,18 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     double2 *ylm = reinterpret_cast<double2 *>(ctx->partial.as<char>() + mapb);
     double2 *partial = reinterpret_cast<double2 *>(ctx->partial.as<char>() + mapb + ylmb);
     double *kd_dev = reinterpret_cast<double *>(ctx->partial.as<char>() + mapb + ylmb + partb);
-    if (interpolated && kln_host) {  // k_ln / dx per (l, n): the unchecked map levels' table scale
+    // range of the radii; r_min NaN when any radius is NaN
+    double r_min = 0.0, r_max = 0.0;
+    for (int64_t i = 0; interpolated && i < npoints; ++i) {
+        const double r = r_host[i];
+        if (std::isnan(r)) {
+            r_min = NAN;
+            break;
+        }
+        if (i == 0 || r < r_min) r_min = r;
+        if (i == 0 || r > r_max) r_max = r;
+    }
+    if (interpolated) {  // k_ln / dx per (l, n): the unchecked map levels' table scale
         std::vector<double> kd((size_t)lmax * nmax);
         for (int l = 0; l < lmax; ++l)
             for (int n = 0; n < nmax; ++n) kd[(size_t)l * nmax + n] = kln_host[(size_t)l * nmax + n] * ctx->tab_dxinv[l];
@@ -721,7 +732,7 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     }
     for (int l = 0; l < lmax; ++l) {
         // the level is in the table's range when 0 <= r_min and k_max r_max < zmax (NaN radii fail both)
-        const bool in_range = interpolated && kln_host && r_min >= 0.0 &&
+        const bool in_range = interpolated && r_min >= 0.0 &&
                               kln_host[(size_t)l * nmax + nmax - 1] * r_max < ctx->tab_zmax[l];
         auto map_kern = in_range ? k_hp_map<false> : k_hp_map<true>;
         map_kern<<<ceil_div(npix * nmax, 256), 256, 0, st>>>(
