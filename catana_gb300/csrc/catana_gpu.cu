@@ -245,28 +245,47 @@ catana_status_t check_args(int64_t npoints, uint16_t lmax, uint16_t nmax, double
     return CATANA_OK;
 }
 
-// Weighted sum on device for the normalisation (sum of weights), in a fixed order.  One CTA waits
-// for memory a few loads at a time (1M weights: 294 us), so more than WSUM_CHUNK weights are
-// summed by chunks of one CTA each first, and the chunks' sums by one CTA (9 + 6 us).
+// Sum of the weights (the normalisation) and their range (bits of positive doubles in their order; none: lo ~0, hi 0),
+// in a fixed order.  One CTA waits for memory a few loads at a time (1M weights: 294 us), so more than WSUM_CHUNK weights
+// are taken by chunks of one CTA each first, and the chunks by one CTA (9 + 6 us).
+struct WStat {
+    double sum;
+    unsigned long long lo, hi;
+};
 constexpr int WSUM_CHUNK = 8192, WSUM_CTAS = 592;
-__global__ void __launch_bounds__(1024) k_wsum(const double *__restrict__ w, int64_t n, int64_t chunk,
-                                               double *__restrict__ out) {
-    __shared__ double sh[1024];
+__device__ __forceinline__ WStat wstat(const double *w, int64_t i) {
+    const unsigned long long a = (unsigned long long)__double_as_longlong(fabs(w[i]));
+    const bool in = a != 0ull && a < 0x7ff0000000000000ull;
+    return {w[i], in ? a : ~0ull, in ? a : 0ull};
+}
+__device__ __forceinline__ WStat wstat(const WStat *w, int64_t i) { return w[i]; }
+template <class T>
+__global__ void __launch_bounds__(1024) k_wsum(const T *__restrict__ w, int64_t n, int64_t chunk, WStat *__restrict__ out) {
+    __shared__ WStat sh[1024];
     const int64_t b = blockIdx.x * chunk, e = min(n, b + chunk);
-    double s = 0.0;
+    WStat s = {0.0, ~0ull, 0ull};
+    auto add = [&](const WStat &v) {
+        s.sum += v.sum;
+        s.lo = min(s.lo, v.lo);
+        s.hi = max(s.hi, v.hi);
+    };
 #pragma unroll 4
-    for (int64_t i = b + threadIdx.x; i < e; i += 1024) s += w[i];
+    for (int64_t i = b + threadIdx.x; i < e; i += 1024) add(wstat(w, i));
     sh[threadIdx.x] = s;
     __syncthreads();
     for (int k = 512; k > 0; k >>= 1) {
-        if ((int)threadIdx.x < k) sh[threadIdx.x] += sh[threadIdx.x + k];
+        if ((int)threadIdx.x < k) {
+            s = sh[threadIdx.x];
+            add(sh[threadIdx.x + k]);
+            sh[threadIdx.x] = s;
+        }
         __syncthreads();
     }
     if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
-// *out = sum of n weights; scratch: WSUM_CTAS doubles
-catana_status_t weight_sum(const double *w, int64_t n, double *out, double *scratch, cudaStream_t st) {
+// *out = the statistics of n weights; scratch: WSUM_CTAS entries
+catana_status_t weight_stats(const double *w, int64_t n, WStat *out, WStat *scratch, cudaStream_t st) {
     if (n <= WSUM_CHUNK) {
         k_wsum<<<1, 1024, 0, st>>>(w, n, n, out);
         count_launch();
@@ -274,61 +293,23 @@ catana_status_t weight_sum(const double *w, int64_t n, double *out, double *scra
         const int64_t chunk = std::max<int64_t>(WSUM_CHUNK, (n + WSUM_CTAS - 1) / WSUM_CTAS);
         const int ctas = (int)((n + chunk - 1) / chunk);
         k_wsum<<<ctas, 1024, 0, st>>>(w, n, chunk, scratch);
-        k_wsum<<<1, 1024, 0, st>>>(scratch, ctas, ctas, out);
+        k_wsum<<<1, 1024, 0, st>>>((const WStat *)scratch, ctas, ctas, out);
         count_launch(2);
     }
     CG_CUDA_TRY(cudaGetLastError());
     return CATANA_OK;
 }
 
-// WeightRange of device weights: bits of positive doubles in their order, out[0] from ~0 down, out[1] from 0 up
-__global__ void __launch_bounds__(256) k_weight_range(const double *__restrict__ w, int64_t n, unsigned long long *out) {
-    unsigned long long lo = ~0ull, hi = 0ull;
-    for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
-        const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(w[i]));
-        if (b == 0ull || b >= 0x7ff0000000000000ull) continue;
-        lo = min(lo, b);
-        hi = max(hi, b);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&out[0], lo);
-        atomicMax(&out[1], hi);
-    }
+WeightRange weight_range(const WStat &s) {
+    WeightRange r;
+    if (s.hi == 0ull) return r;
+    memcpy(&r.lo, &s.lo, 8);
+    memcpy(&r.hi, &s.hi, 8);
+    return r;
 }
 
-// The ranges of the catalogs' weights (null: none) by one read-back
-catana_status_t weight_ranges(DeviceContext *ctx, const catana_catalog_t *cats, int ncat, WeightRange *out, cudaStream_t st) {
-    CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)16 * ncat));
-    unsigned long long *d = ctx->cat_scratch.as<unsigned long long>();
-    std::vector<unsigned long long> h(2 * (size_t)ncat);
-    for (int c = 0; c < ncat; ++c) h[2 * c] = ~0ull;
-    CG_CUDA_TRY(cudaMemcpyAsync(d, h.data(), (size_t)16 * ncat, cudaMemcpyHostToDevice, st));
-    for (int c = 0; c < ncat; ++c)
-        if (cats[c].weights && cats[c].npoints > 0) {
-            k_weight_range<<<std::min(4 * ctx->sm_count, ceil_div(cats[c].npoints, 256)), 256, 0, st>>>(cats[c].weights,
-                                                                                                       cats[c].npoints, d + 2 * c);
-            count_launch();
-        }
-    CG_CUDA_TRY(cudaGetLastError());
-    CG_CUDA_TRY(cudaMemcpyAsync(h.data(), d, (size_t)16 * ncat, cudaMemcpyDeviceToHost, st));
-    CG_CUDA_TRY(cudaStreamSynchronize(st));
-    for (int c = 0; c < ncat; ++c) {
-        out[c] = WeightRange();
-        if (h[2 * c + 1] == 0ull) continue;
-        memcpy(&out[c].lo, &h[2 * c], 8);
-        memcpy(&out[c].hi, &h[2 * c + 1], 8);
-    }
-    return CATANA_OK;
-}
-
-// Core of both raw entry points: device inputs, device outputs; wr: of the weights where the caller has them on
-// the host, or null.
-catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double *w_d, const WeightRange *wr, int64_t npoints,
-                           int lmax, int nmax, double rmax, uint32_t flags, double *kln_d, double *cln_d, double *f_d,
+// Core of both raw entry points: device inputs, device outputs.
+catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double *w_d, int64_t npoints, int lmax, int nmax, double rmax, uint32_t flags, double *kln_d, double *cln_d, double *f_d,
                            int *err_d, cudaStream_t st) {
     const bool split = (flags & CATANA_FORM_MASK) == CATANA_FORM_SPLIT;
     WsOrder ws_order(ctx, st);
@@ -353,28 +334,27 @@ catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double
         s = split_raw_accumulate(ctx, pts_d, w_d, npoints, lmax, nmax, rmax, kln_d, facc, err_d, st,
                                  (flags & CATANA_SPLIT_ACCURATE) != 0);
     } else {
-        WeightRange w;
-        if (wr) {
-            w = *wr;
-        } else if (w_d && npoints > 0) {
-            catana_catalog_t c = {};
-            c.weights = w_d;
-            c.npoints = npoints;
-            s = weight_ranges(ctx, &c, 1, &w, st);
-            if (s != CATANA_OK) return s;
-        }
-        s = fp64_raw_accumulate(ctx, pts_d, w_d, w, npoints, lmax, nmax, rmax, resolve_jl(flags, npoints), kln_d, facc,
-                                err_d, st);
+        s = fp64_raw_accumulate(ctx, pts_d, w_d, nullptr, npoints, lmax, nmax, rmax, resolve_jl(flags, npoints), kln_d,
+                                facc, err_d, st);
     }
     if (s != CATANA_OK) return s;
     double wsum = (double)npoints;
     if (w_d && npoints > 0) {
-        CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)8 * (1 + WSUM_CTAS)));
-        double *ws = ctx->cat_scratch.as<double>();
-        s = weight_sum(w_d, npoints, ws, ws + 1, st);
+        CG_CUDA_TRY(ctx->cat_scratch.ensure(sizeof(WStat) * (1 + WSUM_CTAS)));
+        WStat *ws = ctx->cat_scratch.as<WStat>(), wh;
+        s = weight_stats(w_d, npoints, ws, ws + 1, st);
         if (s != CATANA_OK) return s;
-        CG_CUDA_TRY(cudaMemcpyAsync(&wsum, ws, sizeof(double), cudaMemcpyDeviceToHost, st));
+        CG_CUDA_TRY(cudaMemcpyAsync(&wh, ws, sizeof(wh), cudaMemcpyDeviceToHost, st));
         CG_CUDA_TRY(cudaStreamSynchronize(st));
+        wsum = wh.sum;
+        // the weights' range comes with their sum; one that the tensor cores should not have taken: again
+        const WeightRange wr = weight_range(wh);
+        if (!split && !plain_tc_holds(wr)) {
+            CG_CUDA_TRY(cudaMemsetAsync(facc, 0, fbytes, st));
+            s = fp64_raw_accumulate(ctx, pts_d, w_d, &wr, npoints, lmax, nmax, rmax, resolve_jl(flags, npoints), kln_d,
+                                    facc, err_d, st);
+            if (s != CATANA_OK) return s;
+        }
     }
     // an empty catalog divides by zero like the reference (f = 0 * inf = NaN)
     const double nf = norm_factor(rmax, wsum);
@@ -427,8 +407,8 @@ catana_status_t check_catalogs(const catana_catalog_t *cats, int32_t ncat) {
     return CATANA_OK;
 }
 
-// Core of both batched entry points: device pointers in the records; wr as in raw_device, one per catalog.
-catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats, const WeightRange *wr, int ncat, uint32_t flags,
+// Core of both batched entry points: device pointers in the records.
+catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats, int ncat, uint32_t flags,
                                double waves, int *err_d, cudaStream_t st) {
     const bool split = (flags & CATANA_FORM_MASK) == CATANA_FORM_SPLIT;
     if (split && (ctx->cc_major != 10 || ctx->cc_minor != 3)) {
@@ -458,6 +438,19 @@ catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats,
         if (fc) CG_CUDA_TRY(cudaMemsetAsync(facc[c], 0, fc * sizeof(double), st));
     }
     catana_status_t s;
+    auto plain = [&](int c, const WeightRange *wr) -> catana_status_t {
+        const catana_catalog_t &C = cats[c];
+        catana_status_t r = fp64_raw_accumulate(ctx, C.points, C.weights, wr, C.npoints, C.lmax, C.nmax, C.rmax,
+                                                resolve_jl(flags, C.npoints), C.k_ln, facc[c], err_d, st);
+        if (r != CATANA_OK) return r;
+        if (C.kmax > 0.0 && C.lmax > 0 && C.nmax > 0) {
+            k_kcut<<<dim3(ceil_div((int64_t)C.lmax * C.nmax, 256), C.lmax), 256, 0, st>>>(
+                reinterpret_cast<double2 *>(facc[c]), C.k_ln, C.nmax, C.kmax);
+            count_launch();
+            CG_CUDA_TRY(cudaGetLastError());
+        }
+        return CATANA_OK;
+    };
     if (split) {
         // catalogs whose Legendre rows exceed 16 GB enter as chunks (same accumulator)
         std::vector<SplitCatInput> v;
@@ -485,24 +478,9 @@ catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats,
                       err_d, st);
         if (s != CATANA_OK) return s;
     } else {
-        std::vector<WeightRange> w(ncat);
-        bool ask = false;
-        for (int c = 0; c < ncat; ++c) ask |= (!wr && cats[c].weights && cats[c].npoints > 0);
-        if (ask) {
-            s = weight_ranges(ctx, cats, ncat, w.data(), st);
-            if (s != CATANA_OK) return s;
-        }
         for (int c = 0; c < ncat; ++c) {
-            const catana_catalog_t &C = cats[c];
-            s = fp64_raw_accumulate(ctx, C.points, C.weights, wr ? wr[c] : w[c], C.npoints, C.lmax, C.nmax, C.rmax,
-                                    resolve_jl(flags, C.npoints), C.k_ln, facc[c], err_d, st);
+            s = plain(c, nullptr);
             if (s != CATANA_OK) return s;
-            if (C.kmax > 0.0 && C.lmax > 0 && C.nmax > 0) {
-                k_kcut<<<dim3(ceil_div((int64_t)C.lmax * C.nmax, 256), C.lmax), 256, 0, st>>>(
-                    reinterpret_cast<double2 *>(facc[c]), C.k_ln, C.nmax, C.kmax);
-                count_launch();
-                CG_CUDA_TRY(cudaGetLastError());
-            }
         }
     }
     // weight sums (one read-back for all catalogs), then normalise and form C_ln
@@ -513,18 +491,26 @@ catana_status_t batched_device(DeviceContext *ctx, const catana_catalog_t *cats,
         any_w |= (cats[c].weights && cats[c].npoints > 0);
     }
     if (any_w) {
-        CG_CUDA_TRY(ctx->cat_scratch.ensure((size_t)8 * (ncat + WSUM_CTAS)));
-        double *ws = ctx->cat_scratch.as<double>();
+        CG_CUDA_TRY(ctx->cat_scratch.ensure(sizeof(WStat) * (ncat + WSUM_CTAS)));
+        WStat *ws = ctx->cat_scratch.as<WStat>();
         for (int c = 0; c < ncat; ++c)
             if (cats[c].weights && cats[c].npoints > 0) {
-                s = weight_sum(cats[c].weights, cats[c].npoints, ws + c, ws + ncat, st);
+                s = weight_stats(cats[c].weights, cats[c].npoints, ws + c, ws + ncat, st);
                 if (s != CATANA_OK) return s;
             }
-        std::vector<double> wh(ncat);
-        CG_CUDA_TRY(cudaMemcpyAsync(wh.data(), ws, (size_t)8 * ncat, cudaMemcpyDeviceToHost, st));
+        std::vector<WStat> wh(ncat);
+        CG_CUDA_TRY(cudaMemcpyAsync(wh.data(), ws, sizeof(WStat) * ncat, cudaMemcpyDeviceToHost, st));
         CG_CUDA_TRY(cudaStreamSynchronize(st));
         for (int c = 0; c < ncat; ++c)
-            if (cats[c].weights && cats[c].npoints > 0) wsum[c] = wh[c];
+            if (cats[c].weights && cats[c].npoints > 0) {
+                wsum[c] = wh[c].sum;
+                // as in raw_device: weights that the tensor cores should not have taken
+                const WeightRange wr = weight_range(wh[c]);
+                if (split || plain_tc_holds(wr)) continue;
+                CG_CUDA_TRY(cudaMemsetAsync(facc[c], 0, catana_gpu_flmn_size(cats[c].lmax, cats[c].nmax) * 16, st));
+                s = plain(c, &wr);
+                if (s != CATANA_OK) return s;
+            }
     }
     for (int c = 0; c < ncat; ++c) {
         const catana_catalog_t &C = cats[c];
@@ -659,7 +645,7 @@ catana_status_t catana_gpu_sfb_raw_dev(const double *points_dev, const double *w
         err_d = ctx->misc.as<int>();
         CG_CUDA_TRY(cudaMemsetAsync(err_d, 0, sizeof(int), st));
     }
-    return raw_device(ctx, points_dev, weights_dev, nullptr, npoints, lmax, nmax, rmax, flags, k_ln_dev, c_ln_dev, f_lmn_dev,
+    return raw_device(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, flags, k_ln_dev, c_ln_dev, f_lmn_dev,
                       err_d, st);
 }
 
@@ -694,9 +680,7 @@ catana_status_t catana_gpu_sfb_raw(const double *points, const double *weights, 
         CG_CUDA_TRY(cudaMemcpyAsync(pts_d, points, (size_t)npoints * 3 * sizeof(double), cudaMemcpyHostToDevice, st));
     if (weights && npoints > 0)
         CG_CUDA_TRY(cudaMemcpyAsync(w_d, weights, (size_t)npoints * sizeof(double), cudaMemcpyHostToDevice, st));
-    WeightRange wr;
-    if (weights && (flags & CATANA_FORM_MASK) != CATANA_FORM_SPLIT) wr.add(weights, npoints);
-    s = raw_device(ctx, pts_d, w_d, &wr, npoints, lmax, nmax, rmax, flags, kln_d, cln_d, f_d, err_d, st);
+    s = raw_device(ctx, pts_d, w_d, npoints, lmax, nmax, rmax, flags, kln_d, cln_d, f_d, err_d, st);
     if (s != CATANA_OK) return s;
     int err_h = 0;
     CG_CUDA_TRY(cudaMemcpyAsync(&err_h, err_d, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -730,7 +714,7 @@ catana_status_t catana_gpu_sfb_raw_batched_dev(const catana_catalog_t *cats, int
         err_d = ctx->misc.as<int>();
         CG_CUDA_TRY(cudaMemsetAsync(err_d, 0, sizeof(int), st));
     }
-    return batched_device(ctx, cats, nullptr, ncat, flags, waves, err_d, st);
+    return batched_device(ctx, cats, ncat, flags, waves, err_d, st);
 }
 
 catana_status_t catana_gpu_sfb_raw_batched(const catana_catalog_t *cats, int32_t ncat, uint32_t flags, double waves,
@@ -777,11 +761,7 @@ catana_status_t catana_gpu_sfb_raw_batched(const catana_catalog_t *cats, int32_t
         dc[c].f_lmn = reinterpret_cast<double *>(op);
         op += al(catana_gpu_flmn_size(C.lmax, C.nmax) * 2 * sizeof(double));
     }
-    std::vector<WeightRange> wr(ncat);
-    if ((flags & CATANA_FORM_MASK) != CATANA_FORM_SPLIT)
-        for (int c = 0; c < ncat; ++c)
-            if (cats[c].weights) wr[c].add(cats[c].weights, cats[c].npoints);
-    s = batched_device(ctx, dc.data(), wr.data(), ncat, flags, waves, err_d, st);
+    s = batched_device(ctx, dc.data(), ncat, flags, waves, err_d, st);
     if (s != CATANA_OK) return s;
     int err_h = 0;
     CG_CUDA_TRY(cudaMemcpyAsync(&err_h, err_d, sizeof(int), cudaMemcpyDeviceToHost, st));

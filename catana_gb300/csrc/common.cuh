@@ -166,15 +166,13 @@ struct WeightRange {
         if (a < lo) lo = a;
         if (a > hi) hi = a;
     }
-    void add(const double *w, int64_t n) {
-        for (int64_t i = 0; i < n; ++i) add(w[i]);
-    }
 };
 
 // Plain raw form (sfb_fp64.cu).  All pointers device.  Accumulates into f_acc (complex, packed by l,
-// un-normalised); the caller normalises.  wr: of weights_dev, unused without weights.
+// un-normalised); the caller normalises.  wr: of weights_dev, or null where the caller does not know it yet and will
+// start again if plain_tc_holds() says no to it.
 catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
-                                    const WeightRange &wr, int64_t npoints, int lmax, int nmax, double rmax, JlMode jl,
+                                    const WeightRange *wr, int64_t npoints, int lmax, int nmax, double rmax, JlMode jl,
                                     const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st);
 // The same sum with its contraction on the tensor cores (plain_tc.cu), where the device has them and
 // lmax <= 512; with JL_MODE_POLY the caller has prepared ctx->poly and passes the largest radius (else rtop = 0).

@@ -289,6 +289,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
 
     if (warp < TC_OPW) {
         uint32_t use = 0;  // tiles written so far
+        const uint32_t withheld = a.stall && warp == 0 ? 1u : 0u;
         int ofs = 0;       // units dealt so far, mod TC_OPW
         bool dead = false;
         const uint32_t lk = (uint32_t)(lane >> 3), lr = (uint32_t)(lane & 7);  // K row of this point: group, row
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                 } else if (!mine) {
                     wait(&empty[bf], (it - 1) & 1, dead);
                 }
-                if (lane == 0 && !(a.stall && warp == 0 && use == 1)) tc_arrive(&full[bf]);
+                if (lane == 0 && use != withheld) tc_arrive(&full[bf]);
             }
         });
         if (dead && lane == 0) *a.err = CATANA_ERR_CUDA;
@@ -592,7 +593,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
             if (live && row < 2 * b.mcount) {
                 const int ring = seq & (int)(TC_RING - 1);
                 const uint4 *tn = s_n + ring * TC_NB + nb;
-                const int m = b.mb0 + (row >> 1), esh = ew > 0 ? 32 : 0;
+                const int m = b.mb0 + (row >> 1), esh = ew > 0 ? 32 : 0, ebase = (53 - esh) << 20;
                 const double am = scalbn(a.coef[(size_t)b.l * (b.l + 1) / 2 + m].y,
                                          __double2loint(s_m[ring * TC_MB + (row >> 1)].y) + ew - esh);
                 const int w2 = 2 * (b.l + 1);
@@ -616,7 +617,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                         }
 #pragma unroll
                         for (int c = 0; c < 4; ++c)  // 2^(EJ - 54 + esh) is a normal number: EJ >= -900
-                            v[c] *= __hiloint2double((int)tn[c4 + c].w - ((53 - esh) << 20), 0);
+                            v[c] *= __hiloint2double((int)tn[c4 + c].w - ebase, 0);
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
                             if (nb + c4 + c < b.ncount) out[(size_t)(c4 + c) * w2] = v[c] * am;

@@ -490,7 +490,7 @@ catana_status_t ensure_poly_tables(DeviceContext *ctx, int lmax, int nint, cudaS
 }
 
 catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
-                                    const WeightRange &wr, int64_t npoints, int lmax, int nmax, double rmax, JlMode jl,
+                                    const WeightRange *wr, int64_t npoints, int lmax, int nmax, double rmax, JlMode jl,
                                     const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st) {
     const bool interpolated = (jl == JL_MODE_LERP);
     catana_status_t s = ensure_coefs(ctx, lmax, st);
@@ -532,7 +532,7 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
         if (s != CATANA_OK) return s;
         rtop = max_r;
     }
-    if (plain_tc_takes(ctx, lmax, nmax, rmax) && plain_tc_pays(npoints, lmax, nmax, jl) && (!weights_dev || plain_tc_holds(wr))) {
+    if (plain_tc_takes(ctx, lmax, nmax, rmax) && plain_tc_pays(npoints, lmax, nmax, jl) && (!weights_dev || !wr || plain_tc_holds(*wr))) {
         s = plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, rtop, kln_dev, f_acc_dev,
                                 err_dev, st);
         if (s != CATANA_ERR_NOMEM) return s;

@@ -171,7 +171,7 @@ catana_status_t accum_add(Accum *A, const T *points, const T *weights, int64_t n
         // JL_AUTO picks the table form here (streamed catalogs are large)
         const uint32_t jl = A->flags & CATANA_JL_MASK;
         const JlMode mode = jl == CATANA_JL_POLY ? JL_MODE_POLY : jl == CATANA_JL_EXACT ? JL_MODE_EXACT : JL_MODE_LERP;
-        s = fp64_raw_accumulate(ctx, p64, w64, wr, n, A->lmax, A->nmax, A->rmax, mode, A->kln.as<double>(),
+        s = fp64_raw_accumulate(ctx, p64, w64, &wr, n, A->lmax, A->nmax, A->rmax, mode, A->kln.as<double>(),
                                 A->facc.as<double>(), err_d, A->comp_st);
     }
     if (s != CATANA_OK) return s;
@@ -242,7 +242,7 @@ catana_status_t accum_add_records(Accum *A, const void *records, int64_t n, cons
             const uint32_t jl = A->flags & CATANA_JL_MASK;
             const JlMode mode =
                 jl == CATANA_JL_POLY ? JL_MODE_POLY : jl == CATANA_JL_EXACT ? JL_MODE_EXACT : JL_MODE_LERP;
-            s = fp64_raw_accumulate(ctx, pts, nullptr, WeightRange(), kept, A->lmax, A->nmax, A->rmax, mode,
+            s = fp64_raw_accumulate(ctx, pts, nullptr, nullptr, kept, A->lmax, A->nmax, A->rmax, mode,
                                     A->kln.as<double>(), A->facc.as<double>(), err_d, A->comp_st);
         }
         if (s != CATANA_OK) return s;

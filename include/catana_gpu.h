@@ -111,7 +111,7 @@ catana_status_t catana_gpu_sfb_raw(const double *points, const double *weights, 
 
 /* Same computation on device-resident data: all pointers are device pointers,
  * the work is enqueued on `stream` and the call returns without synchronising
- * except where the host needs a value (the weights' range and sum, max r with
+ * except where the host needs a value (the weights' sum and range, max r with
  * JL_POLY, a table that is not cached yet); *status_dev (device
  * int, may be NULL) receives CATANA_ERR_DOMAIN when an argument left the table. */
 catana_status_t catana_gpu_sfb_raw_dev(const double *points_dev, const double *weights_dev, int64_t npoints,
