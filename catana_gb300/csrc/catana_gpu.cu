@@ -245,9 +245,9 @@ catana_status_t check_args(int64_t npoints, uint16_t lmax, uint16_t nmax, double
     return CATANA_OK;
 }
 
-// Sum of the weights (the normalisation) and their range (bits of positive doubles in their order; none: lo ~0, hi 0),
-// in a fixed order.  One CTA waits for memory a few loads at a time (1M weights: 294 us), so more than WSUM_CHUNK weights
-// are taken by chunks of one CTA each first, and the chunks by one CTA (9 + 6 us).
+// Sum of the weights (the normalisation) and their range (bits of positive doubles in their order; none: lo ~0, hi
+// 0), in a fixed order.  One CTA waits for memory a few loads at a time (1M weights: 294 us), so more than
+// WSUM_CHUNK weights are taken by chunks of one CTA each first, and the chunks by one CTA (9 + 6 us).
 struct WStat {
     double sum;
     unsigned long long lo, hi;
@@ -309,7 +309,8 @@ WeightRange weight_range(const WStat &s) {
 }
 
 // Core of both raw entry points: device inputs, device outputs.
-catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double *w_d, int64_t npoints, int lmax, int nmax, double rmax, uint32_t flags, double *kln_d, double *cln_d, double *f_d,
+catana_status_t raw_device(DeviceContext *ctx, const double *pts_d, const double *w_d, int64_t npoints, int lmax,
+                           int nmax, double rmax, uint32_t flags, double *kln_d, double *cln_d, double *f_d,
                            int *err_d, cudaStream_t st) {
     const bool split = (flags & CATANA_FORM_MASK) == CATANA_FORM_SPLIT;
     WsOrder ws_order(ctx, st);

@@ -205,8 +205,9 @@ struct PixelCatalog {
     const int64_t *tw_off;
 };
 // The pixelized sum (un-normalised, times k_ln) as a sum over points at their pixels' centres.
-catana_status_t plain_tc_pixels(DeviceContext *ctx, const PixelCatalog &pix, int64_t npoints, int lmax, int nmax, double rmax,
-                                JlMode jl, const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st);
+catana_status_t plain_tc_pixels(DeviceContext *ctx, const PixelCatalog &pix, int64_t npoints, int lmax, int nmax,
+                                double rmax, JlMode jl, const double *kln_dev, double *f_acc_dev, int *err_dev,
+                                cudaStream_t st);
 
 // One catalog of a split-form run (device pointers; f_acc zeroed by the caller).
 struct SplitCatInput {
@@ -259,8 +260,8 @@ catana_status_t healpix_pix2ang_dev(int64_t nside, const int64_t *pix, int64_t n
 // kln_host (L x M) and r_host, host copies of k_ln and of the radii: map levels that lie inside the j_l table skip
 // the per-point range test.
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
-                                const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax, double rmax,
-                                bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
+                                const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax,
+                                double rmax, bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
                                 const double *r_host, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st);
 

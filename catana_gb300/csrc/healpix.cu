@@ -58,7 +58,7 @@ __global__ void k_pix2ang(int64_t nside, const int64_t *pix, int64_t n, double *
     pix2ang_ring_dev(nside, pix[i], &theta[i], &phi[i]);
 }
 
-// keys = RING pixel of each point, vals = point index; counts[pix] += 1
+// keys = RING pixel of each point, vals = point index
 __global__ void k_bin_keys(int64_t nside, const double *pts, int64_t n, uint32_t *keys, uint32_t *vals,
                            int *err) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -279,13 +279,12 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
 }
 
-// Power-of-two ring of N pixels: the complex sequence z_j = map_j(n) + i map_j(n + 1)
-// (two radial orders) goes through an in-place decimation-in-time FFT, loaded in
-// bit-reversed order, radix-4 passes (each two radix-2 stages of half-lengths h and 2h
-// fused into one butterfly: inputs 1, 2, 3 times W_4h^2j, W_4h^j, W_4h^3j, then sums with
-// +-1 and +-i) and one radix-2 pass when log2 N is odd.  The two real transforms are A[s] = (Z[s] + conj Z[N-s]) / 2 and
-// B[s] = (Z[s] - conj Z[N-s]) / 2i; the m-extraction, the sign rules and the product
-// with Y_lm(ring) are those of k_hp_ring.
+// Power-of-two ring of N pixels: the complex sequence z_j = map_j(n) + i map_j(n + 1) (two radial orders) goes
+// through an in-place decimation-in-time FFT, loaded in bit-reversed order, radix-4 passes (each two radix-2 stages
+// of half-lengths h and 2h fused into one butterfly: inputs 1, 2, 3 times W_4h^2j, W_4h^j, W_4h^3j, then sums with
+// +-1 and +-i) and one radix-2 pass when log2 N is odd.  The two real transforms are A[s] = (Z[s] + conj Z[N-s]) /
+// 2 and B[s] = (Z[s] - conj Z[N-s]) / 2i; the m-extraction, the sign rules and the product with Y_lm(ring) are
+// those of k_hp_ring.
 __global__ void __launch_bounds__(HF_T) k_hp_fft(const double *__restrict__ map, int nmax, int l,
                                                 const int *__restrict__ rings,
                                                 const int64_t *__restrict__ ring_start,
@@ -621,18 +620,20 @@ catana_status_t healpix_bin_dev(DeviceContext *ctx, int64_t nside, const double 
     return CATANA_OK;
 }
 
-// Against the maps and FFTs below, the pixel sum on the tensor cores: ms 114 / 400 at nside 256, 1M points, l 128, n 64;
-// nside 64, 1.6M points, l 24: n 4 2.9 / 6.7, n 48 8.2 / 30; nside 16, 3M points (977 a pixel), l 10: n 4 4.0 / 8.7, n 48 8.0 /
-// 24; nside 1, 20k points, l 24, n 4: 0.44 / 12.  The maps win where little is summed: one or two levels (nside 16, 300
-// points, l 2, n 8: 171 us / 132), and many radial orders of few points, whose blocks of 64 a CTA of the tensor-core
-// kernel walks in turn (nside 1, 3 points, l 24, n 1500: 5820 / 940).  Microseconds, fitted to 595 calls (nside 1 to 256, 3 to
-// 10000 points, l 1 to 500, n 1 to 1500, both j_l modes), all but five of them within 5% of the faster path; max_pix, the points
-// of the fullest pixel, which the maps sum one after the other.  With more points the maps were ahead at l <= 2 only, by a
-// quarter at most (nside 16, 30000 points, l 2, n 8: 253 / 193; 1M points: 1365 / 1510).
+// Against the maps and FFTs below, the pixel sum on the tensor cores: ms 114 / 400 at nside 256, 1M points, l 128,
+// n 64; nside 64, 1.6M points, l 24: n 4 2.9 / 6.7, n 48 8.2 / 30; nside 16, 3M points (977 a pixel), l 10: n 4 4.0
+// / 8.7, n 48 8.0 / 24; nside 1, 20k points, l 24, n 4: 0.44 / 12.  The maps win where little is summed: one or two
+// levels (nside 16, 300 points, l 2, n 8: 171 us / 132), and many radial orders of few points, whose blocks of 64 a
+// CTA of the tensor-core kernel walks in turn (nside 1, 3 points, l 24, n 1500: 5820 / 940).  Microseconds, fitted
+// to 595 calls (nside 1 to 256, 3 to 10000 points, l 1 to 500, n 1 to 1500, both j_l modes), all but five of them
+// within 5% of the faster path; max_pix, the points of the fullest pixel, which the maps sum one after the other.
+// With more points the maps were ahead at l <= 2 only, by a quarter at most (nside 16, 30000 points, l 2, n 8: 253
+// / 193; 1M points: 1365 / 1510).
 bool pixel_sum_pays(int64_t nside, int64_t npoints, int64_t max_pix, int lmax, int nmax, bool interpolated) {
     if (npoints > 16384) return true;
     const double ns = (double)nside, npix = 12.0 * ns * ns, n = (double)npoints, l = lmax, m = nmax;
-    const double tc = 200.0 + plain_tc_blocks(lmax, nmax) * ((nmax <= 32 ? 6.5 : 12.0) + 3e-4 * std::min(n, npix + n / 64.0)) +
+    const double block = (nmax <= 32 ? 6.5 : 12.0) + 3e-4 * std::min(n, npix + n / 64.0);
+    const double tc = 200.0 + plain_tc_blocks(lmax, nmax) * block +
                       n * m * l * (interpolated ? 3.3e-6 : 4.7e-5 * l) + 4.4e-4 * npix;
     const double level = 21.0 + 0.8 * std::min(l, 40.0) + max_pix * (interpolated ? 0.34 : 0.34 + 0.36 * (l + 7.0)) +
                          npix * m * 1.6e-5 + n * m * (interpolated ? 1.4e-5 : 3.3e-5 * l) + ns * l * m * 3.1e-4;
@@ -640,8 +641,8 @@ bool pixel_sum_pays(int64_t nside, int64_t npoints, int64_t max_pix, int lmax, i
 }
 
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
-                                const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax, double rmax,
-                                bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
+                                const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax,
+                                double rmax, bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
                                 const double *r_host, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st) {
     if (lmax == 0 || nmax == 0) return CATANA_OK;
@@ -666,7 +667,8 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     const int *order = reinterpret_cast<const int *>(rb + R.off_order);
     // As a sum over points at their pixels' centres on the tensor cores (plain_tc.cu) where that takes the sizes and is
     // the faster one: it sums the j_l of a pixel's points first.
-    if (plain_tc_takes(ctx, lmax, nmax, rmax) && pixel_sum_pays(nside, npoints, max_pix, lmax, nmax, interpolated) && npoints <= (int64_t)0xFFFFFFFEll) {
+    if (plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (int64_t)0xFFFFFFFEll &&
+        pixel_sum_pays(nside, npoints, max_pix, lmax, nmax, interpolated)) {
         if (npoints > 0) {
             PixelCatalog px;
             px.r = r_sorted_dev;

@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(IG_BLOCK) k_ingest_mark(const void *__restrict
         const bool small = rf > 1e-15f && rf < 1e18f;  // rf stands for r to within 3e-7 of it
         double r = 0.0;
         keep = 1;
-        if (small && !sp.has_gauss && !sp.has_window && sp.has_tophat && fabs((double)rf - sp.tophat_r0) > 1e-5 * (double)rf) {
+        if (small && !sp.has_gauss && !sp.has_window && sp.has_tophat &&
+            fabs((double)rf - sp.tophat_r0) > 1e-5 * (double)rf) {
             keep = (double)rf < sp.tophat_r0;
         } else {
             r = record_radius(sp.layout, a, b, c);

@@ -60,8 +60,8 @@ __global__ void k_dsb_nodes(DsbRule R, const double *__restrict__ wt, int64_t q0
 
 // a row of j_l(k x) per k, and the same times the weights: a pair is then one FP64 operation a node instead of two
 // (1024 pairs of 32 k, 30k nodes: 124 -> 74 us)
-__global__ void k_dsb_bessel(const double *__restrict__ k, const double *__restrict__ x, const double *__restrict__ w, int64_t nq,
-                             int l, double *__restrict__ o, double *__restrict__ ow) {
+__global__ void k_dsb_bessel(const double *__restrict__ k, const double *__restrict__ x, const double *__restrict__ w,
+                             int64_t nq, int l, double *__restrict__ o, double *__restrict__ ow) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= nq) return;
     const double j = jl_direct(l, k[blockIdx.y] * x[i]);
@@ -72,8 +72,9 @@ __global__ void k_dsb_bessel(const double *__restrict__ k, const double *__restr
 constexpr int DSB_T = 128;
 
 // out[p] (+)= sum_q W[i1][q] J[i2][q], W = w J; first = 0 adds to the chunks before
-__global__ void __launch_bounds__(DSB_T) k_dsb_pairs(const double *__restrict__ J, const double *__restrict__ W, int64_t nq,
-                                                     const uint32_t *__restrict__ i1, const uint32_t *__restrict__ i2, int first,
+__global__ void __launch_bounds__(DSB_T) k_dsb_pairs(const double *__restrict__ J, const double *__restrict__ W,
+                                                     int64_t nq, const uint32_t *__restrict__ i1,
+                                                     const uint32_t *__restrict__ i2, int first,
                                                      double *__restrict__ out) {
     __shared__ double s[DSB_T / 32];
     const int64_t p = blockIdx.x;
@@ -130,8 +131,8 @@ struct DsbCall {
 constexpr size_t DSB_MAXK = 31250;
 
 // The integrals of pairs with k <= kmax (host arrays), by one rule
-catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, const double *k1, const double *k2, int64_t npairs,
-                          const std::vector<double> &ks, double *out, cudaStream_t st) {
+catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, const double *k1, const double *k2,
+                          int64_t npairs, const std::vector<double> &ks, double *out, cudaStream_t st) {
     // each pair's two places among the distinct k
     std::vector<uint32_t> idx(2 * (size_t)npairs);
     for (int64_t i = 0; i < npairs; ++i) {
@@ -187,8 +188,8 @@ catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, con
 }
 
 // The same for any number of distinct k: in runs of pairs where they are too many for a pass
-catana_status_t dsb_pairs(DeviceContext *ctx, const DsbCall &C, double kmax, const double *k1, const double *k2, int64_t npairs,
-                          double *out, cudaStream_t st) {
+catana_status_t dsb_pairs(DeviceContext *ctx, const DsbCall &C, double kmax, const double *k1, const double *k2,
+                          int64_t npairs, double *out, cudaStream_t st) {
     auto distinct = [&](int64_t b, int64_t e) {
         std::vector<double> ks(k1 + b, k1 + e);
         ks.insert(ks.end(), k2 + b, k2 + e);
@@ -249,8 +250,8 @@ catana_status_t catana_gpu_sbessel_integrals(const double *w_table, int64_t w_n,
     C.wdx = (w_max - w_min) / (double)(w_n - 1);
     C.rmax = r_max;
     if (C.cuts(kmax) < 8.0) return dsb_pairs(ctx, C, kmax, k1, k2, npairs, out, st);
-    // The pairs by the octal order of their pieces per segment: a pair is not integrated on pieces that only a much larger k
-    // of the call asks for.
+    // The pairs by the octal order of their pieces per segment: a pair is not integrated on pieces that only a much
+    // larger k of the call asks for.
     std::vector<int> order(npairs);
     int lo = INT_MAX, hi = 0;
     for (int64_t i = 0; i < npairs; ++i) {

@@ -155,7 +155,8 @@ struct Digits {
 // FP64 load where pred holds, 0 elsewhere (rows that this kernel also writes)
 __device__ __forceinline__ double ld_if(const double *p, bool pred) {
     double v;
-    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.f64 %0, 0d0000000000000000;\n@q ld.global.L1::no_allocate.f64 %0, [%1];\n}"
+    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.f64 %0, 0d0000000000000000;\n"
+                 "@q ld.global.L1::no_allocate.f64 %0, [%1];\n}"
                  : "=d"(v)
                  : "l"(p), "r"((int)pred)
                  : "memory");
@@ -407,7 +408,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                             // |q| 2^(61 - EP), then times the 58-bit phase, upper 64 bits: < 2^55
                             const uint32_t qh = (uint32_t)__double2hiint(q[h]), ql = (uint32_t)__double2loint(q[h]);
                             const int s = __double2loint(tm[4 * u + h].y) + 1022 - (int)((qh >> 20) & 0x7ffu);
-                            const uint64_t p = shr64(((uint64_t)((qh & 0xfffffu) | 0x100000u) << 40) | ((uint64_t)ql << 8), s);
+                            const uint64_t mant = ((uint64_t)((qh & 0xfffffu) | 0x100000u) << 40) | ((uint64_t)ql << 8);
+                            const uint64_t p = shr64(mant, s);
                             // both factors as signed halves: three products, no sign to carry along
                             const uint64_t ps = signed_halves(qh >> 31 ? -(int64_t)p : (int64_t)p);
                             const int32_t p1 = (int32_t)(ps >> 32), p0 = (int32_t)ps;
@@ -437,7 +439,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                                     v[h0 + h] = j_digits(fma(y[h].y, f[h], y[h].x), tn[8 * o + h0 + h].w);
                             }
                         } else {
-                            const uint64_t *jp = a.jarr + (((size_t)(l - a.l0) * a.tiles + t) * a.nmax + b.n0 + 8 * o) * TC_KT + lane;
+                            const size_t row = ((size_t)(l - a.l0) * a.tiles + t) * a.nmax + b.n0 + 8 * o;
+                            const uint64_t *jp = a.jarr + row * TC_KT + lane;
 #pragma unroll
                             for (int h = 0; h < 8; ++h) v[h] = 8 * o + h < b.ncount ? __ldg(jp + h * TC_KT) : TC_OFF_J;
                         }
@@ -742,10 +745,11 @@ __device__ __forceinline__ uint64_t phase_word(double v) { return signed_halves(
 // phase of the run's middle comes from the exactly reduced fraction frac(m phi / 2 pi) and is rotated
 // by e^{+-i phi} for the others (at most four times).
 __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ pts, const double *__restrict__ w,
-                                                    const uint32_t *__restrict__ perm, int64_t n, int tiles, int tslab, int lmp,
-                                                    const TcSlab *__restrict__ slab, int er, int lerp, double rlim,
-                                                    uint64_t *__restrict__ rint, double *__restrict__ rabs, double2 *__restrict__ xs,
-                                                    ulonglong2 *__restrict__ phase, int *__restrict__ poison, int *__restrict__ err) {
+                                                    const uint32_t *__restrict__ perm, int64_t n, int tiles, int tslab,
+                                                    int lmp, const TcSlab *__restrict__ slab, int er, int lerp,
+                                                    double rlim, uint64_t *__restrict__ rint, double *__restrict__ rabs,
+                                                    double2 *__restrict__ xs, ulonglong2 *__restrict__ phase,
+                                                    int *__restrict__ poison, int *__restrict__ err) {
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= tiles) return;
     const int64_t i = (int64_t)t * TC_KT + lane;
@@ -814,9 +818,9 @@ __device__ __forceinline__ int64_t pixel_of(const TcPixels &px, int64_t q) {
 // first (a warp sums as long as its longest), of like ones by the head's radius in 256 steps (the lanes of a
 // warp then share cells of the j_l table where entries hold few points: 34 -> 32 ms below); the other points
 // come last.  Also each radius in the table's units.
-__global__ void k_ptc_cells(TcPixels px, int64_t n, double inv_rmax, int er, int lerp, double rlim, uint32_t *__restrict__ keys,
-                            uint32_t *__restrict__ vals, uint64_t *__restrict__ rint, int *__restrict__ poison,
-                            unsigned long long *__restrict__ count, int *__restrict__ err) {
+__global__ void k_ptc_cells(TcPixels px, int64_t n, double inv_rmax, int er, int lerp, double rlim,
+                            uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, uint64_t *__restrict__ rint,
+                            int *__restrict__ poison, unsigned long long *__restrict__ count, int *__restrict__ err) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t p = q < n ? pixel_of(px, q) : 0, k = q < n ? q - px.offs[p] : 1;
     // every thread of the block takes part, whatever its bisection took
@@ -825,7 +829,8 @@ __global__ void k_ptc_cells(TcPixels px, int64_t n, double inv_rmax, int er, int
     if (q >= n) return;
     const double r = px.r[q], rs = r * inv_rmax * 256.0;
     const uint32_t rb = rs >= 255.0 ? 255u : (rs > 0.0 ? (uint32_t)rs : 0u);
-    keys[q] = (k % TC_CELL == 0 ? (uint32_t)(TC_CELL - min((int64_t)TC_CELL, px.offs[p + 1] - q)) : (uint32_t)TC_CELL) << 8 | rb;
+    const int64_t cnt = k % TC_CELL == 0 ? min((int64_t)TC_CELL, px.offs[p + 1] - q) : 0;
+    keys[q] = (uint32_t)(TC_CELL - cnt) << 8 | rb;
     vals[q] = (uint32_t)q;
     const bool bad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
     if (bad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
@@ -876,8 +881,8 @@ __global__ void __launch_bounds__(256) k_ptc_cell_slabs(TcPixels px, const uint2
 // theta, phase e^{-i m phi_0} e^{-2 pi i j s / N}) with phi_0 the ring's first centre, j the pixel's place among
 // the ring's N and s the frequency that the m-extraction reads (sfb_reverse_fft.cpp:192-207): m mod N up to
 // N / 2, then N - m mod N, conjugated only where `conj` says so.  Both factors come from tables (ring_ph, tw).
-__global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t *__restrict__ perm, int64_t n, int tiles, int lmp,
-                                                    uint2 *__restrict__ cell, double2 *__restrict__ xs,
+__global__ void __launch_bounds__(256) k_ptc_pixels(TcPixels px, const uint32_t *__restrict__ perm, int64_t n,
+                                                    int tiles, int lmp, uint2 *__restrict__ cell, double2 *__restrict__ xs,
                                                     ulonglong2 *__restrict__ phase) {
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= tiles) return;
@@ -1108,7 +1113,8 @@ __global__ void __launch_bounds__(256) k_ptc_jl_poly(TcJ a, const TcPoly *__rest
     const uint32_t kh = (uint32_t)(km >> 32), kl = (uint32_t)km, rh = (uint32_t)(r >> 32), rl = (uint32_t)r;
     const uint64_t tt = (uint64_t)rl * kh + (uint64_t)rh * kl, res = (uint64_t)rh * kh + (tt >> 32);
     // 60 - er - ek bits of res are fraction (up to 64: k r < 1/16 when sh < 0)
-    uint64_t fr = sh >= 0 ? (res << sh) | ((uint64_t)(uint32_t)tt << 32 >> (64 - sh) & (sh ? ~0ull : 0ull)) : shr64(res, -sh);
+    const uint64_t low = (uint64_t)(uint32_t)tt << 32;
+    uint64_t fr = sh >= 0 ? (res << sh) | (low >> (64 - sh) & (sh ? ~0ull : 0ull)) : shr64(res, -sh);
     uint32_t j = sh > 0 ? (uint32_t)(res >> (64 - sh)) : 0u;
     fr += 0x8000000000000000ull;
     j += fr < 0x8000000000000000ull ? 1u : 0u;
@@ -1222,11 +1228,11 @@ bool plain_tc_takes(const DeviceContext *ctx, int lmax, int nmax, double rmax) {
            rmax < 1e100;
 }
 
-// A term is held to 2^-55 of its slab's bound, which goes with the slab's heaviest weight.  Where the heavy points add little
-// to a mode -- they lie near a pole and m is high, or where j_l is still small -- a mode has only the light
-// ones' terms, with as many bits less as they are lighter; FP64 held them all.  Up to eight bits, 2^-47 of such a mode's terms
-// (7e-15), stay inside the errors that both paths have from their recurrences (5e-15 to 1e-14 of f); a catalog whose
-// weights differ by more takes the FP64 path.
+// A term is held to 2^-55 of its slab's bound, which goes with the slab's heaviest weight.  Where the heavy points
+// add little to a mode -- they lie near a pole and m is high, or where j_l is still small -- a mode has only the
+// light ones' terms, with as many bits less as they are lighter; FP64 held them all.  Up to eight bits, 2^-47 of
+// such a mode's terms (7e-15), stay inside the errors that both paths have from their recurrences (5e-15 to 1e-14
+// of f); a catalog whose weights differ by more takes the FP64 path.
 bool plain_tc_holds(const WeightRange &wr) { return !(wr.hi > 256.0 * wr.lo); }
 
 double plain_tc_blocks(int lmax, int nmax) {
@@ -1235,12 +1241,13 @@ double plain_tc_blocks(int lmax, int nmax) {
 }
 
 // Few points with many radial orders, and catalogs of a few levels, are the FP64 path's: a CTA of the tensor-core
-// kernel walks its blocks of 64 complex m and 64 radial orders one after the other, 11 to 15 us each (5 to 7 with one
-// or two column steps), where the FP64 path has a CTA for each, and takes 35 us a level below l = 32 and 89 above it, or its
-// FP64 work.  Microseconds, fitted to 742 calls (l 1 to 512, n 1 to 3000, 1 to 8192 points, the three j_l modes): the
-// path chosen is at most 1.2 times slower than the other, in all but 13 of them within 5%.  For instance, tensor
-// cores / FP64: 100 points, n 200: l 8 404 / 269, l 100 7405 / 7334, l 300 43400 / 26200; n 1000: l 24 6340 / 1070, l 128
-// 48300 / 10300, with 4000 points 70100 / 178000; n 64, l 512 33400 / 44900; l 1, n 16 81 / 44, l 8 120 / 184.
+// kernel walks its blocks of 64 complex m and 64 radial orders one after the other, 11 to 15 us each (5 to 7 with
+// one or two column steps), where the FP64 path has a CTA for each, and takes 35 us a level below l = 32 and 89
+// above it, or its FP64 work.  Microseconds, fitted to 742 calls (l 1 to 512, n 1 to 3000, 1 to 8192 points, the
+// three j_l modes): the path chosen is at most 1.2 times slower than the other, in all but 13 of them within 5%.
+// For instance, tensor cores / FP64: 100 points, n 200: l 8 404 / 269, l 100 7405 / 7334, l 300 43400 / 26200; n
+// 1000: l 24 6340 / 1070, l 128 48300 / 10300, with 4000 points 70100 / 178000; n 64, l 512 33400 / 44900; l 1, n
+// 16 81 / 44, l 8 120 / 184.
 bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl) {
     const bool few = nmax <= 32, exact = jl == JL_MODE_EXACT;
     const double n = (double)npoints, l = lmax, values = n * nmax * l;
@@ -1249,7 +1256,8 @@ bool plain_tc_pays(int64_t npoints, int lmax, int nmax, JlMode jl) {
     double base = (few ? 22.0 : 35.0) * std::min(lmax, 32) + (few ? 80.0 : 89.0) * std::max(lmax - 32, 0);
     if (jl == JL_MODE_POLY) base += 6.0 * l;
     if (exact) base += 13.0 * l * l * std::min(nmax, 64) / 64.0 * (npoints < 32 ? 0.28 : 1.0);
-    const double work = n * 64.0 * ((nmax + 63) / 64) * l * (6.2e-5 + 2.4e-6 * (l + 1.0)) + (exact ? values * 3.4e-5 * l : 0.0);
+    const double work = n * 64.0 * ((nmax + 63) / 64) * l * (6.2e-5 + 2.4e-6 * (l + 1.0)) +
+                        (exact ? values * 3.4e-5 * l : 0.0);
     return tc < 23.0 + std::sqrt(std::sqrt(base * base * base * base + work * work * work * work));
 }
 
@@ -1260,9 +1268,9 @@ namespace {
 // CATANA_ERR_NOMEM: nothing has been added, and the caller has another path.
 // pix == nullptr: points_dev are npoints x 3; otherwise the pixelized catalog.  "Points" below are what the main
 // kernel takes as such: the catalog's points, or a pixelized one's entries.
-catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev, const PixelCatalog *pix,
-                              int64_t nall, int lmax, int nmax, double rmax, JlMode jl, double rtop, const double *kln_dev,
-                              double *f_acc_dev, int *err_dev, cudaStream_t st) {
+catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, const double *weights_dev,
+                              const PixelCatalog *pix, int64_t nall, int lmax, int nmax, double rmax, JlMode jl,
+                              double rtop, const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st) {
     // the test hook (catana_gpu_test_plain_stall) arms one run
     const uint64_t stall_ns = g_plain_stall_ns.exchange(0);
     const bool lerp = jl == JL_MODE_LERP, fused = lerp && !pix;  // fused: the main kernel evaluates j_l itself
@@ -1317,14 +1325,15 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         px.ring_ph = ph;
         px.tw = pix->tw;
         px.tw_off = pix->tw_off;
-        k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, 1.0 / rmax, er, lerp ? 1 : 0, rlim, keys, perm, rint, poison,
-                                                         count, err_dev);
+        k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, 1.0 / rmax, er, lerp ? 1 : 0, rlim, keys, perm, rint,
+                                                         poison, count, err_dev);
         count_launch(2);
         CG_CUDA_TRY(cudaGetLastError());
         unsigned long long cells = 0;
         CG_CUDA_TRY(cudaMemcpyAsync(&cells, count, sizeof(cells), cudaMemcpyDeviceToHost, st));
-        s = radix_sort_pairs(keys, perm, reinterpret_cast<uint32_t *>(hs + 2 * kb), reinterpret_cast<uint32_t *>(hs + 3 * kb), nall,
-                             16, reinterpret_cast<uint32_t *>(hs + 4 * kb), st);
+        s = radix_sort_pairs(keys, perm, reinterpret_cast<uint32_t *>(hs + 2 * kb),
+                             reinterpret_cast<uint32_t *>(hs + 3 * kb), nall, 16,
+                             reinterpret_cast<uint32_t *>(hs + 4 * kb), st);
         if (s != CATANA_OK) return s;
         CG_CUDA_TRY(cudaStreamSynchronize(st));
         npoints = (int64_t)cells;
@@ -1403,8 +1412,8 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             s = radix_sort_pairs(keys, perm, tk, tv, nc, bits, hist, st);
             if (s != CATANA_OK) return s;
             k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
-            k_ptc_points<<<pg, 32 * pw, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim, rint_d, rabs_d,
-                                             xs_d, ph_d, poison, err_dev);
+            k_ptc_points<<<pg, 32 * pw, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim,
+                                                 rint_d, rabs_d, xs_d, ph_d, poison, err_dev);
         }
         count_launch(2);
         CG_CUDA_TRY(cudaGetLastError());
@@ -1434,7 +1443,9 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             int l1 = l0 + 1;
             auto pdoubles = [&](int e) { return (int64_t)nmax * ((int64_t)e * (e + 1) - (int64_t)l0 * (l0 + 1)); };
             const double jbytes = fused ? 0.0 : 8.0 * tiles * TC_KT * nmax;
-            while (l1 < lmax && pdoubles(l1 + 1) * 8.0 * nslabs < scale * 256e6 && jbytes * (l1 + 1 - l0) < scale * 2e9) ++l1;
+            while (l1 < lmax && pdoubles(l1 + 1) * 8.0 * nslabs < scale * 256e6 &&
+                   jbytes * (l1 + 1 - l0) < scale * 2e9)
+                ++l1;
             a.l0 = l0;
             a.l1 = l1;
             a.pslab = pdoubles(l1);
@@ -1469,7 +1480,8 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
                 else if (pix)
                     k_ptc_jl_cells_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(j);
                 else if (jl == JL_MODE_POLY)
-                    k_ptc_jl_poly<<<ceil_div(cnt, 256), 256, 0, st>>>(j, ctx->tc_poly.as<TcPoly>(), ctx->tc_poly_nint, err_dev);
+                    k_ptc_jl_poly<<<ceil_div(cnt, 256), 256, 0, st>>>(j, ctx->tc_poly.as<TcPoly>(), ctx->tc_poly_nint,
+                                                                      err_dev);
                 else
                     k_ptc_jl_exact<<<ceil_div(cnt, 256), 256, 0, st>>>(j);
                 count_launch();
@@ -1499,8 +1511,9 @@ catana_status_t plain_tc_accumulate(DeviceContext *ctx, const double *points_dev
                          err_dev, st);
 }
 
-catana_status_t plain_tc_pixels(DeviceContext *ctx, const PixelCatalog &pix, int64_t npoints, int lmax, int nmax, double rmax,
-                                JlMode jl, const double *kln_dev, double *f_acc_dev, int *err_dev, cudaStream_t st) {
+catana_status_t plain_tc_pixels(DeviceContext *ctx, const PixelCatalog &pix, int64_t npoints, int lmax, int nmax,
+                                double rmax, JlMode jl, const double *kln_dev, double *f_acc_dev, int *err_dev,
+                                cudaStream_t st) {
     return tc_accumulate(ctx, nullptr, nullptr, &pix, npoints, lmax, nmax, rmax, jl, 0.0, kln_dev, f_acc_dev, err_dev, st);
 }
 

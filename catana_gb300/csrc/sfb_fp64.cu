@@ -1,6 +1,6 @@
 // sfb_fp64.cu -- the plain raw SFB in FP64 on CUDA cores: the sizes that the tensor-core kernel does not take
-// (plain_tc.cu; lmax > 512, nmax > 4096, extreme rmax) or is slower at (plain_tc_pays), other devices and the allocation-free entry.  Also the
-// j_l tables of both, and the normalisation.
+// (plain_tc.cu; lmax > 512, nmax > 4096, extreme rmax) or is slower at (plain_tc_pays), other devices and the
+// allocation-free entry.  Also the j_l tables of both, and the normalisation.
 //
 // Reference: _sfb_raw, sfb_raw.cpp:13-108.  The reference loops l outermost and,
 // per point, evaluates j_l(k_ln r) for every n (:67-69), P_lm by gsl_sf_legendre_sphPlm
@@ -532,7 +532,8 @@ catana_status_t fp64_raw_accumulate(DeviceContext *ctx, const double *points_dev
         if (s != CATANA_OK) return s;
         rtop = max_r;
     }
-    if (plain_tc_takes(ctx, lmax, nmax, rmax) && plain_tc_pays(npoints, lmax, nmax, jl) && (!weights_dev || !wr || plain_tc_holds(*wr))) {
+    if (plain_tc_takes(ctx, lmax, nmax, rmax) && plain_tc_pays(npoints, lmax, nmax, jl) &&
+        (!weights_dev || !wr || plain_tc_holds(*wr))) {
         s = plain_tc_accumulate(ctx, points_dev, weights_dev, npoints, lmax, nmax, rmax, jl, rtop, kln_dev, f_acc_dev,
                                 err_dev, st);
         if (s != CATANA_ERR_NOMEM) return s;

@@ -169,7 +169,8 @@ namespace {
 // 262144 pairs take as few rounds as leave at most 64 tiles, whose histogram the scan takes in one round.
 // 5000 pairs, a pass: 35 us by tiles of 4096, 12 so.
 int radix_tile(int64_t n) {
-    return RS_THREADS * (int)std::min<int64_t>(RS_ROUNDS, std::max<int64_t>(1, (n + 64 * RS_THREADS - 1) / (64 * RS_THREADS)));
+    const int64_t rounds = (n + 64 * RS_THREADS - 1) / (64 * RS_THREADS);
+    return RS_THREADS * (int)std::min<int64_t>(RS_ROUNDS, std::max<int64_t>(1, rounds));
 }
 }  // namespace
 

@@ -112,7 +112,9 @@ catana_status_t accum_add(Accum *A, const T *points, const T *weights, int64_t n
     CG_CUDA_TRY(A->slot[k].ensure(pb + wb + 256));
     char *dst = A->slot[k].as<char>();
     CG_CUDA_TRY(cudaMemcpyAsync(dst, points, pb, cudaMemcpyHostToDevice, A->copy_st));
-    if (weights) CG_CUDA_TRY(cudaMemcpyAsync(dst + ((pb + 255) & ~size_t(255)), weights, wb, cudaMemcpyHostToDevice, A->copy_st));
+    if (weights)
+        CG_CUDA_TRY(cudaMemcpyAsync(dst + ((pb + 255) & ~size_t(255)), weights, wb, cudaMemcpyHostToDevice,
+                                    A->copy_st));
     CG_CUDA_TRY(cudaEventRecord(A->copied[k], A->copy_st));
     CG_CUDA_TRY(cudaStreamWaitEvent(A->comp_st, A->copied[k], 0));
     const T *pd = reinterpret_cast<const T *>(dst);

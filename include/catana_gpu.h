@@ -63,7 +63,7 @@ typedef enum {
  * 8-bit digits that are exact; FP64 on CUDA cores past lmax 512, for weights
  * that differ by more than 2^8, and where that is faster).  SPLIT: tensor-core
  * tcgen05 contraction of 3-term FP16 hi+lo products with FP32 accumulation,
- * folded per 32-point tile and reduced in FP64; j_l from piecewise degree-6
+ * folded per 32-point tile, slabs summed in three FP32 words and scaled in FP64; j_l from piecewise degree-6
  * polynomials on unit intervals with FP32 coefficients, accurate to ~1e-7 of its
  * envelope (the JL flags do not apply); lmax <= 512, nmax <= 256 (above lmax 256
  * the Legendre rows carry a 2-bit exponent per value). */
