@@ -10,7 +10,8 @@ HEALPix method (py_decomposition.cpp:135-153, sfb_decomposition.cpp:22-26).
 Keyword extensions (absent in the reference, defaults reproduce it):
   weights=None         per-point weights; f is normalised by V/sum(w)
   precision='plain'    'plain': to FP64 accuracy, the contraction as exact products of
-                       8-bit digits on the tensor cores (the drop-in);
+                       8-bit digits on the tensor cores (the drop-in; FP64 on CUDA
+                       cores past lmax 512 or with weights that differ by more than 2^8);
                        'split': tcgen05 tensor cores, 3-term FP16 hi+lo products;
                        'split_accurate': the same with Reinsch-modified Legendre
                        rows: half the f_lmn error at high l (ten times less near
@@ -199,7 +200,7 @@ def sfb_decomposition_batched(point_containers, lmax, nmax, rmax, kmax=None, wei
     precision='split' runs all catalogs level by level in grouped tcgen05 launches,
     captured as one CUDA graph (graph=False launches the levels directly); waves sets
     the work items per SM and mblock (128 or 64) the most complex m per work item (the
-    MMA tile's N); waves <= 0 autotunes both.  precision='plain' runs the FP64 path per
+    MMA tile's N); waves <= 0 autotunes both.  precision='plain' runs the plain form per
     catalog.
     Returns a list of KClkk.
     """

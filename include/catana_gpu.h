@@ -172,7 +172,7 @@ typedef struct {
  * autotunes both -- the schedule and the tile shape -- by timing the contraction at
  * three sample levels for each candidate, once per distinct catalog set
  * (catana_gpu_batch_waves() and catana_gpu_batch_mblk() report the choice).  Plain form: the
- * catalogs run one after another through the FP64 path (waves ignored).
+ * catalogs run one after another as catana_gpu_sfb_raw runs them (waves ignored).
  * Host pointers in the catalog records; blocks until the results are in place. */
 catana_status_t catana_gpu_sfb_raw_batched(const catana_catalog_t *cats, int32_t ncat, uint32_t flags, double waves,
                                            catana_gpu_stream_t stream);
