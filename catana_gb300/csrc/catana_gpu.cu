@@ -950,14 +950,11 @@ catana_status_t catana_gpu_sfb_healpix(int64_t nside, const int64_t *pix_offsets
         set_error("pix_offsets[0] must be 0");
         return CATANA_ERR_ARG;
     }
-    int64_t max_pix = 0;
-    for (int64_t p = 0; p < npix; ++p) {
+    for (int64_t p = 0; p < npix; ++p)
         if (pix_offsets[p + 1] < pix_offsets[p]) {
             set_error("pix_offsets must be non-decreasing");
             return CATANA_ERR_ARG;
         }
-        max_pix = std::max(max_pix, pix_offsets[p + 1] - pix_offsets[p]);
-    }
     if (npoints > 0 && !r_sorted) {
         set_error("null r_sorted");
         return CATANA_ERR_ARG;
@@ -988,7 +985,7 @@ catana_status_t catana_gpu_sfb_healpix(int64_t nside, const int64_t *pix_offsets
     CG_CUDA_TRY(cudaMemcpyAsync(kln_d, kh.data(), lm * sizeof(double), cudaMemcpyHostToDevice, st));
     CG_CUDA_TRY(cudaMemsetAsync(f_d, 0, fc * 2 * sizeof(double), st));
     const double nf = norm_factor(rmax, (double)npoints);
-    s = healpix_sfb_dev(ctx, nside, off_d, rs_d, npoints, max_pix, lmax, nmax, rmax, resolve_interp(flags, npoints),
+    s = healpix_sfb_dev(ctx, nside, off_d, rs_d, pix_offsets, npoints, lmax, nmax, rmax, resolve_interp(flags, npoints),
                         (flags & CATANA_HEALPIX_CONJ_FIX) != 0, kln_d, kh.data(), r_sorted, nf, f_d, cln_d, err_d,
                         st);
     if (s != CATANA_OK) return s;

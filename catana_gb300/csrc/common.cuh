@@ -256,12 +256,11 @@ catana_status_t healpix_ang2pix_dev(int64_t nside, const double *theta, const do
                                     int64_t *pix, int *err_dev, cudaStream_t st);
 catana_status_t healpix_pix2ang_dev(int64_t nside, const int64_t *pix, int64_t n, double *theta, double *phi,
                                     cudaStream_t st);
-// max_pix: points of the fullest pixel.
-// kln_host (L x M) and r_host, host copies of k_ln and of the radii: map levels that lie inside the j_l table skip
-// the per-point range test.
+// offsets_host, kln_host (L x M) and r_host: host copies of the offsets (the fullest pixel), of k_ln and of the radii
+// (map levels that lie inside the j_l table skip the per-point range test).
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
-                                const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax,
-                                double rmax, bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
+                                const double *r_sorted_dev, const int64_t *offsets_host, int64_t npoints, int lmax,
+                                int nmax, double rmax, bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
                                 const double *r_host, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st);
 

@@ -641,8 +641,8 @@ bool pixel_sum_pays(int64_t nside, int64_t npoints, int64_t max_pix, int lmax, i
 }
 
 catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t *offsets_dev,
-                                const double *r_sorted_dev, int64_t npoints, int64_t max_pix, int lmax, int nmax,
-                                double rmax, bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
+                                const double *r_sorted_dev, const int64_t *offsets_host, int64_t npoints, int lmax,
+                                int nmax, double rmax, bool interpolated, bool conj_fix, const double *kln_dev, const double *kln_host,
                                 const double *r_host, double norm, double *f_dev, double *c_ln_dev, int *err_dev,
                                 cudaStream_t st) {
     if (lmax == 0 || nmax == 0) return CATANA_OK;
@@ -667,8 +667,15 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     const int *order = reinterpret_cast<const int *>(rb + R.off_order);
     // As a sum over points at their pixels' centres on the tensor cores (plain_tc.cu) where that takes the sizes and is
     // the faster one: it sums the j_l of a pixel's points first.
-    if (plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (int64_t)0xFFFFFFFEll &&
-        pixel_sum_pays(nside, npoints, max_pix, lmax, nmax, interpolated)) {
+    // The maps' time grows with the fullest pixel, so that one is looked for only where an even catalog would go to them.
+    auto pays = [&](int64_t max_pix) { return pixel_sum_pays(nside, npoints, max_pix, lmax, nmax, interpolated); };
+    bool entries = plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (int64_t)0xFFFFFFFEll;
+    if (entries && !pays(ceil_div(npoints, npix))) {
+        int64_t most = 0;
+        for (int64_t p = 0; p < npix; ++p) most = std::max(most, offsets_host[p + 1] - offsets_host[p]);
+        entries = pays(most);
+    }
+    if (entries) {
         if (npoints > 0) {
             PixelCatalog px;
             px.r = r_sorted_dev;
