@@ -93,6 +93,17 @@ struct TcSlab {
     int ec;             // at most 2^ec points in an entry of a pixelized catalog (0 otherwise)
 };
 
+// One call's words on the device, zero at first
+struct TcCall {
+    int poison;  // TC_POISON_*
+    int etop;    // 2048 + the largest EW of its slabs so far
+    unsigned long long count;  // a pixelized catalog's entries
+};
+
+// 2^e in two factors that are normal numbers, |e| <= 2000
+__device__ __forceinline__ double pow2_lo(int e) { return __hiloint2double((1023 + (e >> 1)) << 20, 0); }
+__device__ __forceinline__ double pow2_hi(int e) { return __hiloint2double((1023 + e - (e >> 1)) << 20, 0); }
+
 struct TcArgs {
     int l0, l1;                 // levels of the launch
     int nmax, lmp;              // radial orders; row pitch in m (lmax rounded up to 4)
@@ -112,7 +123,8 @@ struct TcArgs {
     double *partial;            // [slab][l - l0][n][2 (l + 1)]
     int64_t pslab;              // doubles per slab in partial
     uint64_t wait_ns;           // limit of every wait
-    int stall;                  // test hook: withhold the first tile's hand-off of every CTA
+    int stall;                  // test hook: the MMAs wait for a hand-off that nothing makes
+    const TcCall *call;
     int *err;
 };
 
@@ -290,7 +302,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
 
     if (warp < TC_OPW) {
         uint32_t use = 0;  // tiles written so far
-        const uint32_t withheld = a.stall && warp == 0 ? 1u : 0u;
         int ofs = 0;       // units dealt so far, mod TC_OPW
         bool dead = false;
         const uint32_t lk = (uint32_t)(lane >> 3), lr = (uint32_t)(lane & 7);  // K row of this point: group, row
@@ -476,7 +487,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                 } else if (!mine) {
                     wait(&empty[bf], (it - 1) & 1, dead);
                 }
-                if (lane == 0 && use != withheld) tc_arrive(&full[bf]);
+                if (lane == 0) tc_arrive(&full[bf]);
             }
         });
         if (dead && lane == 0) *a.err = CATANA_ERR_CUDA;
@@ -485,6 +496,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
     } else if (warp < TC_FOLD0) {
         uint32_t use = 0, groups = 0;  // tiles taken, groups issued
         bool dead = false;
+        if (a.stall) wait(&drain, 0, dead);
         tc_blocks(a, [&](const TcBlock &b, int) {
             const uint32_t at0 = (uint32_t)(TC_DG * b.nb0 + 63) >> 6, natoms = at0 + ((uint32_t)(TC_DG * b.nb1 + 63) >> 6);
             for (int g = t0; g < t1; g += TC_GROUP) {
@@ -542,7 +554,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
         const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
         // Slab sums are kept in units of 2^64, 2^-54 of the largest term: a group adds at most 2^61, and what
         // passes 2^60 goes to a count per sum (signed bytes, four to a word; at most two a group).
-        const int ew = a.slab[slab].ew;
+        // relative to the call's largest, which k_ptc_reduce applies: 2^(EP + EW) leaves FP64's range otherwise
+        const int ew = a.slab[slab].ew + 2048 - a.call->etop;
         const int set = warp >= TC_FOLD0 + 4 ? 1 : 0;
         tc_blocks(a, [&](const TcBlock &b, int seq) {
             const bool live = qd * 32 < 2 * b.mcount;  // warp-uniform: the quadrant holds rows of the block
@@ -591,14 +604,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                 tc05::fence_before();
                 tc_arrive(&dfree[reg]);
             }
-            // the slab's sums: value = (acc + top 2^60) 2^(-54 + EJ + EP + EW) A_lm, the powers in two factors that
-            // FP64 holds for weights of any size
+            // the slab's sums: value = (acc + top 2^60) 2^(-54 + EJ + EP + EW) A_lm
             if (live && row < 2 * b.mcount) {
                 const int ring = seq & (int)(TC_RING - 1);
                 const uint4 *tn = s_n + ring * TC_NB + nb;
-                const int m = b.mb0 + (row >> 1), esh = ew > 0 ? 32 : 0, ebase = (53 - esh) << 20;
+                const int m = b.mb0 + (row >> 1);
                 const double am = scalbn(a.coef[(size_t)b.l * (b.l + 1) / 2 + m].y,
-                                         __double2loint(s_m[ring * TC_MB + (row >> 1)].y) + ew - esh);
+                                         __double2loint(s_m[ring * TC_MB + (row >> 1)].y) + ew);
                 const int w2 = 2 * (b.l + 1);
                 double *out = a.partial + (size_t)slab * a.pslab +
                               (size_t)a.nmax * ((size_t)b.l * (b.l + 1) - (size_t)a.l0 * (a.l0 + 1)) + 2 * b.mb0 + row +
@@ -619,8 +631,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_ptc_main(TcArgs a) {
                             }
                         }
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)  // 2^(EJ - 54 + esh) is a normal number: EJ >= -900
-                            v[c] *= __hiloint2double((int)tn[c4 + c].w - ebase, 0);
+                        for (int c = 0; c < 4; ++c)  // 2^(EJ - 54) is a normal number: EJ >= -900
+                            v[c] *= __hiloint2double((int)(tn[c4 + c].w - (53u << 20)), 0);
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
                             if (nb + c4 + c < b.ncount) out[(size_t)(c4 + c) * w2] = v[c] * am;
@@ -680,7 +692,7 @@ __global__ void k_ptc_keys(const double *__restrict__ pts, int64_t n, double inv
 // poison the result, k_ptc_points); so are, with the table, radii outside it (a domain error).
 __global__ void __launch_bounds__(256) k_ptc_slabs(const double *__restrict__ pts, const double *__restrict__ w,
                                                    const uint32_t *__restrict__ perm, int64_t n, int64_t per, double rlim,
-                                                   TcSlab *__restrict__ out) {
+                                                   TcSlab *__restrict__ out, TcCall *__restrict__ call) {
     const int64_t i0 = blockIdx.x * per, i1 = min(n, i0 + per);
     double lo = INFINITY, hi = 0.0, mw = 0.0;
     for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
@@ -714,8 +726,9 @@ __global__ void __launch_bounds__(256) k_ptc_slabs(const double *__restrict__ pt
         TcSlab o;
         o.rmin = lo <= hi ? lo : 0.0;
         o.rmax = hi;
-        o.ew = mw > 0.0 ? ilogb(mw) + 1 : 0;  // mw < 2^ew
+        o.ew = mw > 0.0 ? ilogb(mw) + 1 : -1100;  // mw < 2^ew
         o.ec = 0;
+        atomicMax(&call->etop, 2048 + o.ew);
         out[blockIdx.x] = o;
     }
 }
@@ -749,7 +762,7 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
                                                     int lmp, const TcSlab *__restrict__ slab, int er, int lerp,
                                                     double rlim, uint64_t *__restrict__ rint, double *__restrict__ rabs,
                                                     double2 *__restrict__ xs, ulonglong2 *__restrict__ phase,
-                                                    int *__restrict__ poison, int *__restrict__ err) {
+                                                    TcCall *__restrict__ call, int *__restrict__ err) {
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= tiles) return;
     const int64_t i = (int64_t)t * TC_KT + lane;
@@ -768,13 +781,14 @@ __global__ void __launch_bounds__(256) k_ptc_points(const double *__restrict__ p
     const bool use = in && !(bad & TC_POISON_W) && !rbad;
     const double ct = cos(th);
     if (blockIdx.y == 0) {
-        if (in && bad) atomicOr(poison, bad);
+        if (in && bad) atomicOr(&call->poison, bad);
         if (in && rbad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
         rint[i] = rbad || !(fabs(r) < ldexp(1.0, er)) ? 0ull : (uint64_t)(int64_t)ldexp(fmax(r, 0.0), 62 - er);
         rabs[i] = r;
         xs[i] = use && !(bad & TC_POISON_THETA) ? make_double2(ct, sqrt((1.0 - ct) * (1.0 + ct))) : make_double2(0.0, 0.0);
     }
-    wv = use ? ldexp(wv, -slab[t / tslab].ew) : 0.0;  // in [-1, 1], exact for weights of any size
+    const int e = -slab[t / tslab].ew;
+    wv = use ? wv * pow2_lo(e) * pow2_hi(e) : 0.0;  // in [-1, 1], exact for weights of any size
     const double phi = use && !(bad & TC_POISON_PHI) ? ph : 0.0;
     // frac(phi / 2 pi) 2^64 (mod 2^64), 1 / 2 pi as a pair of doubles: rounded at 2^-64 of a turn
     const double p = phi * 0.15915494309189535, pl = fma(phi, 0.15915494309189535, -p) - phi * 9.839338337591243e-18;
@@ -820,12 +834,12 @@ __device__ __forceinline__ int64_t pixel_of(const TcPixels &px, int64_t q) {
 // come last.  Also each radius in the table's units.
 __global__ void k_ptc_cells(TcPixels px, int64_t n, double inv_rmax, int er, int lerp, double rlim,
                             uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, uint64_t *__restrict__ rint,
-                            int *__restrict__ poison, unsigned long long *__restrict__ count, int *__restrict__ err) {
+                            TcCall *__restrict__ call, int *__restrict__ err) {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t p = q < n ? pixel_of(px, q) : 0, k = q < n ? q - px.offs[p] : 1;
     // every thread of the block takes part, whatever its bisection took
     const int heads = __syncthreads_count(k % TC_CELL == 0);
-    if (threadIdx.x == 0 && heads) atomicAdd(count, (unsigned long long)heads);
+    if (threadIdx.x == 0 && heads) atomicAdd(&call->count, (unsigned long long)heads);
     if (q >= n) return;
     const double r = px.r[q], rs = r * inv_rmax * 256.0;
     const uint32_t rb = rs >= 255.0 ? 255u : (rs > 0.0 ? (uint32_t)rs : 0u);
@@ -834,13 +848,14 @@ __global__ void k_ptc_cells(TcPixels px, int64_t n, double inv_rmax, int er, int
     vals[q] = (uint32_t)q;
     const bool bad = lerp ? !(r >= 0.0 && r < rlim) : !isfinite(r);
     if (bad && lerp) *err = CATANA_ERR_DOMAIN;  // outside every table
-    if (bad && !lerp) atomicOr(poison, TC_POISON_W);
+    if (bad && !lerp) atomicOr(&call->poison, TC_POISON_W);
     rint[q] = bad || !(fabs(r) < ldexp(1.0, er)) ? 0ull : (uint64_t)(int64_t)ldexp(fmax(r, 0.0), 62 - er);
 }
 
 // Per slab of entries what k_ptc_slabs finds for points (weights are 1)
 __global__ void __launch_bounds__(256) k_ptc_cell_slabs(TcPixels px, const uint2 *__restrict__ cell, int64_t n, int64_t per,
-                                                        double rlim, TcSlab *__restrict__ out) {
+                                                        double rlim, TcSlab *__restrict__ out,
+                                                        TcCall *__restrict__ call) {
     const int64_t i0 = blockIdx.x * per, i1 = min(n, i0 + per);
     double lo = INFINITY, hi = 0.0;
     for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
@@ -872,6 +887,7 @@ __global__ void __launch_bounds__(256) k_ptc_cell_slabs(TcPixels px, const uint2
         o.rmin = lo <= hi ? lo : 0.0;
         o.rmax = hi;
         o.ew = 1;
+        atomicMax(&call->etop, 2048 + o.ew);
         o.ec = 32 - __clz((int)cell[i0].y - 1);  // the slab's first entry is its fullest
         out[blockIdx.x] = o;
     }
@@ -943,7 +959,7 @@ __global__ void k_ptc_pairs(const double *__restrict__ y, int npts, int64_t tota
 // f[l][m][n] += k_ln sum over slabs, in eight interleaved parts added in order; one CTA per 32 (m, n) of
 // a level.  Points that are not finite make their terms NaN: theta every l > 0, phi every m > 0, w all.
 __global__ void __launch_bounds__(256) k_ptc_reduce(const double *__restrict__ partial, int64_t pslab, int nslabs, int l0,
-                                                    int nmax, const double *__restrict__ kln, const int *__restrict__ poison,
+                                                    int nmax, const double *__restrict__ kln, const TcCall *__restrict__ call,
                                                     double2 *__restrict__ f) {
     __shared__ double2 s[8][33];
     const int l = l0 + blockIdx.y, cnt = (l + 1) * nmax;
@@ -972,13 +988,14 @@ __global__ void __launch_bounds__(256) k_ptc_reduce(const double *__restrict__ p
             const int n = e / (l + 1), m = e - n * (l + 1);
             const double k = kln[(size_t)l * nmax + n];
             double2 *o = f + (size_t)nmax * l * (l + 1) / 2 + (size_t)m * nmax + n;
-            const int bad = *poison;
+            const int bad = call->poison, e = call->etop - 2048;
             double2 v = *o;
             if ((bad & TC_POISON_W) || ((bad & TC_POISON_THETA) && l > 0) || ((bad & TC_POISON_PHI) && m > 0)) {
                 v = make_double2(NAN, NAN);
             } else {
-                v.x += k * sr;
-                v.y += k * si;
+                const double ks = k * pow2_lo(e);
+                v.x += ks * sr * pow2_hi(e);
+                v.y += ks * si * pow2_hi(e);
             }
             *o = v;
         }
@@ -1296,11 +1313,11 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     const int er = std::max(ilogb(rmax) + 3, rtop > 0.0 ? ilogb(rtop) + 1 : -1000);
     const double rlim = lerp ? ldexp(1.0, er) : INFINITY;
     // A pixelized catalog is sorted into entries first, in the workspace of the HEALPix calls (which end before they
-    // return): [sort scratch][radii][ring phases][poison, count]
+    // return): [sort scratch][radii][ring phases][TcCall]
     TcPixels px = {};
     const uint32_t *entries = nullptr;
     const uint64_t *entry_r = nullptr;
-    int *poison = nullptr;
+    TcCall *call = nullptr;
     if (pix) {
         const size_t kb = tc_al((size_t)nall * 4), hb = tc_al(radix_hist_words(nall) * 4), rb = tc_al((size_t)nall * 8);
         const size_t phb = tc_al((size_t)pix->nrings * lmax * sizeof(double2));
@@ -1309,9 +1326,8 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         uint32_t *keys = reinterpret_cast<uint32_t *>(hs), *perm = reinterpret_cast<uint32_t *>(hs + kb);
         uint64_t *rint = reinterpret_cast<uint64_t *>(hs + 4 * kb + hb);
         double2 *ph = reinterpret_cast<double2 *>(hs + 4 * kb + hb + rb);
-        poison = reinterpret_cast<int *>(hs + 4 * kb + hb + rb + phb);
-        unsigned long long *count = reinterpret_cast<unsigned long long *>(poison) + 1;
-        CG_CUDA_TRY(cudaMemsetAsync(poison, 0, 16, st));  // and the entries' count
+        call = reinterpret_cast<TcCall *>(hs + 4 * kb + hb + rb + phb);
+        CG_CUDA_TRY(cudaMemsetAsync(call, 0, sizeof(TcCall), st));
         k_ptc_ring_phases<<<ceil_div((int64_t)pix->nrings * lmax, 128), 128, 0, st>>>(pix->ring_phi, pix->nrings, lmax, ph);
         px.r = pix->r;
         px.offs = pix->offs;
@@ -1326,11 +1342,11 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         px.tw = pix->tw;
         px.tw_off = pix->tw_off;
         k_ptc_cells<<<ceil_div(nall, 256), 256, 0, st>>>(px, nall, 1.0 / rmax, er, lerp ? 1 : 0, rlim, keys, perm, rint,
-                                                         poison, count, err_dev);
+                                                         call, err_dev);
         count_launch(2);
         CG_CUDA_TRY(cudaGetLastError());
         unsigned long long cells = 0;
-        CG_CUDA_TRY(cudaMemcpyAsync(&cells, count, sizeof(cells), cudaMemcpyDeviceToHost, st));
+        CG_CUDA_TRY(cudaMemcpyAsync(&cells, &call->count, sizeof(cells), cudaMemcpyDeviceToHost, st));
         s = radix_sort_pairs(keys, perm, reinterpret_cast<uint32_t *>(hs + 2 * kb),
                              reinterpret_cast<uint32_t *>(hs + 3 * kb), nall, 16,
                              reinterpret_cast<uint32_t *>(hs + 4 * kb), st);
@@ -1352,8 +1368,8 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         const int waves = ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES);
         return ceil_div(tiles, (int64_t)ctx->sm_count * waves);
     };
-    // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][poison]
-    size_t kb, hb, o_rint, o_rabs, o_xs, o_rows, o_ph, o_sl, o_mx, o_poi;
+    // workspace: [perm and sort scratch][records][rows][phases][slabs][maxima][TcCall]
+    size_t kb, hb, o_rint, o_rabs, o_xs, o_rows, o_ph, o_sl, o_mx, o_call;
     for (;; scale *= 0.25) {
         const double slabs_c = std::max((double)ctx->sm_count, scale * 2e9 / slab_bytes);
         double fit = std::min(scale * 4e9 / (32.0 * lmp), slabs_c * TC_SLAB_TILES * TC_KT);
@@ -1366,11 +1382,11 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         o_rows = o_xs + tc_al(np * 16), o_ph = o_rows + tc_al(2 * np * lmp * 8), o_sl = o_ph + tc_al(np * lmp * 16);
         // a last pass of fewer points may have more slabs, up to this many
         const int slabs = std::min(tiles, ctx->sm_count * ceil_div(tiles, (int64_t)ctx->sm_count * TC_SLAB_TILES));
-        o_mx = o_sl + tc_al((size_t)slabs * sizeof(TcSlab)), o_poi = o_mx + tc_al((size_t)slabs * 3 * TC_LMAX * 4);
+        o_mx = o_sl + tc_al((size_t)slabs * sizeof(TcSlab)), o_call = o_mx + tc_al((size_t)slabs * 3 * TC_LMAX * 4);
         const double sums = std::max(slab_bytes * slabs, std::min(scale * 256e6, 0.5 * (lmax + 1) * slab_bytes * slabs));
         const double ntab = std::min(sums, slab_bytes * slabs);
         const double jl = fused ? 0.0 : 8.0 * np * nmax;
-        cudaError_t e = ctx->tc_ws.ensure(o_poi + 256);
+        cudaError_t e = ctx->tc_ws.ensure(o_call + 256);
         if (e == cudaSuccess) e = ctx->partial.ensure((size_t)(sums + ntab) + 512);
         if (e == cudaSuccess) e = ctx->tc_jarr.ensure((size_t)std::max(jl, std::min(scale * 2e9, jl * lmax)));
         if (e == cudaSuccess) break;
@@ -1383,8 +1399,8 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
     uint32_t *hist = reinterpret_cast<uint32_t *>(ws + 4 * kb);
     TcSlab *slabs = reinterpret_cast<TcSlab *>(ws + o_sl);
     if (!pix) {
-        poison = reinterpret_cast<int *>(ws + o_poi);
-        CG_CUDA_TRY(cudaMemsetAsync(poison, 0, 16, st));
+        call = reinterpret_cast<TcCall *>(ws + o_call);
+        CG_CUDA_TRY(cudaMemsetAsync(call, 0, sizeof(TcCall), st));
     }
     for (int64_t c0 = 0; c0 < npoints; c0 += chunk) {
         const int64_t nc = std::min(chunk, npoints - c0);
@@ -1401,7 +1417,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         uint2 *cell = reinterpret_cast<uint2 *>(ws + o_rabs);
         if (pix) {
             k_ptc_pixels<<<pg, 32 * pw, 0, st>>>(px, entries + c0, nc, tiles, lmp, cell, xs_d, ph_d);
-            k_ptc_cell_slabs<<<nslabs, 256, 0, st>>>(px, cell, nc, (int64_t)tslab * TC_KT, rlim, slabs);
+            k_ptc_cell_slabs<<<nslabs, 256, 0, st>>>(px, cell, nc, (int64_t)tslab * TC_KT, rlim, slabs, call);
         } else {
             const double *pts = points_dev + 3 * c0, *w = weights_dev ? weights_dev + c0 : nullptr;
             // Neighbours share cells of the j_l table and slabs take a bound each.  A tile of 32 of few points
@@ -1411,9 +1427,9 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             count_launch();
             s = radix_sort_pairs(keys, perm, tk, tv, nc, bits, hist, st);
             if (s != CATANA_OK) return s;
-            k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs);
+            k_ptc_slabs<<<nslabs, 256, 0, st>>>(pts, w, perm, nc, (int64_t)tslab * TC_KT, rlim, slabs, call);
             k_ptc_points<<<pg, 32 * pw, 0, st>>>(pts, w, perm, nc, tiles, tslab, lmp, slabs, er, lerp ? 1 : 0, rlim,
-                                                 rint_d, rabs_d, xs_d, ph_d, poison, err_dev);
+                                                 rint_d, rabs_d, xs_d, ph_d, call, err_dev);
         }
         count_launch(2);
         CG_CUDA_TRY(cudaGetLastError());
@@ -1433,6 +1449,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
         a.err = err_dev;
         a.wait_ns = stall_ns ? stall_ns : TC_WAIT_NS;
         a.stall = stall_ns ? 1 : 0;
+        a.call = call;
         a.tab = nullptr;
         const double *dxinv = nullptr;
         if (lerp) {
@@ -1493,7 +1510,7 @@ catana_status_t tc_accumulate(DeviceContext *ctx, const double *points_dev, cons
             else k_ptc_main<false><<<nslabs, TC_THREADS, TC_SMEM, st>>>(a);
             prof_end(st, 2.0 * (double)nc * (double)pdoubles(l1));
             k_ptc_reduce<<<dim3(std::min(64, ceil_div((int64_t)l1 * nmax, 32)), l1 - l0), 256, 0, st>>>(
-                a.partial, a.pslab, nslabs, l0, nmax, kln_dev, poison, reinterpret_cast<double2 *>(f_acc_dev));
+                a.partial, a.pslab, nslabs, l0, nmax, kln_dev, call, reinterpret_cast<double2 *>(f_acc_dev));
             count_launch(2);
             CG_CUDA_TRY(cudaGetLastError());
             l0 = l1;
