@@ -151,7 +151,7 @@ catana_status_t dsb_group(DeviceContext *ctx, const DsbCall &C, double kmax, con
     R.nseg = std::max<int64_t>(1, sl - R.seg0 + 1);
     const double kappa = C.kappa(kmax), cuts = C.cuts(kmax);
     R.p = kappa <= 0.002 ? 2 : kappa <= 0.046 ? 3 : kappa <= 0.23 ? 4 : 8;
-    if (!(cuts < 2e9) || cuts * (double)R.nseg * R.p > 1e11) {
+    if (cuts * (double)R.nseg * R.p > 1e11) {
         set_error("sbessel_integrals: k r_max too large");
         return CATANA_ERR_ARG;
     }
@@ -249,6 +249,10 @@ catana_status_t catana_gpu_sbessel_integrals(const double *w_table, int64_t w_n,
     C.wmin = w_min;
     C.wdx = (w_max - w_min) / (double)(w_n - 1);
     C.rmax = r_max;
+    if (!(C.cuts(kmax) < 2e9)) {
+        set_error("sbessel_integrals: k r_max too large");
+        return CATANA_ERR_ARG;
+    }
     if (C.cuts(kmax) < 8.0) return dsb_pairs(ctx, C, kmax, k1, k2, npairs, out, st);
     // The pairs by the octal order of their pieces per segment: a pair is not integrated on pieces that only a much
     // larger k of the call asks for.

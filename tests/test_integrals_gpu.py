@@ -98,3 +98,11 @@ def test_distinct_k_beyond_a_pass_memory(cuda_device):
     some = np.concatenate([np.arange(0, 50000, 2500), [15624, 15625, 49999]])
     one = np.array([besseltools.double_sbessel_integrator(fi, 2, 100.0, k1[i], k2[i]) for i in some])
     assert np.max(np.abs(got[some] - one)) <= 1e-13 * np.max(np.abs(one))
+
+
+def test_wave_numbers_past_any_rule_are_refused(cuda_device):
+    """Also where the pieces are past every integer: an error before anything is computed."""
+    fi = catana.FunctionInterpolator(lambda r: 1.0 + 0.0 * r, 11, 0.0, 100.0)
+    for k in (1e10, 1e300, 1.7e308):
+        with pytest.raises(ValueError):
+            besseltools.double_sbessel_integrator(fi, 0, 100.0, np.array([1.0, k]), np.array([1.0, 1.0]))
