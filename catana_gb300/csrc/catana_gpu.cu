@@ -201,7 +201,7 @@ WsOrder::WsOrder(DeviceContext *ctx, cudaStream_t st) : ctx_(ctx), st_(st) {
 WsOrder::~WsOrder() {
     // not into a capture: an event recorded there cannot be waited for outside it (such a call has failed anyway)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st_, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+    if (ctx_->ws_event && cudaStreamIsCapturing(st_, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
         cudaEventRecord(ctx_->ws_event, st_);
 }
 

@@ -670,7 +670,7 @@ catana_status_t healpix_sfb_dev(DeviceContext *ctx, int64_t nside, const int64_t
     // The maps' time grows with the fullest pixel, so that one is looked for only where an even catalog would go to them.
     auto pays = [&](int64_t max_pix) { return pixel_sum_pays(nside, npoints, max_pix, lmax, nmax, interpolated); };
     bool entries = plain_tc_takes(ctx, lmax, nmax, rmax) && npoints <= (int64_t)0xFFFFFFFEll;
-    if (entries && !pays(ceil_div(npoints, npix))) {
+    if (entries && npoints > 0 && !pays(ceil_div(npoints, npix))) {
         int64_t most = 0;
         for (int64_t p = 0; p < npix; ++p) most = std::max(most, offsets_host[p + 1] - offsets_host[p]);
         entries = pays(most);

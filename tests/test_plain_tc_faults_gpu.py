@@ -359,3 +359,12 @@ def test_the_faster_path_for_few_pixelized_points(cuda_device, nside, n, lmax, n
     f = O.sfb_healpix(nside, ppc.offsets, ppc.r_sorted, 2, nmax, 1000.0, interpolated=interp == "on")[2]
     for l in range(2):
         assert np.max(np.abs(res.f_lmn[l] - f[l])) <= 1e-10 * np.max(np.abs(f[l])), l
+
+
+@pytest.mark.parametrize("lmax,nmax", [(1, 1), (3, 200), (520, 2)])
+def test_an_empty_pixelized_catalog(cuda_device, lmax, nmax):
+    """No point on any path: the normalisation's 1 / N times 0, as in the reference."""
+    ppc = catana.PixelizedPointContainer(4)
+    ppc.offsets, ppc.r_sorted = np.zeros(12 * 16 + 1, dtype=np.int64), np.zeros(0)
+    res = catana.sfb_decomposition(ppc, lmax, nmax, 1000.0, True, False)
+    assert np.all(np.isnan(res.c_ln)) and all(np.all(np.isnan(f)) for f in res.f_lmn)
